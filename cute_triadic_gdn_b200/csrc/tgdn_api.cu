@@ -41,24 +41,42 @@ int* tgdn_status_word() {
 }
 
 int tgdn_check_device() {
+  static signed char cached[64] = {0};         // per device: 1 = compute capability 10.x, -1 = another one
+  static thread_local int bound = -1;          // the device whose context this thread has made current
   int dev = 0, major = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   // Make the device's primary context current on the calling thread.  The tensor-map encoder is a driver call and
   // fails with "invalid context" on a thread that has not touched the runtime yet (an autograd worker whose tensors all
   // came out of the allocator's cache); setting the current device again is the documented way to bind the context.
-  if (cudaSetDevice(dev) != cudaSuccess) return 0;
+  if (bound != dev) {
+    if (cudaSetDevice(dev) != cudaSuccess) return 0;
+    bound = dev;
+  }
+  if (dev >= 0 && dev < 64 && cached[dev] != 0) return cached[dev] > 0;
   if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return 0;
+  if (dev >= 0 && dev < 64) cached[dev] = major == 10 ? 1 : -1;
   return major == 10;
 }
 
+// The attribute is sticky, so it is set once per kernel and device (`configured`: one flag per device, owned by the caller).
+int tgdn_dynamic_smem(const void* kernel, int bytes, bool* configured) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && configured[dev]) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  if (dev >= 0 && dev < 64) configured[dev] = true;
+  return 0;
+}
+
 int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows,
-                        int swizzle128) {
+                        int swizzle128, int row_tokens) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return TGDN_ERR_DRIVER;
   if (reinterpret_cast<uintptr_t>(base) & 15) return TGDN_ERR_ALIGN;
   if (swizzle128 && box_cols != 64) return TGDN_ERR_SHAPE;
   const cuuint64_t dims[4] = {128, static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[3] = {256, static_cast<cuuint64_t>(H) * 256, static_cast<cuuint64_t>(T) * H * 256};
+  const cuuint64_t strides[3] = {256, static_cast<cuuint64_t>(H) * 256,
+                                 static_cast<cuuint64_t>(row_tokens ? row_tokens : T) * H * 256};
   const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_cols), 1, static_cast<cuuint32_t>(box_rows), 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
@@ -67,13 +85,13 @@ int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H,
   return r == CUDA_SUCCESS ? 0 : TGDN_ERR_DRIVER;
 }
 
-int tgdn_make_gate_map(CUtensorMap* map, const float* base, int B, int T, int H, int E) {
+int tgdn_make_gate_map(CUtensorMap* map, const float* base, int B, int T, int H, int E, int row_tokens) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return TGDN_ERR_DRIVER;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || E % 4) return TGDN_ERR_ALIGN;
   const cuuint64_t row = static_cast<cuuint64_t>(E) * 4;
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(E), static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(B)};
-  const cuuint64_t strides[3] = {row, static_cast<cuuint64_t>(H) * row, static_cast<cuuint64_t>(T) * H * row};
+  const cuuint64_t strides[3] = {row, static_cast<cuuint64_t>(H) * row, static_cast<cuuint64_t>(row_tokens ? row_tokens : T) * H * row};
   const cuuint32_t box[4] = {static_cast<cuuint32_t>(E), 1, 64, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), dims, strides, box, estr,
@@ -100,8 +118,8 @@ int tgdn_make_rows_map(CUtensorMap* map, const void* base, int C, int T, int B, 
   return r == CUDA_SUCCESS ? 0 : TGDN_ERR_DRIVER;
 }
 
-int tgdn_check_core_shape(int B, int T, int H, int E, int NC, int packed) {
-  if (B <= 0 || T <= 0 || H <= 0 || NC <= 0) return TGDN_ERR_SHAPE;
+int tgdn_check_core_shape(int B, int T, int H, int E, int NC, int packed, int row_tokens) {
+  if (B <= 0 || T <= 0 || H <= 0 || NC <= 0 || row_tokens < T) return TGDN_ERR_SHAPE;
   if (E != 1 && E != 2 && E != 4 && E != 8 && E != 12 && E != 16) return TGDN_ERR_SHAPE;
   if (packed) {
     if (B != 1 || NC < (T + 63) / 64) return TGDN_ERR_SHAPE;

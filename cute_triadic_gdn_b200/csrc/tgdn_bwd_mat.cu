@@ -137,7 +137,7 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   // Every global value this thread needs later is requested here, in one batch, from clamped (always valid) addresses,
   // and masked when it is used: a load that waits until its consumer is reached costs a full memory round trip, which
   // under the streaming load of the other blocks is microseconds.
-  const int64_t tok = static_cast<int64_t>(b) * p.T + t0;
+  const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
   constexpr int GATE_ITERS = (64 * E + MAT_THREADS - 1) / MAT_THREADS;
   constexpr int NV_MAX = 8;                                // value blocks of the reverse recurrence (4 or 8)
   float da_in[GATE_ITERS], dc_in[GATE_ITERS];              // row-sum gradients of the state-gradient kernel, used at the end
@@ -487,7 +487,7 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
             bulk_prefetch(p.dc + item2 * (64 * E), 64 * E * 4);
             bulk_prefetch(p.dr + item2 * p.NV * (64 * E), static_cast<uint32_t>(p.NV) * 64 * E * 4);
           }
-          const int64_t tok2 = static_cast<int64_t>(b2) * p.T + t2;
+          const int64_t tok2 = static_cast<int64_t>(b2) * p.TS + t2;
           for (int rr = lane; rr < rows2; rr += 32) {
             const int64_t ro = (tok2 + rr) * p.H + h2;
             prefetch_l2(p.k2 + ro * E);
@@ -750,22 +750,22 @@ template <int E>
 static int launch_mat(const CUtensorMap* maps, const MatParams& p, cudaStream_t s) {
   const int smem = static_cast<int>(sizeof(MatSmem<E>)) + 1024;
   static_assert(sizeof(MatSmem<E>) + 1024 <= 232448, "shared memory budget of one CTA exceeded");
-  cudaError_t e = cudaFuncSetAttribute(mat_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  static bool configured[64] = {};
+  if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(mat_kernel<E>), smem, configured)) return rc;
   const long long items = static_cast<long long>(p.B) * p.NC * p.H;
   mat_kernel<E><<<static_cast<int>(items < p.ahead ? items : p.ahead), MAT_THREADS, smem, s>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], maps[6], maps[7], p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 
-extern "C" int tgdn_bwd_matrix(const void* q, const void* k, const void* dO, const void* dU, const void* W, const void* U,
-                               const void* AP, const float* k2, const float* q2, const float* beta, const float* gc,
-                               const void* dkq, const float* da, const float* dc, const float* dd, const float* dr,
-                               float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC, void* dq,
-                               void* dk, float* dk2, float* dq2, float* dg, float* dbeta, void* stream) {
+int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const void* dU, const void* W, const void* U, const void* AP,
+                         const float* k2, const float* q2, const float* beta, const float* gc, const void* dkq, const float* da,
+                         const float* dc, const float* dd, const float* dr, float scale, const int32_t* chunk_map, int B, int T,
+                         int H, int E, int NC, int row_tokens, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
+                         void* stream) {
   if (!q || !k || !dO || !dU || !W || !U || !AP || !k2 || !q2 || !beta || !gc || !dkq || !da || !dc || !dd || !dr ||
       !dq || !dk || !dk2 || !dq2 || !dg || !dbeta)
     return TGDN_ERR_NULL;
-  int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr);
+  int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr, row_tokens);
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(AP) | reinterpret_cast<uintptr_t>(dkq) | reinterpret_cast<uintptr_t>(dq) |
        reinterpret_cast<uintptr_t>(dk)) & 15)
@@ -773,18 +773,18 @@ extern "C" int tgdn_bwd_matrix(const void* q, const void* k, const void* dO, con
   const long long crows = static_cast<long long>(B) * NC * H * 64;
   if (crows > 0x7fffffffLL) return TGDN_ERR_SHAPE;
   CUtensorMap maps[8];
-  if ((rc = tgdn_make_token_map(&maps[0], k, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&maps[1], q, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&maps[2], dO, B, T, H, 64, 64, 1))) return rc;
+  if ((rc = tgdn_make_token_map(&maps[0], k, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&maps[1], q, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&maps[2], dO, B, T, H, 64, 64, 1, row_tokens))) return rc;
   // chunk-layout tensors are plain (rows, 128) matrices: one batch row, one head
   if ((rc = tgdn_make_token_map(&maps[3], dU, 1, static_cast<int>(crows), 1, 64, 64, 1))) return rc;
   if ((rc = tgdn_make_token_map(&maps[4], W, 1, static_cast<int>(crows), 1, 64, 64, 1))) return rc;
   if ((rc = tgdn_make_token_map(&maps[5], U, 1, static_cast<int>(crows), 1, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&maps[6], dk, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&maps[7], dq, B, T, H, 64, 64, 1))) return rc;
+  if ((rc = tgdn_make_token_map(&maps[6], dk, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&maps[7], dq, B, T, H, 64, 64, 1, row_tokens))) return rc;
   MatParams p{k2, q2, beta, gc, static_cast<const __nv_bfloat16*>(AP), static_cast<const __nv_bfloat16*>(dkq), da, dc, dd, dr,
               static_cast<__nv_bfloat16*>(dq), static_cast<__nv_bfloat16*>(dk), dk2, dq2, dg, dbeta, chunk_map,
-              B, T, H, NC, 128 / tgdn_value_block(E), scale, tgdn_status_word(), tgdn_sm_count()};
+              B, T, H, NC, 128 / tgdn_value_block(E), row_tokens, scale, tgdn_status_word(), tgdn_sm_count()};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1: return launch_mat<1>(maps, p, s);
@@ -795,4 +795,13 @@ extern "C" int tgdn_bwd_matrix(const void* q, const void* k, const void* dO, con
     case 16: return launch_mat<16>(maps, p, s);
     default: return TGDN_ERR_SHAPE;
   }
+}
+
+extern "C" int tgdn_bwd_matrix(const void* q, const void* k, const void* dO, const void* dU, const void* W, const void* U,
+                               const void* AP, const float* k2, const float* q2, const float* beta, const float* gc,
+                               const void* dkq, const float* da, const float* dc, const float* dd, const float* dr,
+                               float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC, void* dq,
+                               void* dk, float* dk2, float* dq2, float* dg, float* dbeta, void* stream) {
+  return tgdn_bwd_matrix_rows(q, k, dO, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, scale, chunk_map, B, T, H, E, NC, T,
+                              dq, dk, dk2, dq2, dg, dbeta, stream);
 }

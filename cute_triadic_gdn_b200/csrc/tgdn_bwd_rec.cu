@@ -296,7 +296,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     int t0, rows;
     chunk_info(i, t0, rows);
     const int last = max(rows, 1) - 1;
-    const int64_t ro = (static_cast<int64_t>(b) * p.T + t0 + min(t, last)) * p.H + h;
+    const int64_t ro = (static_cast<int64_t>(b) * p.TS + t0 + min(t, last)) * p.H + h;
     if (krow) prefetch_l2(p.beta + ro);
   };
   // This thread's piece of a row of an operand image (i = t, j = v) that TMA filled: CW value columns as raw bf16
@@ -394,7 +394,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     int t0, rows;
     chunk_info(i, t0, rows);
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
-    const int64_t tok = static_cast<int64_t>(b) * p.T + t0;
+    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
     const bool live = t < rows;
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     const int nbi = C::NB == 2 ? st : 0;             // which copy of Pm, A and the gate factors this chunk uses
@@ -741,29 +741,24 @@ static int launch_rec(const CUtensorMap& mk, const CUtensorMap& mq,
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static_assert((STAGES == 1 ? 2 : 1) * C::TMEM_COLS <= 512, "tensor memory budget of one SM exceeded");
   static_assert(64 % NWG == 0 && (64 / NWG) % 16 == 0, "the readout of P splits 64 token columns over the warpgroups in pieces of 16");
-  static bool configured[64] = {};                  // per device: the attribute is sticky, set it once
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(rec_kernel<E, VC, NWG, STAGES, NSG>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return tgdn_cuda_error(e);
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
+  static bool configured[64] = {};
+  if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(rec_kernel<E, VC, NWG, STAGES, NSG>), C::SMEM_BYTES, configured))
+    return rc;
   const int grid = p.n_seq * p.H * (HEAD / VC);
   rec_kernel<E, VC, NWG, STAGES, NSG><<<grid, C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 
-extern "C" int tgdn_bwd_recurrent_state(const void* q, const void* k, const void* dO, const float* k2, const float* q2,
-                                        const float* beta, const float* gc, const void* AP, const void* Pm, const void* U,
-                                        float scale, const int32_t* doc_offsets, const int32_t* chunk_map, int n_docs, int B,
-                                        int T, int H, int E, int NC, void* dV, void* dU, void* ds, void* dkg, float* dr,
-                                        const float* grad_state_in, float* grad_state_out, void* stream) {
+int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
+                            const float* gc, const void* AP, const void* Pm, const void* U, float scale, const int32_t* doc_offsets,
+                            const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, void* dV,
+                            void* dU, void* ds, void* dkg, float* dr, const float* grad_state_in, float* grad_state_out,
+                            void* stream) {
   if ((reinterpret_cast<uintptr_t>(grad_state_in) | reinterpret_cast<uintptr_t>(grad_state_out)) & 15) return TGDN_ERR_ALIGN;
   if (!q || !k || !dO || !k2 || !q2 || !beta || !gc || !AP || !Pm || !U || !dV || !dU || !ds || !dkg || !dr) return TGDN_ERR_NULL;
   const bool packed = chunk_map != nullptr;
   if (packed && (!doc_offsets || n_docs < 1)) return TGDN_ERR_NULL;
-  int rc = tgdn_check_core_shape(B, T, H, E, NC, packed);
+  int rc = tgdn_check_core_shape(B, T, H, E, NC, packed, row_tokens);
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(dO) | reinterpret_cast<uintptr_t>(AP) | reinterpret_cast<uintptr_t>(Pm) |
        reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(dV) | reinterpret_cast<uintptr_t>(dU) |
@@ -771,19 +766,19 @@ extern "C" int tgdn_bwd_recurrent_state(const void* q, const void* k, const void
        reinterpret_cast<uintptr_t>(q2) | reinterpret_cast<uintptr_t>(gc)) & 15)
     return TGDN_ERR_ALIGN;
   CUtensorMap mk, mq;
-  if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1))) return rc;
+  if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1, row_tokens))) return rc;
   // dO (token layout) and U, dU (chunk layout: item * 64 + t rows of 128 columns) in boxes of 8 columns x 64 rows
   const int64_t crows = static_cast<int64_t>(B) * NC * H * 64;
   if (crows > 0x7fffffffLL) return TGDN_ERR_SHAPE;
   CUtensorMap mdo, mu, mdu;
-  if ((rc = tgdn_make_token_map(&mdo, dO, B, T, H, 8, 64, 0))) return rc;
+  if ((rc = tgdn_make_token_map(&mdo, dO, B, T, H, 8, 64, 0, row_tokens))) return rc;
   if ((rc = tgdn_make_token_map(&mu, U, 1, static_cast<int>(crows), 1, 8, 64, 0))) return rc;
   if ((rc = tgdn_make_token_map(&mdu, dU, 1, static_cast<int>(crows), 1, 8, 64, 0))) return rc;
   RecParams p{static_cast<const __nv_bfloat16*>(dO), k2, q2, beta, gc, static_cast<const __nv_bfloat16*>(AP),
               static_cast<const __nv_bfloat16*>(Pm), static_cast<const __nv_bfloat16*>(U),
               static_cast<__nv_bfloat16*>(dV), static_cast<__nv_bfloat16*>(dU), static_cast<__nv_bfloat16*>(ds),
-              static_cast<__nv_bfloat16*>(dkg), dr, doc_offsets, chunk_map, B, T, H, NC, packed ? n_docs : B, scale,
+              static_cast<__nv_bfloat16*>(dkg), dr, doc_offsets, chunk_map, B, T, H, NC, packed ? n_docs : B, row_tokens, scale,
               tgdn_status_word(), grad_state_in, grad_state_out};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
@@ -798,6 +793,15 @@ extern "C" int tgdn_bwd_recurrent_state(const void* q, const void* k, const void
     case 16: return launch_rec<16, 16, 4, 2, 2>(mk, mq, mdo, mu, mdu, p, s);
     default: return TGDN_ERR_SHAPE;
   }
+}
+
+extern "C" int tgdn_bwd_recurrent_state(const void* q, const void* k, const void* dO, const float* k2, const float* q2,
+                                        const float* beta, const float* gc, const void* AP, const void* Pm, const void* U,
+                                        float scale, const int32_t* doc_offsets, const int32_t* chunk_map, int n_docs, int B,
+                                        int T, int H, int E, int NC, void* dV, void* dU, void* ds, void* dkg, float* dr,
+                                        const float* grad_state_in, float* grad_state_out, void* stream) {
+  return tgdn_bwd_recurrent_rows(q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, doc_offsets, chunk_map, n_docs, B, T, H, E, NC, T,
+                                 dV, dU, ds, dkg, dr, grad_state_in, grad_state_out, stream);
 }
 
 extern "C" int tgdn_bwd_recurrent(const void* q, const void* k, const void* dO, const float* k2, const float* q2,

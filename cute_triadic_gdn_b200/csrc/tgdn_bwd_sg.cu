@@ -188,7 +188,7 @@ sg_kernel(const __grid_constant__ CUtensorMap map_dv, const __grid_constant__ CU
     // ---- workers: prologue.  All global loads go out together, from clamped (always valid) addresses, and are masked when
     // they are used; the tensor core is meanwhile adding the value-block images and forming the first P tiles, which need
     // no gate.
-    const int64_t tok = static_cast<int64_t>(b) * p.T + t0;
+    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
     uint32_t kw[32];                                   // this thread's K row (Q row) over the key columns wg*64 .. +64, packed bf16 pairs
     if (worker) {
       const int tl = min(t, rows - 1);
@@ -502,20 +502,20 @@ template <int E>
 static int launch_sg(const CUtensorMap& mdv, const CUtensorMap& mdo, const SgParams& p, cudaStream_t s) {
   const int smem = static_cast<int>(sizeof(SgSmem<E>)) + 1024;
   static_assert(sizeof(SgSmem<E>) + 1024 <= 232448, "shared memory budget of one CTA exceeded");
-  cudaError_t e = cudaFuncSetAttribute(sg_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  static bool configured[64] = {};
+  if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(sg_kernel<E>), smem, configured)) return rc;
   const long long items = static_cast<long long>(p.B) * p.NC * p.H;
   const int grid = static_cast<int>(items < p.ahead ? items : p.ahead);      // persistent: one CTA per SM
   sg_kernel<E><<<grid, SG_BLOCK, smem, s>>>(mdv, mdo, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 
-extern "C" int tgdn_bwd_state_grads(const void* q, const void* k, const void* dO, const void* dV,
-                                    const void* h, const void* ds, const void* dkg, const float* k2, const float* q2,
-                                    const float* gc, float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC, void* dkq,
-                                    float* da, float* dc, float* dd, void* stream) {
+int tgdn_bwd_state_grads_rows(const void* q, const void* k, const void* dO, const void* dV, const void* h, const void* ds,
+                              const void* dkg, const float* k2, const float* q2, const float* gc, float scale,
+                              const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, void* dkq, float* da,
+                              float* dc, float* dd, void* stream) {
   if (!q || !k || !dO || !dV || !h || !ds || !dkg || !k2 || !q2 || !gc || !dkq || !da || !dc || !dd) return TGDN_ERR_NULL;
-  int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr);
+  int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr, row_tokens);
   if (rc) return rc;
   if (static_cast<long long>(B) * NC * H * 64 > 0x7fffffffLL) return TGDN_ERR_SHAPE;   // item indices are 32-bit in the kernel
   if ((reinterpret_cast<uintptr_t>(dO) | reinterpret_cast<uintptr_t>(dV) |
@@ -524,12 +524,12 @@ extern "C" int tgdn_bwd_state_grads(const void* q, const void* k, const void* dO
     return TGDN_ERR_ALIGN;
   if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(q)) & 15) return TGDN_ERR_ALIGN;
   CUtensorMap mdv, mdo;
-  if ((rc = tgdn_make_token_map(&mdv, dV, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&mdo, dO, B, T, H, 64, 64, 1))) return rc;
+  if ((rc = tgdn_make_token_map(&mdv, dV, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&mdo, dO, B, T, H, 64, 64, 1, row_tokens))) return rc;
   SgParams p{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(dO), static_cast<const __nv_bfloat16*>(dV),
              static_cast<const __nv_bfloat16*>(h),
              static_cast<const __nv_bfloat16*>(ds), static_cast<const __nv_bfloat16*>(dkg), k2, q2, gc,
-             static_cast<__nv_bfloat16*>(dkq), da, dc, dd, chunk_map, B, T, H, NC, HEAD / tgdn_value_block(E), scale,
+             static_cast<__nv_bfloat16*>(dkq), da, dc, dd, chunk_map, B, T, H, NC, HEAD / tgdn_value_block(E), row_tokens, scale,
              tgdn_status_word(), tgdn_sm_count()};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
@@ -541,4 +541,11 @@ extern "C" int tgdn_bwd_state_grads(const void* q, const void* k, const void* dO
     case 16: return launch_sg<16>(mdv, mdo, p, s);
     default: return TGDN_ERR_SHAPE;
   }
+}
+
+extern "C" int tgdn_bwd_state_grads(const void* q, const void* k, const void* dO, const void* dV,
+                                    const void* h, const void* ds, const void* dkg, const float* k2, const float* q2,
+                                    const float* gc, float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC, void* dkq,
+                                    float* da, float* dc, float* dd, void* stream) {
+  return tgdn_bwd_state_grads_rows(q, k, dO, dV, h, ds, dkg, k2, q2, gc, scale, chunk_map, B, T, H, E, NC, T, dkq, da, dc, dd, stream);
 }

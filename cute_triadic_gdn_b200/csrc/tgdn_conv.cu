@@ -549,8 +549,8 @@ extern "C" int tgdn_conv_fwd(const void* x, const void* weight, void* y, const i
   ConvArgs a{static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(y), nullptr, cu_seqlens, n_docs, T, C,
              act_channels, tpg, tgdn_status_word()};
   const int smem = CONV_FWD_STAGES * CONV_FWD_ROWS * CONV_CH * 2 + 128;
-  cudaError_t e = cudaFuncSetAttribute(conv_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  static bool configured[64] = {};
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(conv_fwd_kernel), smem, configured))) return rc;
   dim3 grid((C + CONV_CH - 1) / CONV_CH, groups, B);
   conv_fwd_kernel<<<grid, CONV_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(mx, a);
   return tgdn_cuda_error(cudaGetLastError());
@@ -579,8 +579,8 @@ static int conv_bwd_launch(const void* x, const void* weight, const void* dy, vo
   ConvArgs a{static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(dx), scratch, cu_seqlens, n_docs, T, C,
              act_channels, tpg, tgdn_status_word()};
   const int smem = CONV_BWD_STAGES * (CONV_BWD_XROWS + CONV_BWD_GROWS) * CONV_CH * 2 + 128;
-  cudaError_t e = cudaFuncSetAttribute(conv_bwd_kernel<CONV_BWD_NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  static bool configured[64] = {};
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(conv_bwd_kernel<CONV_BWD_NP>), smem, configured))) return rc;
   dim3 grid((C + CONV_CH - 1) / CONV_CH, groups, B);
   conv_bwd_kernel<CONV_BWD_NP><<<grid, CONV_THREADS * 2 / CONV_BWD_NP, smem, s>>>(mx, mg, a);
   rc = tgdn_cuda_error(cudaGetLastError());
@@ -919,11 +919,11 @@ static int glue_launch(const void* x, const void* weight, const int32_t* cu, int
              static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), static_cast<__nv_bfloat16*>(v), k2, q2,
              static_cast<__nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stride_b, stride_t, tgdn_status_word()};
   const int smem = CONV_FWD_STAGES * CONV_FWD_ROWS * CONV_CH * 2 + 128;
-  cudaError_t e = cudaFuncSetAttribute(glue_main_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  static bool configured[64] = {};
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(glue_main_kernel<BWD>), smem, configured))) return rc;
   dim3 grid((main_channels + CONV_CH - 1) / CONV_CH, groups, B);
   glue_main_kernel<BWD><<<grid, CONV_THREADS, smem, s>>>(mx, a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return tgdn_cuda_error(e);
+  if ((rc = tgdn_cuda_error(cudaGetLastError()))) return rc;
   const int64_t n = static_cast<int64_t>(B) * T * 2 * H;
   const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, static_cast<int64_t>(tgdn_sm_count()) * 16));
   switch (E) {

@@ -272,12 +272,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     int t0, rows;
     chunk_info(i, t0, rows);
     const int last = max(rows, 1) - 1;
-    const int64_t ro = (static_cast<int64_t>(b) * p.T + t0 + min(t, last)) * p.H + h;
+    const int64_t ro = (static_cast<int64_t>(b) * p.TS + t0 + min(t, last)) * p.H + h;
     if (!beta_tma) prefetch_l2(p.beta + ro);
     if (!C::TMA_V) prefetch_l2(p.v + ro * HEAD + v0g);
   };
   auto load_vrow = [&](int t0, int rows, uint32_t* out /* CW/2 words */) {   // CW value columns of row t (clamped), raw bf16
-    const int64_t tok = static_cast<int64_t>(b) * p.T + t0;
+    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
     const __nv_bfloat16* vp = p.v + ((tok + min(t, max(rows, 1) - 1)) * p.H + h) * HEAD + v0g;
     if constexpr (CW == 16) {
       const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(vp)), u1 = __ldg(reinterpret_cast<const uint4*>(vp) + 1);
@@ -324,7 +324,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     int t0, rows;
     chunk_info(i, t0, rows);
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
-    const int64_t tok = static_cast<int64_t>(b) * p.T + t0;
+    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
     const bool live = t < rows;
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     uint8_t* ap = smem + C::OFF_AP + st * C::AP_BYTES;
@@ -577,21 +577,16 @@ static int launch_fwd(const CUtensorMap& mk, const CUtensorMap& mq, const void* 
   static_assert(MINB == 1 || C::SMEM_BYTES <= 115712, "two CTAs per SM need at most 113 KB each");
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static_assert(MINB * C::TMEM_COLS <= 512, "tensor memory budget of one SM exceeded");
-  static bool configured[64] = {};                  // per device: the attribute is sticky, set it once
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64 || !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(fwd_kernel<E, CW, NCH, WPC, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return tgdn_cuda_error(e);
-    if (dev >= 0 && dev < 64) configured[dev] = true;
-  }
+  static bool configured[64] = {};
+  if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(fwd_kernel<E, CW, NCH, WPC, STAGES, MINB>), C::SMEM_BYTES, configured))
+    return rc;
   CUtensorMap mv = mk, mb = mk;                     // placeholders where the rows are not loaded by TMA
   if (C::TMA_V) {
-    const int rc = tgdn_make_token_map(&mv, v, p.B, p.T, p.H, CW, 64, 0);
+    const int rc = tgdn_make_token_map(&mv, v, p.B, p.T, p.H, CW, 64, 0, p.TS);
     if (rc) return rc;
   }
   if (C::TMA_BETA && p.beta_tma) {
-    const int rc = tgdn_make_gate_map(&mb, p.beta, p.B, p.T, p.H / 4, 4);    // (B, T, H) read as (B, T, H/4, 4)
+    const int rc = tgdn_make_gate_map(&mb, p.beta, p.B, p.T, p.H / 4, 4, p.TS);    // (B, T, H) read as (B, T, H/4, 4)
     if (rc) return rc;
   }
   const int grid = p.n_seq * p.H * (HEAD / C::VC);
@@ -600,14 +595,14 @@ static int launch_fwd(const CUtensorMap& mk, const CUtensorMap& mq, const void* 
 }
 
 
-extern "C" int tgdn_fwd_state(const void* q, const void* k, const void* v, const float* k2, const float* q2,
-                              const float* beta, const float* gc, const void* AP, float scale, const int32_t* doc_offsets,
-                              const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, void* o, void* W,
-                              void* U, void* h, const float* state_in, float* state_out, void* stream) {
+int tgdn_fwd_rows(const void* q, const void* k, const void* v, const float* k2, const float* q2, const float* beta, const float* gc,
+                  const void* AP, float scale, const int32_t* doc_offsets, const int32_t* chunk_map, int n_docs, int B, int T, int H,
+                  int E, int NC, int row_tokens, void* o, void* W, void* U, void* h, const float* state_in, float* state_out,
+                  void* stream) {
   if (!q || !k || !v || !k2 || !q2 || !beta || !gc || !AP || !o) return TGDN_ERR_NULL;
   const bool packed = chunk_map != nullptr;
   if (packed && (!doc_offsets || n_docs < 1)) return TGDN_ERR_NULL;
-  int rc = tgdn_check_core_shape(B, T, H, E, NC, packed);
+  int rc = tgdn_check_core_shape(B, T, H, E, NC, packed, row_tokens);
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(AP) |
        reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(h) |
@@ -615,12 +610,12 @@ extern "C" int tgdn_fwd_state(const void* q, const void* k, const void* v, const
        reinterpret_cast<uintptr_t>(state_in) | reinterpret_cast<uintptr_t>(state_out)) & 15)
     return TGDN_ERR_ALIGN;
   CUtensorMap mk, mq;
-  if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1))) return rc;
+  if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1, row_tokens))) return rc;
   FwdParams p{static_cast<const __nv_bfloat16*>(v), k2, q2, beta, gc, static_cast<const __nv_bfloat16*>(AP),
               static_cast<__nv_bfloat16*>(o), static_cast<__nv_bfloat16*>(W), static_cast<__nv_bfloat16*>(U),
               static_cast<__nv_bfloat16*>(h), state_in, state_out, doc_offsets, chunk_map, B, T, H, NC,
-              packed ? n_docs : B, scale, tgdn_status_word(),
+              packed ? n_docs : B, row_tokens, scale, tgdn_status_word(),
               (H % 4 == 0 && (reinterpret_cast<uintptr_t>(beta) & 15) == 0) ? 1 : 0};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
@@ -641,6 +636,14 @@ extern "C" int tgdn_fwd_state(const void* q, const void* k, const void* v, const
     case 16: return launch_fwd<16, 8, 2, 2, 2, 1>(mk, mq, v, p, s);
     default: return TGDN_ERR_SHAPE;
   }
+}
+
+extern "C" int tgdn_fwd_state(const void* q, const void* k, const void* v, const float* k2, const float* q2,
+                              const float* beta, const float* gc, const void* AP, float scale, const int32_t* doc_offsets,
+                              const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, void* o, void* W,
+                              void* U, void* h, const float* state_in, float* state_out, void* stream) {
+  return tgdn_fwd_rows(q, k, v, k2, q2, beta, gc, AP, scale, doc_offsets, chunk_map, n_docs, B, T, H, E, NC, T, o, W, U, h,
+                       state_in, state_out, stream);
 }
 
 extern "C" int tgdn_fwd(const void* q, const void* k, const void* v, const float* k2, const float* q2, const float* beta,

@@ -15,12 +15,14 @@ int tgdn_cuda_error(cudaError_t e);
 int* tgdn_status_word();
 
 // Tensor map over a (B, T, H, 128) bf16 tensor in token layout: box = [box_cols columns][1 head][box_rows tokens][1 row].
-// swizzle128 = 1 asks for the 128-byte swizzle (box_cols must then be 64).
-int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows, int swizzle128);
+// swizzle128 = 1 asks for the 128-byte swizzle (box_cols must then be 64).  row_tokens: tokens from one batch row to the next
+// (0: T), for a token range of longer rows.
+int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows, int swizzle128,
+                        int row_tokens = 0);
 
 // Tensor map over a (B, T, H, E) f32 gate tensor (k2, q2) in token layout, E a multiple of 4: box = [E][1 head][64 tokens][1 row],
 // which lands in shared memory as 64 dense rows of E floats.
-int tgdn_make_gate_map(CUtensorMap* map, const float* base, int B, int T, int H, int E);
+int tgdn_make_gate_map(CUtensorMap* map, const float* base, int B, int T, int H, int E, int row_tokens = 0);
 
 // Tensor map over a (B, T, C) bf16 tensor with element strides (stride_b, stride_t, 1): box = [box_cols][box_rows][1], no swizzle.
 int tgdn_make_rows_map(CUtensorMap* map, const void* base, int C, int T, int B, int64_t stride_t, int64_t stride_b, int box_cols,
@@ -28,3 +30,31 @@ int tgdn_make_rows_map(CUtensorMap* map, const void* base, int C, int T, int B, 
 
 // True when the current device is compute capability 10.x; also binds the device's primary context to the calling thread.
 int tgdn_check_device();
+
+// Opts a kernel in to `bytes` of dynamic shared memory on the current device, once per device (configured[64]).
+int tgdn_dynamic_smem(const void* kernel, int bytes, bool* configured);
+
+// The core stages on a token range of longer rows: the arguments of the entry points of the same name (include/tgdn.h) plus
+// row_tokens >= T, the tokens from one batch row to the next in every token-layout tensor (inputs and outputs; the chunk-layout
+// tensors are those of the T tokens alone).  Dense rows; the entry points of the public ABI are these with row_tokens = T.
+int tgdn_masks_rows(const void* q, const void* k, const float* k2, const float* q2, const float* g, const float* beta, float scale,
+                    const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, float* gc, void* AP, void* Pm,
+                    void* stream);
+int tgdn_fwd_rows(const void* q, const void* k, const void* v, const float* k2, const float* q2, const float* beta, const float* gc,
+                  const void* AP, float scale, const int32_t* doc_offsets, const int32_t* chunk_map, int n_docs, int B, int T, int H,
+                  int E, int NC, int row_tokens, void* o, void* W, void* U, void* h, const float* state_in, float* state_out,
+                  void* stream);
+int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
+                            const float* gc, const void* AP, const void* Pm, const void* U, float scale, const int32_t* doc_offsets,
+                            const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, void* dV,
+                            void* dU, void* ds, void* dkg, float* dr, const float* grad_state_in, float* grad_state_out,
+                            void* stream);
+int tgdn_bwd_state_grads_rows(const void* q, const void* k, const void* dO, const void* dV, const void* h, const void* ds,
+                              const void* dkg, const float* k2, const float* q2, const float* gc, float scale,
+                              const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, void* dkq, float* da,
+                              float* dc, float* dd, void* stream);
+int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const void* dU, const void* W, const void* U, const void* AP,
+                         const float* k2, const float* q2, const float* beta, const float* gc, const void* dkq, const float* da,
+                         const float* dc, const float* dd, const float* dr, float scale, const int32_t* chunk_map, int B, int T,
+                         int H, int E, int NC, int row_tokens, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
+                         void* stream);

@@ -39,6 +39,7 @@ struct MaskParams {
   __nv_bfloat16* Pm;
   const int32_t* cmap;      // (3, NC) chunk map of a packed row, or nullptr
   int B, T, H, NC;
+  int TS;                   // tokens from one batch row to the next in the token-layout tensors (T: packed tightly)
   float scale;
   int* status;
 };
@@ -59,6 +60,7 @@ struct FwdParams {
   const int32_t* offsets;   // packed: first chunk of every document (n_seq + 1 entries), else nullptr
   const int32_t* cmap;
   int B, T, H, NC, n_seq;   // n_seq = documents (packed) or batch rows (dense)
+  int TS;                   // tokens from one batch row to the next in the token-layout tensors
   float scale;
   int* status;
   int beta_tma;             // beta rows of a chunk arrive by TMA (H a multiple of 4, base 16-byte aligned), else by global loads
@@ -80,7 +82,7 @@ struct RecParams {
   float* dr;                // f32 [item][128/VC][64][E] (out): sum_v U*(K G_e) per value block
   const int32_t* offsets;
   const int32_t* cmap;
-  int B, T, H, NC, n_seq;
+  int B, T, H, NC, n_seq, TS;
   float scale;
   int* status;
   const float* g_in;        // f32 [sequence][H][E][128 d][128 v]: dL/dS after the last token (a later segment's hand-off), or nullptr (zero)
@@ -103,7 +105,7 @@ struct SgParams {
   float* dc;                // f32 [item][64][E] (out)
   float* dd;                // f32 [item][E] (out)
   const int32_t* cmap;
-  int B, T, H, NC, NV;
+  int B, T, H, NC, NV, TS;
   float scale;
   int* status;
   int ahead;                // CTAs to launch (the SM count): the kernel is persistent, CTA c takes items c, c + ahead, ...
@@ -127,7 +129,7 @@ struct MatParams {
   float* dg;
   float* dbeta;
   const int32_t* cmap;
-  int B, T, H, NC, NV;
+  int B, T, H, NC, NV, TS;
   float scale;
   int* status;
   int ahead;                // CTAs to launch (the SM count): the kernel is persistent, CTA c takes items c, c + ahead, ...
@@ -136,7 +138,7 @@ struct MatParams {
 }  // namespace tgdn
 
 // E in {1,2,4,8,12,16}; dense rows need T % 64 == 0 and NC == T/64; packed rows need B == 1.
-int tgdn_check_core_shape(int B, int T, int H, int E, int NC, int packed);
+int tgdn_check_core_shape(int B, int T, int H, int E, int NC, int packed, int row_tokens);
 // Width of the value-axis block one CTA of the recurrences owns, by E.
 int tgdn_value_block(int E);
 int tgdn_sm_count();

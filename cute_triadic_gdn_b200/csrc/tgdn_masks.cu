@@ -177,7 +177,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
 
   // gates of the chunk: rows past the document end count as g = 0, k2 = q2 = beta = 0.  All loads are requested first, from
   // clamped (always valid) addresses, and masked when stored: the block pays one memory round trip, not one per iteration.
-  const int64_t tok = static_cast<int64_t>(b) * p.T + t0;
+  const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
   {
     constexpr int GATE_ITERS = (64 * E + MASK_THREADS - 1) / MASK_THREADS;
     float g_in[GATE_ITERS], k2_in[GATE_ITERS], q2_in[GATE_ITERS];
@@ -475,24 +475,24 @@ using namespace tgdn;
 template <int E>
 static int launch_masks(const CUtensorMap& mk, const CUtensorMap& mq, const MaskParams& p, cudaStream_t s) {
   const int smem = static_cast<int>(sizeof(MaskSmem<E>)) + 1024;
-  cudaError_t e = cudaFuncSetAttribute(masks_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return tgdn_cuda_error(e);
+  static bool configured[64] = {};
+  if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(masks_kernel<E>), smem, configured)) return rc;
   masks_kernel<E><<<p.B * p.NC * p.H, MASK_THREADS, smem, s>>>(mk, mq, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 
-extern "C" int tgdn_masks(const void* q, const void* k, const float* k2, const float* q2, const float* g,
-                          const float* beta, float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC,
-                          float* gc, void* AP, void* Pm, void* stream) {
+int tgdn_masks_rows(const void* q, const void* k, const float* k2, const float* q2, const float* g, const float* beta, float scale,
+                    const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, float* gc, void* AP, void* Pm,
+                    void* stream) {
   if (!q || !k || !k2 || !q2 || !g || !beta || !gc || !AP || !Pm) return TGDN_ERR_NULL;
-  int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr);
+  int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr, row_tokens);
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(AP) | reinterpret_cast<uintptr_t>(Pm)) & 15) return TGDN_ERR_ALIGN;
   CUtensorMap mk, mq;
-  if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1))) return rc;
-  if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1))) return rc;
+  if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1, row_tokens))) return rc;
+  if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1, row_tokens))) return rc;
   MaskParams p{k2, q2, g, beta, gc, static_cast<__nv_bfloat16*>(AP), static_cast<__nv_bfloat16*>(Pm), chunk_map,
-               B, T, H, NC, scale, tgdn_status_word()};
+               B, T, H, NC, row_tokens, scale, tgdn_status_word()};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1: return launch_masks<1>(mk, mq, p, s);
@@ -503,4 +503,10 @@ extern "C" int tgdn_masks(const void* q, const void* k, const float* k2, const f
     case 16: return launch_masks<16>(mk, mq, p, s);
     default: return TGDN_ERR_SHAPE;
   }
+}
+
+extern "C" int tgdn_masks(const void* q, const void* k, const float* k2, const float* q2, const float* g,
+                          const float* beta, float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC,
+                          float* gc, void* AP, void* Pm, void* stream) {
+  return tgdn_masks_rows(q, k, k2, q2, g, beta, scale, chunk_map, B, T, H, E, NC, T, gc, AP, Pm, stream);
 }
