@@ -1,4 +1,5 @@
-"""ctypes binding of libtgdn_b200.so (the C ABI declared in include/tgdn.h).
+"""Loads the compiled parts of the package: libtgdn_b200.so through ctypes (`lib`: the C ABI declared in include/tgdn.h) and the
+host path _tgdn_torch.so, a torch extension (`host`: operators, autograd and launches; csrc/tgdn_torch.cpp).
 
 The library is the only implementation of the hot path: there is no fallback.  If the shared object is missing it is
 built once with nvcc (cute_triadic_gdn_b200/build.py); if that is impossible the import fails loudly.
@@ -69,7 +70,7 @@ def _load():
     try:
         mod.build()
     except Exception as exc:
-        if not os.path.exists(LIB_PATH):
+        if not (os.path.exists(LIB_PATH) and os.path.exists(mod.HOST_OUT)):
             raise
         if not mod.up_to_date():
             raise RuntimeError("libtgdn_b200.so is older than its sources and could not be rebuilt "
@@ -78,10 +79,15 @@ def _load():
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)
         fn.restype, fn.argtypes = res, args
-    return lib
+    import torch  # noqa: F401  (the extension needs torch's libraries in the process)
+    spec = importlib.util.spec_from_file_location(mod.HOST_MODULE, mod.HOST_OUT)
+    host = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(host)
+    host.set_library_error(TgdnError)
+    return lib, host
 
 
-lib = _load()
+lib, host = _load()
 
 
 def check(code, what):

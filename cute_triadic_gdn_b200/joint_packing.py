@@ -6,9 +6,8 @@ prepare_documents): same checks, same errors, no host read of the offsets.
 from __future__ import annotations
 
 import torch
-from torch.library import custom_op
 
-from . import _lib
+from . import _lib  # noqa: F401  (registers the operator)
 
 CHUNK = 64
 NC_BUCKET = 16
@@ -22,22 +21,12 @@ def chunk_capacity(tokens, documents):
     return NC_BUCKET * (-(-worst // NC_BUCKET))
 
 
-@custom_op("tgdn_b200::joint_metadata", mutates_args=(), device_types="cuda")
-def _metadata(cu_seqlens: torch.Tensor, tokens: int) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    documents = cu_seqlens.numel() - 1
-    capacity = chunk_capacity(tokens, documents)
-    dev = cu_seqlens.device
-    offsets = torch.empty(documents + 1, dtype=torch.int32, device=dev)
-    mapping = torch.empty((3, capacity), dtype=torch.int32, device=dev)
-    valid = torch.empty(1, dtype=torch.bool, device=dev)
-    with torch.cuda.device(dev):
-        _lib.check(_lib.lib.tgdn_metadata(_lib.ptr(cu_seqlens), int(cu_seqlens.dtype == torch.int64), documents,
-                                          int(tokens), _lib.ptr(offsets), _lib.ptr(mapping), capacity, _lib.ptr(valid),
-                                          _lib.stream_of(cu_seqlens)), "tgdn_metadata")
-    return offsets, mapping, valid
+def _metadata(cu_seqlens, tokens):
+    """(first chunk of every document, chunk map, validity flag) of a packed row, built on the device (csrc/tgdn_torch.cpp)."""
+    return torch.ops.tgdn_b200.joint_metadata(cu_seqlens, int(tokens))
 
 
-@_metadata.register_fake
+@torch.library.register_fake("tgdn_b200::joint_metadata")
 def _metadata_shapes(cu_seqlens, tokens):
     n = cu_seqlens.numel() - 1
     like = cu_seqlens.new_empty
@@ -45,7 +34,7 @@ def _metadata_shapes(cu_seqlens, tokens):
 
 
 def _validate(inputs, cu_seqlens):
-    """What can be checked without reading the offsets: a ValueError for the conditions the reference rejects
+    """(While tracing; prepare_documents in csrc/tgdn_torch.cpp is the same natively.)  What can be checked without reading the offsets: a ValueError for the conditions the reference rejects
     (ops/joint_packing.py:38-49).  The values themselves are checked on the device."""
     row = inputs[0]
     if row.shape[0] != 1 or row.shape[1] < 1:
@@ -65,6 +54,6 @@ def prepare_documents(inputs, cu_seqlens):
     copied and nothing is read back.  Offsets that do not start at 0, end at T and strictly increase trip a device-side
     assertion, as in the reference (ops/joint_packing.py:52-62)."""
     _validate(inputs, cu_seqlens)
-    offsets, mapping, valid = _metadata(cu_seqlens, inputs[0].shape[1])
+    offsets, mapping, valid = torch.ops.tgdn_b200.joint_metadata(cu_seqlens, inputs[0].shape[1])
     torch._assert_async(valid, "cu_seqlens must start at 0, end at T, and strictly increase")
     return offsets, mapping
