@@ -95,16 +95,15 @@ struct FwdCfg {
   static constexpr int OFF_GT = (OFF_BW + NCH * BW_BYTES + 127) & ~127;
   // per stage: the value rows of the CTA's columns, one box of 64 rows x CW columns per chain (TMA; a row of a box is at
   // least 16 bytes), and the beta rows of the chunk for the four heads h & ~3 .. (TMA when H is a multiple of 4)
-  static constexpr bool TMA_V = CW >= 8;
   static constexpr int VBOX_BYTES = 64 * CW * 2;
-  static constexpr int VT_BYTES = TMA_V ? NCH * VBOX_BYTES : 0;
+  static constexpr int VT_BYTES = NCH * VBOX_BYTES;
   static constexpr int OFF_VT = OFF_GT + STAGES * GT_STRIDE;
   static constexpr int OFF_BT = OFF_VT + STAGES * VT_BYTES;
   static constexpr bool TMA_BETA = OFF_BT + STAGES * 1024 + 128 + 1024 <= 232448;   // where the beta rows still fit
   static constexpr int BT_BYTES = TMA_BETA ? 1024 : 0;
   static constexpr int OFF_CTRL = OFF_BT + STAGES * BT_BYTES;
   static constexpr int SMEM_BYTES = OFF_CTRL + 128 + 1024;    // + control block + alignment slack
-  static_assert(CW == 4 || CW == 8 || CW == 16, "a chain owns 4, 8 or 16 value columns");
+  static_assert(CW == 8 || CW == 16, "a chain owns 8 or 16 value columns");
   static_assert(E % WPC == 0 && (WPC == 1 || ET % 2 == 0), "the slices split evenly over the chain's warpgroups");
   static_assert(TPC % 16 == 0 && TPC <= 256, "columns per chain: a multiple of 16 (MMA N)");
   static_assert(TPT % 16 == 0 && TPT <= 64, "columns per thread: a multiple of 16 (tensor-memory loads), at most 64 registers of state");
@@ -122,12 +121,14 @@ struct FwdCtrl {
 template <int E, int CW, int NCH, int WPC, int STAGES, int MINB>
 __global__ void __launch_bounds__(NCH * WPC * 128, MINB)
 fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_beta,
-           const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q, FwdParams p) {
+           const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
+           const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_w,
+           const __grid_constant__ CUtensorMap map_u, FwdParams p) {
   using C = FwdCfg<E, CW, NCH, WPC, STAGES>;
   constexpr int TPC = C::TPC, VC = C::VC, ET = C::ET, TPT = C::TPT, CT = C::CHAIN_THREADS;
   // Roles inside a chain: its key-row warps (0, 1) have the longer epilogues (gate factors r_e, the operand images of W
   // and of r_e U), so the query-row warps take the extra work: warp 2 issues the MMAs and polls their barrier, warp 3
-  // hands stages back and issues the loads.
+  // hands stages back and issues the loads and stores.
   constexpr int ISSUE_WARP = 2, REFILL_WARP = 3;
   const bool beta_tma = C::TMA_BETA && p.beta_tma;
   constexpr bool LATE_R = E >= 12;                   // read r_e after the epilogue of (1) (register pressure at many slices)
@@ -178,7 +179,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
 #pragma unroll
     for (int e = 0; e < ET; ++e)
 #pragma unroll
-      for (int c = 0; c < CW; ++c) S[e * CW + c] = __ldg(src + e * (HEAD * HEAD) + c);
+      for (int c = 0; c < CW; c += 4) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(src + e * (HEAD * HEAD) + c));
+        S[e * CW + c] = x.x; S[e * CW + c + 1] = x.y; S[e * CW + c + 2] = x.z; S[e * CW + c + 3] = x.w;
+      }
   } else {
 #pragma unroll
     for (int j = 0; j < TPT; ++j) S[j] = 0.f;
@@ -186,28 +190,17 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
   // the second 8-column block of the (2) operand is never written: keep it zero (its products land in unused columns)
   for (int i = (tid & (CT - 1)); i < C::BW_BYTES / 16; i += CT) reinterpret_cast<uint4*>(bw_img)[i] = make_uint4(0, 0, 0, 0);
 
-  // saved state / operand image of this thread's S: pieces of 8 columns (one 16-byte store each into the image)
-  auto state_item_ptr = [&](int64_t item) {
-    return reinterpret_cast<uint8_t*>(p.h) + item * (static_cast<int64_t>(E) * 32768);
-  };
-  auto store_state_slices = [&](uint8_t* hbase, int j0, const uint32_t* packed /* 8 words = 16 columns from j0 */) {
+  // The operand image of S is also the saved state: its 8-column blocks (128 key rows x 16 bytes) are the [v / 8][d][v % 8]
+  // blocks of h, so the state of a chunk leaves by bulk copies straight from the image (one thread, 2 KB each).
+  auto save_state = [&](int64_t item) {
+    uint8_t* dst = reinterpret_cast<uint8_t*>(p.h) + item * (static_cast<int64_t>(E) * 32768) + (v0g >> 3) * 2048;
 #pragma unroll
-    for (int j = 0; j < 16; j += CW) {
-      const int e = e0 + (j0 + j) / CW;
-      uint8_t* dst = hbase + e * 32768 + (v0g >> 3) * 2048 + row * 16 + (v0g & 7) * 2;
-      if constexpr (CW == 16) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        *reinterpret_cast<uint4*>(dst + 2048) = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-      } else if constexpr (CW == 8) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[j / 2], packed[j / 2 + 1], packed[j / 2 + 2], packed[j / 2 + 3]);
-      } else {
-        *reinterpret_cast<uint2*>(dst) = make_uint2(packed[j / 2], packed[j / 2 + 1]);
-      }
-    }
+    for (int e = 0; e < E; ++e)
+#pragma unroll
+      for (int cb = 0; cb < CW / 8; ++cb) bulk_store(dst + e * 32768 + cb * 2048, s_img + (e * (CW / 8) + cb) * 2048, 2048);
   };
   {
     const uint32_t base = smem_u32(s_img) + (row >> 3) * 128 + (row & 7) * 16;
-    uint8_t* hbase = p.h != nullptr ? state_item_ptr((static_cast<int64_t>(b) * p.NC + first) * p.H + h) : nullptr;
 #pragma unroll
     for (int j0 = 0; j0 < TPT; j0 += 16) {
       uint32_t packed[8];
@@ -215,7 +208,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       for (int j = 0; j < 16; j += 2) packed[j / 2] = pack_bf16(S[j0 + j], S[j0 + j + 1]);
       st_shared_v4(base + ((col0 + j0) >> 3) * 2048, packed[0], packed[1], packed[2], packed[3]);
       st_shared_v4(base + ((col0 + j0 + 8) >> 3) * 2048, packed[4], packed[5], packed[6], packed[7]);
-      if (hbase != nullptr) store_state_slices(hbase, j0, packed);
     }
   }
   fence_async_smem();
@@ -243,11 +235,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
     mbar_expect_tx(&ctrl.bar_load[st], C::KQ_BYTES + C::AP_BYTES + C::GT_BYTES + C::VT_BYTES + (beta_tma ? C::BT_BYTES : 0));
-    if constexpr (C::TMA_V) {
 #pragma unroll
-      for (int c = 0; c < NCH; ++c)
-        tma_load_4d(smem + C::OFF_VT + st * C::VT_BYTES + c * C::VBOX_BYTES, &map_v, &ctrl.bar_load[st], vb * VC + c * CW, h, t0, b);
-    }
+    for (int c = 0; c < NCH; ++c)
+      tma_load_4d(smem + C::OFF_VT + st * C::VT_BYTES + c * C::VBOX_BYTES, &map_v, &ctrl.bar_load[st], vb * VC + c * CW, h, t0, b);
     if (beta_tma) tma_load_4d(smem + C::OFF_BT + st * C::BT_BYTES, &map_beta, &ctrl.bar_load[st], 0, h >> 2, t0, b);
     bulk_load(smem + C::OFF_GT + st * C::GT_STRIDE, p.gc + item * gate_item_floats(E) + 64 * E, C::GT_BYTES, &ctrl.bar_load[st]);
     tma_load_4d(kq, &map_k, &ctrl.bar_load[st], 0, h, t0, b);
@@ -274,42 +264,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     const int last = max(rows, 1) - 1;
     const int64_t ro = (static_cast<int64_t>(b) * p.TS + t0 + min(t, last)) * p.H + h;
     if (!beta_tma) prefetch_l2(p.beta + ro);
-    if (!C::TMA_V) prefetch_l2(p.v + ro * HEAD + v0g);
   };
-  auto load_vrow = [&](int t0, int rows, uint32_t* out /* CW/2 words */) {   // CW value columns of row t (clamped), raw bf16
-    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
-    const __nv_bfloat16* vp = p.v + ((tok + min(t, max(rows, 1) - 1)) * p.H + h) * HEAD + v0g;
-    if constexpr (CW == 16) {
-      const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(vp)), u1 = __ldg(reinterpret_cast<const uint4*>(vp) + 1);
-      out[0] = u0.x; out[1] = u0.y; out[2] = u0.z; out[3] = u0.w; out[4] = u1.x; out[5] = u1.y; out[6] = u1.z; out[7] = u1.w;
-    } else if constexpr (CW == 8) {
-      const uint4 u0 = __ldg(reinterpret_cast<const uint4*>(vp));
-      out[0] = u0.x; out[1] = u0.y; out[2] = u0.z; out[3] = u0.w;
-    } else {
-      const uint2 u0 = __ldg(reinterpret_cast<const uint2*>(vp));
-      out[0] = u0.x; out[1] = u0.y;
-    }
-  };
-  auto store_row_global = [&](__nv_bfloat16* ptr, const float* src) {         // CW consecutive bf16
+  // CW packed bf16 (CW/2 words) of one row -> 8-column blocks `stride` bytes apart
+  auto store_packed = [&](uint32_t dst, uint32_t stride, const uint32_t* w) {
 #pragma unroll
-    for (int c = 0; c < CW; c += 8) {
-      if constexpr (CW >= 8)
-        *reinterpret_cast<uint4*>(ptr + c) = make_uint4(pack_bf16(src[c], src[c + 1]), pack_bf16(src[c + 2], src[c + 3]),
-                                                        pack_bf16(src[c + 4], src[c + 5]), pack_bf16(src[c + 6], src[c + 7]));
-      else
-        *reinterpret_cast<uint2*>(ptr) = make_uint2(pack_bf16(src[0], src[1]), pack_bf16(src[2], src[3]));
-    }
-  };
-  // CW consecutive columns n0.. of row r of an image whose 8-column blocks are SJ bytes apart
-  auto store_row_image = [&](uint32_t row_base, int n0, uint32_t SJ, const float* src, float f) {
-    if constexpr (CW >= 8) {
-#pragma unroll
-      for (int c = 0; c < CW; c += 8)
-        st_shared_v4(row_base + ((n0 + c) >> 3) * SJ, pack_bf16(f * src[c], f * src[c + 1]), pack_bf16(f * src[c + 2], f * src[c + 3]),
-                     pack_bf16(f * src[c + 4], f * src[c + 5]), pack_bf16(f * src[c + 6], f * src[c + 7]));
-    } else {
-      st_shared_v2(row_base + (n0 >> 3) * SJ + (n0 & 7) * 2, pack_bf16(f * src[0], f * src[1]), pack_bf16(f * src[2], f * src[3]));
-    }
+    for (int c = 0; c < CW / 2; c += 4) st_shared_v4(dst + (c >> 2) * stride, w[c], w[c + 1], w[c + 2], w[c + 3]);
   };
 
   if (tid == 0) {
@@ -326,6 +285,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
     const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
     const bool live = t < rows;
+    const bool o_tile = rows == CHUNK;               // a chunk cut short by a document end cannot leave as a tile
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     uint8_t* ap = smem + C::OFF_AP + st * C::AP_BYTES;
 
@@ -347,12 +307,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     __syncwarp();                                    // the other lanes must not run ahead into a spin wait
     // The chain finished with the previous chunk's tiles when its third MMA group completed.  It says so now, under this
     // MMA, where its warps have time to spare; the last chain to say so refills that stage with the chunk STAGES ahead.
-    if (i > 0 && cwarp_u == REFILL_WARP && elect_one()) {
-      const uint32_t done = atomicAdd(&ctrl.released[(i - 1) % STAGES], 1u) + 1u;
-      if (done % NCH == 0) {
-        if (i - 1 + STAGES < count) issue_loads(i - 1 + STAGES);
-        if (i + STAGES < count) prefetch_tiles(i + STAGES);
+    // (o left from the stage's value rows, W and U from the place of beta*W: the stores must have read them.)
+    if (cwarp_u == REFILL_WARP && elect_one()) {
+      if (i > 0) {
+        bulk_wait_group_read();
+        const uint32_t done = atomicAdd(&ctrl.released[(i - 1) % STAGES], 1u) + 1u;
+        if (done % NCH == 0) {
+          if (i - 1 + STAGES < count) issue_loads(i - 1 + STAGES);
+          if (i + STAGES < count) prefetch_tiles(i + STAGES);
+        }
       }
+      if (p.h != nullptr) save_state(item);
+      bulk_commit_group();
     }
     __syncwarp();
     // Under the MMA: this row's gate factors, value row and beta from the stage.
@@ -360,6 +326,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     float ga[ET];                                    // this thread's slices.  K rows: a_e = k2 exp(gc); Q rows: c_e = scale q2 exp(gc)
     float gr[ET];                                    // K rows: r_e = k2 exp(gL - gc)
     float bt = 0.f;
+    // This chain's value rows in the stage (64 rows x CW columns): read here, then the place from which W and, after it, o
+    // leave.  One 16-byte store per row into the tile and one TMA store replace a store per thread into a row of its own,
+    // which cost 32 wavefronts of the L1 data path per warp (768 of about 4900 per chunk at E = 8).
+    uint8_t* vbox = smem + C::OFF_VT + st * C::VT_BYTES + chain * C::VBOX_BYTES;
+    const uint32_t vrow = smem_u32(vbox) + t * (CW * 2);
     uint32_t vraw[CW / 2];
     if constexpr (WPC > 1) {
 #pragma unroll
@@ -375,14 +346,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
           } else {
             bt = __ldg(p.beta + (tok + min(t, max(rows, 1) - 1)) * p.H + h);
           }
-          if constexpr (C::TMA_V) {
-            const uint32_t va = smem_u32(smem + C::OFF_VT + st * C::VT_BYTES + chain * C::VBOX_BYTES) + t * (CW * 2);
 #pragma unroll
-            for (int c = 0; c < CW / 2; c += 4)
-              asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(vraw[c]), "=r"(vraw[c + 1]), "=r"(vraw[c + 2]), "=r"(vraw[c + 3]) : "r"(va + c * 4));
-          } else {
-            load_vrow(t0, rows, vraw);
-          }
+          for (int c = 0; c < CW / 2; c += 4)
+            asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(vraw[c]), "=r"(vraw[c + 1]), "=r"(vraw[c + 2]), "=r"(vraw[c + 3]) : "r"(vrow + c * 4));
         }
         if (!live) bt = 0.f;
       } else {
@@ -436,9 +402,22 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       }
     }
     if (krow && sw == 0) {
-      // W -> saved (bf16), beta*W -> operand image (i = s, j = v)
-      store_row_image(smem_u32(bw_img) + (t >> 3) * 128 + (t & 7) * 16, 0, 1024, acc, bt);
-      if (p.W != nullptr) store_row_global(p.W + (item * 64 + t) * HEAD + v0g, acc);
+      // beta*W -> operand image (i = s, j = v); W -> the value tile, to be saved (bf16)
+      uint32_t w[CW / 2];
+#pragma unroll
+      for (int c = 0; c < CW; c += 2) w[c >> 1] = pack_bf16(bt * acc[c], bt * acc[c + 1]);
+      store_packed(smem_u32(bw_img) + t * 16, 1024, w);
+      if (p.W != nullptr) {
+#pragma unroll
+        for (int c = 0; c < CW; c += 2) w[c >> 1] = pack_bf16(acc[c], acc[c + 1]);
+        if constexpr (CW == 8) {                     // behind the operand, where the product's unused columns read
+          store_packed(smem_u32(bw_img) + 1024 + t * 16, 1024, w);
+        } else {
+          __nv_bfloat16* dst = p.W + (item * 64 + t) * HEAD + v0g;
+#pragma unroll
+          for (int c = 0; c < CW / 2; c += 4) *reinterpret_cast<uint4*>(dst + 2 * c) = make_uint4(w[c], w[c + 1], w[c + 2], w[c + 3]);
+        }
+      }
     }
     fence_async_smem();
     tc_fence_before();
@@ -455,6 +434,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
         umma_bf16(tmem_c + TPC, desc_advance(da, kk * 4096), desc_advance(db, kk * 256), idesc, kk > 0);
       umma_commit(&ctrl.bar_mma[chain]);
     }
+    __syncwarp();
+    if (CW == 8 && p.W != nullptr && cwarp_u == REFILL_WARP && elect_one())
+      tma_store_4d(&map_w, bw_img + 1024, v0g, 0, static_cast<int>(item) * 64, 0);
     __syncwarp();
     if constexpr (LATE_R) {                          // r_e only now, from the stage: sixteen registers fewer are live
       if (krow) lds_part<ET>(gf + C::GF_R + t * E + e0, gr);   // through the epilogue of (1)
@@ -473,34 +455,29 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
         uint32_t uw[CW / 2];
 #pragma unroll
         for (int c = 0; c < CW; c += 2) uw[c >> 1] = pack_bf16(u[c], u[c + 1]);
-        if (p.U != nullptr && sw == 0) {
-          __nv_bfloat16* dst = p.U + (item * 64 + t) * HEAD + v0g;
-          if constexpr (CW >= 8) {
-#pragma unroll
-            for (int c = 0; c < CW / 2; c += 4) *reinterpret_cast<uint4*>(dst + 2 * c) = make_uint4(uw[c], uw[c + 1], uw[c + 2], uw[c + 3]);
-          } else {
-            *reinterpret_cast<uint2*>(dst) = make_uint2(uw[0], uw[1]);
-          }
-        }
+        // (the operand beta*W has been read: its place takes U, which leaves from there by TMA)
+        if (p.U != nullptr && sw == 0) store_packed(smem_u32(bw_img) + t * 16, 1024, uw);
         const uint32_t base = smem_u32(vn_img) + (t >> 3) * 128 + (t & 7) * 16;
 #pragma unroll
         for (int e = 0; e < ET; ++e) {
           const uint32_t rr = pack_bf16(gr[e], gr[e]);
           const int n0 = (e0 + e) * CW;
-          if constexpr (CW >= 8) {
 #pragma unroll
-            for (int c = 0; c < CW / 2; c += 4)
-              st_shared_v4(base + ((n0 + 2 * c) >> 3) * 1024, mul_bf16x2(uw[c], rr), mul_bf16x2(uw[c + 1], rr), mul_bf16x2(uw[c + 2], rr),
-                           mul_bf16x2(uw[c + 3], rr));
-          } else {
-            st_shared_v2(base + (n0 >> 3) * 1024 + (n0 & 7) * 2, mul_bf16x2(uw[0], rr), mul_bf16x2(uw[1], rr));
-          }
+          for (int c = 0; c < CW / 2; c += 4)
+            st_shared_v4(base + ((n0 + 2 * c) >> 3) * 1024, mul_bf16x2(uw[c], rr), mul_bf16x2(uw[c + 1], rr), mul_bf16x2(uw[c + 2], rr),
+                         mul_bf16x2(uw[c + 3], rr));
         }
       } else if (live && sw == WPC - 1) {
-        float ov[CW];
+        uint32_t ow[CW / 2];
 #pragma unroll
-        for (int c = 0; c < CW; ++c) ov[c] = acc[c] + u[c];
-        store_row_global(p.o + ((tok + t) * p.H + h) * HEAD + v0g, ov);
+        for (int c = 0; c < CW; c += 2) ow[c >> 1] = pack_bf16(acc[c] + u[c], acc[c + 1] + u[c + 1]);
+        if (o_tile) {
+          store_packed(vrow, 16, ow);
+        } else {
+          __nv_bfloat16* dst = p.o + ((tok + t) * p.H + h) * HEAD + v0g;
+#pragma unroll
+          for (int c = 0; c < CW / 2; c += 4) *reinterpret_cast<uint4*>(dst + 2 * c) = make_uint4(ow[c], ow[c + 1], ow[c + 2], ow[c + 3]);
+        }
       }
     }
     fence_async_smem();
@@ -519,6 +496,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       umma_commit(&ctrl.bar_mma[chain]);
     }
     __syncwarp();
+    if (cwarp_u == REFILL_WARP && elect_one()) {
+      if (o_tile) tma_store_4d(&map_o, vbox, v0g, h, t0, b);
+      if (p.U != nullptr) {
+#pragma unroll
+        for (int cb = 0; cb < CW / 8; ++cb) tma_store_4d(&map_u, bw_img + cb * 1024, v0g + cb * 8, 0, static_cast<int>(item) * 64, 0);
+      }
+      bulk_commit_group();
+      bulk_wait_group_read_but<1>();                 // the saved state has been read: the image takes the next one
+    }
+    __syncwarp();
     if (cwarp_u == ISSUE_WARP) mbar_wait(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     chain_sync<CT>(chain);
     ++mma_phase;
@@ -527,7 +514,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       float dch[ET];                                 // exp(gL) of this thread's slices
       lds_part<ET>(gf + C::GF_D + e0, dch);
       const uint32_t base = smem_u32(s_img) + (row >> 3) * 128 + (row & 7) * 16;
-      uint8_t* hbase = (p.h != nullptr && i + 1 < count) ? state_item_ptr(item + p.H) : nullptr;
       float ds[2][16];
       tmem_ld<16>(tmem_row + col0, ds[0]);
 #pragma unroll
@@ -546,21 +532,22 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
         // operand image (i = d, j = n') for the next chunk's (1)
         st_shared_v4(base + ((col0 + j0) >> 3) * 2048, packed[0], packed[1], packed[2], packed[3]);
         st_shared_v4(base + ((col0 + j0 + 8) >> 3) * 2048, packed[4], packed[5], packed[6], packed[7]);
-        // saved state of the next chunk: slice e as [v/8][d][v%8]
-        if (hbase != nullptr) store_state_slices(hbase, j0, packed);
       }
     }
     fence_async_smem();
     tc_fence_before();
     chain_sync<CT>(chain);
   }
+  if (cwarp_u == REFILL_WARP && elect_one()) bulk_wait_group();   // the last stores read shared memory of this CTA
+  __syncwarp();
   // final state for the caller (f32, same form as the initial state)
   if (p.s_out != nullptr) {
     float* dst = p.s_out + ((static_cast<int64_t>(seq) * p.H + h) * E + e0) * (HEAD * HEAD) + row * HEAD + v0g;
 #pragma unroll
     for (int e = 0; e < ET; ++e)
 #pragma unroll
-      for (int c = 0; c < CW; ++c) dst[e * (HEAD * HEAD) + c] = S[e * CW + c];
+      for (int c = 0; c < CW; c += 4)
+        *reinterpret_cast<float4*>(dst + e * (HEAD * HEAD) + c) = make_float4(S[e * CW + c], S[e * CW + c + 1], S[e * CW + c + 2], S[e * CW + c + 3]);
   }
   tc_fence_before();
   __syncthreads();
@@ -573,24 +560,27 @@ using namespace tgdn;
 
 template <int E, int CW, int NCH, int WPC, int STAGES, int MINB>
 static int launch_fwd(const CUtensorMap& mk, const CUtensorMap& mq, const void* v, const FwdParams& p, cudaStream_t s) {
+  int rc;
   using C = FwdCfg<E, CW, NCH, WPC, STAGES>;
   static_assert(MINB == 1 || C::SMEM_BYTES <= 115712, "two CTAs per SM need at most 113 KB each");
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static_assert(MINB * C::TMEM_COLS <= 512, "tensor memory budget of one SM exceeded");
   static bool configured[64] = {};
-  if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(fwd_kernel<E, CW, NCH, WPC, STAGES, MINB>), C::SMEM_BYTES, configured))
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(fwd_kernel<E, CW, NCH, WPC, STAGES, MINB>), C::SMEM_BYTES, configured)))
     return rc;
-  CUtensorMap mv = mk, mb = mk;                     // placeholders where the rows are not loaded by TMA
-  if (C::TMA_V) {
-    const int rc = tgdn_make_token_map(&mv, v, p.B, p.T, p.H, CW, 64, 0, p.TS);
-    if (rc) return rc;
-  }
+  CUtensorMap mv, mo, mb = mk, mw = mk, mu = mk;    // placeholders where a tensor is not loaded or stored by TMA
+  if ((rc = tgdn_make_token_map(&mv, v, p.B, p.T, p.H, CW, 64, 0, p.TS))) return rc;
+  if ((rc = tgdn_make_token_map(&mo, p.o, p.B, p.T, p.H, CW, 64, 0, p.TS))) return rc;
   if (C::TMA_BETA && p.beta_tma) {
-    const int rc = tgdn_make_gate_map(&mb, p.beta, p.B, p.T, p.H / 4, 4, p.TS);    // (B, T, H) read as (B, T, H/4, 4)
-    if (rc) return rc;
+    if ((rc = tgdn_make_gate_map(&mb, p.beta, p.B, p.T, p.H / 4, 4, p.TS))) return rc;    // (B, T, H) read as (B, T, H/4, 4)
   }
+  // chunk-layout tensors are plain (rows, 128) matrices: one batch row, one head
+  const int64_t crows = static_cast<int64_t>(p.B) * p.NC * p.H * 64;
+  if ((p.W != nullptr || p.U != nullptr) && crows > 0x7fffffffLL) return TGDN_ERR_SHAPE;
+  if (p.W != nullptr && (rc = tgdn_make_token_map(&mw, p.W, 1, static_cast<int>(crows), 1, CW, 64, 0))) return rc;
+  if (p.U != nullptr && (rc = tgdn_make_token_map(&mu, p.U, 1, static_cast<int>(crows), 1, 8, 64, 0))) return rc;
   const int grid = p.n_seq * p.H * (HEAD / C::VC);
-  fwd_kernel<E, CW, NCH, WPC, STAGES, MINB><<<grid, C::THREADS, C::SMEM_BYTES, s>>>(mv, mb, mk, mq, p);
+  fwd_kernel<E, CW, NCH, WPC, STAGES, MINB><<<grid, C::THREADS, C::SMEM_BYTES, s>>>(mv, mb, mk, mq, mo, mw, mu, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 
@@ -618,18 +608,23 @@ int tgdn_fwd_rows(const void* q, const void* k, const void* v, const float* k2, 
               packed ? n_docs : B, row_tokens, scale, tgdn_status_word(),
               (H % 4 == 0 && (reinterpret_cast<uintptr_t>(beta) & 15) == 0) ? 1 : 0};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // Width of the value block, up to four slices.  One CTA per SM: the grid runs in whole waves.  A CTA of 64 columns (four chains
+  // of 16, twice the columns per MMA for the same operand reads of [K;Q]) takes longer per chunk than the narrow one (32), but by
+  // less than twice: measured 1.40 (E = 1), 1.19 (E = 2) and 1.25 (E = 4) times.  So the wide one wins when it saves waves by
+  // more than that (always, once the grid is a few waves); a grid that fills one wave either way keeps the narrow one.
+  // B=4, T=4096, H=16 (two waves or one), forward with the saved tensors: E = 1 264 -> 188 us, E = 2 310 -> 205 us.
+  const long long sms = tgdn_sm_count(), seqs = static_cast<long long>(p.n_seq) * p.H;
+  const long long narrow = (seqs * 4 + sms - 1) / sms, wide = (seqs * 2 + sms - 1) / sms;
   switch (E) {
-    case 1: return launch_fwd<1, 16, 2, 1, 2, 1>(mk, mq, v, p, s);
-    case 2: return launch_fwd<2, 8, 4, 1, 2, 1>(mk, mq, v, p, s);
-    case 4: {
-      // One CTA per SM: the grid runs in whole waves.  Where a block of 32 value columns needs a second, partly filled wave
-      // and a block of 64 does not, the wider block wins although its chunks take a little longer (B=4, H=16: 256 CTAs on
-      // 148 SMs are two waves, 128 CTAs are one).
-      const long long sms = tgdn_sm_count(), seqs = static_cast<long long>(p.n_seq) * p.H;
-      const long long waves32 = (seqs * 4 + sms - 1) / sms, waves64 = (seqs * 2 + sms - 1) / sms;
-      if (waves64 * 5 < waves32 * 4) return launch_fwd<4, 16, 4, 1, 2, 1>(mk, mq, v, p, s);
+    case 1:      // (its narrow block is two chains of 16 columns)
+      if (wide * 7 < narrow * 5) return launch_fwd<1, 16, 4, 1, 2, 1>(mk, mq, v, p, s);
+      return launch_fwd<1, 16, 2, 1, 2, 1>(mk, mq, v, p, s);
+    case 2:
+      if (wide * 6 < narrow * 5) return launch_fwd<2, 16, 4, 1, 2, 1>(mk, mq, v, p, s);
+      return launch_fwd<2, 8, 4, 1, 2, 1>(mk, mq, v, p, s);
+    case 4:
+      if (wide * 5 < narrow * 4) return launch_fwd<4, 16, 4, 1, 2, 1>(mk, mq, v, p, s);
       return launch_fwd<4, 8, 4, 1, 2, 1>(mk, mq, v, p, s);
-    }
     // (two warpgroups per chain at E = 8, sixteen columns per thread, measured 17% slower than four one-warpgroup chains)
     case 8: return launch_fwd<8, 8, 4, 1, 2, 1>(mk, mq, v, p, s);
     case 12: return launch_fwd<12, 8, 2, 2, 2, 1>(mk, mq, v, p, s);

@@ -1,0 +1,33 @@
+"""Both sides of the size rules by which the library picks a kernel variant, at the sizes where they can go wrong."""
+import pytest
+import torch
+
+from cute_triadic_gdn_b200 import _lib, chunk_gdn_joint, gdn_joint_call
+from oracle import triadic_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("E", [1, 2, 4])
+@pytest.mark.parametrize("docs", [None, [0, 1, 64, 129, 200, 263, 384]])
+def test_wide_value_blocks_of_the_forward(E, docs):
+    """Enough sequences for more than one wave of narrow value blocks: the 64-column variant runs, dense and with chunks cut
+    short by document ends, with the state handed in and out."""
+    B, T, H = (1, 384, 16) if docs else (6, 128, 16)
+    ins = [t.cuda() for t in orc.make_inputs(B, T, H, E, seed=70 + E, dist="mild")]
+    do = orc.make_grad_output((B, T, H, 128), 5)
+    cu = torch.tensor(docs, dtype=torch.int32) if docs else None
+    leaves = [t.clone().requires_grad_(True) for t in ins]
+    o = gdn_joint_call(*leaves, cu_seqlens=None if cu is None else cu.cuda())
+    o.backward(do.cuda())
+    o_ref, g_ref = orc.reference_with_grads(orc.chunk_reference, [t.cpu() for t in ins], do, cu_seqlens=cu, dtype=torch.float32)
+    assert _lib.device_status() == 0
+    assert orc.rel_l2(o.detach().float().cpu(), o_ref) < 1e-2
+    for name, leaf, ref in zip("q k v k2 q2 g beta".split(), leaves, g_ref):
+        assert orc.rel_l2(leaf.grad.float().cpu(), ref) < 2e-2, name
+    if docs is None:                                   # the two halves of the row, chained by the state, are the whole row
+        with torch.no_grad():
+            _, s_all = chunk_gdn_joint(*ins, output_final_state=True)
+            o1, s1 = chunk_gdn_joint(*[t[:, :64].contiguous() for t in ins], output_final_state=True)
+            o2, s2 = chunk_gdn_joint(*[t[:, 64:].contiguous() for t in ins], initial_state=s1, output_final_state=True)
+        assert torch.equal(torch.cat([o1, o2], 1), o.detach()) and torch.equal(s2, s_all)
