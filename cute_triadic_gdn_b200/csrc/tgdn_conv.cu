@@ -1,15 +1,17 @@
-// Width-4 causal depthwise convolution with SiLU on the leading channels: forward and backward.
+// Width-4 causal depthwise convolution with SiLU on the leading channels, forward and backward, and the same with the layer glue
+// that follows it fused in (conv -> SiLU / softplus -> l2 norms -> q, k, v, k2, q2).
 //
-// Replaces the reference's Triton kernels cute_triadic_gdn/ops/conv_split_act.py:20-55 (_fwd_kernel) and :58-107
-// (_bwd_kernel).  HBM-bound, so the kernels are built around bytes in flight: a CTA owns a tile of 256 channels and
-// walks a run of 32-token tiles; the [tokens + halo][256 channels] input tiles arrive by TMA (cp.async.bulk.tensor, no
-// swizzle) into a multi-stage shared-memory ring, several tiles ahead of the arithmetic, and rows before the start of a
-// batch row come back as zeros from the tensor map's out-of-range fill.  Each warp computes 8 of the 32 output rows
-// for the tile's 256 channels (8 channels = one 16-byte vector per lane) and stores them with coalesced 512-byte rows.
-// The backward recomputes the bf16-rounded pre-activation from the same x window (the reference launches a second
-// forward for it), so x and dy are read once and dx written once; the weight gradient is accumulated in registers
-// over all tiles of the CTA, reduced across its warps in shared memory and written as one f32 partial per CTA; a
-// second small kernel sums the partials in a fixed order.
+// Replaces the reference's Triton kernels cute_triadic_gdn/ops/conv_split_act.py:20-55 (_fwd_kernel) and :58-107 (_bwd_kernel).
+//
+// A warp walks a run of tokens of its channels with the three rows of the window (and, backward, the last three gradients and the
+// weight gradient) in registers: each row is read once and nothing is computed twice but the three rows behind the end of a
+// run.  Its rows arrive by TMA in a ring of its own (RING kernels: 128 channels per warp; what the tensor maps can describe) or
+// by loads asked for a batch ahead (WALKERS: everything else).  The version before staged 32-token tiles per CTA, eight rows per
+// warp: eleven rows computed for eight in the backward, a CTA barrier per tile, and padded copies of every tensor where the
+// channel count was not a multiple of eight.  Measured at (1, 32768, 13056), of the HBM copy rate: backward 558 -> 424 us (70 ->
+// 92%), forward 302 -> 300 us (87%; two transcendental operations per element are the co-limit); at (3, 1000, 1930), padded
+// copies included, forward and backward 130 -> 32 us.
+// The weight gradient is accumulated in f32 per run and the runs' partials are summed in a fixed order by a second small kernel.
 #include <algorithm>
 #include <mutex>
 
@@ -20,254 +22,97 @@
 namespace tgdn {
 
 constexpr int CONV_W = 4;
-constexpr int CONV_THREADS = 256;      // 8 warps = 4 row groups x 2 channel halves
-constexpr int CONV_CH = 256;           // channels per CTA tile (2 halves x 32 lanes x 4)
-constexpr int CONV_VEC = 4;            // channels per thread (one 8-byte vector)
-constexpr int CONV_TOK = 32;           // output tokens per tile (4 row groups x 8 rows)
-constexpr int CONV_FWD_ROWS = CONV_TOK + 3;       // x rows t0-3 .. t0+31
-constexpr int CONV_BWD_XROWS = CONV_TOK + 6;      // x rows t0-3 .. t0+34
-constexpr int CONV_BWD_GROWS = CONV_TOK + 3;      // dy rows t0 .. t0+34
-constexpr int CONV_FWD_STAGES = 3;     // 54 KB per CTA: four CTAs per SM
-constexpr int CONV_BWD_STAGES = 3;     // 112 KB per CTA: two CTAs per SM
-constexpr int CONV_BWD_NP = 2;         // channel pairs per thread of the backward (512 threads per CTA)
+constexpr int CONV_TOK = 32;           // granularity of the token groups that size the scratch of the public ABI
 
-// Four channels of a thread as two packed pairs: the arithmetic runs on the two-wide f32 instructions (one instruction per
-// pair, each lane an ordinary IEEE fma), which halves the instruction count of the kernels' inner loops.
-struct Vec4 {
-  float2 p[2];                  // channels (0,1) and (2,3)
+// ---- V channels of one row: raw bf16 words and f32 pairs -----------------------------------------------------------------
+// The arithmetic runs on the two-wide f32 instructions (one instruction per pair, each lane an ordinary IEEE fma).
+template <int V> struct RawRow;
+template <> struct RawRow<4> { uint2 w; };
+template <> struct RawRow<2> { uint32_t w; };
+template <> struct RawRow<1> { unsigned short w; };
+template <int V> struct Pairs { float2 p[(V + 1) / 2]; };
+
+template <int V>
+__device__ __forceinline__ RawRow<V> load_raw(const __nv_bfloat16* p) {      // streamed: not kept in L1
+  RawRow<V> r;
+  if constexpr (V == 4)
+    asm volatile("ld.global.nc.L1::no_allocate.v2.b32 {%0,%1}, [%2];" : "=r"(r.w.x), "=r"(r.w.y) : "l"(p));
+  else if constexpr (V == 2)
+    asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(r.w) : "l"(p));
+  else
+    asm volatile("ld.global.nc.L1::no_allocate.b16 %0, [%1];" : "=h"(r.w) : "l"(p));
+  return r;
+}
+template <int V>
+__device__ __forceinline__ RawRow<V> zero_raw() {
+  RawRow<V> r;
+  if constexpr (V == 4) r.w = make_uint2(0u, 0u); else r.w = 0;
+  return r;
+}
+template <int V>
+__device__ __forceinline__ Pairs<V> unpack(const RawRow<V>& r) {
+  Pairs<V> o;
+  if constexpr (V == 4) {
+    o.p[0] = make_float2(bf16_lo(r.w.x), bf16_hi(r.w.x));
+    o.p[1] = make_float2(bf16_lo(r.w.y), bf16_hi(r.w.y));
+  } else if constexpr (V == 2) {
+    o.p[0] = make_float2(bf16_lo(r.w), bf16_hi(r.w));
+  } else {
+    o.p[0] = make_float2(bf16_lo(r.w), 0.f);
+  }
+  return o;
+}
+template <int V>
+__device__ __forceinline__ Pairs<V> zero_pairs() {
+  Pairs<V> o;
+#pragma unroll
+  for (int i = 0; i < (V + 1) / 2; ++i) o.p[i] = make_float2(0.f, 0.f);
+  return o;
+}
+template <int V>
+__device__ __forceinline__ void store_row(__nv_bfloat16* p, const Pairs<V>& a) {
+  if constexpr (V == 4)
+    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(a.p[0].x, a.p[0].y), pack_bf16(a.p[1].x, a.p[1].y));
+  else if constexpr (V == 2)
+    *reinterpret_cast<uint32_t*>(p) = pack_bf16(a.p[0].x, a.p[0].y);
+  else
+    *p = __float2bfloat16_rn(a.p[0].x);
+}
+
+// The four taps of V channels as pairs, and the products with the window.
+template <int V> struct Taps { float2 w[(V + 1) / 2][CONV_W]; };
+template <int V>
+__device__ __forceinline__ Taps<V> load_taps(const __nv_bfloat16* weight, int c0, bool live) {
+  float f[V][CONV_W];
+#pragma unroll
+  for (int c = 0; c < V; ++c) {
+    const uint2 u = live ? __ldg(reinterpret_cast<const uint2*>(weight + static_cast<int64_t>(c0 + c) * CONV_W)) : make_uint2(0u, 0u);
+    f[c][0] = bf16_lo(u.x); f[c][1] = bf16_hi(u.x); f[c][2] = bf16_lo(u.y); f[c][3] = bf16_hi(u.y);
+  }
+  Taps<V> t;
+#pragma unroll
+  for (int i = 0; i < (V + 1) / 2; ++i)
+#pragma unroll
+    for (int j = 0; j < CONV_W; ++j) t.w[i][j] = make_float2(f[2 * i][j], 2 * i + 1 < V ? f[2 * i + (V > 1 ? 1 : 0)][j] : 0.f);
+  return t;
+}
+// The window of a walk: x[t-1], x[t-2], x[t-3].
+template <int V> struct Window {
+  Pairs<V> m[3];
+  __device__ __forceinline__ void push(const Pairs<V>& x0) { m[2] = m[1]; m[1] = m[0]; m[0] = x0; }
+  __device__ __forceinline__ float2 conv(const Taps<V>& t, const Pairs<V>& x0, int i) const {
+    float2 acc = __fmul2_rn(m[2].p[i], t.w[i][0]);
+    acc = __ffma2_rn(m[1].p[i], t.w[i][1], acc);
+    acc = __ffma2_rn(m[0].p[i], t.w[i][2], acc);
+    return __ffma2_rn(x0.p[i], t.w[i][3], acc);
+  }
 };
 
-__device__ __forceinline__ Vec4 unpack4(uint2 u) {
-  Vec4 r;
-  r.p[0] = make_float2(bf16_lo(u.x), bf16_hi(u.x));
-  r.p[1] = make_float2(bf16_lo(u.y), bf16_hi(u.y));
-  return r;
-}
-__device__ __forceinline__ Vec4 zero4() {
-  Vec4 r;
-  r.p[0] = r.p[1] = make_float2(0.f, 0.f);
-  return r;
-}
-__device__ __forceinline__ void store4(__nv_bfloat16* p, const Vec4& a) {
-  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(a.p[0].x, a.p[0].y), pack_bf16(a.p[1].x, a.p[1].y));
-}
 // sigmoid with the fast exponential and the fast reciprocal: relative error of a few f32 ulps
 __device__ __forceinline__ float fast_sigmoid(float y) { return __fdividef(1.f, 1.f + __expf(-y)); }
 __device__ __forceinline__ float silu(float y) { return y * fast_sigmoid(y); }
-// Derivative of SiLU for the backward, where the result is rounded to bf16 after further products: the sigmoid comes
-// from one tanh.approx (absolute error about 2^-11) instead of an exponential and a reciprocal.
-__device__ __forceinline__ float silu_grad(float y) {
-  float th;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(0.5f * y));
-  const float s = fmaf(0.5f, th, 0.5f);
-  return s * fmaf(y, 1.f - s, 1.f);
-}
-
-// Walks document boundaries as the token index grows: one binary search per tile, then a compare per token.
-struct DocCursor {
-  const int32_t* cu;
-  int n_docs, d, start, next;
-  __device__ __forceinline__ void init(const int32_t* cu_, int n_docs_, int t, int T) {
-    cu = cu_; n_docs = n_docs_; d = 0; start = 0; next = 0x7fffffff;
-    if (cu == nullptr) return;
-    int lo = 0, hi = n_docs - 1;
-    while (lo < hi) {
-      int mid = (lo + hi + 1) >> 1;
-      if (__ldg(cu + mid) <= t) lo = mid; else hi = mid - 1;
-    }
-    d = lo;
-    start = __ldg(cu + d);
-    next = (d + 1 < n_docs) ? __ldg(cu + d + 1) : 0x7fffffff;
-  }
-  // true when token t is the first token of a document that starts after the one the cursor was on
-  __device__ __forceinline__ bool advance(int t) {
-    if (t < next) return false;
-    do {
-      ++d; start = next;
-      next = (d + 1 < n_docs) ? __ldg(cu + d + 1) : 0x7fffffff;
-    } while (t >= next);
-    return true;
-  }
-};
-
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-
-struct ConvArgs {
-  const __nv_bfloat16* weight;
-  __nv_bfloat16* out;            // y (forward) or dx (backward), contiguous (B, T, C)
-  float* dw_partial;             // backward: [B * groups][C][4]
-  const int32_t* cu;
-  int n_docs, T, C, act_channels, tiles_per_group;
-  int* status;
-};
-
-// w2[p][j]: tap j of the channel pair p (channels c0 + 2p, c0 + 2p + 1)
-__device__ __forceinline__ void load_weights(const __nv_bfloat16* weight, int c0, int C, float2 (*w2)[CONV_W]) {
-  float w[CONV_VEC][CONV_W];
-#pragma unroll
-  for (int c = 0; c < CONV_VEC; ++c)
-#pragma unroll
-    for (int j = 0; j < CONV_W; ++j) w[c][j] = 0.f;
-  if (c0 < C) {                                 // C % 8 == 0 and c0 % 4 == 0: the four channels are all inside
-    const uint4* wp = reinterpret_cast<const uint4*>(weight + static_cast<int64_t>(c0) * CONV_W);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {               // 4 channels x 4 taps = 16 bf16 = 2 vectors
-      uint4 u = __ldg(wp + i);
-      const uint32_t ws[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        int e = i * 8 + j * 2;
-        w[e / 4][e % 4] = bf16_lo(ws[j]);
-        w[(e + 1) / 4][(e + 1) % 4] = bf16_hi(ws[j]);
-      }
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int j = 0; j < CONV_W; ++j) w2[p][j] = make_float2(w[2 * p][j], w[2 * p + 1][j]);
-}
-
-__global__ void __launch_bounds__(CONV_THREADS, 4)
-conv_fwd_kernel(const __grid_constant__ CUtensorMap map_x, ConvArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  constexpr int STAGE_BYTES = CONV_FWD_ROWS * CONV_CH * 2;
-  __shared__ uint64_t full[CONV_FWD_STAGES];
-  __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int half = warp & 1, rg = warp >> 1;
-  const int cbase = blockIdx.x * CONV_CH, c0 = cbase + half * 128 + lane * CONV_VEC, b = blockIdx.z;
-  const int n_tiles = (a.T + CONV_TOK - 1) / CONV_TOK;
-  const int tile_lo = blockIdx.y * a.tiles_per_group, tile_hi = min(n_tiles, tile_lo + a.tiles_per_group);
-  if (tile_lo >= tile_hi) return;
-  if (tid == 0) {
-    for (int s = 0; s < CONV_FWD_STAGES; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-    abort_s = 0;
-  }
-  __syncthreads();
-  WaitCtl ctl{&abort_s, a.status};
-  auto issue = [&](int tile) {                         // thread 0
-    const int s = (tile - tile_lo) % CONV_FWD_STAGES;
-    mbar_expect_tx(&full[s], STAGE_BYTES);
-    tma_load_3d(smem + s * STAGE_BYTES, &map_x, &full[s], cbase, tile * CONV_TOK - 3, b);
-  };
-  if (tid == 0)
-    for (int i = 0; i < CONV_FWD_STAGES && tile_lo + i < tile_hi; ++i) issue(tile_lo + i);
-
-  float2 w2[2][CONV_W];
-  load_weights(a.weight, c0, a.C, w2);
-  __nv_bfloat16* yb = a.out + (static_cast<int64_t>(b) * a.T) * a.C + c0;
-  const int col_off = half * 256 + lane * 8;             // byte offset of this thread's channels inside a tile row
-  const bool live = c0 < a.C;
-  bool act[CONV_VEC];
-#pragma unroll
-  for (int c = 0; c < CONV_VEC; ++c) act[c] = c0 + c < a.act_channels;
-
-  for (int tile = tile_lo; tile < tile_hi; ++tile) {
-    const int k = tile - tile_lo, s = k % CONV_FWD_STAGES;
-    mbar_wait(&full[s], (k / CONV_FWD_STAGES) & 1, ctl, DEV_TIMEOUT_LOAD);
-    const uint8_t* st = smem + s * STAGE_BYTES + col_off;
-    const int t_first = tile * CONV_TOK + rg * 8;         // this warp's first output token; its smem row is rg*8 + 3
-    DocCursor doc;
-    doc.init(a.cu, a.n_docs, min(t_first, a.T - 1), a.T);
-    __nv_bfloat16* yrow = yb + static_cast<int64_t>(t_first) * a.C;
-    // Interior of a document and of the sequence: no start of a document among the warp's eight rows or their three halo
-    // rows (rows before the sequence come back as zeros from the tensor map, which is what a start at token 0 means),
-    // all eight rows exist.  Then the rows need no cursor, no bounds and no window resets; almost every tile is like this.
-    const bool interior = t_first + 8 <= a.T && doc.next >= t_first + 8 && doc.start <= max(t_first - 3, 0);
-    if (interior && live && (act[0] == act[3])) {
-      const bool on = act[0];
-      Vec4 xm[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) xm[j] = unpack4(*reinterpret_cast<const uint2*>(st + (rg * 8 + 2 - j) * (CONV_CH * 2)));
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const Vec4 x0 = unpack4(*reinterpret_cast<const uint2*>(st + (rg * 8 + 3 + i) * (CONV_CH * 2)));
-        Vec4 out;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          float2 acc = __fmul2_rn(xm[2].p[p], w2[p][0]);
-          acc = __ffma2_rn(xm[1].p[p], w2[p][1], acc);
-          acc = __ffma2_rn(xm[0].p[p], w2[p][2], acc);
-          acc = __ffma2_rn(x0.p[p], w2[p][3], acc);
-          out.p[p] = on ? make_float2(silu(acc.x), silu(acc.y)) : acc;
-        }
-        store4(yrow + static_cast<int64_t>(i) * a.C, out);
-        xm[2] = xm[1]; xm[1] = xm[0]; xm[0] = x0;
-      }
-    } else {
-      Vec4 xm[3];                                           // x[t-1], x[t-2], x[t-3]
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int tj = t_first - 1 - j;
-        xm[j] = (tj >= doc.start) ? unpack4(*reinterpret_cast<const uint2*>(st + (rg * 8 + 2 - j) * (CONV_CH * 2))) : zero4();
-      }
-      const int n_rows = min(8, a.T - t_first);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (i >= n_rows) break;
-        if (i > 0 && doc.advance(t_first + i)) { xm[0] = zero4(); xm[1] = zero4(); xm[2] = zero4(); }   // a document starts here
-        const Vec4 x0 = unpack4(*reinterpret_cast<const uint2*>(st + (rg * 8 + 3 + i) * (CONV_CH * 2)));
-        Vec4 out;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          float2 acc = __fmul2_rn(xm[2].p[p], w2[p][0]);
-          acc = __ffma2_rn(xm[1].p[p], w2[p][1], acc);
-          acc = __ffma2_rn(xm[0].p[p], w2[p][2], acc);
-          acc = __ffma2_rn(x0.p[p], w2[p][3], acc);
-          out.p[p] = make_float2(act[2 * p] ? silu(acc.x) : acc.x, act[2 * p + 1] ? silu(acc.y) : acc.y);
-        }
-        if (live) store4(yrow, out);
-        yrow += a.C;
-        xm[2] = xm[1]; xm[1] = xm[0]; xm[0] = x0;
-      }
-    }
-    __syncthreads();                                      // every warp is done with this stage
-    if (tid == 0 && tile + CONV_FWD_STAGES < tile_hi) issue(tile + CONV_FWD_STAGES);
-  }
-}
-
-// NP channel pairs of a thread (the forward's Vec4 is the NP = 2 case with its own helpers).
-template <int NP>
-struct VecP {
-  float2 p[NP];
-};
-template <int NP>
-__device__ __forceinline__ VecP<NP> load_pairs(const uint8_t* s) {
-  VecP<NP> r;
-  if constexpr (NP == 2) {
-    const uint2 u = *reinterpret_cast<const uint2*>(s);
-    r.p[0] = make_float2(bf16_lo(u.x), bf16_hi(u.x));
-    r.p[1] = make_float2(bf16_lo(u.y), bf16_hi(u.y));
-  } else {
-    const uint32_t u = *reinterpret_cast<const uint32_t*>(s);
-    r.p[0] = make_float2(bf16_lo(u), bf16_hi(u));
-  }
-  return r;
-}
-template <int NP>
-__device__ __forceinline__ VecP<NP> zero_pairs() {
-  VecP<NP> r;
-#pragma unroll
-  for (int p = 0; p < NP; ++p) r.p[p] = make_float2(0.f, 0.f);
-  return r;
-}
-template <int NP>
-__device__ __forceinline__ void store_pairs(__nv_bfloat16* dst, const VecP<NP>& a) {
-  if constexpr (NP == 2)
-    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(a.p[0].x, a.p[0].y), pack_bf16(a.p[1].x, a.p[1].y));
-  else
-    *reinterpret_cast<uint32_t*>(dst) = pack_bf16(a.p[0].x, a.p[0].y);
-}
-// SiLU' of the bf16-rounded pre-activations of a channel pair: one packed conversion rounds both, the polynomial part runs
-// on the two-wide f32 instructions (each lane the same bits as silu_grad).
+// SiLU' of the bf16-rounded pre-activations of a pair, for the backward, where the result is rounded to bf16 after further
+// products: the sigmoid comes from one tanh.approx (absolute error about 2^-11) instead of an exponential and a reciprocal.
 __device__ __forceinline__ float2 silu_grad_pair(float2 pre) {
   const uint32_t r = pack_bf16(pre.x, pre.y);
   const float2 y = make_float2(bf16_lo(r), bf16_hi(r));
@@ -281,217 +126,759 @@ __device__ __forceinline__ float2 silu_grad_pair(float2 pre) {
   return __fmul2_rn(s, __ffma2_rn(y, om, one2));
 }
 
-// Backward.  NP = 1: 512 threads = 4 row groups x 4 channel slices of 64, one channel pair per thread, so that the kernel
-// fits 64 registers and two CTAs put 32 warps on an SM: the per-row chain (4 fma, rounding, tanh, 4 more fma) is all
-// fixed-latency dependency, which only more warps per scheduler hide.
-template <int NP>
-__global__ void __launch_bounds__(CONV_THREADS * 2 / NP, 2)
-conv_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_dy, ConvArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  constexpr int X_BYTES = CONV_BWD_XROWS * CONV_CH * 2, G_BYTES = CONV_BWD_GROWS * CONV_CH * 2;
-  constexpr int STAGE_BYTES = X_BYTES + G_BYTES;
-  constexpr int SLICES = 4 / NP, NCH = 2 * NP;                         // channel slices per tile, channels per thread
-  constexpr int ROW = CONV_CH * 2;                                     // bytes of a tile row
-  __shared__ uint64_t full[CONV_BWD_STAGES];
-  __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int slice = warp % SLICES, rg = warp / SLICES;
-  const int cin = slice * (32 * NCH) + lane * NCH;                     // first channel of the thread inside the tile
-  const int cbase = blockIdx.x * CONV_CH, c0 = cbase + cin, b = blockIdx.z;
-  const int n_tiles = (a.T + CONV_TOK - 1) / CONV_TOK;
-  const int tile_lo = blockIdx.y * a.tiles_per_group, tile_hi = min(n_tiles, tile_lo + a.tiles_per_group);
-  if (tid == 0) {
-    for (int s = 0; s < CONV_BWD_STAGES; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-    abort_s = 0;
+// The document of a token, and the next one's first token.
+struct DocCursor {
+  const int32_t* cu;
+  int n_docs, d, start, next;
+  __device__ __forceinline__ void init(const int32_t* cu_, int n_docs_, int t) {
+    cu = cu_; n_docs = n_docs_; d = 0; start = 0; next = 0x7fffffff;
+    if (cu == nullptr) return;
+    int lo = 0, hi = n_docs - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(cu + mid) <= t) lo = mid; else hi = mid - 1;
+    }
+    d = lo;
+    start = __ldg(cu + d);
+    set_next();
   }
-  __syncthreads();
-  WaitCtl ctl{&abort_s, a.status};
-  auto issue = [&](int tile) {                         // thread 0
-    const int s = (tile - tile_lo) % CONV_BWD_STAGES;
-    mbar_expect_tx(&full[s], STAGE_BYTES);
-    tma_load_3d(smem + s * STAGE_BYTES, &map_x, &full[s], cbase, tile * CONV_TOK - 3, b);
-    tma_load_3d(smem + s * STAGE_BYTES + X_BYTES, &map_dy, &full[s], cbase, tile * CONV_TOK, b);
-  };
-  if (tid == 0)
-    for (int i = 0; i < CONV_BWD_STAGES && tile_lo + i < tile_hi; ++i) issue(tile_lo + i);
+  __device__ __forceinline__ void set_next() { next = (d + 1 < n_docs) ? __ldg(cu + d + 1) : 0x7fffffff; }
+  __device__ __forceinline__ void advance(int t) {       // to the document of token t, which is not before the current one
+    while (t >= next) { ++d; start = next; set_next(); }
+  }
+};
 
-  const bool live = c0 < a.C;                          // C % 8 == 0 and c0 % NCH == 0: the thread's channels are all inside
-  float2 w2[NP][CONV_W];
-  {
-    float w[NCH][CONV_W];
+template <int V>
+__device__ __forceinline__ void open_window(Window<V>& win, const __nv_bfloat16* col, int64_t stride, int t, int doc_start, bool live) {
 #pragma unroll
-    for (int c = 0; c < NCH; ++c)
-#pragma unroll
-      for (int j = 0; j < CONV_W; ++j) w[c][j] = 0.f;
-    if (live) {
-      const uint4* wp = reinterpret_cast<const uint4*>(a.weight + static_cast<int64_t>(c0) * CONV_W);
-#pragma unroll
-      for (int i = 0; i < NP; ++i) {                   // two channels x four taps per 16-byte vector
-        const uint4 u = __ldg(wp + i);
-        w[2 * i][0] = bf16_lo(u.x); w[2 * i][1] = bf16_hi(u.x); w[2 * i][2] = bf16_lo(u.y); w[2 * i][3] = bf16_hi(u.y);
-        w[2 * i + 1][0] = bf16_lo(u.z); w[2 * i + 1][1] = bf16_hi(u.z);
-        w[2 * i + 1][2] = bf16_lo(u.w); w[2 * i + 1][3] = bf16_hi(u.w);
+  for (int j = 0; j < 3; ++j) win.m[j] = (live && t - 1 - j >= doc_start) ? unpack<V>(load_raw<V>(col + (t - 1 - j) * stride)) : zero_pairs<V>();
+}
+
+// Which channels of the warp pass through SiLU: 0 none, 1 all, 2 some.
+__device__ __forceinline__ int act_kind(int c0, int channels, bool live, int act_channels) {
+  if (__all_sync(0xffffffffu, !live || c0 + channels <= act_channels)) return 1;
+  if (__all_sync(0xffffffffu, !live || c0 >= act_channels)) return 0;
+  return 2;
+}
+
+// ---- per-warp TMA ring ---------------------------------------------------------------------------------------------------
+// A warp that walks 128 channels (V = 4) of a run of tokens has its rows arrive by TMA, eight at a time, in a ring of its own:
+// nothing couples the warps of a CTA, rows are read from shared memory at constant offsets (no address arithmetic per row),
+// and three to six tiles per warp are in flight.  Rows past the end of a batch row arrive as zeros (the tensor map's fill).
+constexpr int RING_ROWS = 8;
+constexpr int RING_TILE = RING_ROWS * 256;       // bytes: 8 rows x 128 channels
+constexpr int RING_WARPS = 4;                    // warps per CTA
+constexpr int RING_FWD_STAGES = 6, RING_BWD_STAGES = 3;      // 12 KB per warp either way
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
+// TENSORS tiles per stage: x, and in the backward the gradient rows.
+template <int TENSORS, int STAGES>
+struct Ring {
+  static constexpr int STAGE_BYTES = TENSORS * RING_TILE;
+  static constexpr int WARP_BYTES = STAGES * STAGE_BYTES;
+  uint8_t* buf;                                  // this warp's stages
+  uint64_t* full;                                // and their barriers
+  int k;                                         // tiles taken so far
+  __device__ __forceinline__ void init(uint8_t* smem, uint64_t* bars) {
+    const int warp = threadIdx.x >> 5;
+    buf = smem + warp * WARP_BYTES;
+    full = bars + warp * STAGES;
+    k = 0;
+    if ((threadIdx.x & 31) == 0) {
+      for (int s = 0; s < STAGES; ++s) mbar_init(&full[s], 1);
+      mbar_fence_init();
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ uint8_t* stage(int tile) const { return buf + tile % STAGES * STAGE_BYTES; }
+  // issue(tile, stage, barrier): one lane sends off the loads of a tile
+  template <typename F>
+  __device__ __forceinline__ void open(int tiles, F issue) {
+    if (elect_one()) {
+      for (int i = 0; i < STAGES && i < tiles; ++i) {
+        mbar_expect_tx(&full[i], STAGE_BYTES);
+        issue(i, stage(i), &full[i]);
       }
     }
-#pragma unroll
-    for (int p = 0; p < NP; ++p)
-#pragma unroll
-      for (int j = 0; j < CONV_W; ++j) w2[p][j] = make_float2(w[2 * p][j], w[2 * p + 1][j]);
+    __syncwarp();
   }
-  float2 dwa[NP][CONV_W];                                              // weight gradient of the channel pairs
-#pragma unroll
-  for (int p = 0; p < NP; ++p)
-#pragma unroll
-    for (int j = 0; j < CONV_W; ++j) dwa[p][j] = make_float2(0.f, 0.f);
-  __nv_bfloat16* dxb = a.out + (static_cast<int64_t>(b) * a.T) * a.C + c0;
-  const int col_off = cin * 2;
-  bool act[NCH];
-#pragma unroll
-  for (int c = 0; c < NCH; ++c) act[c] = c0 + c < a.act_channels;
-  using V = VecP<NP>;
+  __device__ __forceinline__ const uint8_t* wait(const WaitCtl& ctl) const {
+    mbar_wait(&full[k % STAGES], (k / STAGES) & 1, ctl, DEV_TIMEOUT_LOAD);
+    return stage(k) + (threadIdx.x & 31) * 8;    // this lane's four channels of row 0
+  }
+  template <typename F>
+  __device__ __forceinline__ void release(int tiles, F issue) {       // every lane has read the tile
+    __syncwarp();
+    if (k + STAGES < tiles && elect_one()) {
+      mbar_expect_tx(&full[k % STAGES], STAGE_BYTES);
+      issue(k + STAGES, stage(k), &full[k % STAGES]);
+    }
+    __syncwarp();
+    ++k;
+  }
+};
+__device__ __forceinline__ RawRow<4> ring_row(const uint8_t* tile, int i) {
+  RawRow<4> r;
+  r.w = *reinterpret_cast<const uint2*>(tile + i * 256);
+  return r;
+}
 
-  for (int tile = tile_lo; tile < tile_hi; ++tile) {
-    const int k = tile - tile_lo, s = k % CONV_BWD_STAGES;
-    mbar_wait(&full[s], (k / CONV_BWD_STAGES) & 1, ctl, DEV_TIMEOUT_LOAD);
-    const uint8_t* sx = smem + s * STAGE_BYTES + col_off;              // row r holds x[t0 - 3 + r]
-    const uint8_t* sg = sx + X_BYTES;                                  // row r holds dy[t0 + r]
-    const int t0 = tile * CONV_TOK, u_first = t0 + rg * 8;             // this warp's output tokens u_first .. +7
-    // dx[u] = sum_j dy'[u+j] w[3-j] over tokens of the same document; dy'[t] needs x[t-3..t].  Walk t = u_first .. u_first+10
-    // (three tokens past the warp's rows) with the x window and the last three dy' in registers.
-    DocCursor doc;
-    doc.init(a.cu, a.n_docs, min(u_first, a.T - 1), a.T);
-    // Interior of a document and of the sequence: no start of a document among the eleven tokens the warp walks or their
-    // three halo rows, and all of them exist.  Then no cursor, no bounds and no masks are needed; almost every tile is
-    // like this.
-    const bool interior = u_first + 11 <= a.T && doc.next >= u_first + 11 && doc.start <= max(u_first - 3, 0);
-    if (interior && live && (act[0] == act[NCH - 1])) {
-      const bool on = act[0];
-      V xw[3];
+// Sums of N = 4 or 8 values over the lanes of a warp, every lane gets all of them: halving exchanges (each step sends the half
+// that the partner keeps), then one broadcast per value: 2N + 1 or 2N + 2 shuffles instead of 5N.
+template <int N>
+__device__ __forceinline__ void warp_sums(float (&v)[N]) {
+  static_assert(N == 4 || N == 8, "four or eight values");
+  const int lane = threadIdx.x & 31;
+  int keep = 16;
 #pragma unroll
-      for (int j = 0; j < 3; ++j) xw[j] = load_pairs<NP>(sx + (rg * 8 + 2 - j) * ROW);
-      V gw[3] = {zero_pairs<NP>(), zero_pairs<NP>(), zero_pairs<NP>()};
-      __nv_bfloat16* dxr = dxb + static_cast<int64_t>(u_first) * a.C;
+  for (int n = N / 2; n >= 1; n >>= 1) {
+    const bool up = (lane & keep) != 0;
 #pragma unroll
-      for (int i = 0; i < 11; ++i) {
-        const V x0 = load_pairs<NP>(sx + (rg * 8 + 3 + i) * ROW);
-        V gy = load_pairs<NP>(sg + (rg * 8 + i) * ROW);
-        if (on) {
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n], mine = up ? v[i + n] : v[i];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, send, keep);
+    }
+    keep >>= 1;
+  }
+  float s = v[0];
 #pragma unroll
-          for (int p = 0; p < NP; ++p) {
-            float2 pre = __fmul2_rn(xw[2].p[p], w2[p][0]);
-            pre = __ffma2_rn(xw[1].p[p], w2[p][1], pre);
-            pre = __ffma2_rn(xw[0].p[p], w2[p][2], pre);
-            pre = __ffma2_rn(x0.p[p], w2[p][3], pre);
-            gy.p[p] = __fmul2_rn(gy.p[p], silu_grad_pair(pre));
-          }
+  for (; keep >= 1; keep >>= 1) s += __shfl_xor_sync(0xffffffffu, s, keep);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    int src = 0;
+    if (N == 8) src = ((i >> 2) & 1) * 16 + ((i >> 1) & 1) * 8 + (i & 1) * 4;
+    else src = ((i >> 1) & 1) * 16 + (i & 1) * 8;
+    v[i] = __shfl_sync(0xffffffffu, s, src);
+  }
+}
+
+// ---- ring kernels: channel counts that are multiples of eight ------------------------------------------------------------
+struct RingArgs {
+  const __nv_bfloat16* x;        // the three rows before a run; the rest arrives by TMA
+  const __nv_bfloat16* weight;
+  __nv_bfloat16* out;            // y or dx
+  int64_t out_stride_b, out_stride_t;
+  float* dw_partial;             // [B * runs][dw_channels][4], this launch's channels from dw_c0
+  int dw_channels, dw_c0;
+  const int32_t* cu;
+  int n_docs, T, C, act_channels, units, runs, run;     // units of 128 channels; runs of `run` tokens
+  int64_t stride_b, stride_t;
+  // fused glue: the first 3 H units are the heads of q, k, v
+  int H;
+  float eps;
+  __nv_bfloat16 *q, *k, *v;      // forward outputs (B, T, H, 128)
+  int n_warps;
+  int* status;
+};
+struct RingWork {
+  int unit, run, b, lo, own, c0;
+  bool live;
+  __device__ __forceinline__ RingWork(const RingArgs& a, int wi) {
+    unit = wi % a.units;
+    run = wi / a.units % a.runs;
+    b = wi / a.units / a.runs;
+    lo = run * a.run;
+    own = min(a.T, lo + a.run);
+    c0 = unit * 128 + (threadIdx.x & 31) * 4;
+    live = c0 < a.C;
+  }
+};
+
+// Forward.  GLUE: a warp owns one head of q, k or v, so that the head's norm is a sum over its lanes.
+template <bool GLUE, int ACT>
+__device__ __forceinline__ void ring_fwd_walk(const CUtensorMap* map_x, const RingArgs& a, const RingWork& w, Ring<1, RING_FWD_STAGES>& ring,
+                                              const WaitCtl& ctl) {
+  const int tiles = (w.own - w.lo + RING_ROWS - 1) / RING_ROWS;
+  const bool normed = GLUE && w.unit < 2 * a.H;
+  auto issue = [&](int tile, uint8_t* dst, uint64_t* bar) { tma_load_3d(dst, map_x, bar, w.unit * 128, w.lo + tile * RING_ROWS, w.b); };
+  ring.open(tiles, issue);
+  const Taps<4> taps = load_taps<4>(a.weight, w.c0, w.live);
+  DocCursor doc;
+  doc.init(a.cu, a.n_docs, w.lo);
+  doc.advance(w.lo);
+  Window<4> win;
+  open_window<4>(win, a.x + w.b * a.stride_b + (w.live ? w.c0 : 0), a.stride_t, w.lo, max(doc.start, 0), w.live);
+  __nv_bfloat16* out;
+  int64_t os;
+  if constexpr (GLUE) {
+    const int region = w.unit / a.H, head = w.unit % a.H;
+    out = (region == 0 ? a.q : region == 1 ? a.k : a.v) + ((static_cast<int64_t>(w.b) * a.T + w.lo) * a.H + head) * HEAD + (threadIdx.x & 31) * 4;
+    os = static_cast<int64_t>(a.H) * HEAD;
+  } else {
+    out = a.out + w.b * a.out_stride_b + w.lo * a.out_stride_t + w.c0;
+    os = a.out_stride_t;
+  }
+  auto act_row = [&](const Pairs<4>& x0) {
+    Pairs<4> s;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const float2 acc = win.conv(taps, x0, p);
+      if constexpr (ACT == 0) s.p[p] = acc;
+      else if constexpr (ACT == 1) s.p[p] = make_float2(silu(acc.x), silu(acc.y));
+      else s.p[p] = make_float2(w.c0 + 2 * p < a.act_channels ? silu(acc.x) : acc.x, w.c0 + 2 * p + 1 < a.act_channels ? silu(acc.y) : acc.y);
+    }
+    return s;
+  };
+  auto square = [&](const Pairs<4>& s) {
+    const float2 q = __ffma2_rn(s.p[0], s.p[0], __fmul2_rn(s.p[1], s.p[1]));
+    return q.x + q.y;
+  };
+  auto scaled = [&](const Pairs<4>& s, float r) {
+    Pairs<4> o;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) o.p[p] = __fmul2_rn(s.p[p], make_float2(r, r));
+    return o;
+  };
+  for (int tile = 0; tile < tiles; ++tile) {
+    const int t = w.lo + tile * RING_ROWS;
+    const uint8_t* xt = ring.wait(ctl);
+    if (t + RING_ROWS <= w.own && doc.next >= t + RING_ROWS) {     // every row is there and belongs to the window's document
+      Pairs<4> s[RING_ROWS];
+      float ss[RING_ROWS];
+#pragma unroll
+      for (int i = 0; i < RING_ROWS; ++i) {
+        const Pairs<4> x0 = unpack<4>(ring_row(xt, i));
+        s[i] = act_row(x0);
+        if constexpr (GLUE) ss[i] = square(s[i]);
+        win.push(x0);
+        if (!GLUE) {
+          if (w.live) store_row<4>(out, s[i]);
+          out += os;
         }
-        if (i < 8) {
+      }
+      if constexpr (GLUE) {
+        if (normed) warp_sums<RING_ROWS>(ss);
 #pragma unroll
-          for (int p = 0; p < NP; ++p) {
-            dwa[p][0] = __ffma2_rn(gy.p[p], xw[2].p[p], dwa[p][0]);
-            dwa[p][1] = __ffma2_rn(gy.p[p], xw[1].p[p], dwa[p][1]);
-            dwa[p][2] = __ffma2_rn(gy.p[p], xw[0].p[p], dwa[p][2]);
-            dwa[p][3] = __ffma2_rn(gy.p[p], x0.p[p], dwa[p][3]);
-          }
+        for (int i = 0; i < RING_ROWS; ++i) {
+          store_row<4>(out, normed ? scaled(s[i], rsqrtf(ss[i] + a.eps)) : s[i]);
+          out += os;
         }
-        if (i >= 3) {
-          V out;
-#pragma unroll
-          for (int p = 0; p < NP; ++p) {
-            float2 acc = __fmul2_rn(gw[2].p[p], w2[p][3]);
-            acc = __ffma2_rn(gw[1].p[p], w2[p][2], acc);
-            acc = __ffma2_rn(gw[0].p[p], w2[p][1], acc);
-            acc = __ffma2_rn(gy.p[p], w2[p][0], acc);
-            out.p[p] = acc;
-          }
-          store_pairs<NP>(dxr, out);
-          dxr += a.C;
-        }
-        gw[2] = gw[1]; gw[1] = gw[0]; gw[0] = gy;
-        xw[2] = xw[1]; xw[1] = xw[0]; xw[0] = x0;
       }
     } else {
-      V xw[3];                                                           // x[t-1], x[t-2], x[t-3]
+#pragma unroll 1
+      for (int i = 0; i < RING_ROWS; ++i) {
+        const int r = t + i;
+        if (r >= w.own) break;
+        if (r >= doc.next) {
+          doc.advance(r);
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int tj = u_first - 1 - j;
-        xw[j] = (tj >= doc.start) ? load_pairs<NP>(sx + (rg * 8 + 2 - j) * ROW) : zero_pairs<NP>();
-      }
-      V gw[3] = {zero_pairs<NP>(), zero_pairs<NP>(), zero_pairs<NP>()};  // dy'[t-1], dy'[t-2], dy'[t-3]
-      int ds1 = 0x7fffffff, ds2 = 0x7fffffff;                            // document starts of tokens t-1, t-2
-#pragma unroll
-      for (int i = 0; i < 11; ++i) {
-        const int t = u_first + i;
-        V gy = zero_pairs<NP>(), x0 = zero_pairs<NP>();
-        int ds0 = 0x7fffffff;
-        if (t < a.T) {
-          if (i > 0 && doc.advance(t)) { xw[0] = zero_pairs<NP>(); xw[1] = zero_pairs<NP>(); xw[2] = zero_pairs<NP>(); }
-          ds0 = doc.start;
-          x0 = load_pairs<NP>(sx + (rg * 8 + 3 + i) * ROW);
-          const V g = load_pairs<NP>(sg + (rg * 8 + i) * ROW);
-#pragma unroll
-          for (int p = 0; p < NP; ++p) {                                 // dy'[t] = dy[t] * silu'(bf16(pre-activation[t]))
-            float2 pre = __fmul2_rn(xw[2].p[p], w2[p][0]);
-            pre = __ffma2_rn(xw[1].p[p], w2[p][1], pre);
-            pre = __ffma2_rn(xw[0].p[p], w2[p][2], pre);
-            pre = __ffma2_rn(x0.p[p], w2[p][3], pre);
-            const float2 sgp = silu_grad_pair(pre);
-            gy.p[p] = __fmul2_rn(g.p[p], make_float2(act[2 * p] ? sgp.x : 1.f, act[2 * p + 1] ? sgp.y : 1.f));
-          }
-          if (i < 8) {                                                   // the weight gradient of token t belongs to this warp
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-              dwa[p][0] = __ffma2_rn(gy.p[p], xw[2].p[p], dwa[p][0]);
-              dwa[p][1] = __ffma2_rn(gy.p[p], xw[1].p[p], dwa[p][1]);
-              dwa[p][2] = __ffma2_rn(gy.p[p], xw[0].p[p], dwa[p][2]);
-              dwa[p][3] = __ffma2_rn(gy.p[p], x0.p[p], dwa[p][3]);
-            }
-          }
+          for (int j = 0; j < 3; ++j) win.m[j] = zero_pairs<4>();
         }
-        if (i >= 3) {
-          const int u = t - 3;
-          if (u < a.T && live) {
-            const float m2 = (ds2 <= u) ? 1.f : 0.f, m1 = (ds1 <= u) ? 1.f : 0.f, m0 = (ds0 <= u) ? 1.f : 0.f;
-            const float2 m22 = make_float2(m2, m2), m12 = make_float2(m1, m1), m02 = make_float2(m0, m0);
-            V out;
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-              float2 acc = __fmul2_rn(gw[2].p[p], w2[p][3]);
-              acc = __ffma2_rn(__fmul2_rn(m22, gw[1].p[p]), w2[p][2], acc);
-              acc = __ffma2_rn(__fmul2_rn(m12, gw[0].p[p]), w2[p][1], acc);
-              acc = __ffma2_rn(__fmul2_rn(m02, gy.p[p]), w2[p][0], acc);
-              out.p[p] = acc;
-            }
-            store_pairs<NP>(dxb + static_cast<int64_t>(u) * a.C, out);
-          }
+        const Pairs<4> x0 = unpack<4>(ring_row(xt, i));
+        Pairs<4> s = act_row(x0);
+        if (GLUE && normed) {
+          float sums[4] = {square(s), 0.f, 0.f, 0.f};
+          warp_sums<4>(sums);
+          s = scaled(s, rsqrtf(sums[0] + a.eps));
         }
-        gw[2] = gw[1]; gw[1] = gw[0]; gw[0] = gy;
-        ds2 = ds1; ds1 = ds0;
-        xw[2] = xw[1]; xw[1] = xw[0]; xw[0] = x0;
+        if (w.live) store_row<4>(out, s);
+        out += os;
+        win.push(x0);
       }
     }
-    __syncthreads();
-    if (tid == 0 && tile + CONV_BWD_STAGES < tile_hi) issue(tile + CONV_BWD_STAGES);
+    ring.release(tiles, issue);
   }
-  // weight-gradient partial of this CTA: sum over its four row groups in a fixed order through shared memory
-  float* red = reinterpret_cast<float*>(smem);                         // [4 row groups][256 channels][4 taps]
+}
+
+template <bool GLUE>
+__global__ void __launch_bounds__(RING_WARPS * 32, GLUE ? 5 : 6)
+ring_fwd_kernel(const __grid_constant__ CUtensorMap map_x, RingArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t bars[RING_WARPS * RING_FWD_STAGES];
+  __shared__ int abort_s;
+  if (threadIdx.x == 0) abort_s = 0;
   __syncthreads();
+  const int wi = blockIdx.x * RING_WARPS + __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  if (wi >= a.n_warps) return;
+  const RingWork w(a, wi);
+  WaitCtl ctl{&abort_s, a.status};
+  Ring<1, RING_FWD_STAGES> ring;
+  ring.init(smem, bars);
+  if constexpr (GLUE) {
+    ring_fwd_walk<true, 1>(&map_x, a, w, ring, ctl);
+  } else {
+    const bool all = __all_sync(0xffffffffu, !w.live || w.c0 + 4 <= a.act_channels), none = __all_sync(0xffffffffu, !w.live || w.c0 >= a.act_channels);
+    if (all) ring_fwd_walk<false, 1>(&map_x, a, w, ring, ctl);
+    else if (none) ring_fwd_walk<false, 0>(&map_x, a, w, ring, ctl);
+    else ring_fwd_walk<false, 2>(&map_x, a, w, ring, ctl);
+  }
+}
+
+// Backward.  GLUE: the gradient rows are those of q, k, v (map_g: one map per region); the activations are formed again from the
+// window, s = SiLU(pre), and
+//   ds = r dy - r^3 <s, dy> s,   r = rsqrt(sum s^2 + eps)      (v: ds = dv),      dy' = ds SiLU'(pre)
+// in one pass: x and the gradients are read once and dx written once.  (Two kernels, with the gradient of the convolution's
+// output written and read in between, took 1.09 ms for the 12288 q, k, v channels
+// of (1, 32768, 13056) where this one takes 0.58.)
+// (Rows per reduction of the head norms: four rows take fewer shuffles each but hold s and SiLU' of four rows, 168 registers or
+// spills: 595 to 790 us against 583.)
+constexpr int GR = 2;
+template <bool GLUE, int ACT>
+__device__ __forceinline__ void ring_bwd_walk(const CUtensorMap* map_x, const CUtensorMap* map_g, const RingArgs& a, const RingWork& w,
+                                              Ring<2, RING_BWD_STAGES>& ring, const WaitCtl& ctl, float2 (&dw)[2][CONV_W]) {
+  const int tiles = (w.own + 3 - w.lo + RING_ROWS - 1) / RING_ROWS;
+  const int head = GLUE ? w.unit % a.H : 0;
+  const bool normed = GLUE && w.unit < 2 * a.H;
+  auto issue = [&](int tile, uint8_t* dst, uint64_t* bar) {
+    const int t = w.lo + tile * RING_ROWS;
+    tma_load_3d(dst, map_x, bar, w.unit * 128, t, w.b);
+    if constexpr (GLUE) tma_load_4d(dst + RING_TILE, map_g, bar, 0, head, t, w.b);
+    else tma_load_3d(dst + RING_TILE, map_g, bar, w.unit * 128, t, w.b);
+  };
+  ring.open(tiles, issue);
+  const Taps<4> taps = load_taps<4>(a.weight, w.c0, w.live);
+  DocCursor doc;
+  doc.init(a.cu, a.n_docs, w.lo);
+  doc.advance(w.lo);
+  Window<4> win, gw;                                     // x[t-1..t-3], dy'[t-1..t-3]
+  open_window<4>(win, a.x + w.b * a.stride_b + (w.live ? w.c0 : 0), a.stride_t, w.lo, max(doc.start, 0), w.live);
 #pragma unroll
-  for (int p = 0; p < NP; ++p) {
-    float* dst = red + (rg * CONV_CH + cin + 2 * p) * CONV_W;
-    *reinterpret_cast<float4*>(dst) = make_float4(dwa[p][0].x, dwa[p][1].x, dwa[p][2].x, dwa[p][3].x);
-    *reinterpret_cast<float4*>(dst + CONV_W) = make_float4(dwa[p][0].y, dwa[p][1].y, dwa[p][2].y, dwa[p][3].y);
+  for (int j = 0; j < 3; ++j) gw.m[j] = zero_pairs<4>();
+  int ds1 = 0x7fffffff, ds2 = 0x7fffffff;                // document starts of tokens t-1, t-2
+  __nv_bfloat16* out = a.out + w.b * a.out_stride_b + (w.lo - 3) * a.out_stride_t + w.c0;   // row t - 3
+
+  auto add_dw = [&](const Pairs<4>& gy, const Pairs<4>& x0) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      dw[p][0] = __ffma2_rn(gy.p[p], win.m[2].p[p], dw[p][0]);
+      dw[p][1] = __ffma2_rn(gy.p[p], win.m[1].p[p], dw[p][1]);
+      dw[p][2] = __ffma2_rn(gy.p[p], win.m[0].p[p], dw[p][2]);
+      dw[p][3] = __ffma2_rn(gy.p[p], x0.p[p], dw[p][3]);
+    }
+  };
+  // one row's pre-activation -> gradient factor: plain convolution
+  auto plain_grad = [&](const Pairs<4>& x0, Pairs<4>& gy) {
+    if constexpr (ACT != 0) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        float2 sg = silu_grad_pair(win.conv(taps, x0, p));
+        if constexpr (ACT == 2) {
+          sg.x = w.c0 + 2 * p < a.act_channels ? sg.x : 1.f;
+          sg.y = w.c0 + 2 * p + 1 < a.act_channels ? sg.y : 1.f;
+        }
+        gy.p[p] = __fmul2_rn(gy.p[p], sg);
+      }
+    }
+  };
+  // s = SiLU(pre), sp = SiLU'(pre); this lane's shares of sum s^2 and <s, g>
+  auto glue_act = [&](const Pairs<4>& x0, const Pairs<4>& g, Pairs<4>& s, Pairs<4>& sp, float& ss, float& dot) {
+    float2 s2 = make_float2(0.f, 0.f), d2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const float2 pre = win.conv(taps, x0, p);
+      const float2 sig = make_float2(fast_sigmoid(pre.x), fast_sigmoid(pre.y));
+      s.p[p] = __fmul2_rn(pre, sig);
+      // sig (1 + pre (1 - sig)) = sig + s - s sig
+      sp.p[p] = __ffma2_rn(s.p[p], __ffma2_rn(sig, make_float2(-1.f, -1.f), make_float2(1.f, 1.f)), sig);
+      s2 = __ffma2_rn(s.p[p], s.p[p], s2);
+      d2 = __ffma2_rn(s.p[p], g.p[p], d2);
+    }
+    ss = s2.x + s2.y;
+    dot = d2.x + d2.y;
+  };
+  auto glue_grad = [&](Pairs<4>& gy, const Pairs<4>& s, const Pairs<4>& sp, float ss, float dot) {
+    const float r = rsqrtf(ss + a.eps), f = -r * r * r * dot;
+    const float2 r2 = make_float2(r, r), f2 = make_float2(f, f);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) gy.p[p] = __fmul2_rn(__ffma2_rn(f2, s.p[p], __fmul2_rn(r2, gy.p[p])), sp.p[p]);
+  };
+  auto dx_row = [&](const Pairs<4>& g3, const Pairs<4>& g2, const Pairs<4>& g1, const Pairs<4>& g0) {
+    Pairs<4> o;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      float2 acc = __fmul2_rn(g3.p[p], taps.w[p][3]);
+      acc = __ffma2_rn(g2.p[p], taps.w[p][2], acc);
+      acc = __ffma2_rn(g1.p[p], taps.w[p][1], acc);
+      o.p[p] = __ffma2_rn(g0.p[p], taps.w[p][0], acc);
+    }
+    return o;
+  };
+
+  for (int tile = 0; tile < tiles; ++tile) {
+    const int t = w.lo + tile * RING_ROWS;
+    const uint8_t* xt = ring.wait(ctl);
+    const uint8_t* gt = xt + RING_TILE;
+    // Interior: every row is the warp's own and no document starts among the rows or the three before them.
+    if (tile > 0 && t + RING_ROWS <= w.own && doc.next >= t + RING_ROWS && doc.start <= t - 3) {
+      if constexpr (!GLUE) {
+#pragma unroll
+        for (int i = 0; i < RING_ROWS; ++i) {
+          const Pairs<4> x0 = unpack<4>(ring_row(xt, i));
+          Pairs<4> gy = unpack<4>(ring_row(gt, i));
+          plain_grad(x0, gy);
+          add_dw(gy, x0);
+          const Pairs<4> o = dx_row(gw.m[2], gw.m[1], gw.m[0], gy);
+          if (w.live) store_row<4>(out, o);
+          out += a.out_stride_t;
+          gw.push(gy);
+          win.push(x0);
+        }
+      } else {
+#pragma unroll
+        for (int step = 0; step < RING_ROWS; step += GR) {
+          Pairs<4> s[GR], sp[GR];
+          float sums[2 * GR];
+          const Window<4> keep = win;
+#pragma unroll
+          for (int i = 0; i < GR; ++i) {
+            const Pairs<4> x0 = unpack<4>(ring_row(xt, step + i)), g = unpack<4>(ring_row(gt, step + i));
+            glue_act(x0, g, s[i], sp[i], sums[i], sums[GR + i]);
+            win.push(x0);
+          }
+          if (normed) warp_sums<2 * GR>(sums);
+          win = keep;
+#pragma unroll
+          for (int i = 0; i < GR; ++i) {
+            const Pairs<4> x0 = unpack<4>(ring_row(xt, step + i));
+            Pairs<4> gy = unpack<4>(ring_row(gt, step + i));
+            if (normed) {
+              glue_grad(gy, s[i], sp[i], sums[i], sums[GR + i]);
+            } else {
+#pragma unroll
+              for (int p = 0; p < 2; ++p) gy.p[p] = __fmul2_rn(gy.p[p], sp[i].p[p]);
+            }
+            add_dw(gy, x0);
+            store_row<4>(out, dx_row(gw.m[2], gw.m[1], gw.m[0], gy));
+            out += a.out_stride_t;
+            gw.push(gy);
+            win.push(x0);
+          }
+        }
+      }
+      ds1 = ds2 = doc.start;
+    } else {
+#pragma unroll 1
+      for (int i = 0; i < RING_ROWS; ++i) {
+        const int r = t + i;
+        Pairs<4> x0 = zero_pairs<4>(), gy = zero_pairs<4>();
+        int ds0 = 0x7fffffff;
+        if (r < a.T && r < w.own + 3) {
+          if (r >= doc.next) {                           // a document starts here
+            doc.advance(r);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) win.m[j] = zero_pairs<4>();
+          }
+          ds0 = doc.start;
+          x0 = unpack<4>(ring_row(xt, i));
+          gy = unpack<4>(ring_row(gt, i));
+          if constexpr (!GLUE) {
+            plain_grad(x0, gy);
+          } else {
+            Pairs<4> s, sp;
+            float sums[4] = {0.f, 0.f, 0.f, 0.f};
+            glue_act(x0, gy, s, sp, sums[0], sums[1]);
+            if (normed) {
+              warp_sums<4>(sums);
+              glue_grad(gy, s, sp, sums[0], sums[1]);
+            } else {
+#pragma unroll
+              for (int p = 0; p < 2; ++p) gy.p[p] = __fmul2_rn(gy.p[p], sp.p[p]);
+            }
+          }
+          if (r < w.own) add_dw(gy, x0);                 // the weight gradient of a token belongs to one warp
+        }
+        const int u = r - 3;
+        if (u >= w.lo && u < w.own && w.live) {          // gradients of later documents do not reach back
+          const Pairs<4> z = zero_pairs<4>();
+          store_row<4>(out, dx_row(gw.m[2], ds2 <= u ? gw.m[1] : z, ds1 <= u ? gw.m[0] : z, ds0 <= u ? gy : z));
+        }
+        out += a.out_stride_t;
+        gw.push(gy);
+        win.push(x0);
+        ds2 = ds1;
+        ds1 = ds0;
+      }
+    }
+    ring.release(tiles, issue);
+  }
+}
+
+template <bool GLUE>
+__global__ void __launch_bounds__(RING_WARPS * 32, 4)
+ring_bwd_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g0,
+                const __grid_constant__ CUtensorMap map_g1, const __grid_constant__ CUtensorMap map_g2, RingArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t bars[RING_WARPS * RING_BWD_STAGES];
+  __shared__ int abort_s;
+  if (threadIdx.x == 0) abort_s = 0;
+  __syncthreads();
+  const int wi = blockIdx.x * RING_WARPS + __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  if (wi >= a.n_warps) return;
+  const RingWork w(a, wi);
+  WaitCtl ctl{&abort_s, a.status};
+  Ring<2, RING_BWD_STAGES> ring;
+  ring.init(smem, bars);
+  float2 dw[2][CONV_W];
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int j = 0; j < CONV_W; ++j) dw[p][j] = make_float2(0.f, 0.f);
+  if constexpr (GLUE) {
+    const int region = w.unit / a.H;
+    ring_bwd_walk<true, 1>(&map_x, region == 0 ? &map_g0 : region == 1 ? &map_g1 : &map_g2, a, w, ring, ctl, dw);
+  } else {
+    const bool all = __all_sync(0xffffffffu, !w.live || w.c0 + 4 <= a.act_channels), none = __all_sync(0xffffffffu, !w.live || w.c0 >= a.act_channels);
+    if (all) ring_bwd_walk<false, 1>(&map_x, &map_g0, a, w, ring, ctl, dw);
+    else if (none) ring_bwd_walk<false, 0>(&map_x, &map_g0, a, w, ring, ctl, dw);
+    else ring_bwd_walk<false, 2>(&map_x, &map_g0, a, w, ring, ctl, dw);
+  }
+  if (w.live) {                                          // the weight gradient of this run: 4 channels x 4 taps per lane
+    float* out = a.dw_partial + ((static_cast<int64_t>(w.b) * a.runs + w.run) * a.dw_channels + a.dw_c0 + w.c0) * CONV_W;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      *reinterpret_cast<float4*>(out + 8 * p) = make_float4(dw[p][0].x, dw[p][1].x, dw[p][2].x, dw[p][3].x);
+      *reinterpret_cast<float4*>(out + 8 * p + 4) = make_float4(dw[p][0].y, dw[p][1].y, dw[p][2].y, dw[p][3].y);
+    }
+  }
+}
+
+
+// ---- walkers: what the ring kernels cannot take (channel counts, strides or addresses that are no multiples of 16 bytes) --------
+constexpr int CONV_WARPS = 8;          // sub-runs per CTA
+constexpr int CONV_THREADS = CONV_WARPS * 32;
+constexpr int WALK_ROWS = 4;           // rows per batch
+// Rows of a walk in batches of U, the next batch asked for before the current one is used.  Addresses are clamped to the row
+// `last` (always valid); what lies beyond the walk is masked by the caller.
+template <int V, int U>
+struct RowBatch {
+  RawRow<V> r[U];
+  __device__ __forceinline__ void load(const __nv_bfloat16* col, int64_t stride, int t, int last) {
+    if (t + U - 1 <= last) {
+      const __nv_bfloat16* p = col + t * stride;
+#pragma unroll
+      for (int i = 0; i < U; ++i) { r[i] = load_raw<V>(p); p += stride; }
+    } else {
+#pragma unroll
+      for (int i = 0; i < U; ++i) r[i] = load_raw<V>(col + min(t + i, last) * stride);
+    }
+  }
+};
+
+struct ConvArgs {
+  const __nv_bfloat16* x;
+  const __nv_bfloat16* weight;
+  const __nv_bfloat16* dy;       // backward
+  __nv_bfloat16* out;            // y (forward) or dx (backward), contiguous (B, T, C)
+  float* dw_partial;             // backward: [B * groups][C][4]
+  const int32_t* cu;
+  int n_docs, T, C, act_channels, run;      // run: tokens per CTA
+  int64_t x_stride_b, x_stride_t, dy_stride_b, dy_stride_t;
+};
+
+// This warp's tokens [lo, hi) and channels.
+template <int V>
+struct Walk {
+  int lo, hi, c0;
+  bool live;
+  __device__ __forceinline__ Walk(int T, int C, int run) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int first = blockIdx.y * run, sub = (run + CONV_WARPS - 1) / CONV_WARPS;
+    lo = first + warp * sub;
+    hi = min(T, min(lo + sub, first + run));
+    c0 = (blockIdx.x * 32 + lane) * V;
+    live = c0 < C;
+  }
+};
+
+template <int V, int ACT>
+__device__ __forceinline__ void conv_fwd_walk(const ConvArgs& a, const Walk<V>& w) {
+  constexpr int P = (V + 1) / 2;
+  const Taps<V> taps = load_taps<V>(a.weight, w.c0, w.live);
+  const int64_t xs = a.x_stride_t, ys = a.C;
+  const __nv_bfloat16* col = a.x + blockIdx.z * a.x_stride_b + (w.live ? w.c0 : 0);
+  __nv_bfloat16* out = a.out + static_cast<int64_t>(blockIdx.z) * a.T * a.C + w.c0;
+  DocCursor doc;
+  doc.init(a.cu, a.n_docs, w.lo);
+  for (int t = w.lo; t < w.hi;) {
+    doc.advance(t);
+    const int end = min(w.hi, doc.next);
+    Window<V> win;
+    RowBatch<V, WALK_ROWS> b0, b1;
+    b0.load(col, xs, t, end - 1);
+    open_window<V>(win, col, xs, t, max(doc.start, 0), w.live);
+    auto rows = [&](const RowBatch<V, WALK_ROWS>& b) {
+      __nv_bfloat16* y = out + t * ys;
+      const int n = end - t;
+#pragma unroll
+      for (int i = 0; i < WALK_ROWS; ++i) {
+        const Pairs<V> x0 = unpack<V>(b.r[i]);
+        Pairs<V> o;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          const float2 acc = win.conv(taps, x0, p);
+          if constexpr (ACT == 0) o.p[p] = acc;
+          else if constexpr (ACT == 1) o.p[p] = make_float2(silu(acc.x), silu(acc.y));
+          else o.p[p] = make_float2(w.c0 + 2 * p < a.act_channels ? silu(acc.x) : acc.x, w.c0 + 2 * p + 1 < a.act_channels ? silu(acc.y) : acc.y);
+        }
+        if (w.live && i < n) store_row<V>(y, o);
+        y += ys;
+        win.push(x0);
+      }
+      t += WALK_ROWS;
+    };
+    for (;;) {
+      if (t + WALK_ROWS < end) b1.load(col, xs, t + WALK_ROWS, end - 1);
+      rows(b0);
+      if (t >= end) break;
+      if (t + WALK_ROWS < end) b0.load(col, xs, t + WALK_ROWS, end - 1);
+      rows(b1);
+      if (t >= end) break;
+    }
+    t = end;
+  }
+}
+
+template <int V>
+__global__ void __launch_bounds__(CONV_THREADS, 3)
+conv_fwd_kernel(ConvArgs a) {
+  const Walk<V> w(a.T, a.C, a.run);
+  if (w.lo >= w.hi) return;
+  switch (act_kind(w.c0, V, w.live, a.act_channels)) {
+    case 0: conv_fwd_walk<V, 0>(a, w); break;
+    case 1: conv_fwd_walk<V, 1>(a, w); break;
+    default: conv_fwd_walk<V, 2>(a, w); break;
+  }
+}
+
+// Backward over the rows [lo, hi) of this warp: dx, and the weight gradient of these rows in `dw`.
+//   dy'[t] = dy[t] SiLU'(pre[t])      dw[j] += dy'[t] x[t-3+j]      dx[u] = sum_j dy'[u+j] w[3-j]  over tokens of the same document
+// A walk of one document's rows ends with the three gradients behind its own rows (which the next walk owns; zero past the end
+// of the document).
+template <int V, int ACT>
+__device__ __forceinline__ void conv_bwd_walk(const ConvArgs& a, const Walk<V>& w, float2 (&dw)[(V + 1) / 2][CONV_W]) {
+  constexpr int P = (V + 1) / 2;
+  const Taps<V> taps = load_taps<V>(a.weight, w.c0, w.live);
+  const int64_t xs = a.x_stride_t, gs = a.dy_stride_t, os = a.C;
+  const __nv_bfloat16* col = a.x + blockIdx.z * a.x_stride_b + (w.live ? w.c0 : 0);
+  const __nv_bfloat16* gcol = a.dy + blockIdx.z * a.dy_stride_b + (w.live ? w.c0 : 0);
+  __nv_bfloat16* out = a.out + static_cast<int64_t>(blockIdx.z) * a.T * a.C + w.c0;
+  DocCursor doc;
+  doc.init(a.cu, a.n_docs, w.lo);
+  for (int t = w.lo; t < w.hi;) {
+    doc.advance(t);
+    const int own = min(w.hi, doc.next), real = min(own + 3, min(doc.next, a.T)), first = t;
+    Window<V> win, gw;                                   // gw: dy'[t-1], dy'[t-2], dy'[t-3]
+    RowBatch<V, WALK_ROWS> x0b, g0b, x1b, g1b;
+    x0b.load(col, xs, t, real - 1);
+    g0b.load(gcol, gs, t, real - 1);
+    open_window<V>(win, col, xs, t, max(doc.start, 0), w.live);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) gw.m[j] = zero_pairs<V>();
+    auto row = [&](const RawRow<V>& xr, const RawRow<V>& gr, int r, bool edge) {
+      const Pairs<V> x0 = unpack<V>(xr);
+      Pairs<V> gy = unpack<V>(gr);
+      if constexpr (ACT != 0) {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          float2 sg = silu_grad_pair(win.conv(taps, x0, p));
+          if constexpr (ACT == 2) {
+            sg.x = w.c0 + 2 * p < a.act_channels ? sg.x : 1.f;
+            sg.y = w.c0 + 2 * p + 1 < a.act_channels ? sg.y : 1.f;
+          }
+          gy.p[p] = __fmul2_rn(gy.p[p], sg);
+        }
+      }
+      if (edge && r >= real) gy = zero_pairs<V>();
+      if (!edge || r < own) {
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          dw[p][0] = __ffma2_rn(gy.p[p], win.m[2].p[p], dw[p][0]);
+          dw[p][1] = __ffma2_rn(gy.p[p], win.m[1].p[p], dw[p][1]);
+          dw[p][2] = __ffma2_rn(gy.p[p], win.m[0].p[p], dw[p][2]);
+          dw[p][3] = __ffma2_rn(gy.p[p], x0.p[p], dw[p][3]);
+        }
+      }
+      if (w.live && r - 3 >= first && (!edge || r - 3 < own)) {
+        Pairs<V> o;
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          float2 acc = __fmul2_rn(gw.m[2].p[p], taps.w[p][3]);
+          acc = __ffma2_rn(gw.m[1].p[p], taps.w[p][2], acc);
+          acc = __ffma2_rn(gw.m[0].p[p], taps.w[p][1], acc);
+          o.p[p] = __ffma2_rn(gy.p[p], taps.w[p][0], acc);
+        }
+        store_row<V>(out + (r - 3) * os, o);
+      }
+      gw.push(gy);
+      win.push(x0);
+    };
+    auto rows = [&](const RowBatch<V, WALK_ROWS>& xb, const RowBatch<V, WALK_ROWS>& gb) {
+      if (t + WALK_ROWS <= own) {
+#pragma unroll
+        for (int i = 0; i < WALK_ROWS; ++i) row(xb.r[i], gb.r[i], t + i, false);
+      } else {
+#pragma unroll
+        for (int i = 0; i < WALK_ROWS; ++i) row(xb.r[i], gb.r[i], t + i, true);
+      }
+      t += WALK_ROWS;
+    };
+    for (;;) {
+      if (t + WALK_ROWS < real) {
+        x1b.load(col, xs, t + WALK_ROWS, real - 1);
+        g1b.load(gcol, gs, t + WALK_ROWS, real - 1);
+      }
+      rows(x0b, g0b);
+      if (t >= own + 3) break;
+      if (t + WALK_ROWS < real) {
+        x0b.load(col, xs, t + WALK_ROWS, real - 1);
+        g0b.load(gcol, gs, t + WALK_ROWS, real - 1);
+      }
+      rows(x1b, g1b);
+      if (t >= own + 3) break;
+    }
+    t = own;
+  }
+}
+
+// Sum of the warps' weight gradients in index order -> this CTA's partial.
+template <int V>
+__device__ __forceinline__ void reduce_dw(const float2 (&dw)[(V + 1) / 2][CONV_W], float* red, float* out, int channels, int cbase) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+  for (int c = 0; c < V; ++c) {
+    float4 v;
+    v.x = (c & 1) ? dw[c / 2][0].y : dw[c / 2][0].x;
+    v.y = (c & 1) ? dw[c / 2][1].y : dw[c / 2][1].x;
+    v.z = (c & 1) ? dw[c / 2][2].y : dw[c / 2][2].x;
+    v.w = (c & 1) ? dw[c / 2][3].y : dw[c / 2][3].x;
+    *reinterpret_cast<float4*>(red + (warp * 32 * V + lane * V + c) * CONV_W) = v;
   }
   __syncthreads();
-  float* out = a.dw_partial + (static_cast<int64_t>(b) * gridDim.y + blockIdx.y) * (static_cast<int64_t>(a.C) * CONV_W);
-  for (int e = tid; e < CONV_CH * CONV_W; e += blockDim.x) {
-    const int ch = cbase + e / CONV_W;
-    if (ch < a.C)
-      out[static_cast<int64_t>(ch) * CONV_W + e % CONV_W] =
-          (red[e] + red[CONV_CH * CONV_W + e]) + (red[2 * CONV_CH * CONV_W + e] + red[3 * CONV_CH * CONV_W + e]);
+  for (int e = tid; e < 32 * V * CONV_W; e += CONV_THREADS) {
+    if (e / CONV_W >= channels) break;
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < CONV_WARPS; ++w) s += red[w * 32 * V * CONV_W + e];
+    out[static_cast<int64_t>(cbase) * CONV_W + e] = s;
   }
+}
+
+template <int V>
+__global__ void __launch_bounds__(CONV_THREADS, V == 4 ? 2 : 3)
+conv_bwd_kernel(ConvArgs a) {
+  __shared__ __align__(16) float red[CONV_WARPS * 32 * V * CONV_W];
+  const Walk<V> w(a.T, a.C, a.run);
+  float2 dw[(V + 1) / 2][CONV_W];
+#pragma unroll
+  for (int p = 0; p < (V + 1) / 2; ++p)
+#pragma unroll
+    for (int j = 0; j < CONV_W; ++j) dw[p][j] = make_float2(0.f, 0.f);
+  if (w.lo < w.hi) {
+    switch (act_kind(w.c0, V, w.live, a.act_channels)) {
+      case 0: conv_bwd_walk<V, 0>(a, w, dw); break;
+      case 1: conv_bwd_walk<V, 1>(a, w, dw); break;
+      default: conv_bwd_walk<V, 2>(a, w, dw); break;
+    }
+  }
+  const int cbase = blockIdx.x * 32 * V;
+  float* out = a.dw_partial + (static_cast<int64_t>(blockIdx.z) * gridDim.y + blockIdx.y) * (static_cast<int64_t>(a.C) * CONV_W);
+  reduce_dw<V>(dw, red, out, a.C - cbase, cbase);
 }
 
 __global__ void conv_dw_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ dw, int n_partial,
@@ -510,98 +897,206 @@ using namespace tgdn;
 static int conv_check(const void* x, const void* weight, const void* y, const int32_t* cu, int n_docs, int B, int T,
                       int C, int64_t stride_b, int64_t stride_t) {
   if (!x || !weight || !y) return TGDN_ERR_NULL;
-  if (B <= 0 || T <= 0 || C <= 0 || C % 8) return TGDN_ERR_SHAPE;
+  if (B <= 0 || T <= 0 || C <= 0) return TGDN_ERR_SHAPE;
   if (cu && (B != 1 || n_docs < 1)) return TGDN_ERR_SHAPE;
   if (B > 65535) return TGDN_ERR_SHAPE;
-  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(y)) & 15)
-    return TGDN_ERR_ALIGN;
-  if ((stride_b % 8) || (stride_t % 8) || stride_t < C) return TGDN_ERR_ALIGN;
+  if (reinterpret_cast<uintptr_t>(weight) & 7) return TGDN_ERR_ALIGN;         // the four taps of a channel are one load
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 1) || stride_t < C) return TGDN_ERR_ALIGN;
   return 0;
 }
+// What the entry points of the public ABI ask for: whole 16-byte pieces.
+static int conv_check_abi(const void* x, const void* weight, const void* y, const int32_t* cu, int n_docs, int B, int T,
+                          int C, int64_t stride_b, int64_t stride_t) {
+  const int rc = conv_check(x, weight, y, cu, n_docs, B, T, C, stride_b, stride_t);
+  if (rc && rc != TGDN_ERR_ALIGN) return rc;
+  if (C % 8) return TGDN_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(y)) & 15) return TGDN_ERR_ALIGN;
+  return ((stride_b % 8) || (stride_t % 8) || stride_t < C) ? TGDN_ERR_ALIGN : 0;
+}
 
-// Token tiles per CTA and number of CTAs along the token axis.  A CTA walks a run of tokens with its ring of tiles in flight,
-// and each CTA of the backward leaves a weight-gradient partial, so runs should be long; but the grid must not end in a
-// nearly empty wave (306 CTAs on 296 resident slots take as long as 592), and the SMs do not finish in step, so several
-// short waves balance better than one long one.  Measured at (1, 32768, 13056): the time falls until about four waves
-// (backward) or six (forward) and is flat beyond, until the partials of the backward start to cost.  So: as many token
-// groups as fill `waves` waves of resident CTAs without spilling into the next, with runs of at least eight tiles.
-static void conv_groups(int B, int T, int C, int ctas_per_sm, int waves, int* groups, int* tiles_per_group) {
+// The ring kernels want what a tensor map wants: 16-byte aligned rows of whole 16-byte pieces (and 8-byte stores).
+static bool ring_ok(int C, std::initializer_list<const void*> ptrs, std::initializer_list<int64_t> strides) {
+  uintptr_t p = 0;
+  int64_t s = C;
+  for (const void* q : ptrs) p |= reinterpret_cast<uintptr_t>(q);
+  for (int64_t q : strides) s |= q;
+  return s % 8 == 0 && p % 16 == 0;
+}
+// Channels per lane of the walkers: 8-byte, 4-byte or 2-byte accesses.
+static int walk_vec(int C, std::initializer_list<const void*> ptrs, std::initializer_list<int64_t> strides) {
+  uintptr_t p = 0;
+  int64_t s = C;
+  for (const void* q : ptrs) p |= reinterpret_cast<uintptr_t>(q);
+  for (int64_t q : strides) s |= q;
+  if (s % 4 == 0 && p % 8 == 0) return 4;
+  return (s % 2 == 0 && p % 4 == 0) ? 2 : 1;
+}
+
+// Runs per batch row of a ring kernel: as many warps as fill the chip `waves` times over with `per_sm` resident warps, runs of
+// at least `least` tokens (a run loads three rows to open its window; the backward walks three more behind its end).
+// Measured at (1, 32768, 13056), us: forward 23 runs 319, 46 310, 92 307, 164 299, 513 311; backward 23 runs 462, 46 452, 92 424,
+// 164 431, 513 518 (each run leaves a weight-gradient partial); at (2, 4096, 4096) the forward falls from 42 (runs of 195) to 33
+// (runs of 32), the backward is flat at 58 between runs of 195 and 63.
+static int ring_runs(int B, int T, int units, int waves, int per_sm, int least) {
+  const int64_t warps = static_cast<int64_t>(waves) * per_sm * tgdn_sm_count();
+  int64_t runs = warps / (static_cast<int64_t>(units) * B);
+  if (runs > T / least) runs = T / least;
+  return static_cast<int>(runs < 1 ? 1 : runs);
+}
+static int fwd_runs(int B, int T, int units) { return ring_runs(B, T, units, 5, 24, 16); }
+static int bwd_runs(int B, int T, int units) { return ring_runs(B, T, units, 4, 16, 48); }
+
+// Token groups for which the caller of the public ABI has scratch: one f32 partial of C x 4 per group and batch row.
+static int scratch_groups(int B, int T, int C) {
   const int n_tiles = (T + CONV_TOK - 1) / CONV_TOK;
-  const int64_t columns = static_cast<int64_t>((C + CONV_CH - 1) / CONV_CH) * B;      // CTAs per token group
-  int64_t g = static_cast<int64_t>(waves) * ctas_per_sm * tgdn_sm_count() / columns;   // 148 on a B200 (and without a device)
+  const int64_t columns = static_cast<int64_t>((C + 255) / 256) * B;
+  int64_t g = static_cast<int64_t>(8) * tgdn_sm_count() / columns;                     // 148 on a B200 (and without a device)
   if (g > n_tiles / 8) g = n_tiles / 8;
   if (g < 1) g = 1;
-  *tiles_per_group = static_cast<int>((n_tiles + g - 1) / g);
-  *groups = (n_tiles + *tiles_per_group - 1) / *tiles_per_group;
+  const int tpg = static_cast<int>((n_tiles + g - 1) / g);
+  return (n_tiles + tpg - 1) / tpg;
 }
-constexpr int CONV_FWD_WAVES = 6, CONV_BWD_WAVES = 4;
+static int64_t partial_bytes(int B, int groups, int C) { return static_cast<int64_t>(B) * groups * C * CONV_W * static_cast<int64_t>(sizeof(float)); }
+
+// Scratch with which the backward runs best; tgdn_conv_bwd_scratch_bytes is the least.
+int64_t tgdn_conv_bwd_best_scratch(int B, int T, int C) {
+  return partial_bytes(B, std::max(scratch_groups(B, T, C), bwd_runs(B, T, (C + 127) / 128)), C);
+}
+
+static RingArgs ring_args(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b,
+                          int64_t stride_t, int runs) {
+  RingArgs a{};
+  a.x = static_cast<const __nv_bfloat16*>(x);
+  a.weight = static_cast<const __nv_bfloat16*>(weight);
+  a.cu = cu; a.n_docs = n_docs; a.T = T; a.C = C;
+  a.units = (C + 127) / 128;
+  a.run = (T + runs - 1) / runs;
+  a.runs = (T + a.run - 1) / a.run;
+  a.stride_b = stride_b; a.stride_t = stride_t;
+  a.out_stride_b = static_cast<int64_t>(T) * C; a.out_stride_t = C;
+  a.dw_channels = C;
+  a.n_warps = a.units * a.runs * B;
+  a.status = tgdn_status_word();
+  return a;
+}
+static unsigned ring_grid(const RingArgs& a) { return static_cast<unsigned>((a.n_warps + RING_WARPS - 1) / RING_WARPS); }
+constexpr int RING_FWD_SMEM = RING_WARPS * RING_FWD_STAGES * RING_TILE, RING_BWD_SMEM = RING_WARPS * RING_BWD_STAGES * RING_TILE * 2;
+
+template <bool GLUE>
+static int ring_fwd_launch(const RingArgs& a, int B, cudaStream_t s) {
+  CUtensorMap mx;
+  int rc = tgdn_make_rows_map(&mx, a.x, a.C, a.T, B, a.stride_t, a.stride_b, 128, RING_ROWS);
+  if (rc) return rc;
+  static bool configured[64] = {};
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(ring_fwd_kernel<GLUE>), RING_FWD_SMEM, configured))) return rc;
+  ring_fwd_kernel<GLUE><<<ring_grid(a), RING_WARPS * 32, RING_FWD_SMEM, s>>>(mx, a);
+  return tgdn_cuda_error(cudaGetLastError());
+}
+template <bool GLUE>
+static int ring_bwd_launch(const RingArgs& a, int B, const CUtensorMap* mg, cudaStream_t s) {
+  CUtensorMap mx;
+  int rc = tgdn_make_rows_map(&mx, a.x, a.C, a.T, B, a.stride_t, a.stride_b, 128, RING_ROWS);
+  if (rc) return rc;
+  static bool configured[64] = {};
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(ring_bwd_kernel<GLUE>), RING_BWD_SMEM, configured))) return rc;
+  ring_bwd_kernel<GLUE><<<ring_grid(a), RING_WARPS * 32, RING_BWD_SMEM, s>>>(mx, mg[0], mg[GLUE ? 1 : 0], mg[GLUE ? 2 : 0], a);
+  return tgdn_cuda_error(cudaGetLastError());
+}
+static int reduce_dw_launch(const float* partial, void* dw, int n_partial, int C, cudaStream_t s) {
+  const int n_elem = C * CONV_W;
+  conv_dw_reduce_kernel<<<(n_elem + 127) / 128, 128, 0, s>>>(partial, static_cast<__nv_bfloat16*>(dw), n_partial, n_elem);
+  return tgdn_cuda_error(cudaGetLastError());
+}
+
+// Tokens per CTA of the walkers: sub-runs of at least 16 rows, a few waves of CTAs.
+static int walk_run(int B, int T, int columns) {
+  int64_t groups = static_cast<int64_t>(32) * tgdn_sm_count() / (static_cast<int64_t>(columns) * B);
+  if (groups < 1) groups = 1;
+  const int64_t run = (T + groups - 1) / groups;
+  return static_cast<int>(std::min<int64_t>(std::max<int64_t>(run, 16 * CONV_WARPS), 256 * CONV_WARPS));
+}
+template <int V>
+static dim3 walk_grid(int B, int C, int groups) { return dim3((C + 32 * V - 1) / (32 * V), groups, B); }
+
+int tgdn_conv_fwd_any(const void* x, const void* weight, void* y, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b,
+                      int64_t stride_t, int act_channels, void* stream) {
+  int rc = conv_check(x, weight, y, cu, n_docs, B, T, C, stride_b, stride_t);
+  if (rc) return rc;
+  if (!tgdn_check_device()) return TGDN_ERR_DEVICE;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (ring_ok(C, {x, y}, {stride_b, stride_t})) {
+    RingArgs a = ring_args(x, weight, cu, n_docs, B, T, C, stride_b, stride_t, fwd_runs(B, T, (C + 127) / 128));
+    a.out = static_cast<__nv_bfloat16*>(y);
+    a.act_channels = act_channels;
+    return ring_fwd_launch<false>(a, B, s);
+  }
+  ConvArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), nullptr, static_cast<__nv_bfloat16*>(y), nullptr,
+             cu, n_docs, T, C, act_channels, 0, stride_b, stride_t, 0, 0};
+  const int V = walk_vec(C, {x, y}, {stride_b, stride_t});
+  a.run = walk_run(B, T, (C + 32 * V - 1) / (32 * V));
+  const int groups = (T + a.run - 1) / a.run;
+  if (V == 4) conv_fwd_kernel<4><<<walk_grid<4>(B, C, groups), CONV_THREADS, 0, s>>>(a);
+  else if (V == 2) conv_fwd_kernel<2><<<walk_grid<2>(B, C, groups), CONV_THREADS, 0, s>>>(a);
+  else conv_fwd_kernel<1><<<walk_grid<1>(B, C, groups), CONV_THREADS, 0, s>>>(a);
+  return tgdn_cuda_error(cudaGetLastError());
+}
+
+int tgdn_conv_bwd_any(const void* x, const void* weight, const void* dy, void* dx, void* dw, const int32_t* cu, int n_docs, int B, int T,
+                      int C, int64_t stride_b, int64_t stride_t, int64_t dy_stride_b, int64_t dy_stride_t, int act_channels,
+                      void* scratch, int64_t scratch_bytes, void* stream) {
+  int rc = conv_check(x, weight, dx, cu, n_docs, B, T, C, stride_b, stride_t);
+  if (rc) return rc;
+  if (!dy || !dw) return TGDN_ERR_NULL;
+  if ((reinterpret_cast<uintptr_t>(dy) & 1) || dy_stride_t < C) return TGDN_ERR_ALIGN;
+  if (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 15) || scratch_bytes < partial_bytes(B, scratch_groups(B, T, C), C)) return TGDN_ERR_SCRATCH;
+  if (!tgdn_check_device()) return TGDN_ERR_DEVICE;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int room = static_cast<int>(std::min<int64_t>(scratch_bytes / partial_bytes(B, 1, C), 1 << 20));
+  if (ring_ok(C, {x, dy, dx}, {stride_b, stride_t, dy_stride_b, dy_stride_t})) {
+    RingArgs a = ring_args(x, weight, cu, n_docs, B, T, C, stride_b, stride_t, std::min(room, bwd_runs(B, T, (C + 127) / 128)));
+    a.out = static_cast<__nv_bfloat16*>(dx);
+    a.act_channels = act_channels;
+    a.dw_partial = static_cast<float*>(scratch);
+    CUtensorMap mg;
+    if ((rc = tgdn_make_rows_map(&mg, dy, C, T, B, dy_stride_t, dy_stride_b, 128, RING_ROWS))) return rc;
+    if ((rc = ring_bwd_launch<false>(a, B, &mg, s))) return rc;
+    return reduce_dw_launch(a.dw_partial, dw, B * a.runs, C, s);
+  }
+  ConvArgs a{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), static_cast<const __nv_bfloat16*>(dy),
+             static_cast<__nv_bfloat16*>(dx), static_cast<float*>(scratch), cu, n_docs, T, C, act_channels, 0, stride_b, stride_t,
+             dy_stride_b, dy_stride_t};
+  const int V = walk_vec(C, {x, dy, dx}, {stride_b, stride_t, dy_stride_b, dy_stride_t});
+  int groups = std::min(room, (T + walk_run(B, T, (C + 32 * V - 1) / (32 * V)) - 1) / walk_run(B, T, (C + 32 * V - 1) / (32 * V)));
+  a.run = (T + groups - 1) / groups;
+  groups = (T + a.run - 1) / a.run;
+  if (V == 4) conv_bwd_kernel<4><<<walk_grid<4>(B, C, groups), CONV_THREADS, 0, s>>>(a);
+  else if (V == 2) conv_bwd_kernel<2><<<walk_grid<2>(B, C, groups), CONV_THREADS, 0, s>>>(a);
+  else conv_bwd_kernel<1><<<walk_grid<1>(B, C, groups), CONV_THREADS, 0, s>>>(a);
+  if ((rc = tgdn_cuda_error(cudaGetLastError()))) return rc;
+  return reduce_dw_launch(a.dw_partial, dw, B * groups, C, s);
+}
 
 extern "C" int tgdn_conv_fwd(const void* x, const void* weight, void* y, const int32_t* cu_seqlens, int n_docs, int B,
                              int T, int C, int64_t stride_b, int64_t stride_t, int act_channels, void* stream) {
-  int rc = conv_check(x, weight, y, cu_seqlens, n_docs, B, T, C, stride_b, stride_t);
-  if (rc) return rc;
-  // the device query also binds the CUDA context to the calling thread, which the tensor-map encoder needs
-  if (!tgdn_check_device()) return TGDN_ERR_DEVICE;
-  CUtensorMap mx;
-  if ((rc = tgdn_make_rows_map(&mx, x, C, T, B, stride_t, stride_b, CONV_CH, CONV_FWD_ROWS))) return rc;
-  int groups, tpg;
-  conv_groups(B, T, C, 4, CONV_FWD_WAVES, &groups, &tpg);
-  ConvArgs a{static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(y), nullptr, cu_seqlens, n_docs, T, C,
-             act_channels, tpg, tgdn_status_word()};
-  const int smem = CONV_FWD_STAGES * CONV_FWD_ROWS * CONV_CH * 2 + 128;
-  static bool configured[64] = {};
-  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(conv_fwd_kernel), smem, configured))) return rc;
-  dim3 grid((C + CONV_CH - 1) / CONV_CH, groups, B);
-  conv_fwd_kernel<<<grid, CONV_THREADS, smem, static_cast<cudaStream_t>(stream)>>>(mx, a);
-  return tgdn_cuda_error(cudaGetLastError());
+  const int rc = conv_check_abi(x, weight, y, cu_seqlens, n_docs, B, T, C, stride_b, stride_t);
+  return rc ? rc : tgdn_conv_fwd_any(x, weight, y, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, act_channels, stream);
 }
 
 extern "C" int64_t tgdn_conv_bwd_scratch_bytes(int B, int T, int C) {
   if (B <= 0 || T <= 0 || C <= 0) return 0;
-  int groups, tpg;
-  conv_groups(B, T, C, 2, CONV_BWD_WAVES, &groups, &tpg);
-  return static_cast<int64_t>(B) * groups * C * CONV_W * static_cast<int64_t>(sizeof(float));
-}
-
-// Shared by tgdn_conv_bwd and tgdn_conv_bwd_static: both kernels of the backward with the partials in `scratch`.
-static int conv_bwd_launch(const void* x, const void* weight, const void* dy, void* dx, void* dw, const int32_t* cu_seqlens,
-                           int n_docs, int B, int T, int C, int64_t stride_b, int64_t stride_t, int64_t dy_stride_b,
-                           int64_t dy_stride_t, int act_channels, float* scratch, cudaStream_t s) {
-  // the device query also binds the CUDA context to the calling thread (autograd runs the backward on a worker thread
-  // that may not have made a runtime call yet), which the tensor-map encoder needs
-  if (!tgdn_check_device()) return TGDN_ERR_DEVICE;
-  CUtensorMap mx, mg;
-  int rc;
-  if ((rc = tgdn_make_rows_map(&mx, x, C, T, B, stride_t, stride_b, CONV_CH, CONV_BWD_XROWS))) return rc;
-  if ((rc = tgdn_make_rows_map(&mg, dy, C, T, B, dy_stride_t, dy_stride_b, CONV_CH, CONV_BWD_GROWS))) return rc;
-  int groups, tpg;
-  conv_groups(B, T, C, 2, CONV_BWD_WAVES, &groups, &tpg);
-  ConvArgs a{static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(dx), scratch, cu_seqlens, n_docs, T, C,
-             act_channels, tpg, tgdn_status_word()};
-  const int smem = CONV_BWD_STAGES * (CONV_BWD_XROWS + CONV_BWD_GROWS) * CONV_CH * 2 + 128;
-  static bool configured[64] = {};
-  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(conv_bwd_kernel<CONV_BWD_NP>), smem, configured))) return rc;
-  dim3 grid((C + CONV_CH - 1) / CONV_CH, groups, B);
-  conv_bwd_kernel<CONV_BWD_NP><<<grid, CONV_THREADS * 2 / CONV_BWD_NP, smem, s>>>(mx, mg, a);
-  rc = tgdn_cuda_error(cudaGetLastError());
-  if (rc) return rc;
-  const int n_elem = C * CONV_W;
-  conv_dw_reduce_kernel<<<(n_elem + 255) / 256, 256, 0, s>>>(scratch, static_cast<__nv_bfloat16*>(dw), B * groups, n_elem);
-  return tgdn_cuda_error(cudaGetLastError());
+  return partial_bytes(B, scratch_groups(B, T, C), C);
 }
 
 extern "C" int tgdn_conv_bwd(const void* x, const void* weight, const void* dy, void* dx, void* dw,
                              const int32_t* cu_seqlens, int n_docs, int B, int T, int C, int64_t stride_b,
                              int64_t stride_t, int64_t dy_stride_b, int64_t dy_stride_t, int act_channels, void* scratch,
                              int64_t scratch_bytes, void* stream) {
-  int rc = conv_check(x, weight, dx, cu_seqlens, n_docs, B, T, C, stride_b, stride_t);
+  int rc = conv_check_abi(x, weight, dx, cu_seqlens, n_docs, B, T, C, stride_b, stride_t);
   if (rc) return rc;
   if (!dy || !dw) return TGDN_ERR_NULL;
   if ((reinterpret_cast<uintptr_t>(dy) & 15) || (dy_stride_b % 8) || (dy_stride_t % 8) || dy_stride_t < C) return TGDN_ERR_ALIGN;
-  if (!scratch || scratch_bytes < tgdn_conv_bwd_scratch_bytes(B, T, C) || (reinterpret_cast<uintptr_t>(scratch) & 15))
-    return TGDN_ERR_SCRATCH;
-  return conv_bwd_launch(x, weight, dy, dx, dw, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, dy_stride_b, dy_stride_t,
-                         act_channels, static_cast<float*>(scratch), static_cast<cudaStream_t>(stream));
+  return tgdn_conv_bwd_any(x, weight, dy, dx, dw, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, dy_stride_b, dy_stride_t,
+                           act_channels, scratch, scratch_bytes, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -648,251 +1143,211 @@ extern "C" int tgdn_conv_bwd_static(const void* x, const void* weight, const voi
                                     const int32_t* cu_seqlens, int n_docs, int B, int T, int C, int64_t stride_b,
                                     int64_t stride_t, int64_t dy_stride_b, int64_t dy_stride_t, int act_channels,
                                     void* stream) {
-  int rc = conv_check(x, weight, dx, cu_seqlens, n_docs, B, T, C, stride_b, stride_t);
+  int rc = conv_check_abi(x, weight, dx, cu_seqlens, n_docs, B, T, C, stride_b, stride_t);
   if (rc) return rc;
   if (!dy || !dw) return TGDN_ERR_NULL;
   if ((reinterpret_cast<uintptr_t>(dy) & 15) || (dy_stride_b % 8) || (dy_stride_t % 8) || dy_stride_t < C) return TGDN_ERR_ALIGN;
   if (tgdn_conv_bwd_scratch_bytes(B, T, C) > static_cast<int64_t>(TGDN_CONV_STATIC_SCRATCH_BYTES)) return TGDN_ERR_STATIC_LIMIT;
   float* scratch = nullptr;
   if ((rc = conv_static_scratch(&scratch))) return rc;
-  return conv_bwd_launch(x, weight, dy, dx, dw, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, dy_stride_b, dy_stride_t,
-                         act_channels, scratch, static_cast<cudaStream_t>(stream));
+  // (the partials of a caller with the least scratch: the same runs, the same sums)
+  return tgdn_conv_bwd_any(x, weight, dy, dx, dw, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, dy_stride_b, dy_stride_t,
+                           act_channels, scratch, tgdn_conv_bwd_scratch_bytes(B, T, C), stream);
 }
 
-// ----------------------------------------------------------------------------------------------------------------------
-// The layer glue around the convolution, fused: x (B, T, C) with C = H (3*128 + 2E) channels laid out as
-// [q: H x 128 | k: H x 128 | v: H x 128 | k2: H x E | q2: H x E] goes straight to the tensors the core takes:
+
+// ---- the layer glue ------------------------------------------------------------------------------------------------------
+// x (B, T, C) with C = H (3*128 + 2E) channels laid out as [q: H x 128 | k: H x 128 | v: H x 128 | k2: H x E | q2: H x E] goes straight
+// to the tensors the core takes:
 //   q, k  = l2norm(SiLU(conv))   bf16 (B, T, H, 128)         v = SiLU(conv)   bf16 (B, T, H, 128)
 //   k2, q2 = l2norm(softplus(conv))   f32 (B, T, H, E)        l2norm(s) = s * rsqrt(sum s^2 + eps)
-// which the reference only describes (cute_triadic_gdn/ops/conv_split_act.py:3-5: "q, k, v (SiLU) and its second key and
-// query (no activation, softplus afterwards)"); its callers run the split, the activations and the norms as separate
-// elementwise passes over (T, C).  Here nothing of the convolution's output is written in between.
-//
-// Main kernel (both directions): the forward's tiling, a warp owning one head's 128 channels of 8 token rows, so that a
-// head's norm is a sum over the 32 lanes.  Forward: writes q, k, v.  Backward: recomputes s = SiLU(conv) from the same x
-// window, takes the gradients of q, k, v and writes the gradient of s, which is what the convolution's own backward takes:
-//   ds = r dy - r^3 <s, dy> s,   r = rsqrt(sum s^2 + eps)              (v: ds = dv)
-// Gate kernel (both directions): one thread per (token, head, k2 | q2), E channels each, straight from global memory (the
-// gate channels are 2E of 384 + 2E per head).  Backward writes dc = du * sigmoid(c) with du as above for u = softplus(c).
-// ----------------------------------------------------------------------------------------------------------------------
+// which the reference only describes (cute_triadic_gdn/ops/conv_split_act.py:3-5) and leaves to separate elementwise passes.
+// q, k, v: the ring kernels above with GLUE.  k2, q2 (2E of 384 + 2E channels per head): the kernel below; its backward leaves the
+// gradient of the convolution's output, compact, for a plain ring backward over those channels.
 namespace tgdn {
 
-struct GlueArgs {
-  const __nv_bfloat16* weight;
-  const int32_t* cu;
-  int n_docs, T, C, H, E, tiles_per_group;
-  float eps;
-  // forward: outputs; backward: the gradients of the same tensors
-  __nv_bfloat16 *q, *k, *v;      // (B, T, H, 128) each
-  float *k2, *q2;                // (B, T, H, E) each
-  __nv_bfloat16* dy;             // backward: (B, T, C) gradient for the convolution's backward
-  const __nv_bfloat16* x;        // gate kernel: the input itself (element strides below)
-  int64_t stride_b, stride_t;
-  int* status;
-};
-
-template <bool BWD>
-__global__ void __launch_bounds__(CONV_THREADS, BWD ? 3 : 4)
-glue_main_kernel(const __grid_constant__ CUtensorMap map_x, GlueArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  constexpr int STAGE_BYTES = CONV_FWD_ROWS * CONV_CH * 2;
-  __shared__ uint64_t full[CONV_FWD_STAGES];
+// The gradient of the convolution's output at the q, k, v channels alone: ds = r dy - r^3 <s, dy> s, s = SiLU(conv).
+__global__ void __launch_bounds__(RING_WARPS * 32, 4)
+glue_norm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g0,
+                 const __grid_constant__ CUtensorMap map_g1, const __grid_constant__ CUtensorMap map_g2, RingArgs a) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t bars[RING_WARPS * RING_BWD_STAGES];
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int half = warp & 1, rg = warp >> 1;
-  const int cbase = blockIdx.x * CONV_CH, c0 = cbase + half * 128 + lane * CONV_VEC, b = blockIdx.z;
-  const int n_tiles = (a.T + CONV_TOK - 1) / CONV_TOK;
-  const int tile_lo = blockIdx.y * a.tiles_per_group, tile_hi = min(n_tiles, tile_lo + a.tiles_per_group);
-  if (tile_lo >= tile_hi) return;
-  if (tid == 0) {
-    for (int s = 0; s < CONV_FWD_STAGES; ++s) mbar_init(&full[s], 1);
-    mbar_fence_init();
-    abort_s = 0;
-  }
+  if (threadIdx.x == 0) abort_s = 0;
   __syncthreads();
+  const int wi = blockIdx.x * RING_WARPS + __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+  if (wi >= a.n_warps) return;
+  const RingWork w(a, wi);
   WaitCtl ctl{&abort_s, a.status};
-  auto issue = [&](int tile) {                         // thread 0
-    const int s = (tile - tile_lo) % CONV_FWD_STAGES;
-    mbar_expect_tx(&full[s], STAGE_BYTES);
-    tma_load_3d(smem + s * STAGE_BYTES, &map_x, &full[s], cbase, tile * CONV_TOK - 3, b);
+  Ring<2, RING_BWD_STAGES> ring;
+  ring.init(smem, bars);
+  const int region = w.unit / a.H, head = w.unit % a.H, tiles = (w.own - w.lo + RING_ROWS - 1) / RING_ROWS;
+  const CUtensorMap* map_g = region == 0 ? &map_g0 : region == 1 ? &map_g1 : &map_g2;
+  auto issue = [&](int tile, uint8_t* dst, uint64_t* bar) {
+    const int t = w.lo + tile * RING_ROWS;
+    tma_load_3d(dst, &map_x, bar, w.unit * 128, t, w.b);
+    tma_load_4d(dst + RING_TILE, map_g, bar, 0, head, t, w.b);
   };
-  if (tid == 0)
-    for (int i = 0; i < CONV_FWD_STAGES && tile_lo + i < tile_hi; ++i) issue(tile_lo + i);
-
-  // this warp's head: unit = which 128-channel block of [q heads | k heads | v heads]
-  const int unit = (cbase + half * 128) >> 7;
-  const bool live = unit < 3 * a.H;                    // a last, half-filled channel tile
-  const int region = live ? unit / a.H : 0, head = live ? unit % a.H : 0;
-  const bool normed = region < 2;
-  float2 w2[2][CONV_W];
-  load_weights(a.weight, c0, live ? a.C : 0, w2);
-  __nv_bfloat16* tb = (region == 0 ? a.q : region == 1 ? a.k : a.v) + ((static_cast<int64_t>(b) * a.T) * a.H + head) * HEAD + lane * CONV_VEC;
-  __nv_bfloat16* dyb = BWD ? a.dy + (static_cast<int64_t>(b) * a.T) * a.C + c0 : nullptr;
-  const int col_off = half * 256 + lane * 8;
-  const int64_t trow = static_cast<int64_t>(a.H) * HEAD;    // elements between token rows of q, k, v
-
-  for (int tile = tile_lo; tile < tile_hi; ++tile) {
-    const int k = tile - tile_lo, s = k % CONV_FWD_STAGES;
-    mbar_wait(&full[s], (k / CONV_FWD_STAGES) & 1, ctl, DEV_TIMEOUT_LOAD);
-    const uint8_t* st = smem + s * STAGE_BYTES + col_off;
-    const int t_first = tile * CONV_TOK + rg * 8;
-    DocCursor doc;
-    doc.init(a.cu, a.n_docs, min(t_first, a.T - 1), a.T);
-    Vec4 xm[3];                                           // x[t-1], x[t-2], x[t-3]
+  ring.open(tiles, issue);
+  const Taps<4> taps = load_taps<4>(a.weight, w.c0, w.live);
+  DocCursor doc;
+  doc.init(a.cu, a.n_docs, w.lo);
+  doc.advance(w.lo);
+  Window<4> win;
+  open_window<4>(win, a.x + w.b * a.stride_b + w.c0, a.stride_t, w.lo, max(doc.start, 0), true);
+  __nv_bfloat16* out = a.out + (static_cast<int64_t>(w.b) * a.T + w.lo) * a.out_stride_t + w.c0;
+  for (int tile = 0; tile < tiles; ++tile) {
+    const uint8_t* xt = ring.wait(ctl);
+    const int t = w.lo + tile * RING_ROWS;
+#pragma unroll 4
+    for (int i = 0; i < RING_ROWS; ++i) {
+      if (t + i >= w.own) break;
+      if (t + i >= doc.next) {
+        doc.advance(t + i);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int tj = t_first - 1 - j;
-      xm[j] = (tj >= doc.start) ? unpack4(*reinterpret_cast<const uint2*>(st + (rg * 8 + 2 - j) * (CONV_CH * 2))) : zero4();
-    }
-    const int n_rows = live ? min(8, a.T - t_first) : 0;
-    // Interior of a document and of the sequence (almost every tile): no document starts among the warp's eight rows or
-    // their three halo rows and all eight rows exist, so the rows need no cursor and no bounds.
-    const bool interior = live && t_first + 8 <= a.T && doc.next >= t_first + 8 && doc.start <= max(t_first - 3, 0);
-    // the gradient rows of this warp's eight tokens are asked for before the arithmetic needs them
-    uint2 gin[8];
-    if constexpr (BWD) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        gin[i] = (i < n_rows) ? __ldg(reinterpret_cast<const uint2*>(tb + (t_first + i) * trow)) : make_uint2(0u, 0u);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (!interior) {                                     // warp-uniform
-        if (i >= n_rows) break;
-        if (i > 0 && doc.advance(t_first + i)) { xm[0] = zero4(); xm[1] = zero4(); xm[2] = zero4(); }   // a document starts here
+        for (int j = 0; j < 3; ++j) win.m[j] = zero_pairs<4>();
       }
-      const Vec4 x0 = unpack4(*reinterpret_cast<const uint2*>(st + (rg * 8 + 3 + i) * (CONV_CH * 2)));
-      Vec4 sv;
-      float ss = 0.f;
+      const Pairs<4> x0 = unpack<4>(ring_row(xt, i));
+      Pairs<4> g = unpack<4>(ring_row(xt + RING_TILE, i)), s;
+      if (region < 2) {
+        float2 s2 = make_float2(0.f, 0.f), d2 = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        float2 acc = __fmul2_rn(xm[2].p[p], w2[p][0]);
-        acc = __ffma2_rn(xm[1].p[p], w2[p][1], acc);
-        acc = __ffma2_rn(xm[0].p[p], w2[p][2], acc);
-        acc = __ffma2_rn(x0.p[p], w2[p][3], acc);
-        sv.p[p] = make_float2(silu(acc.x), silu(acc.y));
-        ss = fmaf(sv.p[p].x, sv.p[p].x, fmaf(sv.p[p].y, sv.p[p].y, ss));
-      }
-      if constexpr (!BWD) {
-        float r = 1.f;
-        if (normed) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-          r = rsqrtf(ss + a.eps);
+        for (int p = 0; p < 2; ++p) {
+          const float2 pre = win.conv(taps, x0, p);
+          s.p[p] = make_float2(silu(pre.x), silu(pre.y));
+          s2 = __ffma2_rn(s.p[p], s.p[p], s2);
+          d2 = __ffma2_rn(s.p[p], g.p[p], d2);
         }
-        Vec4 out;
-        out.p[0] = make_float2(sv.p[0].x * r, sv.p[0].y * r);
-        out.p[1] = make_float2(sv.p[1].x * r, sv.p[1].y * r);
-        store4(tb + (t_first + i) * trow, out);
-      } else {
-        Vec4 g = unpack4(gin[i]);
-        if (normed) {
-          float dot = fmaf(sv.p[0].x, g.p[0].x, fmaf(sv.p[0].y, g.p[0].y, fmaf(sv.p[1].x, g.p[1].x, sv.p[1].y * g.p[1].y)));
+        float sums[4] = {s2.x + s2.y, d2.x + d2.y, 0.f, 0.f};
+        warp_sums<4>(sums);
+        const float r = rsqrtf(sums[0] + a.eps), f = -r * r * r * sums[1];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            dot += __shfl_xor_sync(0xffffffffu, dot, o);
-          }
-          const float r = rsqrtf(ss + a.eps), f = r * r * r * dot;
-#pragma unroll
-          for (int p = 0; p < 2; ++p) g.p[p] = make_float2(fmaf(r, g.p[p].x, -f * sv.p[p].x), fmaf(r, g.p[p].y, -f * sv.p[p].y));
-        }
-        store4(dyb + static_cast<int64_t>(t_first + i) * a.C, g);
+        for (int p = 0; p < 2; ++p) g.p[p] = __ffma2_rn(make_float2(f, f), s.p[p], __fmul2_rn(make_float2(r, r), g.p[p]));
       }
-      xm[2] = xm[1]; xm[1] = xm[0]; xm[0] = x0;
+      store_row<4>(out, g);
+      out += a.out_stride_t;
+      win.push(x0);
     }
-    __syncthreads();                                      // every warp is done with this stage
-    if (tid == 0 && tile + CONV_FWD_STAGES < tile_hi) issue(tile + CONV_FWD_STAGES);
+    ring.release(tiles, issue);
   }
 }
 
+struct GateArgs {
+  const __nv_bfloat16* x;        // (B, T, C), element strides below
+  const __nv_bfloat16* weight;
+  const int32_t* cu;
+  int n_docs, B, T, H, run, runs;
+  int64_t stride_b, stride_t;
+  float eps;
+  float *k2, *q2;                // (B, T, H, E): outputs, or (backward) their gradients
+  __nv_bfloat16* dy;             // backward: gradient at the gate channels, row t at dy + t * dy_stride_t (batch rows T of them apart)
+  int64_t dy_stride_t;
+  bool vec;                      // k2, q2 allow 16-byte accesses
+};
+
+// E consecutive bf16 / f32 in the widest pieces that E allows (the gate channels start at a multiple of E).
+template <int E> struct GateRow { uint32_t w[(E + 1) / 2]; };
+template <int E>
+__device__ __forceinline__ GateRow<E> load_gate_row(const __nv_bfloat16* p) {
+  GateRow<E> r;
+  if constexpr (E % 4 == 0) {
+#pragma unroll
+    for (int i = 0; i < E / 4; ++i) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(p) + i);
+      r.w[2 * i] = u.x; r.w[2 * i + 1] = u.y;
+    }
+  } else if constexpr (E == 2) {
+    r.w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+  } else {
+    r.w[0] = *reinterpret_cast<const unsigned short*>(p);
+  }
+  return r;
+}
+
+// One thread per (unit = k2 | q2 head, run of tokens): the window of its E channels stays in registers, the next row is asked for
+// while the current one is used; neighbouring threads read neighbouring channels.  (One thread per token loaded every row
+// four times and searched the document of every token: 97 us forward at (1, 32768) tokens, H = 32, E = 12.)
 template <int E, bool BWD>
-__global__ void __launch_bounds__(256)
-glue_gate_kernel(GlueArgs a, int B) {
-  const int64_t n = static_cast<int64_t>(B) * a.T * 2 * a.H;
-  const int gbase = 3 * a.H * HEAD;                    // first gate channel
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int u, t, b;                                        // u = which * H + head: consecutive threads, consecutive channel groups
-    if (n <= 0x7fffffffLL) {                            // 64-bit divisions cost a few hundred cycles each: avoid them where 32 bits do
-      const int i32 = static_cast<int>(idx), bt = i32 / (2 * a.H);
-      u = i32 - bt * (2 * a.H);
-      b = bt / a.T;
-      t = bt - b * a.T;
+__global__ void __launch_bounds__(128)
+glue_gate_kernel(GateArgs a) {
+  const int units = 2 * a.H, idx = blockIdx.x * 128 + threadIdx.x;
+  if (idx >= units * a.runs * a.B) return;
+  const int u = idx % units, b = idx / units / a.runs, lo = idx / units % a.runs * a.run, hi = min(a.T, lo + a.run);
+  const int head = u % a.H, c0 = 3 * a.H * HEAD + u * E;
+  float w[E][CONV_W];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(a.weight + static_cast<int64_t>(c0 + e) * CONV_W));
+    w[e][0] = bf16_lo(v.x); w[e][1] = bf16_hi(v.x); w[e][2] = bf16_lo(v.y); w[e][3] = bf16_hi(v.y);
+  }
+  const __nv_bfloat16* xb = a.x + b * a.stride_b + c0;
+  DocCursor doc;
+  doc.init(a.cu, a.n_docs, lo);
+  doc.advance(lo);
+  GateRow<E> m[3];                                       // x[t-1], x[t-2], x[t-3]
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    if (lo - 1 - j >= max(doc.start, 0)) {
+      m[j] = load_gate_row<E>(xb + (lo - 1 - j) * a.stride_t);
     } else {
-      u = static_cast<int>(idx % (2 * a.H));
-      const int64_t bt = idx / (2 * a.H);
-      t = static_cast<int>(bt % a.T);
-      b = static_cast<int>(bt / a.T);
-    }
-    const int which = u / a.H, head = u % a.H;
-    const int c0 = gbase + u * E;
-    int start = 0;                                      // first token of t's document
-    if (a.cu != nullptr) {
-      int lo = 0, hi = a.n_docs - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(a.cu + mid) <= t) lo = mid; else hi = mid - 1;
-      }
-      start = __ldg(a.cu + lo);
-    }
-    float c[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) c[e] = 0.f;
-    const __nv_bfloat16* xb = a.x + b * a.stride_b + c0;
-    // taps of the E channels: four bf16 = one 8-byte load per channel (c0 * 4 taps * 2 bytes is a multiple of 8)
-    float w[E][CONV_W];
+      for (int i = 0; i < (E + 1) / 2; ++i) m[j].w[i] = 0u;
+    }
+  }
+  float* gp = (u < a.H ? a.k2 : a.q2) + ((static_cast<int64_t>(b) * a.T + lo) * a.H + head) * E;
+  __nv_bfloat16* dyr = BWD ? a.dy + (static_cast<int64_t>(b) * a.T + lo) * a.dy_stride_t + u * E : nullptr;
+  GateRow<E> next = load_gate_row<E>(xb + lo * a.stride_t);
+  for (int t = lo; t < hi; ++t) {
+    const GateRow<E> x0 = next;
+    if (t + 1 < hi) next = load_gate_row<E>(xb + (t + 1) * a.stride_t);
+    float g[E];
+    if constexpr (BWD) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) g[e] = gp[e];
+    }
+    if (t >= doc.next) {
+      doc.advance(t);
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int i = 0; i < (E + 1) / 2; ++i) m[j].w[i] = 0u;
+    }
+    auto at = [](const GateRow<E>& r, int e) { return (e & 1) ? bf16_hi(r.w[e / 2]) : bf16_lo(r.w[e / 2]); };
+    float c[E], uu[E], ss = 0.f;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      const uint2 u2 = __ldg(reinterpret_cast<const uint2*>(a.weight + static_cast<int64_t>(c0 + e) * CONV_W));
-      w[e][0] = bf16_lo(u2.x); w[e][1] = bf16_hi(u2.x); w[e][2] = bf16_lo(u2.y); w[e][3] = bf16_hi(u2.y);
-    }
-#pragma unroll
-    for (int j = 0; j < CONV_W; ++j) {
-      const int tj = t - 3 + j;
-      if (tj < start) continue;
-      const __nv_bfloat16* xr = xb + tj * a.stride_t;
-      if constexpr (E % 4 == 0) {                       // rows and c0 are multiples of 4 channels: 8-byte loads
-#pragma unroll
-        for (int e = 0; e < E; e += 4) {
-          const uint2 u2 = __ldg(reinterpret_cast<const uint2*>(xr + e));
-          c[e] = fmaf(bf16_lo(u2.x), w[e][j], c[e]);
-          c[e + 1] = fmaf(bf16_hi(u2.x), w[e + 1][j], c[e + 1]);
-          c[e + 2] = fmaf(bf16_lo(u2.y), w[e + 2][j], c[e + 2]);
-          c[e + 3] = fmaf(bf16_hi(u2.y), w[e + 3][j], c[e + 3]);
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < E; ++e) c[e] = fmaf(__bfloat162float(xr[e]), w[e][j], c[e]);
-      }
-    }
-    float uu[E], ss = 0.f;
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
+      c[e] = fmaf(at(x0, e), w[e][3], fmaf(at(m[0], e), w[e][2], fmaf(at(m[1], e), w[e][1], at(m[2], e) * w[e][0])));
       uu[e] = c[e] > 15.f ? c[e] : __logf(1.f + __expf(c[e]));     // softplus; absolute error below 1e-7 at either end
       ss = fmaf(uu[e], uu[e], ss);
     }
     const float r = rsqrtf(ss + a.eps);
-    float* gp = (which == 0 ? a.k2 : a.q2) + ((static_cast<int64_t>(b) * a.T + t) * a.H + head) * E;
     if constexpr (!BWD) {
+      if (E % 4 == 0 && a.vec) {
 #pragma unroll
-      for (int e = 0; e < E; ++e) gp[e] = uu[e] * r;
+        for (int e = 0; e < E; e += 4) *reinterpret_cast<float4*>(gp + e) = make_float4(uu[e] * r, uu[e + 1] * r, uu[e + 2] * r, uu[e + 3] * r);
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) gp[e] = uu[e] * r;
+      }
     } else {
-      float g[E], dot = 0.f;
+      float dot = 0.f;
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        g[e] = gp[e];
-        dot = fmaf(uu[e], g[e], dot);
-      }
-      const float f = r * r * r * dot;
-      __nv_bfloat16* dyr = a.dy + (static_cast<int64_t>(b) * a.T + t) * a.C + c0;
+      for (int e = 0; e < E; ++e) dot = fmaf(uu[e], g[e], dot);
+      const float f = -r * r * r * dot;
+      float o[E];
 #pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const float du = fmaf(r, g[e], -f * uu[e]);
-        dyr[e] = __float2bfloat16_rn(du * fast_sigmoid(c[e]));      // d softplus = sigmoid
+      for (int e = 0; e < E; ++e) o[e] = fmaf(r, g[e], f * uu[e]) * fast_sigmoid(c[e]);     // d softplus = sigmoid
+      if constexpr (E % 4 == 0) {
+#pragma unroll
+        for (int e = 0; e < E; e += 4) *reinterpret_cast<uint2*>(dyr + e) = make_uint2(pack_bf16(o[e], o[e + 1]), pack_bf16(o[e + 2], o[e + 3]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < E; ++e) dyr[e] = __float2bfloat16_rn(o[e]);
       }
+      dyr += a.dy_stride_t;
     }
+    gp += static_cast<int64_t>(a.H) * E;
+    m[2] = m[1]; m[1] = m[0]; m[0] = x0;
   }
 }
 
@@ -900,40 +1355,41 @@ glue_gate_kernel(GlueArgs a, int B) {
 
 using namespace tgdn;
 
-template <bool BWD>
-static int glue_launch(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b,
-                       int64_t stride_t, int H, int E, float eps, void* q, void* k, void* v, float* k2, float* q2, void* dy,
-                       cudaStream_t s) {
-  if (!q || !k || !v || !k2 || !q2 || (BWD && !dy)) return TGDN_ERR_NULL;
-  int rc = conv_check(x, weight, q, cu, n_docs, B, T, C, stride_b, stride_t);
+static int glue_check(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b,
+                      int64_t stride_t, int H, int E, const void* q, const void* k, const void* v, const void* k2, const void* q2) {
+  if (!q || !k || !v || !k2 || !q2) return TGDN_ERR_NULL;
+  const int rc = conv_check_abi(x, weight, q, cu, n_docs, B, T, C, stride_b, stride_t);
   if (rc) return rc;
   if (H <= 0 || C != H * (3 * HEAD + 2 * E)) return TGDN_ERR_SHAPE;
-  if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(dy)) & 15) return TGDN_ERR_ALIGN;
-  if (!tgdn_check_device()) return TGDN_ERR_DEVICE;
-  CUtensorMap mx;
-  if ((rc = tgdn_make_rows_map(&mx, x, C, T, B, stride_t, stride_b, CONV_CH, CONV_FWD_ROWS))) return rc;
-  const int main_channels = 3 * H * HEAD;
-  int groups, tpg;
-  conv_groups(B, T, main_channels, 4, CONV_FWD_WAVES, &groups, &tpg);
-  GlueArgs a{static_cast<const __nv_bfloat16*>(weight), cu, n_docs, T, C, H, E, tpg, eps,
-             static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), static_cast<__nv_bfloat16*>(v), k2, q2,
-             static_cast<__nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stride_b, stride_t, tgdn_status_word()};
-  const int smem = CONV_FWD_STAGES * CONV_FWD_ROWS * CONV_CH * 2 + 128;
-  static bool configured[64] = {};
-  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(glue_main_kernel<BWD>), smem, configured))) return rc;
-  dim3 grid((main_channels + CONV_CH - 1) / CONV_CH, groups, B);
-  glue_main_kernel<BWD><<<grid, CONV_THREADS, smem, s>>>(mx, a);
-  if ((rc = tgdn_cuda_error(cudaGetLastError()))) return rc;
-  const int64_t n = static_cast<int64_t>(B) * T * 2 * H;
-  const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, static_cast<int64_t>(tgdn_sm_count()) * 16));
+  if (E != 1 && E != 2 && E != 4 && E != 8 && E != 12 && E != 16) return TGDN_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) return TGDN_ERR_ALIGN;
+  return tgdn_check_device() ? 0 : TGDN_ERR_DEVICE;
+}
+static RingArgs glue_args(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b,
+                          int64_t stride_t, int H, float eps, int runs) {
+  RingArgs a = ring_args(x, weight, cu, n_docs, B, T, C, stride_b, stride_t, runs);
+  a.units = 3 * H;                                       // one head of q, k or v each
+  a.n_warps = a.units * a.runs * B;
+  a.H = H;
+  a.eps = eps;
+  return a;
+}
+// Gate channels: runs of 32 tokens, shorter where that leaves the chip idle.
+template <bool BWD>
+static int gate_launch(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int64_t stride_b, int64_t stride_t,
+                       int H, int E, float eps, float* k2, float* q2, void* dy, int64_t dy_stride_t, cudaStream_t s) {
+  GateArgs g{static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(weight), cu, n_docs, B, T, H, 32, 0, stride_b, stride_t,
+             eps, k2, q2, static_cast<__nv_bfloat16*>(dy), dy_stride_t, ((reinterpret_cast<uintptr_t>(k2) | reinterpret_cast<uintptr_t>(q2)) & 15) == 0};
+  while (g.run > 8 && static_cast<int64_t>(2) * H * B * ((T + g.run - 1) / g.run) < static_cast<int64_t>(tgdn_sm_count()) * 256) g.run /= 2;
+  g.runs = (T + g.run - 1) / g.run;
+  const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(2) * H * B * g.runs + 127) / 128);
   switch (E) {
-    case 1: glue_gate_kernel<1, BWD><<<blocks, 256, 0, s>>>(a, B); break;
-    case 2: glue_gate_kernel<2, BWD><<<blocks, 256, 0, s>>>(a, B); break;
-    case 4: glue_gate_kernel<4, BWD><<<blocks, 256, 0, s>>>(a, B); break;
-    case 8: glue_gate_kernel<8, BWD><<<blocks, 256, 0, s>>>(a, B); break;
-    case 12: glue_gate_kernel<12, BWD><<<blocks, 256, 0, s>>>(a, B); break;
-    case 16: glue_gate_kernel<16, BWD><<<blocks, 256, 0, s>>>(a, B); break;
-    default: return TGDN_ERR_SHAPE;
+    case 1: glue_gate_kernel<1, BWD><<<blocks, 128, 0, s>>>(g); break;
+    case 2: glue_gate_kernel<2, BWD><<<blocks, 128, 0, s>>>(g); break;
+    case 4: glue_gate_kernel<4, BWD><<<blocks, 128, 0, s>>>(g); break;
+    case 8: glue_gate_kernel<8, BWD><<<blocks, 128, 0, s>>>(g); break;
+    case 12: glue_gate_kernel<12, BWD><<<blocks, 128, 0, s>>>(g); break;
+    default: glue_gate_kernel<16, BWD><<<blocks, 128, 0, s>>>(g); break;
   }
   return tgdn_cuda_error(cudaGetLastError());
 }
@@ -941,14 +1397,71 @@ static int glue_launch(const void* x, const void* weight, const int32_t* cu, int
 extern "C" int tgdn_glue_fwd(const void* x, const void* weight, const int32_t* cu_seqlens, int n_docs, int B, int T, int C,
                              int64_t stride_b, int64_t stride_t, int H, int E, float eps, void* q, void* k, void* v, float* k2,
                              float* q2, void* stream) {
-  return glue_launch<false>(x, weight, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, H, E, eps, q, k, v, k2, q2, nullptr,
-                            static_cast<cudaStream_t>(stream));
+  int rc = glue_check(x, weight, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, H, E, q, k, v, k2, q2);
+  if (rc) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  RingArgs a = glue_args(x, weight, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, H, eps, fwd_runs(B, T, 3 * H));
+  a.q = static_cast<__nv_bfloat16*>(q); a.k = static_cast<__nv_bfloat16*>(k); a.v = static_cast<__nv_bfloat16*>(v);
+  if ((rc = ring_fwd_launch<true>(a, B, s))) return rc;
+  return gate_launch<false>(x, weight, cu_seqlens, n_docs, B, T, stride_b, stride_t, H, E, eps, k2, q2, nullptr, 0, s);
+}
+
+static int glue_grad_maps(CUtensorMap* mg, const void* dq, const void* dk, const void* dv, int B, int T, int H) {
+  const void* g[3] = {dq, dk, dv};
+  for (int i = 0; i < 3; ++i)
+    if (const int rc = tgdn_make_token_map(&mg[i], g[i], B, T, H, 128, RING_ROWS, 0)) return rc;
+  return 0;
 }
 
 extern "C" int tgdn_glue_bwd_norm(const void* x, const void* weight, const int32_t* cu_seqlens, int n_docs, int B, int T, int C,
                                   int64_t stride_b, int64_t stride_t, int H, int E, float eps, const void* dq, const void* dk,
                                   const void* dv, const float* dk2, const float* dq2, void* dy, void* stream) {
-  return glue_launch<true>(x, weight, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, H, E, eps, const_cast<void*>(dq),
-                           const_cast<void*>(dk), const_cast<void*>(dv), const_cast<float*>(dk2), const_cast<float*>(dq2), dy,
-                           static_cast<cudaStream_t>(stream));
+  int rc = glue_check(x, weight, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, H, E, dq, dk, dv, dk2, dq2);
+  if (rc) return rc;
+  if (!dy) return TGDN_ERR_NULL;
+  if (reinterpret_cast<uintptr_t>(dy) & 15) return TGDN_ERR_ALIGN;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  RingArgs a = glue_args(x, weight, cu_seqlens, n_docs, B, T, C, stride_b, stride_t, H, eps, fwd_runs(B, T, 3 * H));
+  a.out = static_cast<__nv_bfloat16*>(dy);
+  CUtensorMap mx, mg[3];
+  if ((rc = glue_grad_maps(mg, dq, dk, dv, B, T, H))) return rc;
+  if ((rc = tgdn_make_rows_map(&mx, x, C, T, B, stride_t, stride_b, 128, RING_ROWS))) return rc;
+  static bool configured[64] = {};
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(glue_norm_kernel), RING_BWD_SMEM, configured))) return rc;
+  glue_norm_kernel<<<ring_grid(a), RING_WARPS * 32, RING_BWD_SMEM, s>>>(mx, mg[0], mg[1], mg[2], a);
+  if ((rc = tgdn_cuda_error(cudaGetLastError()))) return rc;
+  return gate_launch<true>(x, weight, cu_seqlens, n_docs, B, T, stride_b, stride_t, H, E, eps, const_cast<float*>(dk2), const_cast<float*>(dq2),
+                           static_cast<__nv_bfloat16*>(dy) + 3 * H * HEAD, C, s);
+}
+
+int tgdn_glue_bwd(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b, int64_t stride_t,
+                  int H, int E, float eps, const void* dq, const void* dk, const void* dv, const float* dk2, const float* dq2, void* dx,
+                  void* dw, void* dy_gates, void* scratch, int64_t scratch_bytes, void* stream) {
+  int rc = glue_check(x, weight, cu, n_docs, B, T, C, stride_b, stride_t, H, E, dq, dk, dv, dk2, dq2);
+  if (rc) return rc;
+  if (!dx || !dw || !dy_gates) return TGDN_ERR_NULL;
+  if ((reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(dy_gates)) & 15) return TGDN_ERR_ALIGN;
+  if (!scratch || (reinterpret_cast<uintptr_t>(scratch) & 15) || scratch_bytes < partial_bytes(B, 1, C)) return TGDN_ERR_SCRATCH;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int room = static_cast<int>(std::min<int64_t>(scratch_bytes / partial_bytes(B, 1, C), 1 << 20));
+  // q, k, v channels
+  RingArgs a = glue_args(x, weight, cu, n_docs, B, T, C, stride_b, stride_t, H, eps, std::min(room, bwd_runs(B, T, 3 * H)));
+  a.out = static_cast<__nv_bfloat16*>(dx);
+  a.dw_partial = static_cast<float*>(scratch);
+  CUtensorMap mg[3];
+  if ((rc = glue_grad_maps(mg, dq, dk, dv, B, T, H))) return rc;
+  if ((rc = ring_bwd_launch<true>(a, B, mg, s))) return rc;
+  // gate channels: the gradient of the convolution's output, then a plain backward over the same runs
+  const int G = 2 * H * E, c0 = 3 * H * HEAD;
+  if ((rc = gate_launch<true>(x, weight, cu, n_docs, B, T, stride_b, stride_t, H, E, eps, const_cast<float*>(dk2), const_cast<float*>(dq2),
+                              dy_gates, G, s)))
+    return rc;
+  RingArgs g = ring_args(a.x + c0, a.weight + static_cast<int64_t>(c0) * CONV_W, cu, n_docs, B, T, G, stride_b, stride_t, a.runs);
+  g.run = a.run; g.runs = a.runs; g.n_warps = g.units * g.runs * B;
+  g.out = a.out + c0;
+  g.out_stride_b = a.out_stride_b; g.out_stride_t = a.out_stride_t;
+  g.dw_partial = a.dw_partial; g.dw_channels = C; g.dw_c0 = c0;
+  if ((rc = tgdn_make_rows_map(&mg[0], dy_gates, G, T, B, G, static_cast<int64_t>(T) * G, 128, RING_ROWS))) return rc;
+  if ((rc = ring_bwd_launch<false>(g, B, mg, s))) return rc;
+  return reduce_dw_launch(a.dw_partial, dw, B * a.runs, C, s);
 }

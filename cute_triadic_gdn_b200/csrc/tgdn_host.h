@@ -58,3 +58,19 @@ int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const voi
                          const float* dc, const float* dd, const float* dr, float scale, const int32_t* chunk_map, int B, int T,
                          int H, int E, int NC, int row_tokens, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
                          void* stream);
+
+// The convolution for any channel count, strides and 2-byte aligned rows (weight: 8-byte aligned); the entry points of the public ABI
+// are these for whole 16-byte pieces.  The backward uses as many weight-gradient partials as the scratch holds, up to
+// tgdn_conv_bwd_best_scratch.
+int tgdn_conv_fwd_any(const void* x, const void* weight, void* y, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b,
+                      int64_t stride_t, int act_channels, void* stream);
+int tgdn_conv_bwd_any(const void* x, const void* weight, const void* dy, void* dx, void* dw, const int32_t* cu, int n_docs, int B, int T,
+                      int C, int64_t stride_b, int64_t stride_t, int64_t dy_stride_b, int64_t dy_stride_t, int act_channels,
+                      void* scratch, int64_t scratch_bytes, void* stream);
+int64_t tgdn_conv_bwd_best_scratch(int B, int T, int C);
+
+// The whole backward of tgdn_glue_fwd: from the gradients of q, k, v, k2, q2 to dx (B, T, C) and dw (C, 4) without the gradient of the
+// convolution's output in between (except for the gate channels: dy_gates, bf16 (B, T, 2 H E)).  scratch as for the convolution.
+int tgdn_glue_bwd(const void* x, const void* weight, const int32_t* cu, int n_docs, int B, int T, int C, int64_t stride_b, int64_t stride_t,
+                  int H, int E, float eps, const void* dq, const void* dk, const void* dv, const float* dk2, const float* dq2, void* dx,
+                  void* dw, void* dy_gates, void* scratch, int64_t scratch_bytes, void* stream);

@@ -587,28 +587,25 @@ Tensor decode(Tensor q, Tensor k, Tensor v, Tensor k2, Tensor q2, Tensor g, Tens
 struct ConvInput {
   Tensor x, weight, cu;
   int n_docs = 0;
-  int64_t pad = 0;                                        // zero channels added so that the kernels' row length is a multiple of 8
 };
 
-bool rows_aligned(const Tensor& t) {
-  return t.stride(2) == 1 && t.stride(1) % 8 == 0 && t.stride(0) % 8 == 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
-}
+bool aligned(const Tensor& t, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % bytes == 0; }
+bool rows_aligned(const Tensor& t) { return t.stride(2) == 1 && t.stride(1) % 8 == 0 && t.stride(0) % 8 == 0 && aligned(t, 16); }
+// Rows of consecutive channels that do not overlap: what the kernels read in place.
+bool rows_readable(const Tensor& t) { return t.stride(2) == 1 && t.stride(1) >= t.size(2); }
 
-ConvInput conv_prep(const Tensor& x, const Tensor& weight, const OptTensor& cu) {
+// `pieces`: the rows must be whole 16-byte pieces (the fused kernels); otherwise any readable row will do.
+ConvInput conv_prep(const Tensor& x, const Tensor& weight, const OptTensor& cu, bool pieces = false) {
   TORCH_CHECK_VALUE(x.dim() == 3 && weight.dim() == 2 && weight.size(0) == x.size(2) && weight.size(1) == 4,
                     "x must be (B, T, C) and weight (C, 4)");
   TORCH_CHECK_VALUE(x.scalar_type() == at::kBFloat16, "x must be bf16");
   TORCH_CHECK_VALUE(x.is_cuda() && weight.device() == x.device(), "x and weight must be on the same CUDA device");
   ConvInput c;
   c.x = x;
-  c.weight = weight.to(at::kBFloat16);
-  c.pad = (8 - x.size(2) % 8) % 8;
-  if (c.pad) {
-    c.x = at::constant_pad_nd(c.x, {0, c.pad});
-    c.weight = at::constant_pad_nd(c.weight, {0, 0, 0, c.pad});
-  }
-  c.weight = c.weight.contiguous();
-  if (!rows_aligned(c.x)) c.x = c.x.contiguous();
+  if (!rows_readable(c.x)) c.x = c.x.contiguous();
+  if (pieces && !rows_aligned(c.x)) c.x = c.x.clone(at::MemoryFormat::Contiguous);
+  c.weight = weight.to(at::kBFloat16).contiguous();
+  if (!aligned(c.weight, 16)) c.weight = c.weight.clone();
   if (has(cu)) {
     TORCH_CHECK_VALUE(c.x.size(0) == 1, "cu_seqlens requires a packed row: B=1");
     TORCH_CHECK_VALUE(cu->dim() == 1 && cu->numel() >= 2 && cu->device() == x.device(),
@@ -624,30 +621,24 @@ Tensor conv_fwd(const Tensor& x, const Tensor& weight, int64_t act_channels, con
   ConvInput c = conv_prep(x, weight, cu);
   const int64_t B = c.x.size(0), T = c.x.size(1), C = c.x.size(2);
   Tensor y = empty({B, T, C}, c.x, at::kBFloat16);
-  check_rc(tgdn_conv_fwd(ptr(c.x), ptr(c.weight), ptr(y), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T),
-                         static_cast<int>(C), c.x.stride(0), c.x.stride(1), static_cast<int>(act_channels), stream_of(c.x)),
+  check_rc(tgdn_conv_fwd_any(ptr(c.x), ptr(c.weight), ptr(y), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T),
+                             static_cast<int>(C), c.x.stride(0), c.x.stride(1), static_cast<int>(act_channels), stream_of(c.x)),
            "tgdn_conv_fwd");
-  return c.pad ? y.narrow(2, 0, C - c.pad).contiguous() : y;
+  return y;
 }
 
 std::tuple<Tensor, Tensor> conv_bwd(const Tensor& x, const Tensor& dy_in, const Tensor& weight, int64_t act_channels, const OptTensor& cu) {
   const c10::cuda::OptionalCUDAGuard guard(x.is_cuda() ? std::optional<c10::Device>(x.device()) : std::nullopt);
   ConvInput c = conv_prep(x, weight, cu);
-  Tensor dy = dy_in;
-  if (c.pad) dy = at::constant_pad_nd(dy, {0, c.pad});
-  if (!rows_aligned(dy)) dy = dy.contiguous();
+  const Tensor dy = rows_readable(dy_in) ? dy_in : dy_in.contiguous();
   const int64_t B = c.x.size(0), T = c.x.size(1), C = c.x.size(2);
   Tensor dx = empty({B, T, C}, c.x, at::kBFloat16), dw = empty({C, 4}, c.x, at::kBFloat16);
-  const int64_t nbytes = tgdn_conv_bwd_scratch_bytes(static_cast<int>(B), static_cast<int>(T), static_cast<int>(C));
+  const int64_t nbytes = tgdn_conv_bwd_best_scratch(static_cast<int>(B), static_cast<int>(T), static_cast<int>(C));
   Tensor scratch = empty({nbytes / 4}, c.x, at::kFloat);
-  check_rc(tgdn_conv_bwd(ptr(c.x), ptr(c.weight), ptr(dy), ptr(dx), ptr(dw), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B),
-                         static_cast<int>(T), static_cast<int>(C), c.x.stride(0), c.x.stride(1), dy.stride(0), dy.stride(1),
-                         static_cast<int>(act_channels), ptr(scratch), nbytes, stream_of(c.x)),
+  check_rc(tgdn_conv_bwd_any(ptr(c.x), ptr(c.weight), ptr(dy), ptr(dx), ptr(dw), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B),
+                             static_cast<int>(T), static_cast<int>(C), c.x.stride(0), c.x.stride(1), dy.stride(0), dy.stride(1),
+                             static_cast<int>(act_channels), ptr(scratch), nbytes, stream_of(c.x)),
            "tgdn_conv_bwd");
-  if (c.pad) {
-    dx = dx.narrow(2, 0, C - c.pad).contiguous();
-    dw = dw.narrow(0, 0, C - c.pad).contiguous();
-  }
   return {dx, dw.to(weight.scalar_type())};
 }
 
@@ -663,7 +654,7 @@ void glue_dims(const Tensor& x, int64_t H, int64_t E) {
 Five norm_fwd(const Tensor& x, const Tensor& weight, int64_t heads, int64_t slices, double eps, const OptTensor& cu) {
   const c10::cuda::OptionalCUDAGuard guard(x.is_cuda() ? std::optional<c10::Device>(x.device()) : std::nullopt);
   glue_dims(x, heads, slices);
-  ConvInput c = conv_prep(x, weight, cu);
+  ConvInput c = conv_prep(x, weight, cu, true);
   const int64_t B = c.x.size(0), T = c.x.size(1), C = c.x.size(2);
   Tensor q = empty({B, T, heads, 128}, x, at::kBFloat16), k = empty({B, T, heads, 128}, x, at::kBFloat16),
          v = empty({B, T, heads, 128}, x, at::kBFloat16), k2 = empty({B, T, heads, slices}, x, at::kFloat),
@@ -678,17 +669,20 @@ Five norm_fwd(const Tensor& x, const Tensor& weight, int64_t heads, int64_t slic
 std::tuple<Tensor, Tensor> norm_bwd(const Tensor& x, const Tensor& weight, const Tensor& dq, const Tensor& dk, const Tensor& dv,
                                     const Tensor& dk2, const Tensor& dq2, int64_t heads, int64_t slices, double eps, const OptTensor& cu) {
   const c10::cuda::OptionalCUDAGuard guard(x.is_cuda() ? std::optional<c10::Device>(x.device()) : std::nullopt);
-  ConvInput c = conv_prep(x, weight, cu);
+  glue_dims(x, heads, slices);
+  ConvInput c = conv_prep(x, weight, cu, true);
   const int64_t B = c.x.size(0), T = c.x.size(1), C = c.x.size(2);
   auto bf = [](const Tensor& t) { return t.to(at::kBFloat16).contiguous(); };
   auto f32 = [](const Tensor& t) { return t.to(at::kFloat).contiguous(); };
   const Tensor q = bf(dq), k = bf(dk), v = bf(dv), k2 = f32(dk2), q2 = f32(dq2);
-  Tensor dy = empty({B, T, C}, c.x, at::kBFloat16);
-  check_rc(tgdn_glue_bwd_norm(ptr(c.x), ptr(c.weight), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T),
-                              static_cast<int>(C), c.x.stride(0), c.x.stride(1), static_cast<int>(heads), static_cast<int>(slices),
-                              static_cast<float>(eps), ptr(q), ptr(k), ptr(v), fptr(k2), fptr(q2), ptr(dy), stream_of(c.x)),
-           "tgdn_glue_bwd_norm");
-  auto [dx, dw] = conv_bwd(c.x, dy, c.weight, 3 * heads * 128, or_nullopt(c.cu));
+  Tensor dx = empty({B, T, C}, c.x, at::kBFloat16), dw = empty({C, 4}, c.x, at::kBFloat16);
+  Tensor dy_gates = empty({B, T, 2 * heads * slices}, c.x, at::kBFloat16);
+  const int64_t nbytes = tgdn_conv_bwd_best_scratch(static_cast<int>(B), static_cast<int>(T), static_cast<int>(C));
+  Tensor scratch = empty({nbytes / 4}, c.x, at::kFloat);
+  check_rc(tgdn_glue_bwd(ptr(c.x), ptr(c.weight), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T), static_cast<int>(C),
+                         c.x.stride(0), c.x.stride(1), static_cast<int>(heads), static_cast<int>(slices), static_cast<float>(eps), ptr(q),
+                         ptr(k), ptr(v), fptr(k2), fptr(q2), ptr(dx), ptr(dw), ptr(dy_gates), ptr(scratch), nbytes, stream_of(c.x)),
+           "tgdn_glue_bwd");
   return {dx, dw.to(weight.scalar_type())};
 }
 

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from cute_triadic_gdn_b200 import _lib, chunk_gdn_joint, gdn_joint_call
+from cute_triadic_gdn_b200 import _lib, chunk_gdn_joint, conv_split_act_call, gdn_joint_call
 from oracle import triadic_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -31,3 +31,33 @@ def test_wide_value_blocks_of_the_forward(E, docs):
             o1, s1 = chunk_gdn_joint(*[t[:, :64].contiguous() for t in ins], output_final_state=True)
             o2, s2 = chunk_gdn_joint(*[t[:, 64:].contiguous() for t in ins], initial_state=s1, output_final_state=True)
         assert torch.equal(torch.cat([o1, o2], 1), o.detach()) and torch.equal(s2, s_all)
+
+
+@pytest.mark.parametrize("B,T,C,act,docs", [
+    (2, 37, 1930, 1920, None),                         # 4-byte rows
+    (1, 150, 77, 40, [0, 1, 3, 64, 65, 150]),          # 2-byte rows, SiLU ends inside a warp's channels
+    (1, 130, 516, 516, [0, 127, 128, 130]),            # 8-byte rows
+    (1, 3, 130, 0, None),
+    (1, 777, 264, 100, [0, 2, 48, 49, 95, 96, 97, 700, 777]),   # whole 16-byte pieces, documents that start at the edges of runs
+    (3, 97, 128, 128, None),
+])
+def test_convolution_rows_of_every_alignment(B, T, C, act, docs):
+    g = torch.Generator().manual_seed(T + C)
+    x = torch.randn(B, T, C, generator=g).to(torch.bfloat16)
+    w = (0.5 * torch.randn(C, 4, generator=g)).to(torch.bfloat16)
+    dy = torch.randn(B, T, C, generator=g).to(torch.bfloat16)
+    cu = torch.tensor(docs, dtype=torch.int32) if docs else None
+    y_ref = orc.conv_reference(x, w, act, cu)
+    dx_ref, dw_ref = orc.conv_reference_backward(x, w, act, dy, cu)
+    wide = torch.zeros(B, T, C + 3, dtype=torch.bfloat16, device="cuda")
+    wide[..., 1:C + 1] = x.cuda()
+    outs = []
+    for xg in (x.cuda(), wide[..., 1:C + 1]):          # contiguous, and rows of a wider tensor at an odd address
+        xg, wg = xg.detach().requires_grad_(True), w.cuda().requires_grad_(True)
+        y = conv_split_act_call(xg, wg, act, None if cu is None else cu.cuda())
+        outs.append((y.detach(), *torch.autograd.grad(y, (xg, wg), dy.cuda())))
+        assert _lib.device_status() == 0
+        assert orc.rel_l2(outs[-1][0].float().cpu(), y_ref.float()) < 2e-3
+        assert orc.rel_l2(outs[-1][1].float().cpu(), dx_ref.float()) < 4e-3
+        assert orc.rel_l2(outs[-1][2].float().cpu(), dw_ref.float()) < 8e-3
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
