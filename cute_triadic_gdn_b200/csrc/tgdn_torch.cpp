@@ -178,12 +178,12 @@ struct Reverse { Tensor dV, dU, ds, dkg, dr; };
 // no document uses are neither written here nor read by the later stages.
 Reverse run_reverse(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& k2, const Tensor& q2, const Tensor& beta,
                     const Tensor& gc, const Tensor& AP, const Tensor& Pm, const Tensor& U, double scale, const OptTensor& chunk_starts,
-                    const OptTensor& token_map, const OptTensor& grad_state_in, const OptTensor& grad_state_out, Tensor dV = Tensor()) {
+                    const OptTensor& token_map, const OptTensor& grad_state_in, const OptTensor& grad_state_out) {
   const c10::cuda::CUDAGuard guard(q.device());
   const Dims d = dims(q, k2, token_map, chunk_starts);
   const int64_t NV = value_blocks(d.E);
   Reverse r;
-  r.dV = dV.defined() ? dV : empty(dO.sizes(), dO, at::kBFloat16);
+  r.dV = empty(dO.sizes(), dO, at::kBFloat16);
   r.dU = empty({d.B, d.NC, d.H, CHUNK, 128}, q, at::kBFloat16);
   r.ds = empty({d.B, d.NC, d.H, d.E, 16, 128, 8}, q, at::kBFloat16);
   r.dkg = empty({d.B, d.NC, d.H, NV, 8, 128, 8}, q, at::kBFloat16);    // image [token / 8][key row][token % 8] per value block
@@ -254,11 +254,32 @@ void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tens
     AP = m.AP;
     Pm = m.Pm;
   }
-  Reverse r = run_reverse(q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, chunk_starts, token_map, grad_state_in, grad_state_out, out.v);
-  StateGrads s = run_state_grads(q, k, dO, r.dV, h, r.ds, r.dkg, k2, q2, gc, scale, token_map);
-  r.ds.reset();
-  r.dkg.reset();
-  run_matrix(q, k, dO, r.dU, W, U, AP, k2, q2, beta, gc, s, r.dr, scale, token_map, out);
+  // What travels between the three kernels, in two allocations (the first one, by far the larger, is given back before the last
+  // kernel's temporaries matter).
+  const c10::cuda::CUDAGuard guard(q.device());
+  const Dims d = dims(q, k2, token_map, chunk_starts);
+  const int64_t items = static_cast<int64_t>(d.B) * d.NC * d.H, NV = value_blocks(d.E);
+  const float sc = static_cast<float>(scale);
+  const int32_t *starts = ptr<int32_t>(chunk_starts), *map = ptr<int32_t>(token_map);
+  void* stream = stream_of(q);
+  Tensor big = empty({items * (d.E * 32768 + NV * 16384)}, q, at::kByte);              // ds, dkg
+  Tensor small = empty({items * (16384 + 32768 + (NV + 2) * 64 * d.E * 4 + d.E * 4)}, q, at::kByte);   // dU, dkq, dr, da, dc, dd
+  uint8_t *ds = ptr<uint8_t>(big), *dkg = ds + items * d.E * 32768;
+  uint8_t *dU = ptr<uint8_t>(small), *dkq = dU + items * 16384;
+  float *dr = reinterpret_cast<float*>(dkq + items * 32768), *da = dr + items * NV * 64 * d.E, *dc = da + items * 64 * d.E,
+        *dd = dc + items * 64 * d.E;
+  check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U), sc, starts, map,
+                                   d.n_docs, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, ptr(out.v), dU, ds, dkg, dr, ptr<float>(grad_state_in),
+                                   ptr<float>(grad_state_out), stream),
+           "tgdn_bwd_recurrent");
+  check_rc(tgdn_bwd_state_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(out.v), ptr(h), ds, dkg, fptr(k2), fptr(q2), fptr(gc), sc, map, d.B, d.T, d.H,
+                                     d.E, d.NC, d.row_tokens, dkq, da, dc, dd, stream),
+           "tgdn_bwd_state_grads");
+  big.reset();
+  check_rc(tgdn_bwd_matrix_rows(ptr(q), ptr(k), ptr(dO), dU, ptr(W), ptr(U), ptr(AP), fptr(k2), fptr(q2), fptr(beta), fptr(gc), dkq, da, dc, dd, dr,
+                                sc, map, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2),
+                                ptr<float>(out.g), ptr<float>(out.beta), stream),
+           "tgdn_bwd_matrix");
 }
 
 // ---- operators of the core --------------------------------------------------------------------------------------------
