@@ -118,7 +118,7 @@ struct FwdCtrl {
   int abort;
 };
 
-template <int E, int CW, int NCH, int WPC, int STAGES, int MINB>
+template <int E, int CW, int NCH, int WPC, int STAGES, int MINB, bool PACKED>
 __global__ void __launch_bounds__(NCH * WPC * 128, MINB)
 fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_beta,
            const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
@@ -152,7 +152,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
   constexpr int NV = HEAD / VC;
   const int vb = blockIdx.x % NV, h = (blockIdx.x / NV) % p.H, seq_rank = blockIdx.x / (NV * p.H);
   int b = seq_rank, first = 0, count = p.NC, seq = seq_rank;
-  if (p.cmap != nullptr) {
+  if constexpr (PACKED) {
     const int doc = p.cmap[2 * p.NC + seq_rank];    // longest documents first
     if (doc < 0 || doc >= p.n_seq) return;
     b = 0;
@@ -222,7 +222,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
 
   auto chunk_info = [&](int i, int& t0, int& rows) {
     const int n = first + i;
-    if (p.cmap != nullptr) { t0 = p.cmap[n]; rows = p.cmap[p.NC + n]; } else { t0 = n * CHUNK; rows = CHUNK; }
+    t0 = n * CHUNK;
+    rows = CHUNK;
+    if constexpr (!PACKED) return;                  // dense rows hold whole chunks
+    t0 = p.cmap[n];
+    rows = p.cmap[p.NC + n];
     if (t0 < 0 || rows < 0 || rows > CHUNK || t0 + rows > p.T) {
       atomicCAS(p.status, DEV_OK, DEV_BAD_CHUNK_MAP);
       t0 = 0; rows = 0;
@@ -277,15 +281,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
   }
   if (count > 1) prefetch_rows(1);
   uint32_t mma_phase = 0;
+  int t0_next = 0, rows_next = CHUNK;               // packed rows: the chunk's place is looked up a chunk ahead
+  if constexpr (PACKED) chunk_info(0, t0_next, rows_next);
 
   for (int i = 0; i < count; ++i) {
     const int st = i % STAGES;
-    int t0, rows;
-    chunk_info(i, t0, rows);
-    const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
-    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
-    const bool live = t < rows;
-    const bool o_tile = rows == CHUNK;               // a chunk cut short by a document end cannot leave as a tile
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     uint8_t* ap = smem + C::OFF_AP + st * C::AP_BYTES;
 
@@ -305,6 +305,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       umma_commit(&ctrl.bar_mma[chain]);
     }
     __syncwarp();                                    // the other lanes must not run ahead into a spin wait
+    const int t0 = PACKED ? t0_next : (first + i) * CHUNK, rows = PACKED ? rows_next : CHUNK;
+    const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
+    const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
+    const bool live = t < rows;
+    const bool o_tile = rows == CHUNK;               // a chunk cut short by a document end cannot leave as a tile
     // The chain finished with the previous chunk's tiles when its third MMA group completed.  It says so now, under this
     // MMA, where its warps have time to spare; the last chain to say so refills that stage with the chunk STAGES ahead.
     // (o left from the stage's value rows, W and U from the place of beta*W: the stores must have read them.)
@@ -438,6 +443,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     if (CW == 8 && p.W != nullptr && cwarp_u == REFILL_WARP && elect_one())
       tma_store_4d(&map_w, bw_img + 1024, v0g, 0, static_cast<int>(item) * 64, 0);
     __syncwarp();
+    if (PACKED && i + 1 < count) chunk_info(i + 1, t0_next, rows_next);
     if constexpr (LATE_R) {                          // r_e only now, from the stage: sixteen registers fewer are live
       if (krow) lds_part<ET>(gf + C::GF_R + t * E + e0, gr);   // through the epilogue of (1)
     }
@@ -558,15 +564,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
 
 using namespace tgdn;
 
-template <int E, int CW, int NCH, int WPC, int STAGES, int MINB>
-static int launch_fwd(const CUtensorMap& mk, const CUtensorMap& mq, const void* v, const FwdParams& p, cudaStream_t s) {
+template <int E, int CW, int NCH, int WPC, int STAGES, int MINB, bool PACKED>
+static int launch_fwd_rows(const CUtensorMap& mk, const CUtensorMap& mq, const void* v, const FwdParams& p, cudaStream_t s) {
   int rc;
   using C = FwdCfg<E, CW, NCH, WPC, STAGES>;
   static_assert(MINB == 1 || C::SMEM_BYTES <= 115712, "two CTAs per SM need at most 113 KB each");
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static_assert(MINB * C::TMEM_COLS <= 512, "tensor memory budget of one SM exceeded");
   static bool configured[64] = {};
-  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(fwd_kernel<E, CW, NCH, WPC, STAGES, MINB>), C::SMEM_BYTES, configured)))
+  if ((rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(fwd_kernel<E, CW, NCH, WPC, STAGES, MINB, PACKED>), C::SMEM_BYTES, configured)))
     return rc;
   CUtensorMap mv, mo, mb = mk, mw = mk, mu = mk;    // placeholders where a tensor is not loaded or stored by TMA
   if ((rc = tgdn_make_token_map(&mv, v, p.B, p.T, p.H, CW, 64, 0, p.TS))) return rc;
@@ -580,10 +586,16 @@ static int launch_fwd(const CUtensorMap& mk, const CUtensorMap& mq, const void* 
   if (p.W != nullptr && (rc = tgdn_make_token_map(&mw, p.W, 1, static_cast<int>(crows), 1, CW, 64, 0))) return rc;
   if (p.U != nullptr && (rc = tgdn_make_token_map(&mu, p.U, 1, static_cast<int>(crows), 1, 8, 64, 0))) return rc;
   const int grid = p.n_seq * p.H * (HEAD / C::VC);
-  fwd_kernel<E, CW, NCH, WPC, STAGES, MINB><<<grid, C::THREADS, C::SMEM_BYTES, s>>>(mv, mb, mk, mq, mo, mw, mu, p);
+  fwd_kernel<E, CW, NCH, WPC, STAGES, MINB, PACKED><<<grid, C::THREADS, C::SMEM_BYTES, s>>>(mv, mb, mk, mq, mo, mw, mu, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 
+
+template <int E, int CW, int NCH, int WPC, int STAGES, int MINB>
+static int launch_fwd(const CUtensorMap& mk, const CUtensorMap& mq, const void* v, const FwdParams& p, cudaStream_t s) {
+  return p.cmap != nullptr ? launch_fwd_rows<E, CW, NCH, WPC, STAGES, MINB, true>(mk, mq, v, p, s)
+                           : launch_fwd_rows<E, CW, NCH, WPC, STAGES, MINB, false>(mk, mq, v, p, s);
+}
 
 int tgdn_fwd_rows(const void* q, const void* k, const void* v, const float* k2, const float* q2, const float* beta, const float* gc,
                   const void* AP, float scale, const int32_t* doc_offsets, const int32_t* chunk_map, int n_docs, int B, int T, int H,

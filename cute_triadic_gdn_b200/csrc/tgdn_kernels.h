@@ -139,6 +139,4 @@ struct MatParams {
 
 // E in {1,2,4,8,12,16}; dense rows need T % 64 == 0 and NC == T/64; packed rows need B == 1.
 int tgdn_check_core_shape(int B, int T, int H, int E, int NC, int packed, int row_tokens);
-// Width of the value-axis block one CTA of the recurrences owns, by E.
-int tgdn_value_block(int E);
 int tgdn_sm_count();
