@@ -32,10 +32,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// 64x64 f32 matrix in shared memory, column index XOR-swizzled with the row so that both "lanes along a row" and
-// "lanes along a column" accesses are conflict-free.
-__device__ __forceinline__ int mat_idx(int i, int j) { return i * 64 + (j ^ (i & 31)); }
-__device__ __forceinline__ int t_idx(int k, int j) { return k * 32 + ((j ^ k) & 31); }
+// 64x64 f32 matrix in shared memory with rows 68 floats apart: whole rows are read and written in 16-byte pieces by 32 lanes on 32
+// rows without bank conflicts, and so are the A fragments of the merges (8 rows x 4 columns; the B fragments meet twice).
+constexpr int MAT_LD = 68, T_LD = 36;
+__device__ __forceinline__ int mat_idx(int i, int j) { return i * MAT_LD + j; }
+__device__ __forceinline__ int t_idx(int k, int j) { return k * T_LD + j; }
 __device__ __forceinline__ void st_shared_b16(uint32_t saddr, float v) {      // v is a bf16 value held as f32
   const unsigned short b = __bfloat16_as_ushort(__float2bfloat16_rn(v));
   asm volatile("st.shared.b16 [%0], %1;" ::"r"(saddr), "h"(b) : "memory");
@@ -52,7 +53,7 @@ __device__ __forceinline__ void mma_tf32(float* c, const uint32_t* a, const uint
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// c (16x8 tile, standard fragment) += A(16x8) B(8x8) with A(i,k), B(k,j) given as element functors
+// c[0..3] (large terms) and c[4..7] (small terms), 16x8 tiles in standard fragments, += A(16x8) B(8x8) with A(i,k), B(k,j) given as element functors
 template <typename FA, typename FB>
 __device__ __forceinline__ void mma_step_3x(float* c, FA a_at, FB b_at, int lane) {
   const int gid = lane >> 2, tig = lane & 3;
@@ -63,8 +64,8 @@ __device__ __forceinline__ void mma_step_3x(float* c, FA a_at, FB b_at, int lane
   tf32_split(a_at(gid + 8, tig + 4), ah[3], al[3]);
   tf32_split(b_at(tig, gid), bh[0], bl[0]);
   tf32_split(b_at(tig + 4, gid), bh[1], bl[1]);
-  mma_tf32(c, al, bh);
-  mma_tf32(c, ah, bl);
+  mma_tf32(c + 4, al, bh);                                // the small terms apart: two accumulation chains instead of one of thrice the length
+  mma_tf32(c + 4, ah, bl);
   mma_tf32(c, ah, bh);
 }
 
@@ -73,11 +74,11 @@ struct MaskSmem {
   // KQ tile (two 64-column blocks of 128 rows x 128 B) while the Gram product runs; L and X afterwards
   union {
     uint8_t kq[32768];
-    struct { float L[4096]; float X[4096]; } m;
+    struct { float L[64 * MAT_LD]; float X[64 * MAT_LD]; } m;
   } u;
-  float Pm[4096];
-  float T[1024];
+  alignas(16) float T[32 * T_LD];
   uint8_t img_ap[16384];   // [A; PA] image (i = row 0..127, j = column), SI = 128, SJ = 2048
+  uint8_t gpad[E > 8 ? 12288 : 16];   // room for the G images at twelve and sixteen slices
   uint8_t img_pm[8192];    // Pm image (i = t, j = s), SI = 128, SJ = 1024; read as 128 rows by the PA product: keep >= 8 KB behind it
   float gc2[64 * E];       // log2-domain cumulative gate
   float k2[64 * E];
@@ -89,13 +90,13 @@ struct MaskSmem {
   int abort;
   int steep;               // a 16-row block decays by more than 2^-100 (or gc is not monotone): direct decay path
   // Operands of the mask-sum products (see the kernel), in buffers that are written only after those products are done:
-  //   G images: four blocks of (128 rows x KP) bf16, image (i = row, j = k), SI = 128, SJ = 2048, over Pm, T, img_ap
+  //   G images: four blocks of (128 rows x KP) bf16, image (i = row, j = k), SI = 128, SJ = 2048, over T, img_ap, gpad
   //   H images: two of (64 rows x KP) bf16, image (i = s, j = k), SI = 128, SJ = 1024, over img_pm
   static constexpr int KP = 2 * E <= 16 ? 16 : 32;         // [hi | lo] halves of the E factors, padded to the MMA's K = 16
   static constexpr int G_BYTES = KP / 8 * 2048, H_BYTES = KP / 8 * 1024;
-  __device__ uint8_t* img_g() { return reinterpret_cast<uint8_t*>(Pm); }
+  __device__ uint8_t* img_g() { return reinterpret_cast<uint8_t*>(T); }
   __device__ uint8_t* img_h() { return img_pm; }
-  static_assert(4 * G_BYTES <= 16384 + 4096 + 16384 && 2 * H_BYTES <= 8192, "operand images fit the buffers they borrow");
+  static_assert(4 * G_BYTES <= static_cast<int>(sizeof(T) + sizeof(img_ap) + sizeof(gpad)) && 2 * H_BYTES <= 8192, "operand images fit the buffers they borrow");
 };
 
 // X21 = -X22 (L21 X11) for the diagonal blocks of size 2n (n = 16: two blocks, n = 32: one), one 16x8 tile per warp.
@@ -105,12 +106,14 @@ __device__ __forceinline__ void tri_merge_mma(const float* L, float* X, float* T
   const int gid = lane >> 2, tig = lane & 3;
   const int m = warp / (MT * NT), mt = (warp / NT) % MT, nt = warp % NT, r = m * 2 * N;
   if (warp < TASKS) {
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    float c[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int kb = nt; kb < NT; ++kb)                           // X11 is lower triangular: rows k < column block are zero
       mma_step_3x(c,
                   [&](int i, int k) { return L[mat_idx(r + N + 16 * mt + i, r + 8 * kb + k)]; },
                   [&](int k, int j) { return X[mat_idx(r + 8 * kb + k, r + 8 * nt + j)]; }, lane);
-    float* Tm = T + m * 512;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += c[4 + i];
+    float* Tm = T + m * 16 * T_LD;
     Tm[t_idx(16 * mt + gid, 8 * nt + 2 * tig)] = c[0];
     Tm[t_idx(16 * mt + gid, 8 * nt + 2 * tig + 1)] = c[1];
     Tm[t_idx(16 * mt + gid + 8, 8 * nt + 2 * tig)] = c[2];
@@ -118,12 +121,14 @@ __device__ __forceinline__ void tri_merge_mma(const float* L, float* X, float* T
   }
   __syncthreads();
   if (warp < TASKS) {
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
-    const float* Tm = T + m * 512;
+    float c[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const float* Tm = T + m * 16 * T_LD;
     for (int kb = 0; kb <= 2 * mt + 1; ++kb)                   // X22 is lower triangular: columns k > row block are zero
       mma_step_3x(c,
                   [&](int i, int k) { return X[mat_idx(r + N + 16 * mt + i, r + N + 8 * kb + k)]; },
                   [&](int k, int j) { return Tm[t_idx(8 * kb + k, 8 * nt + j)]; }, lane);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += c[4 + i];
     X[mat_idx(r + N + 16 * mt + gid, r + 8 * nt + 2 * tig)] = -c[0];
     X[mat_idx(r + N + 16 * mt + gid, r + 8 * nt + 2 * tig + 1)] = -c[1];
     X[mat_idx(r + N + 16 * mt + gid + 8, r + 8 * nt + 2 * tig)] = -c[2];
@@ -133,7 +138,7 @@ __device__ __forceinline__ void tri_merge_mma(const float* L, float* X, float* T
 }
 
 template <int E>
-__global__ void __launch_bounds__(MASK_THREADS, 2)
+__global__ void __launch_bounds__(MASK_THREADS, E > 8 ? 2 : 3)
 masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q, MaskParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using SM = MaskSmem<E>;
@@ -318,11 +323,24 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   __syncwarp();                                           // the other lanes must not run ahead into a spin wait
   mbar_wait_spin(&sm.bar_mma, 0, ctl, DEV_TIMEOUT_MMA);
   tc_fence_after();
-  // The KQ tile and the operand images are dead from here (every thread has seen the products complete): L, X, Pm take
+  // The KQ tile and the operand images are dead from here (every thread has seen the products complete): L, X, the Pm image take
   // their places.  Rows 0..63 -> M (strictly lower) -> L, rows 64..127 -> Mp (lower) -> Pm.
   {
     const float rowscale = isq ? p.scale : sm.beta[t];
-    float* dst = isq ? sm.Pm : sm.u.m.L;
+    // eight columns of a row: Pm rounded into its operand image, L as it is (the inverse X fills in the blocks on and below the
+    // diagonal of zeros)
+    auto put = [&](int sb, const float* v) {
+      if (isq) {
+        st_shared_v4(smem_u32(sm.img_pm) + (t >> 3) * 128 + (t & 7) * 16 + (sb >> 3) * 1024, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]),
+                     pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+      } else {
+        float* l = sm.u.m.L + mat_idx(t, sb);
+        float* x = sm.u.m.X + mat_idx(t, sb);
+        *reinterpret_cast<float4*>(l) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(l + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        *reinterpret_cast<float4*>(x) = *reinterpret_cast<float4*>(x + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    };
     const int tmax = (warp & 1) ? 63 : 31;                  // largest row of this warp
     if (sm.steep == 0) {
 #pragma unroll
@@ -338,9 +356,9 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         for (int c = 0; c < 8; ++c) {
           const int s = sb + c;
           const bool in = sb <= tmax && (isq ? (s <= t) : (s < t));
-          dst[mat_idx(t, s)] = in ? rowscale * pr8[c] * m8[c] : 0.f;
-          if (!isq) sm.u.m.X[mat_idx(t, s)] = 0.f;        // the inverse fills in the blocks on and below the diagonal
+          pr8[c] = in ? rowscale * pr8[c] * m8[c] : 0.f;
         }
+        put(sb, pr8);
       }
     } else {
       float my2[E], mygc[E];
@@ -366,9 +384,9 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
               acc = fmaf(my2[e] * sm.k2[s * E + e], fast_exp2(mygc[e] - sm.gc2[s * E + e]), acc);
             val = rowscale * pr8[c] * acc;
           }
-          dst[mat_idx(t, s)] = val;
-          if (!isq) sm.u.m.X[mat_idx(t, s)] = 0.f;
+          pr8[c] = val;
         }
+        put(sb, pr8);
       }
     }
   }
@@ -410,20 +428,13 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   tri_merge_mma<16>(L, X, sm.T, warp, lane);
   tri_merge_mma<32>(L, X, sm.T, warp, lane);
 
-  // bf16 images of A (rows 0..63 of the [A;PA] image) and Pm: one 16-byte piece per thread and step
+  // bf16 image of A (rows 0..63 of the [A;PA] image): one 16-byte piece per thread and step
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int piece = it * MASK_THREADS + tid, i = piece & 63, jb = piece >> 6;
-    float va[8], vp[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      va[c] = X[mat_idx(i, jb * 8 + c)];
-      vp[c] = sm.Pm[mat_idx(i, jb * 8 + c)];
-    }
-    st_shared_v4(smem_u32(sm.img_ap) + (i >> 3) * 128 + (i & 7) * 16 + jb * 2048, pack_bf16(va[0], va[1]),
-                 pack_bf16(va[2], va[3]), pack_bf16(va[4], va[5]), pack_bf16(va[6], va[7]));
-    st_shared_v4(smem_u32(sm.img_pm) + (i >> 3) * 128 + (i & 7) * 16 + jb * 1024, pack_bf16(vp[0], vp[1]),
-                 pack_bf16(vp[2], vp[3]), pack_bf16(vp[4], vp[5]), pack_bf16(vp[6], vp[7]));
+    const float4 a0 = *reinterpret_cast<const float4*>(X + mat_idx(i, jb * 8)), a1 = *reinterpret_cast<const float4*>(X + mat_idx(i, jb * 8 + 4));
+    st_shared_v4(smem_u32(sm.img_ap) + (i >> 3) * 128 + (i & 7) * 16 + jb * 2048, pack_bf16(a0.x, a0.y), pack_bf16(a0.z, a0.w),
+                 pack_bf16(a1.x, a1.y), pack_bf16(a1.z, a1.w));
   }
   fence_async_smem();
   tc_fence_before();
