@@ -33,6 +33,44 @@ __device__ __forceinline__ float mexp2(float x) {
 }
 __device__ __forceinline__ int midx(int i, int j) { return i * 64 + (j ^ (i & 31)); }
 
+// A row of E gate values as pairs: sums over the slices run on the two-wide f32 instructions, half as many instructions for the
+// same products (each lane an ordinary f32 fma).
+template <int E> struct GateVec {
+  static constexpr int N = (E + 1) / 2;
+  float2 p[N];
+  __device__ __forceinline__ void set(int e, float v) { if (e & 1) p[e / 2].y = v; else p[e / 2].x = v; }
+  __device__ __forceinline__ float get(int e) const { return (e & 1) ? p[e / 2].y : p[e / 2].x; }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[i] = make_float2(0.f, 0.f);
+  }
+  __device__ __forceinline__ float dot(const GateVec& o) const {
+    float2 a = __fmul2_rn(p[0], o.p[0]);
+#pragma unroll
+    for (int i = 1; i < N; ++i) a = __ffma2_rn(p[i], o.p[i], a);
+    return E == 1 ? a.x : a.x + a.y;
+  }
+  __device__ __forceinline__ void add_scaled(float f, const GateVec& o) {
+    const float2 ff = make_float2(f, f);
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[i] = __ffma2_rn(ff, o.p[i], p[i]);
+  }
+  __device__ __forceinline__ void load(const float* row) {       // a dense table row (the same row for the whole warp)
+    if constexpr (E % 4 == 0) {
+#pragma unroll
+      for (int i = 0; i < N; i += 2) {
+        const float4 x = *reinterpret_cast<const float4*>(row + 2 * i);
+        p[i] = make_float2(x.x, x.y);
+        p[i + 1] = make_float2(x.z, x.w);
+      }
+    } else if constexpr (E == 2) {
+      p[0] = *reinterpret_cast<const float2*>(row);
+    } else {
+      p[0] = make_float2(row[0], 0.f);
+    }
+  }
+};
+
 template <int E>
 struct MatSmem {
   static constexpr int ES = E | 1;
@@ -243,18 +281,6 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     mygc[e] = sm.gc2[t * ES + e];
   }
   const bool fast = sm.steep == 0;                         // block-uniform
-  auto table_row = [&](const float* tab, int row, float* out) {   // E floats of a dense table row (the same row for the whole warp)
-    if constexpr (E % 4 == 0) {
-#pragma unroll
-      for (int e = 0; e < E; e += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(tab + row * E + e);
-        out[e] = x.x; out[e + 1] = x.y; out[e + 2] = x.z; out[e + 3] = x.w;
-      }
-    } else {
-#pragma unroll
-      for (int e = 0; e < E; ++e) out[e] = tab[row * E + e];
-    }
-  };
   const int warp_tmin = (warp & 1) ? 32 : 0;               // smallest row index t in this warp
   const uint32_t a5 = smem_u32(sm.u1.a5);
   const int warp_tmax = (warp & 1) ? 63 : 31;              // largest row index t in this warp
@@ -274,34 +300,32 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     for (int e = 0; e < E; ++e) r1v[e] = 0.f;
     float xrow[16];
     if (fast) {
-      float F[E], G[E], accr[E];
+      GateVec<E> F, G, accr;
+      F.clear(); G.clear(); accr.clear();
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        F[e] = mexp2(fminf(mygc[e] - sm.gc2[s0 * ES + e], 0.f));   // rows above the block (masked below) would give > 0
-        G[e] = my2[e] * F[e];
-        accr[e] = 0.f;
+        const float f = mexp2(fminf(mygc[e] - sm.gc2[s0 * ES + e], 0.f));   // rows above the block (masked below) would give > 0
+        F.set(e, f);
+        G.set(e, my2[e] * f);
       }
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int s = s0 + j;
         float x = 0.f, dmpv = 0.f;
         if (s0 <= warp_tmax) {
-          float hk[E];
-          table_row(sm.hkv, s, hk);
-          float mp = 0.f;
-#pragma unroll
-          for (int e = 0; e < E; ++e) mp = fmaf(G[e], hk[e], mp);
+          GateVec<E> hk;
+          hk.load(sm.hkv + s * E);
+          const float mp = G.dot(hk);
           const float in = (s <= t) ? p.scale * gr[j] : 0.f;
           x = in * mp;
           dmpv = live * in * pr[j];
-#pragma unroll
-          for (int e = 0; e < E; ++e) accr[e] = fmaf(dmpv, hk[e], accr[e]);
+          accr.add_scaled(dmpv, hk);
         }
         xrow[j] = x;
         sm.u2.f.dmp[midx(t, s)] = dmpv;
       }
 #pragma unroll
-      for (int e = 0; e < E; ++e) r1v[e] = F[e] * accr[e];
+      for (int e = 0; e < E; ++e) r1v[e] = F.get(e) * accr.get(e);
     } else {
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -343,9 +367,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     // query thread (64+s, cq): partial c1[s,e] over t' in quarter cq: dmp[t',s] exp(gc[t']-gc[s]) q2[t',e]
     {
       const int s = t;
-      float c1v[E];
-#pragma unroll
-      for (int e = 0; e < E; ++e) c1v[e] = 0.f;
+      GateVec<E> c1v;
+      c1v.clear();
       if (fast) {
         // the same sixteen rows t' for every lane (dmp is zero above the diagonal); nothing to do where the whole warp
         // lies below the quarter
@@ -354,26 +377,25 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
           for (int j = 0; j < 16; ++j) {
             const int tt = s0 + j;
             const float dv = sm.u2.f.dmp[midx(tt, s)];
-            float qx[E];
-            table_row(sm.qxv, tt, qx);
-#pragma unroll
-            for (int e = 0; e < E; ++e) c1v[e] = fmaf(dv, qx[e], c1v[e]);
+            GateVec<E> qx;
+            qx.load(sm.qxv + tt * E);
+            c1v.add_scaled(dv, qx);
           }
         }
         if (s0 + 15 >= s) {
 #pragma unroll
-          for (int e = 0; e < E; ++e) c1v[e] *= mexp2(sm.gc2[s0 * ES + e] - mygc[e]);
+          for (int e = 0; e < E; ++e) c1v.set(e, c1v.get(e) * mexp2(sm.gc2[s0 * ES + e] - mygc[e]));
         }
       } else {
         for (int tt = max(s, s0); tt < s0 + 16; ++tt) {
           const float dv = sm.u2.f.dmp[midx(tt, s)];
   #pragma unroll
           for (int e = 0; e < E; ++e)
-            c1v[e] = fmaf(dv * sm.q2[tt * ES + e], mexp2(sm.gc2[tt * ES + e] - mygc[e]), c1v[e]);
+            c1v.set(e, fmaf(dv * sm.q2[tt * ES + e], mexp2(sm.gc2[tt * ES + e] - mygc[e]), c1v.get(e)));
         }
       }
 #pragma unroll
-      for (int e = 0; e < E; ++e) sm.part[1][cq][s * ES + e] = c1v[e];
+      for (int e = 0; e < E; ++e) sm.part[1][cq][s * ES + e] = c1v.get(e);
     }
     mma_phase += 2;                                        // G3 and G4 complete without the query rows watching
   } else {
@@ -511,34 +533,32 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
 #pragma unroll
       for (int j = 0; j < 16; ++j) dpk[j] = 0.f;
       if (fast) {
-        float F[E], G[E], accr[E];
+        GateVec<E> F, G, accr;
+        F.clear(); G.clear(); accr.clear();
 #pragma unroll
         for (int e = 0; e < E; ++e) {
-          F[e] = mexp2(fminf(mygc[e] - sm.gc2[s0 * ES + e], 0.f));
-          G[e] = my2[e] * F[e];
-          accr[e] = 0.f;
+          const float f = mexp2(fminf(mygc[e] - sm.gc2[s0 * ES + e], 0.f));
+          F.set(e, f);
+          G.set(e, my2[e] * f);
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const int s = s0 + j;
           float dmv = 0.f;
           if (s0 <= warp_tmax) {
-            float hk[E];
-            table_row(sm.hkv, s, hk);
-            float m = 0.f;
-#pragma unroll
-            for (int e = 0; e < E; ++e) m = fmaf(G[e], hk[e], m);
+            GateVec<E> hk;
+            hk.load(sm.hkv + s * E);
+            const float m = G.dot(hk);
             const float dl = (s < t) ? -dpr[j] : 0.f;
             brow = fmaf(dl * pr[j], m, brow);
             dmv = bt * dl * pr[j];
             dpk[j] = bt * dl * m;                          // zero on and above the diagonal
-#pragma unroll
-            for (int e = 0; e < E; ++e) accr[e] = fmaf(dmv, hk[e], accr[e]);
+            accr.add_scaled(dmv, hk);
           }
           sm.u2.f.dm[midx(t, s)] = dmv;
         }
 #pragma unroll
-        for (int e = 0; e < E; ++e) r2v[e] = F[e] * accr[e];
+        for (int e = 0; e < E; ++e) r2v[e] = F.get(e) * accr.get(e);
       } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
@@ -606,9 +626,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   {
     // thread (s = t, cq): partial c2[s,e] = sum over t' > s of dm[t',s] exp(gc[t']-gc[s]) k2[t',e]; the key-row thread takes
     // the first eight t' of quarter cq, the query-row thread of the same (t, cq) the other eight
-    float c2v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) c2v[e] = 0.f;
+    GateVec<E> c2v;
+    c2v.clear();
     const int lo = s0 + (krow ? 0 : 8);
     if (fast) {
       if (lo + 7 > warp_tmin) {                            // dm is zero on and above the diagonal
@@ -616,26 +635,25 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         for (int j = 0; j < 8; ++j) {
           const int tt = lo + j;
           const float dv = sm.u2.f.dm[midx(tt, t)];
-          float kx[E];
-          table_row(sm.hkv, tt, kx);
-#pragma unroll
-          for (int e = 0; e < E; ++e) c2v[e] = fmaf(dv, kx[e], c2v[e]);
+          GateVec<E> kx;
+          kx.load(sm.hkv + tt * E);
+          c2v.add_scaled(dv, kx);
         }
       }
       if (s0 + 15 > t) {
 #pragma unroll
-        for (int e = 0; e < E; ++e) c2v[e] *= mexp2(sm.gc2[s0 * ES + e] - mygc[e]);
+        for (int e = 0; e < E; ++e) c2v.set(e, c2v.get(e) * mexp2(sm.gc2[s0 * ES + e] - mygc[e]));
       }
     } else {
       for (int tt = max(t + 1, lo); tt < lo + 8; ++tt) {
         const float dv = sm.u2.f.dm[midx(tt, t)];
   #pragma unroll
         for (int e = 0; e < E; ++e)
-          c2v[e] = fmaf(dv * sm.k2[tt * ES + e], mexp2(sm.gc2[tt * ES + e] - mygc[e]), c2v[e]);
+          c2v.set(e, fmaf(dv * sm.k2[tt * ES + e], mexp2(sm.gc2[tt * ES + e] - mygc[e]), c2v.get(e)));
       }
     }
 #pragma unroll
-    for (int e = 0; e < E; ++e) sm.part[krow ? 0 : 1][cq][t * ES + e] = c2v[e];
+    for (int e = 0; e < E; ++e) sm.part[krow ? 0 : 1][cq][t * ES + e] = c2v.get(e);
   }
   __syncthreads();
   // gate gradients: one thread per (row, gate column)
