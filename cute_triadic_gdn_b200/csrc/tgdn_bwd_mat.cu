@@ -15,6 +15,13 @@
 // Row and column sums that span the four column quarters go through four-copy partial tables in shared memory and are
 // added in a fixed order (no atomics: results are bitwise reproducible).
 //
+// What bounds it: one CTA per SM (operands, tables and partial sums fill its shared memory), and inside an item a serial chain of
+// five product groups with the sums over the slices between them (f32 on the ordinary pipes).  Hence the two independent chains,
+// the two-wide f32 instructions for those sums, L2 prefetch of the next item, and 16-byte pieces wherever a thread owns a row; the
+// column sums of dA'*A are exchanges inside the warps, before G3, instead of a matrix in shared memory that is walked by columns
+// after it.  us, before (first these, then the two-wide sums) and after: 16384 items E8 575 -> 519; 4096 items E8 mild 303 -> 268,
+// E4 248 -> 231, E1 222 -> 211; packed E16 900 -> 875.
+//
 // Replaces cute_triadic_gdn/kernels/sm100_joint_bwd_parallel.py:80-405 (matrix_kernel),
 // cute_triadic_gdn/kernels/sm90_joint_bwd_parallel.py:278-372 (mask_grad_kernel) and the reverse pass of
 // cute_triadic_gdn/kernels/sm90_joint_scan.py:21-80; math as listed in cute_triadic_gdn/ops/gdn_joint.py:45-90 differentiated.
@@ -31,7 +38,24 @@ __device__ __forceinline__ float mexp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ int midx(int i, int j) { return i * 64 + (j ^ (i & 31)); }
+// 64x64 f32 matrices with rows 68 floats apart: a lane per row writes 16-byte pieces, a lane per column reads floats, both without
+// bank conflicts.
+constexpr int MAT_LD = 68;
+__device__ __forceinline__ int midx(int i, int j) { return i * MAT_LD + j; }
+// Sums of sixteen values over the lanes of a warp by halving exchanges: lanes 2i and 2i + 1 end with the sum of value
+// (bit 4, 3, 2, 1 of the lane).
+__device__ __forceinline__ float warp_sums16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int n = 8, keep = 16; n >= 1; n >>= 1, keep >>= 1) {
+    const bool up = (lane & keep) != 0;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float send = up ? v[i] : v[i + n], mine = up ? v[i + n] : v[i];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, send, keep);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
 
 // A row of E gate values as pairs: sums over the slices run on the two-wide f32 instructions, half as many instructions for the
 // same products (each lane an ordinary f32 fma).
@@ -81,12 +105,11 @@ struct MatSmem {
   } u1;
   union {
     uint8_t wu[32768];               // [W;U] tile (until G2), then two f32 64x64 matrices
-    struct { float dmp[4096]; float dm[4096]; } f;
+    struct { float dmp[64 * MAT_LD]; float dm[64 * MAT_LD]; } f;
   } u2;
   uint8_t ap[16384];                 // [A;PmA] image, rows 0..63 = A
   uint8_t da[8192];                  // dA image (i = t, j = s), SI = 128, SJ = 1024
-  uint8_t y[8192];                   // Y image (i = s', j = t'), SI = 128, SJ = 1024 (read as 128 rows: daa follows)
-  float daa[4096];                   // dA' * A, for the column sums
+  uint8_t y[8192];                   // Y image (i = s', j = t'), SI = 128, SJ = 1024 (read as 128 rows: the tables follow)
   // decay tables whose rows are read by whole warps at once (dense rows, 16-byte loads):
   alignas(16) float hkv[64 * E];     // until the two chains join: exp2(gc[r0(s)] - gc[s]) * k2[s], r0(s) the first row of
                                      // s's 16-row block; afterwards: k2[t] * exp2(gc[t] - gc[r0(t)])
@@ -95,7 +118,7 @@ struct MatSmem {
   float r1[64 * ES], c1[64 * ES], r2[64 * ES], dgc[64 * ES], drr[64 * ES];
   float part[2][4][64 * ES];         // per column quarter partial sums
   float browp[4][64];
-  float beta[64], brow[64], bcol[64];
+  float beta[64], brow[64], bcolp[2][64];    // bcolp: column sums of dA' * A over the rows of a warp (32 each)
   uint64_t bar_load, bar_mma;
   uint32_t tmem_base;
   int abort;
@@ -274,12 +297,14 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   tc_fence_before();
   __syncthreads();                                         // dudo and wu are dead: a5, dmp, dm take their place
 
-  float my2[E], mygc[E];
+  float my2[E], mygc[E];                                   // this row's k2 (q2) and gc
+  auto read_gates = [&]() {
 #pragma unroll
-  for (int e = 0; e < E; ++e) {
-    my2[e] = krow ? sm.k2[t * ES + e] : sm.q2[t * ES + e];
-    mygc[e] = sm.gc2[t * ES + e];
-  }
+    for (int e = 0; e < E; ++e) {
+      my2[e] = krow ? sm.k2[t * ES + e] : sm.q2[t * ES + e];
+      mygc[e] = sm.gc2[t * ES + e];
+    }
+  };
   const bool fast = sm.steep == 0;                         // block-uniform
   const int warp_tmin = (warp & 1) ? 32 : 0;               // smallest row index t in this warp
   const uint32_t a5 = smem_u32(sm.u1.a5);
@@ -293,12 +318,13 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
 
   if (!krow) {
     // ================================ query-row chain ================================
+    read_gates();
     // query row t, columns s0..s0+15: X -> a5 (row 64+t and, transposed, column 64+t), dmp, partial r1
     const float live = (t < rows) ? 1.f : 0.f;
     float r1v[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) r1v[e] = 0.f;
-    float xrow[16];
+    float xrow[16], dmr[4];                                 // dmr: four values of dmp on their way to shared memory
     if (fast) {
       GateVec<E> F, G, accr;
       F.clear(); G.clear(); accr.clear();
@@ -322,7 +348,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
           accr.add_scaled(dmpv, hk);
         }
         xrow[j] = x;
-        sm.u2.f.dmp[midx(t, s)] = dmpv;
+        dmr[j & 3] = dmpv;
+        if ((j & 3) == 3) *reinterpret_cast<float4*>(sm.u2.f.dmp + midx(t, s - 3)) = make_float4(dmr[0], dmr[1], dmr[2], dmr[3]);
       }
 #pragma unroll
       for (int e = 0; e < E; ++e) r1v[e] = F.get(e) * accr.get(e);
@@ -345,7 +372,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         for (int e = 0; e < E; ++e) r1v[e] = fmaf(dmpv, dec[e], r1v[e]);
       }
       xrow[j] = x;
-      sm.u2.f.dmp[midx(t, s)] = dmpv;
+      dmr[j & 3] = dmpv;
+      if ((j & 3) == 3) *reinterpret_cast<float4*>(sm.u2.f.dmp + midx(t, s - 3)) = make_float4(dmr[0], dmr[1], dmr[2], dmr[3]);
     }
     }
     const uint32_t rowbase = a5 + ((64 + t) >> 3) * 128 + (t & 7) * 16;
@@ -404,21 +432,27 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     {
       const uint32_t apr = smem_u32(sm.ap) + (t >> 3) * 128 + (t & 7) * 16;
       const uint32_t dar = smem_u32(sm.da) + (t >> 3) * 128 + (t & 7) * 16;
+      float prod[16];
 #pragma unroll
       for (int jb = 0; jb < 2; ++jb) {
         uint32_t aw[4];
         asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(aw[0]), "=r"(aw[1]), "=r"(aw[2]), "=r"(aw[3]) : "r"(apr + (2 * cq + jb) * 2048));
+        const float4 b0 = *reinterpret_cast<const float4*>(sm.beta + s0 + jb * 8), b1 = *reinterpret_cast<const float4*>(sm.beta + s0 + jb * 8 + 4);
+        const float bs[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
         float dav[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-          const int j = jb * 8 + c, s = s0 + j;
-          const float a_ts = (c & 1) ? bf16_hi(aw[c >> 1]) : bf16_lo(aw[c >> 1]);
-          sm.daa[midx(t, s)] = gr[j] * a_ts;
-          dav[c] = gr[j] * sm.beta[s];
+          const int j = jb * 8 + c;
+          prod[j] = gr[j] * ((c & 1) ? bf16_hi(aw[c >> 1]) : bf16_lo(aw[c >> 1]));
+          dav[c] = gr[j] * bs[c];
         }
         st_shared_v4(dar + (2 * cq + jb) * 1024, pack_bf16(dav[0], dav[1]), pack_bf16(dav[2], dav[3]), pack_bf16(dav[4], dav[5]),
                      pack_bf16(dav[6], dav[7]));
       }
+      fence_async_smem();
+      // dbeta_col[s] = sum_t dA'[t,s] A[t,s]: this warp's 32 rows
+      const float col = warp_sums16(prod, lane);
+      if (!(lane & 1)) sm.bcolp[warp & 1][s0 + (lane >> 1)] = col;
     }
     fence_async_smem();
     tc_fence_before();
@@ -435,13 +469,6 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       umma_commit(&sm.bar_mma);
     }
     __syncwarp();                                          // the other lanes must not run ahead into a spin wait
-    // meanwhile: dbeta_col[s] = sum_t dA'[t,s] A[t,s] (the 64 key-row threads of the last column quarter)
-    if (cq == 3) {
-      const int s = t;
-      float acc = 0.f;
-      for (int tt = 0; tt < 64; ++tt) acc += sm.daa[midx(tt, s)];
-      sm.bcol[s] = acc;
-    }
     mbar_wait_spin(&sm.bar_mma, mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     ++mma_phase;
     tc_fence_after();
@@ -470,12 +497,13 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       umma_commit(&sm.bar_mma);
     }
     __syncwarp();                                          // the other lanes must not run ahead into a spin wait
+    read_gates();
     mbar_wait_spin(&sm.bar_mma, mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     ++mma_phase;
     tc_fence_after();
-    // ap, da, y and daa (48 KB in a row) are dead from here on: the state part of dK, dQ (32 KB bf16 image written by
+    // ap, da and y (32 KB in a row) are dead from here on: the state part of dK, dQ (32 KB bf16 image written by
     // the state-gradient kernel) is fetched into their place now, so that its HBM round trip runs under the remaining
-    // phases.  (The column sums over daa were finished before the barrier that preceded G4.)
+    // phases.
     if (warp_u == 0 && elect_one()) {
       mbar_expect_tx(&sm.bar_load, 32768);
       bulk_load(sm.ap, reinterpret_cast<const uint8_t*>(p.dkq) + item * 32768, 32768, &sm.bar_load);
@@ -529,6 +557,7 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       float r2v[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) r2v[e] = 0.f;
+      float dmr[4];                                        // four values of dm on their way to shared memory
       float dpk[16];                                       // dPkk, this thread's 16 columns of row t
 #pragma unroll
       for (int j = 0; j < 16; ++j) dpk[j] = 0.f;
@@ -555,7 +584,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
             dpk[j] = bt * dl * m;                          // zero on and above the diagonal
             accr.add_scaled(dmv, hk);
           }
-          sm.u2.f.dm[midx(t, s)] = dmv;
+          dmr[j & 3] = dmv;
+          if ((j & 3) == 3) *reinterpret_cast<float4*>(sm.u2.f.dm + midx(t, s - 3)) = make_float4(dmr[0], dmr[1], dmr[2], dmr[3]);
         }
 #pragma unroll
         for (int e = 0; e < E; ++e) r2v[e] = F.get(e) * accr.get(e);
@@ -579,7 +609,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
 #pragma unroll
           for (int e = 0; e < E; ++e) r2v[e] = fmaf(dmv, dec[e], r2v[e]);
         }
-        sm.u2.f.dm[midx(t, s)] = dmv;
+        dmr[j & 3] = dmv;
+        if ((j & 3) == 3) *reinterpret_cast<float4*>(sm.u2.f.dm + midx(t, s - 3)) = make_float4(dmr[0], dmr[1], dmr[2], dmr[3]);
       }
       }
       const uint32_t rowbase = a5 + (t >> 3) * 128 + (t & 7) * 16;
@@ -678,7 +709,7 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       sm.drr[o] = drv * (k2v * egr);                        // dr*r, summed over the rows below
     }
   }
-  if (tid < 64 && tid < rows) p.dbeta[(tok + tid) * p.H + h] = sm.bcol[tid] + sm.brow[tid];
+  if (tid < 64 && tid < rows) p.dbeta[(tok + tid) * p.H + h] = (sm.bcolp[0][tid] + sm.bcolp[1][tid]) + sm.brow[tid];
   __syncthreads();
   // dg = reverse inclusive cumulative sum of dgc over the chunk, one warp per gate column; the last row first takes the
   // chunk-end terms sum_t dr*r + dd*exp(gL)
