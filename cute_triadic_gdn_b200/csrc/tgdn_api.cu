@@ -69,18 +69,19 @@ int tgdn_dynamic_smem(const void* kernel, int bytes, bool* configured) {
 }
 
 int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows,
-                        int swizzle128, int row_tokens) {
+                        int swizzle, int row_tokens) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return TGDN_ERR_DRIVER;
   if (reinterpret_cast<uintptr_t>(base) & 15) return TGDN_ERR_ALIGN;
-  if (swizzle128 && box_cols != 64) return TGDN_ERR_SHAPE;
+  if (swizzle && box_cols != 64 && box_cols != 32 && box_cols != 16) return TGDN_ERR_SHAPE;
   const cuuint64_t dims[4] = {128, static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(T), static_cast<cuuint64_t>(B)};
   const cuuint64_t strides[3] = {256, static_cast<cuuint64_t>(H) * 256,
                                  static_cast<cuuint64_t>(row_tokens ? row_tokens : T) * H * 256};
   const cuuint32_t box[4] = {static_cast<cuuint32_t>(box_cols), 1, static_cast<cuuint32_t>(box_rows), 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, !swizzle ? CU_TENSOR_MAP_SWIZZLE_NONE
+                  : box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : TGDN_ERR_DRIVER;
 }

@@ -271,6 +271,17 @@ __device__ __forceinline__ void umma_ksteps(uint32_t d_tmem, uint64_t adesc, uin
               (accumulate || k > 0) ? 1u : 0u);
 }
 
+// Two f32 fused multiply-adds in one instruction (each lane an ordinary fma): the epilogues of the recurrences are bound by
+// instruction issue.
+__device__ __forceinline__ void fma_pair(float& a0, float& a1, float f, float x0, float x1) {        // a += f * x
+  const float2 r = __ffma2_rn(make_float2(f, f), make_float2(x0, x1), make_float2(a0, a1));
+  a0 = r.x; a1 = r.y;
+}
+__device__ __forceinline__ void scale_add_pair(float& a0, float& a1, float f, float x0, float x1) {  // a = f * a + x
+  const float2 r = __ffma2_rn(make_float2(f, f), make_float2(a0, a1), make_float2(x0, x1));
+  a0 = r.x; a1 = r.y;
+}
+
 // ------------------------------------------------------------------------------------------------
 // small helpers
 // ------------------------------------------------------------------------------------------------

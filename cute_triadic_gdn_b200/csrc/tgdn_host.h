@@ -15,9 +15,9 @@ int tgdn_cuda_error(cudaError_t e);
 int* tgdn_status_word();
 
 // Tensor map over a (B, T, H, 128) bf16 tensor in token layout: box = [box_cols columns][1 head][box_rows tokens][1 row].
-// swizzle128 = 1 asks for the 128-byte swizzle (box_cols must then be 64).  row_tokens: tokens from one batch row to the next
+// swizzle = 1 asks for the swizzle as wide as a row of the box (box_cols 64, 32 or 16).  row_tokens: tokens from one batch row to the next
 // (0: T), for a token range of longer rows.
-int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows, int swizzle128,
+int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows, int swizzle,
                         int row_tokens = 0);
 
 // Tensor map over a (B, T, H, E) f32 gate tensor (k2, q2) in token layout, E a multiple of 4: box = [E][1 head][64 tokens][1 row],

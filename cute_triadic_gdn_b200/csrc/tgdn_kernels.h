@@ -45,7 +45,8 @@ struct MaskParams {
 };
 
 struct FwdParams {
-  const __nv_bfloat16* v;   // token layout
+  const __nv_bfloat16* q;   // token layout, like k and v
+  const __nv_bfloat16* k;
   const float* k2;
   const float* q2;
   const float* beta;
