@@ -86,6 +86,33 @@ int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H,
   return r == CUDA_SUCCESS ? 0 : TGDN_ERR_DRIVER;
 }
 
+static int encode_5d(CUtensorMap* map, const void* base, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box) {
+  EncodeTiledFn fn = encode_tiled();
+  if (!fn) return TGDN_ERR_DRIVER;
+  if (reinterpret_cast<uintptr_t>(base) & 15) return TGDN_ERR_ALIGN;
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : TGDN_ERR_DRIVER;
+}
+
+int tgdn_make_image_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_blocks, int row_tokens) {
+  const cuuint64_t row = static_cast<cuuint64_t>(H) * 256;
+  const cuuint64_t dims[5] = {8, static_cast<cuuint64_t>(T), 16, static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
+  const cuuint64_t strides[4] = {row, 16, 256, static_cast<cuuint64_t>(row_tokens ? row_tokens : T) * row};
+  const cuuint32_t box[5] = {8, 64, static_cast<cuuint32_t>(box_blocks), 1, 1};
+  return encode_5d(map, base, dims, strides, box);
+}
+
+int tgdn_make_a_half_map(CUtensorMap* map, const void* base, long long items) {
+  if (items > 0x7fffffffLL) return TGDN_ERR_SHAPE;
+  const cuuint64_t dims[5] = {256, 2, 2, 8, static_cast<cuuint64_t>(items)};
+  const cuuint64_t strides[4] = {512, 1024, 2048, 16384};
+  const cuuint32_t box[5] = {256, 2, 1, 8, 1};
+  return encode_5d(map, base, dims, strides, box);
+}
+
 int tgdn_make_gate_map(CUtensorMap* map, const float* base, int B, int T, int H, int E, int row_tokens) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return TGDN_ERR_DRIVER;

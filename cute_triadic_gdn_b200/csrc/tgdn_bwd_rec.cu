@@ -34,6 +34,10 @@
 // products' operand reads and the operand images fill to two thirds.  Reverse recurrence, us, one lockstep CTA of four warpgroups
 // that looked the chunk up when it began -> this version: B2 T8192 H32 E8 1241 -> 1092; B1 T32768 packed H8 E12 1132 -> 997;
 // H16 E16 2497 -> 2414; B4 T4096 H16 E4 394 -> 285, E2 318 -> 226, E1 299 -> 202 (the last three with 64 value columns per CTA).
+// Every copy operation costs the warp that issues it some sixty cycles and the chain waits for its last warp, so the images of dO and U,
+// the A half and dU move with one operation each, whatever their width (22 -> 9 a chunk at E = 8); with that and the two-wide f32
+// multiply-adds: E8 1095 -> 1075, E16 2418 -> 2395, E4 291 -> 275, E2 229 -> 209, E1 204 -> 178 us.  (Pulling later chunks into L2 by
+// prefetch instructions made it 3 to 8 % slower: the loads are a chunk ahead already.)
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
 #include "tgdn_kernels.h"
@@ -158,11 +162,12 @@ template <int E, int VC, int NCH, int NSG, bool PACKED>
 __global__ void __launch_bounds__(512, 1)
 rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
            const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_u,
-           const __grid_constant__ CUtensorMap map_du, RecParams p) {
+           const __grid_constant__ CUtensorMap map_du, const __grid_constant__ CUtensorMap map_a, RecParams p) {
   using C = RecCfg<E, VC, NCH, NSG>;
   constexpr int REC_THREADS = C::THREADS, NWG = C::NWG, CT = C::CHAIN_THREADS, CC = C::CC, CV = C::CV, YW = C::YW;
   constexpr int NCOLS = C::NCOLS, CW = C::CW, TPC = C::TPC, ES = C::ES, NCG = C::NCG, EL = C::EL;
   constexpr int NV = HEAD / VC;
+  constexpr bool TWO_WIDE = TPC * CW < 1024;        // the two-wide multiply-adds of (a) need register pairs: sixteen columns of four slices spill
   constexpr float LOG2E = 1.4426950408889634f;   // the decay threshold below is in the log2 domain
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -267,10 +272,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   };
   auto issue_a = [&](int i, int nb, uint64_t* bar) {          // one thread: the A half of [A;PmA] of local chunk i -> copy nb
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
-    // [A; Pm A] is an image of 128 rows: per 8-column block (2 KB) the first 1 KB holds the rows of A
-    const __nv_bfloat16* ap = p.AP + item * (128 * 64);
-#pragma unroll
-    for (int jb = 0; jb < 8; ++jb) bulk_load(smem + C::OFF_A + nb * C::A_BYTES + jb * 1024, ap + jb * 1024, 1024, bar);
+    tma_load_5d(smem + C::OFF_A + nb * C::A_BYTES, &map_a, bar, 0, 0, 0, 0, static_cast<int>(item));
   };
   auto issue_loads = [&](int i, int st) {           // one thread: the tiles of local chunk i that live in a stage
     int t0, rows;
@@ -278,12 +280,9 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
     mbar_expect_tx(&ctrl.bar_load[st], C::KQ_BYTES + 2 * C::DO_BYTES + C::GT_BYTES + (C::LATE ? 0u : C::A_BYTES + C::PM_BYTES));
-#pragma unroll
-    for (int jb = 0; jb < VC / 8; ++jb) {            // eight value columns x 64 rows = one 1 KB column block of the image
-      tma_load_4d(smem + C::OFF_DO + st * C::DOB + jb * 1024, &map_do, &ctrl.bar_load[st], vb * VC + jb * 8, h, t0, b);
-      tma_load_4d(smem + C::OFF_DU + st * C::DOB + jb * 1024, &map_u, &ctrl.bar_load[st], vb * VC + jb * 8, 0,
-                  static_cast<int>(item * 64), 0);
-    }
+    // (eight value columns x 64 rows = one 1 KB column block of the images)
+    tma_load_5d(smem + C::OFF_DO + st * C::DOB, &map_do, &ctrl.bar_load[st], 0, t0, vb * (VC / 8), h, b);
+    tma_load_5d(smem + C::OFF_DU + st * C::DOB, &map_u, &ctrl.bar_load[st], 0, static_cast<int>(item * 64), vb * (VC / 8), 0, 0);
     tma_load_4d(kq, &map_k, &ctrl.bar_load[st], 0, h, t0, b);
     tma_load_4d(kq + 8192, &map_q, &ctrl.bar_load[st], 0, h, t0, b);
     tma_load_4d(kq + 16384, &map_k, &ctrl.bar_load[st], 64, h, t0, b);
@@ -515,13 +514,23 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
 #pragma unroll
         for (int ee = 0; ee < EP; ++ee) {
           const float re = gr[pc * EP + ee];
-          float dot = 0.f;
+          if constexpr (TWO_WIDE) {
+            float2 dot = make_float2(0.f, 0.f);
 #pragma unroll
-          for (int c = 0; c < CW; ++c) {
-            du[c] = fmaf(re, kp[ee * CW + c], du[c]);
-            dot = fmaf(uv[c], kp[ee * CW + c], dot);
+            for (int c = 0; c < CW; c += 2) {
+              fma_pair(du[c], du[c + 1], re, kp[ee * CW + c], kp[ee * CW + c + 1]);
+              dot = __ffma2_rn(make_float2(uv[c], uv[c + 1]), make_float2(kp[ee * CW + c], kp[ee * CW + c + 1]), dot);
+            }
+            drp[(cgp * 64 + t) * ES + e0 + pc * EP + ee] = dot.x + dot.y;
+          } else {
+            float dot = 0.f;
+#pragma unroll
+            for (int c = 0; c < CW; ++c) {
+              du[c] = fmaf(re, kp[ee * CW + c], du[c]);
+              dot = fmaf(uv[c], kp[ee * CW + c], dot);
+            }
+            drp[(cgp * 64 + t) * ES + e0 + pc * EP + ee] = dot;
           }
-          drp[(cgp * 64 + t) * ES + e0 + pc * EP + ee] = dot;
         }
       }
       if constexpr (NSG > 1) {
@@ -573,9 +582,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     __syncwarp();                                    // the other lanes must not run ahead into a spin wait
     if (PACKED && i > 0) chunk_info(i - 1, t0_next, rows_next);
     if (warp_u == COPY_WARP && elect_one()) {                // dU (chunk layout) straight from its operand image
-#pragma unroll
-      for (int jb = chain * (CV / 8); jb < (chain + 1) * (CV / 8); ++jb)
-        tma_store_4d(&map_du, duimg + jb * 1024, vb * VC + jb * 8, 0, static_cast<int>(item * 64), 0);
+      tma_store_5d(&map_du, duimg + chain * (CV / 8) * 1024, 0, static_cast<int>(item * 64), (vb * VC + chain * CV) / 8, 0, 0);
       bulk_commit_group();
     }
     __syncwarp();
@@ -690,8 +697,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         uint32_t packed[PIECE / 2];
 #pragma unroll
         for (int j = 0; j < PIECE; j += 2) {
-          G[j0 + j] = fmaf(dtab[e0 + (j0 + j) / CW], G[j0 + j], dp[j]);
-          G[j0 + j + 1] = fmaf(dtab[e0 + (j0 + j + 1) / CW], G[j0 + j + 1], dp[j + 1]);
+          scale_add_pair(G[j0 + j], G[j0 + j + 1], dtab[e0 + (j0 + j) / CW], dp[j], dp[j + 1]);
           packed[j / 2] = pack_bf16(G[j0 + j], G[j0 + j + 1]);
         }
         // operand image (i = d, j = n') of the next (a)
@@ -739,19 +745,19 @@ using namespace tgdn;
 
 template <int E, int VC, int NCH, int NSG, bool PACKED>
 static int launch_rec_rows(const CUtensorMap& mk, const CUtensorMap& mq,
-                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const RecParams& p, cudaStream_t s) {
+                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const RecParams& p, cudaStream_t s) {
   using C = RecCfg<E, VC, NCH, NSG>;
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static bool configured[64] = {};
   if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(rec_kernel<E, VC, NCH, NSG, PACKED>), C::SMEM_BYTES, configured)) return rc;
-  rec_kernel<E, VC, NCH, NSG, PACKED><<<p.n_seq * p.H * (HEAD / VC), C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, p);
+  rec_kernel<E, VC, NCH, NSG, PACKED><<<p.n_seq * p.H * (HEAD / VC), C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, ma, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 template <int E, int VC, int NCH, int NSG = 1>
 static int launch_rec(const CUtensorMap& mk, const CUtensorMap& mq,
-                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const RecParams& p, cudaStream_t s) {
-  return p.cmap != nullptr ? launch_rec_rows<E, VC, NCH, NSG, true>(mk, mq, mdo, mu, mdu, p, s)
-                           : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, p, s);
+                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const RecParams& p, cudaStream_t s) {
+  return p.cmap != nullptr ? launch_rec_rows<E, VC, NCH, NSG, true>(mk, mq, mdo, mu, mdu, ma, p, s)
+                           : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, ma, p, s);
 }
 
 int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
@@ -774,13 +780,15 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   CUtensorMap mk, mq;
   if ((rc = tgdn_make_token_map(&mk, k, B, T, H, 64, 64, 1, row_tokens))) return rc;
   if ((rc = tgdn_make_token_map(&mq, q, B, T, H, 64, 64, 1, row_tokens))) return rc;
-  // dO (token layout) and U, dU (chunk layout: item * 64 + t rows of 128 columns) in boxes of 8 columns x 64 rows
+  // dO (token layout) and U, dU (chunk layout: item * 64 + t rows of 128 columns) as operand images of the value block
   const int64_t crows = static_cast<int64_t>(B) * NC * H * 64;
   if (crows > 0x7fffffffLL) return TGDN_ERR_SHAPE;
-  CUtensorMap mdo, mu, mdu;
-  if ((rc = tgdn_make_token_map(&mdo, dO, B, T, H, 8, 64, 0, row_tokens))) return rc;
-  if ((rc = tgdn_make_token_map(&mu, U, 1, static_cast<int>(crows), 1, 8, 64, 0))) return rc;
-  if ((rc = tgdn_make_token_map(&mdu, dU, 1, static_cast<int>(crows), 1, 8, 64, 0))) return rc;
+  CUtensorMap mdo, mu, mdu, ma;
+  const int blocks = value_block / 8, share = E <= 2 && value_block == 32 ? blocks : blocks / 2;   // dU leaves by chain
+  if ((rc = tgdn_make_image_map(&mdo, dO, B, T, H, blocks, row_tokens))) return rc;
+  if ((rc = tgdn_make_image_map(&mu, U, 1, static_cast<int>(crows), 1, blocks))) return rc;
+  if ((rc = tgdn_make_image_map(&mdu, dU, 1, static_cast<int>(crows), 1, share))) return rc;
+  if ((rc = tgdn_make_a_half_map(&ma, AP, static_cast<long long>(B) * NC * H))) return rc;
   RecParams p{static_cast<const __nv_bfloat16*>(dO), k2, q2, beta, gc, static_cast<const __nv_bfloat16*>(AP),
               static_cast<const __nv_bfloat16*>(Pm), static_cast<const __nv_bfloat16*>(U),
               static_cast<__nv_bfloat16*>(dV), static_cast<__nv_bfloat16*>(dU), static_cast<__nv_bfloat16*>(ds),
@@ -789,19 +797,19 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1:
-      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, p, s);
-      return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, p, s);
+      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+      return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, ma, p, s);
     case 2:
-      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, p, s);
-      return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, p, s);
+      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+      return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, ma, p, s);
     case 4:
-      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, p, s);
-      return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, p, s);
+      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+      return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
     // E = 8: 32 value columns per CTA measured 9% faster than two CTAs per SM of 16 columns each (5.26 -> 4.77 ms at B=8, T=8192, H=32,
     // before the chains), and the state-gradient kernel then adds four value-block images per item instead of eight.
-    case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, p, s);
-    case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, p, s);
-    case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, p, s);
+    case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+    case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+    case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
     default: return TGDN_ERR_SHAPE;
   }
 }

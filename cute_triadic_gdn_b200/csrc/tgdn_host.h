@@ -20,6 +20,13 @@ int* tgdn_status_word();
 int tgdn_make_token_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_cols, int box_rows, int swizzle,
                         int row_tokens = 0);
 
+// The same tensors for boxes that land in shared memory as operand images [column / 8][64 tokens][column % 8]: coordinates
+// (0, token, first 8-column block, head, batch row), box_blocks blocks of 1 KB.
+int tgdn_make_image_map(CUtensorMap* map, const void* base, int B, int T, int H, int box_blocks, int row_tokens = 0);
+
+// Tensor map over the [A; Pm A] images whose boxes are the A half of one item (8 KB, an image of 64 rows): coordinates (0, 0, 0, 0, item).
+int tgdn_make_a_half_map(CUtensorMap* map, const void* base, long long items);
+
 // Tensor map over a (B, T, H, E) f32 gate tensor (k2, q2) in token layout, E a multiple of 4: box = [E][1 head][64 tokens][1 row],
 // which lands in shared memory as 64 dense rows of E floats.
 int tgdn_make_gate_map(CUtensorMap* map, const float* base, int B, int T, int H, int E, int row_tokens = 0);
