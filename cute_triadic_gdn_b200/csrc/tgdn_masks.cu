@@ -15,8 +15,12 @@
 // cute_triadic_gdn/ops/gdn_joint.py:36-39, :45-60.
 //   * Gram product [K;Q] K^T: one tcgen05 MMA group (M=128, N=64, K=128) on TMA-staged 128B-swizzled tiles.
 //   * Mask sums: thread (row, column half) with the half's 8-column blocks interleaved so that the triangle is balanced.
-//   * Triangular inverse in f32: four 16x16 diagonal blocks by forward substitution, then the 16->32 and 32->64
+//   * Triangular inverse in f32: eight 8x8 diagonal blocks by forward substitution, an 8->16 step, then the 16->32 and 32->64
 //     merges X21 = -X22 (L21 X11) as warp-level mma.sync m16n8k8 products with a 3-term TF32 split (f32-grade accuracy).
+//   * What bounds it: the chain of these steps, with five block barriers, hidden by three CTAs per SM (two at twelve and sixteen slices),
+//     and the shared-memory wavefronts inside them; hence padded rows in 16-byte pieces everywhere.  us, before (swizzled single
+//     floats, two CTAs per SM) and after: 16384 items E8 355 -> 240; 4096 items E4 179 -> 110, E2 179 -> 105, E1 176 -> 100; packed
+//     E16 561 -> 370, E12 238 -> 171.
 //   * PA = Pm A: a second tcgen05 MMA group on the bf16 images of Pm and A that are about to be stored anyway.
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
@@ -80,10 +84,11 @@ struct MaskSmem {
   uint8_t img_ap[16384];   // [A; PA] image (i = row 0..127, j = column), SI = 128, SJ = 2048
   uint8_t gpad[E > 8 ? 12288 : 16];   // room for the G images at twelve and sixteen slices
   uint8_t img_pm[8192];    // Pm image (i = t, j = s), SI = 128, SJ = 1024; read as 128 rows by the PA product: keep >= 8 KB behind it
-  float gc2[64 * E];       // log2-domain cumulative gate
-  float k2[64 * E];
-  float q2[64 * E];
-  float pad[(3 * 64 * E * 4 >= 8192) ? 1 : (8192 - 3 * 64 * E * 4) / 4];
+  static constexpr int ES = E == 8 || E == 16 ? E + 4 : E;   // rows of 48 and 80 bytes: 32 lanes read a row each without bank conflicts
+  alignas(16) float gc2[64 * ES];    // log2-domain cumulative gate
+  float k2[64 * ES];
+  float q2[64 * ES];
+  float pad[(3 * 64 * ES * 4 >= 8192) ? 1 : (8192 - 3 * 64 * ES * 4) / 4];
   float beta[64];
   uint64_t bar_load, bar_mma;
   uint32_t tmem_base;
@@ -142,6 +147,7 @@ __global__ void __launch_bounds__(MASK_THREADS, E > 8 ? 2 : 3)
 masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q, MaskParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using SM = MaskSmem<E>;
+  constexpr int ES = SM::ES;
   SM& sm = *reinterpret_cast<SM*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ch = warp >> 2;                                 // column half (interleaved 8-column blocks)
@@ -199,10 +205,11 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     for (int it = 0; it < GATE_ITERS; ++it) {
       const int idx = tid + it * MASK_THREADS;
       if (idx < 64 * E) {
+        const int o = idx / E * ES + idx % E;
         const bool ok = idx / E < rows;
-        sm.gc2[idx] = ok ? g_in[it] : 0.f;
-        sm.k2[idx] = ok ? k2_in[it] : 0.f;
-        sm.q2[idx] = ok ? q2_in[it] : 0.f;
+        sm.gc2[o] = ok ? g_in[it] : 0.f;
+        sm.k2[o] = ok ? k2_in[it] : 0.f;
+        sm.q2[o] = ok ? q2_in[it] : 0.f;
       }
     }
     if (tid < 64) sm.beta[tid] = (tid < rows) ? beta_in : 0.f;
@@ -213,7 +220,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   // inclusive scan over the 64 rows, one warp per gate column
   float* gc_out = p.gc + ((static_cast<int64_t>(b) * p.NC + n) * p.H + h) * gate_item_floats(E);
   for (int e = warp; e < E; e += MASK_THREADS / 32) {
-    float v0 = sm.gc2[lane * E + e], v1 = sm.gc2[(lane + 32) * E + e];
+    float v0 = sm.gc2[lane * ES + e], v1 = sm.gc2[(lane + 32) * ES + e];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float a0 = __shfl_up_sync(0xffffffffu, v0, o), a1 = __shfl_up_sync(0xffffffffu, v1, o);
@@ -222,8 +229,8 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     v1 += __shfl_sync(0xffffffffu, v0, 31);
     gc_out[lane * E + e] = v0;
     gc_out[(lane + 32) * E + e] = v1;
-    sm.gc2[lane * E + e] = v0 * LOG2E;
-    sm.gc2[(lane + 32) * E + e] = v1 * LOG2E;
+    sm.gc2[lane * ES + e] = v0 * LOG2E;
+    sm.gc2[(lane + 32) * ES + e] = v1 * LOG2E;
   }
   __syncthreads();
   // Mask sums on the tensor core.  With r0(s) the first row of s's 16-row block,
@@ -239,20 +246,20 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   {
     const uint32_t hb = smem_u32(sm.img_h());
     for (int idx = tid; idx < 64 * E; idx += MASK_THREADS) {
-      const int rr = idx / E, e = idx % E;
-      const float up = sm.gc2[(rr & ~15) * E + e] - sm.gc2[idx];   // >= 0 when gc does not increase
+      const int rr = idx / E, e = idx % E, o = rr * ES + e;
+      const float up = sm.gc2[(rr & ~15) * ES + e] - sm.gc2[o];   // >= 0 when gc does not increase
       // too steep, NaN, or not monotone: a log gate above zero anywhere in the chunk makes gc rise from one row to the
       // next, and the factorised form (which clamps its first factor at one) would then be wrong for rows of later blocks
-      if (!(up <= 100.f) || up < 0.f || (rr > 0 && sm.gc2[idx] > sm.gc2[idx - E])) sm.steep = 1;
+      if (!(up <= 100.f) || up < 0.f || (rr > 0 && sm.gc2[o] > sm.gc2[o - ES])) sm.steep = 1;
       // the gate factors of the recurrences, formed here once instead of by every value block of every recurrence
       {
-        const float eg = fast_exp2(sm.gc2[idx]), k2v = sm.k2[idx];
+        const float eg = fast_exp2(sm.gc2[o]), k2v = sm.k2[o];
         gc_out[64 * E + idx] = k2v * eg;
-        gc_out[128 * E + idx] = k2v * fast_exp2(sm.gc2[63 * E + e] - sm.gc2[idx]);
-        gc_out[192 * E + idx] = p.scale * sm.q2[idx] * eg;
-        if (idx < 16) gc_out[256 * E + idx] = idx < E ? fast_exp2(sm.gc2[63 * E + idx]) : 0.f;
+        gc_out[128 * E + idx] = k2v * fast_exp2(sm.gc2[63 * ES + e] - sm.gc2[o]);
+        gc_out[192 * E + idx] = p.scale * sm.q2[o] * eg;
+        if (idx < 16) gc_out[256 * E + idx] = idx < E ? fast_exp2(sm.gc2[63 * ES + idx]) : 0.f;
       }
-      const float hv = fast_exp2(up) * sm.k2[idx];
+      const float hv = fast_exp2(up) * sm.k2[o];
       const float hi = round_bf16(hv), lo = hv - hi;
       const uint32_t row = hb + (rr >> 3) * 128 + (rr & 7) * 16;
       st_shared_b16(row + (e >> 3) * 1024 + (e & 7) * 2, hi);                                    // first image:  [hi | hi]
@@ -266,8 +273,8 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     float my2[E], mygc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      my2[e] = isq ? sm.q2[t * E + e] : sm.k2[t * E + e];
-      mygc[e] = sm.gc2[t * E + e];
+      my2[e] = isq ? sm.q2[t * ES + e] : sm.k2[t * ES + e];
+      mygc[e] = sm.gc2[t * ES + e];
     }
 #pragma unroll
     for (int ii = 0; ii < 2; ++ii) {
@@ -277,7 +284,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       for (int k = 0; k < KP; ++k) vals[k] = 0.f;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const float g = my2[e] * fast_exp2(fminf(mygc[e] - sm.gc2[(16 * i) * E + e], 0.f));   // rows above the block are masked later
+        const float g = my2[e] * fast_exp2(fminf(mygc[e] - sm.gc2[(16 * i) * ES + e], 0.f));   // rows above the block are masked later
         vals[e] = round_bf16(g);
         vals[E + e] = g - vals[e];
       }
@@ -364,8 +371,8 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       float my2[E], mygc[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        my2[e] = isq ? sm.q2[t * E + e] : sm.k2[t * E + e];
-        mygc[e] = sm.gc2[t * E + e];
+        my2[e] = isq ? sm.q2[t * ES + e] : sm.k2[t * ES + e];
+        mygc[e] = sm.gc2[t * ES + e];
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -381,7 +388,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
             float acc = 0.f;
 #pragma unroll
             for (int e = 0; e < E; ++e)
-              acc = fmaf(my2[e] * sm.k2[s * E + e], fast_exp2(mygc[e] - sm.gc2[s * E + e]), acc);
+              acc = fmaf(my2[e] * sm.k2[s * ES + e], fast_exp2(mygc[e] - sm.gc2[s * ES + e]), acc);
             val = rowscale * pr8[c] * acc;
           }
           pr8[c] = val;
