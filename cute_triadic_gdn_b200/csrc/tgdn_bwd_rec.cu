@@ -44,27 +44,6 @@
 
 namespace tgdn {
 
-// N floats of a gate row in shared memory; 16-byte loads where N allows (the offsets used are then 16-byte aligned too),
-// 8-byte loads otherwise (N even)
-template <int N>
-__device__ __forceinline__ void rec_lds_part(const float* p, float* out) {
-  if constexpr (N == 1) {
-    out[0] = p[0];
-  } else if constexpr (N % 4 == 0) {
-#pragma unroll
-    for (int j = 0; j < N / 4; ++j) {
-      const float4 x = *(reinterpret_cast<const float4*>(p) + j);
-      out[4 * j] = x.x; out[4 * j + 1] = x.y; out[4 * j + 2] = x.z; out[4 * j + 3] = x.w;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < N / 2; ++j) {
-      const float2 x = *(reinterpret_cast<const float2*>(p) + j);
-      out[2 * j] = x.x; out[2 * j + 1] = x.y;
-    }
-  }
-}
-
 // The CTA is two independent CHAINS of two warpgroups, each owning half of the value columns of every slice: own MMAs, own barriers,
 // own named barrier.  While one chain's threads are in an epilogue the tensor core works for the other one.  (One lockstep CTA of
 // four warpgroups took 9.5 k cycles per chunk at E = 8, of which its products were in flight for 4.6 k and its epilogues ran for
@@ -451,9 +430,9 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     float bt = 0.f;
     {
       const float* gf = reinterpret_cast<const float*>(smem + C::OFF_GT + st * C::GT_STRIDE);
-      rec_lds_part<EL>(gf + (krow ? 0 : C::GF_C) + t * E + e0, ga);
+      lds_row<E, EL>(gf + (krow ? 0 : C::GF_C), t, e0, ga);
       if (krow) {
-        rec_lds_part<EL>(gf + C::GF_R + t * E + e0, gr);
+        lds_row<E, EL>(gf + C::GF_R, t, e0, gr);
         bt = __ldg(p.beta + (tok + min(t, max(rows, 1) - 1)) * p.H + h);   // masked where it is used, after (c): nothing here waits for it
         const Piece up = image_piece(duimg);
         // Xu_e = r_e * U -> operand image (i = t, j = n') of (p)

@@ -281,6 +281,41 @@ __device__ __forceinline__ void umma_ksteps(uint32_t d_tmem, uint64_t adesc, uin
               (accumulate || k > 0) ? 1u : 0u);
 }
 
+// N floats from shared memory; 16-byte loads where N and the address allow, else 8-byte loads (N even) or one float
+template <int N>
+__device__ __forceinline__ void lds_part(const float* p, float* out) {
+  if constexpr (N == 1) {
+    out[0] = p[0];
+  } else if constexpr (N % 4 == 0) {
+#pragma unroll
+    for (int j = 0; j < N / 4; ++j) {
+      const float4 x = *(reinterpret_cast<const float4*>(p) + j);
+      out[4 * j] = x.x; out[4 * j + 1] = x.y; out[4 * j + 2] = x.z; out[4 * j + 3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < N / 2; ++j) {
+      const float2 x = *(reinterpret_cast<const float2*>(p) + j);
+      out[2 * j] = x.x; out[2 * j + 1] = x.y;
+    }
+  }
+}
+// N floats from entry e0 on of row t of a dense table of E floats a row, where the lanes of a warp read a row each.  Rows of 32 and
+// 64 bytes put every second or fourth lane on the same banks (sixteen wavefronts a load instead of four): there the lanes take the two
+// 16-byte pieces in an order that depends on the row (ORDERED).
+template <int E, int N, bool ORDERED = E == 8 || E == 16>
+__device__ __forceinline__ void lds_row(const float* table, int t, int e0, float* out) {
+  const float* p = table + t * E + e0;
+  if constexpr (ORDERED && N == 8) {
+    const bool swap = (t & (E == 8 ? 4 : 2)) != 0;
+    const float4 x = *reinterpret_cast<const float4*>(p + (swap ? 4 : 0)), y = *reinterpret_cast<const float4*>(p + (swap ? 0 : 4));
+    out[0] = swap ? y.x : x.x; out[1] = swap ? y.y : x.y; out[2] = swap ? y.z : x.z; out[3] = swap ? y.w : x.w;
+    out[4] = swap ? x.x : y.x; out[5] = swap ? x.y : y.y; out[6] = swap ? x.z : y.z; out[7] = swap ? x.w : y.w;
+  } else {
+    lds_part<N>(p, out);
+  }
+}
+
 // Two f32 fused multiply-adds in one instruction (each lane an ordinary fma): the epilogues of the recurrences are bound by
 // instruction issue.
 __device__ __forceinline__ void fma_pair(float& a0, float& a1, float f, float x0, float x1) {        // a += f * x

@@ -44,26 +44,6 @@ __device__ __forceinline__ void chain_sync(int chain) {     // the threads of on
   asm volatile("bar.sync %0, %1;" ::"r"(chain + 1), "n"(THREADS) : "memory");
 }
 
-// N floats from shared memory; 16-byte loads where N and the address allow, else 8-byte loads (N even) or one float
-template <int N>
-__device__ __forceinline__ void lds_part(const float* p, float* out) {
-  if constexpr (N == 1) {
-    out[0] = p[0];
-  } else if constexpr (N % 4 == 0) {
-#pragma unroll
-    for (int j = 0; j < N / 4; ++j) {
-      const float4 x = *(reinterpret_cast<const float4*>(p) + j);
-      out[4 * j] = x.x; out[4 * j + 1] = x.y; out[4 * j + 2] = x.z; out[4 * j + 3] = x.w;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < N / 2; ++j) {
-      const float2 x = *(reinterpret_cast<const float2*>(p) + j);
-      out[2 * j] = x.x; out[2 * j + 1] = x.y;
-    }
-  }
-}
-
 // WS = 2 warpgroups share one chain and split its SLICES (warpgroup w of a chain owns slices w*E/WS ..): the chain's MMAs
 // then have N = E*CW columns with CW = 8 columns per thread even at twelve and sixteen slices, where a warpgroup alone
 // could hold only four columns of every slice in its registers; the sums over the slices (W, and the state part of o) are
@@ -374,9 +354,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       for (int c = 0; c < CW / 2; ++c) vraw[c] = 0u;
     }
     {
-      lds_part<ET>(gf + (krow ? 0 : C::GF_C) + t * E + e0, ga);
+      // (at eight slices the selects of the ordered form cost the two chains more than its bank conflicts: 570 -> 622 us, 16384 items
+      // without saved state; at sixteen it takes 1662 -> 1585 us, packed)
+      lds_row<E, ET, E == 16>(gf + (krow ? 0 : C::GF_C), t, e0, ga);
       if (krow) {
-        if constexpr (!LATE_R) lds_part<ET>(gf + C::GF_R + t * E + e0, gr);
+        if constexpr (!LATE_R) lds_row<E, ET, E == 16>(gf + C::GF_R, t, e0, gr);
         if (sw == 0) {                               // the warpgroup that completes W: beta and the value row
           if (beta_tma) {
             bt = reinterpret_cast<const float*>(smem + C::OFF_BT + st * C::BT_BYTES)[t * 4 + (h & 3)];
@@ -477,7 +459,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     __syncwarp();
     if (PACKED && i + 1 < count) chunk_info(i + 1, t0_next, rows_next);
     if constexpr (LATE_R) {                          // r_e only now, from the stage: sixteen registers fewer are live
-      if (krow) lds_part<ET>(gf + C::GF_R + t * E + e0, gr);   // through the epilogue of (1)
+      if (krow) lds_row<E, ET, E == 16>(gf + C::GF_R, t, e0, gr);   // through the epilogue of (1)
     }
     if (cwarp_u == ISSUE_WARP) mbar_wait(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     chain_sync<CT>(chain);
