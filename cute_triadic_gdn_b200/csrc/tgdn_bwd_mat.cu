@@ -19,7 +19,7 @@
 // five product groups with the sums over the slices between them (f32 on the ordinary pipes).  Hence the two independent chains,
 // the two-wide f32 instructions for those sums, L2 prefetch of the next item, and 16-byte pieces wherever a thread owns a row; the
 // column sums of dA'*A are exchanges inside the warps, before G3, instead of a matrix in shared memory that is walked by columns
-// after it.  us, before (first these, then the two-wide sums) and after: 16384 items E8 575 -> 519; 4096 items E8 mild 303 -> 268,
+// after it.  us, before (first these, then the two-wide sums) and after: 8192 items E8 575 -> 519; 4096 items E8 mild 303 -> 268,
 // E4 248 -> 231, E1 222 -> 211; packed E16 900 -> 875.
 //
 // Replaces cute_triadic_gdn/kernels/sm100_joint_bwd_parallel.py:80-405 (matrix_kernel),

@@ -22,7 +22,7 @@
 // bounds this kernel, and the independent chains per SM are what hides it.  Next to it come instruction issue (hence the two-wide
 // f32 multiply-adds) and the copy engine: it moves a row of a tile a cycle and writes 32 bytes a cycle, so o, W and U leave as
 // tiles as wide as a chain, the state leaves by stores, and later chunks are pulled into L2 by the threads.
-// us, before all three and after: 16384 items E8 850 -> 764, without saved state 717 -> 573; 4096 items E4 250 -> 209, 190 -> 160;
+// us, before all three and after: 8192 items E8 850 -> 764, without saved state 717 -> 573; 4096 items E4 250 -> 209, 190 -> 160;
 // E2 201 -> 152, 149 -> 129; E1 187 -> 133, 138 -> 111; packed E16 1658 -> 1663, 1450 -> 1264; E12 778 -> 745, 694 -> 569.
 //
 // The gate factors of a chunk (a, r, c per row and slice, d per slice) were formed by the masks kernel and arrive in the
@@ -201,7 +201,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
   // Sixteen of this thread's state columns -> h of a chunk, slice e as [v / 8][d][v % 8].  A warp's 16-byte stores cover 512
   // contiguous bytes, and the threads store: the copy engine writes 32 bytes a cycle, which for the state alone (E * 8 KB per 32
   // value columns and chunk) was a third of the chunk, with o, W and U and the next loads queued behind it.  us, copies -> stores:
-  // 16384 items E8 850 -> 760; 4096 items E4 250 -> 208, E2 201 -> 153, E1 187 -> 134.
+  // 8192 items E8 850 -> 760; 4096 items E4 250 -> 208, E2 201 -> 153, E1 187 -> 134.
   auto save_state = [&](int64_t item, int j0, const uint32_t* w) {
     uint8_t* dst = reinterpret_cast<uint8_t*>(p.h) + (item * E + e0) * 32768 + (v0g >> 3) * 2048 + row * 16;
 #pragma unroll
@@ -354,7 +354,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       for (int c = 0; c < CW / 2; ++c) vraw[c] = 0u;
     }
     {
-      // (at eight slices the selects of the ordered form cost the two chains more than its bank conflicts: 570 -> 622 us, 16384 items
+      // (at eight slices the selects of the ordered form cost the two chains more than its bank conflicts: 570 -> 622 us, 8192 items
       // without saved state; at sixteen it takes 1662 -> 1585 us, packed)
       lds_row<E, ET, E == 16>(gf + (krow ? 0 : C::GF_C), t, e0, ga);
       if (krow) {
@@ -637,7 +637,7 @@ int tgdn_fwd_rows(const void* q, const void* k, const void* v, const float* k2, 
   const long long narrow = (seqs * 4 + sms - 1) / sms, wide = (seqs * 2 + sms - 1) / sms;
   // Chains: two of two warpgroups (WV = 2, twice the columns per MMA) do better than four of one wherever the state is not saved,
   // and at one and two slices; at four and eight slices the state's stores want the four chains' finer interleaving.
-  // us, four chains -> two: 16384 items E8 forward alone 618 -> 573, with saved state 764 -> 780; 4096 items E4 176 -> 160, 209 -> 220,
+  // us, four chains -> two: 8192 items E8 forward alone 618 -> 573, with saved state 764 -> 780; 4096 items E4 176 -> 160, 209 -> 220,
   // E2 135 -> 129, 156 -> 152, E1 127 -> 111, 152 -> 133.
   const bool save = W != nullptr || U != nullptr || h != nullptr;
 #define TGDN_FWD(E, CW, NCH, WS, WV) \

@@ -19,7 +19,7 @@
 //     merges X21 = -X22 (L21 X11) as warp-level mma.sync m16n8k8 products with a 3-term TF32 split (f32-grade accuracy).
 //   * What bounds it: the chain of these steps, with five block barriers, hidden by three CTAs per SM (two at twelve and sixteen slices),
 //     and the shared-memory wavefronts inside them; hence padded rows in 16-byte pieces everywhere.  us, before (swizzled single
-//     floats, two CTAs per SM) and after: 16384 items E8 355 -> 240; 4096 items E4 179 -> 110, E2 179 -> 105, E1 176 -> 100; packed
+//     floats, two CTAs per SM) and after: 8192 items E8 355 -> 240; 4096 items E4 179 -> 110, E2 179 -> 105, E1 176 -> 100; packed
 //     E16 561 -> 370, E12 238 -> 171.
 //   * PA = Pm A: a second tcgen05 MMA group on the bf16 images of Pm and A that are about to be stored anyway.
 #include "tgdn_common.cuh"
