@@ -17,10 +17,10 @@
 //   * Mask sums: thread (row, column half) with the half's 8-column blocks interleaved so that the triangle is balanced.
 //   * Triangular inverse in f32: eight 8x8 diagonal blocks by forward substitution, an 8->16 step, then the 16->32 and 32->64
 //     merges X21 = -X22 (L21 X11) as warp-level mma.sync m16n8k8 products with a 3-term TF32 split (f32-grade accuracy).
-//   * What bounds it: the chain of these steps, with five block barriers, hidden by three CTAs per SM (two at twelve and sixteen slices),
-//     and the shared-memory wavefronts inside them; hence padded rows in 16-byte pieces everywhere.  us, before (swizzled single
-//     floats, two CTAs per SM) and after: 8192 items E8 355 -> 240; 4096 items E4 179 -> 110, E2 179 -> 105, E1 176 -> 100; packed
-//     E16 561 -> 370, E12 238 -> 171.
+//   * What bounds it: the chain of these steps, with five block barriers, hidden by four CTAs per SM (three at twelve and sixteen slices:
+//     registers), and the shared-memory wavefronts inside them; hence one buffer for tile, operand images, L and X and [A; PA] in turn,
+//     and padded rows in 16-byte pieces everywhere.  us, before (swizzled single floats, two CTAs per SM) and after: 8192 items E8
+//     355 -> 220; 4096 items E4 179 -> 105, E2 179 -> 96, E1 176 -> 91; packed E16 561 -> 316, E12 238 -> 145.
 //   * PA = Pm A: a second tcgen05 MMA group on the bf16 images of Pm and A that are about to be stored anyway.
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
@@ -75,33 +75,34 @@ __device__ __forceinline__ void mma_step_3x(float* c, FA a_at, FB b_at, int lane
 
 template <int E>
 struct MaskSmem {
-  // KQ tile (two 64-column blocks of 128 rows x 128 B) while the Gram product runs; L and X afterwards
-  union {
-    uint8_t kq[32768];
-    struct { float L[64 * MAT_LD]; float X[64 * MAT_LD]; } m;
-  } u;
-  alignas(16) float T[32 * T_LD];
-  uint8_t img_ap[16384];   // [A; PA] image (i = row 0..127, j = column), SI = 128, SJ = 2048
-  uint8_t gpad[E > 8 ? 12288 : 16];   // room for the G images at twelve and sixteen slices
-  uint8_t img_pm[8192];    // Pm image (i = t, j = s), SI = 128, SJ = 1024; read as 128 rows by the PA product: keep >= 8 KB behind it
   static constexpr int ES = E == 8 || E == 16 ? E + 4 : E;   // rows of 48 and 80 bytes: 32 lanes read a row each without bank conflicts
-  alignas(16) float gc2[64 * ES];    // log2-domain cumulative gate
-  float k2[64 * ES];
-  float q2[64 * ES];
-  float pad[(3 * 64 * ES * 4 >= 8192) ? 1 : (8192 - 3 * 64 * ES * 4) / 4];
+  // Operands of the mask-sum products (see the kernel):
+  //   G images: four blocks of (128 rows x KP) bf16, image (i = row, j = k), SI = 128, SJ = 2048
+  //   H images: two of (64 rows x KP) bf16, image (i = s, j = k), SI = 128, SJ = 1024
+  static constexpr int KP = 2 * E <= 16 ? 16 : 32;         // [hi | lo] halves of the E factors, padded to the MMA's K = 16
+  static constexpr int G_BYTES = KP / 8 * 2048, H_BYTES = KP / 8 * 1024;
+  // Pm image (i = t, j = s), SI = 128, SJ = 1024; read as 128 rows by the PA product, 8 KB into what follows.  The H images before it.
+  uint8_t img_pm[8192];
+  union {                  // one after the other:
+    uint8_t kq[32768];     //   [K;Q] tile, until the Gram product is done
+    uint8_t g[4 * G_BYTES];   //   G images, until the mask-sum products are done
+    struct { float L[64 * MAT_LD]; float X[64 * MAT_LD]; } m;
+    uint8_t img_ap[16384]; //   [A; PA] image (i = row 0..127, j = column), SI = 128, SJ = 2048, in the place of L
+  } u;
+  union {
+    struct {
+      float gc2[64 * ES];  // log2-domain cumulative gate
+      float k2[64 * ES];
+      float q2[64 * ES];
+    } t;
+    alignas(16) float T[32 * T_LD];   // scratch of the inverse
+  } v;
   float beta[64];
   uint64_t bar_load, bar_mma;
   uint32_t tmem_base;
   int abort;
   int steep;               // a 16-row block decays by more than 2^-100 (or gc is not monotone): direct decay path
-  // Operands of the mask-sum products (see the kernel), in buffers that are written only after those products are done:
-  //   G images: four blocks of (128 rows x KP) bf16, image (i = row, j = k), SI = 128, SJ = 2048, over T, img_ap, gpad
-  //   H images: two of (64 rows x KP) bf16, image (i = s, j = k), SI = 128, SJ = 1024, over img_pm
-  static constexpr int KP = 2 * E <= 16 ? 16 : 32;         // [hi | lo] halves of the E factors, padded to the MMA's K = 16
-  static constexpr int G_BYTES = KP / 8 * 2048, H_BYTES = KP / 8 * 1024;
-  __device__ uint8_t* img_g() { return reinterpret_cast<uint8_t*>(T); }
-  __device__ uint8_t* img_h() { return img_pm; }
-  static_assert(4 * G_BYTES <= static_cast<int>(sizeof(T) + sizeof(img_ap) + sizeof(gpad)) && 2 * H_BYTES <= 8192, "operand images fit the buffers they borrow");
+  static_assert(2 * H_BYTES <= 8192 && 16384 <= 64 * MAT_LD * 4, "images fit the buffers they borrow");
 };
 
 // X21 = -X22 (L21 X11) for the diagonal blocks of size 2n (n = 16: two blocks, n = 32: one), one 16x8 tile per warp.
@@ -143,7 +144,7 @@ __device__ __forceinline__ void tri_merge_mma(const float* L, float* X, float* T
 }
 
 template <int E>
-__global__ void __launch_bounds__(MASK_THREADS, E > 8 ? 2 : 3)
+__global__ void __launch_bounds__(MASK_THREADS, E > 8 ? 3 : 4)
 masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q, MaskParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   using SM = MaskSmem<E>;
@@ -184,7 +185,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   }
   __syncwarp();
   if (warp_u == 0) { tmem_alloc(&sm.tmem_base, 128); tmem_relinquish(); }
-  for (int i = tid; i < 2 * SM::H_BYTES / 16; i += MASK_THREADS) reinterpret_cast<uint4*>(sm.img_h())[i] = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < 2 * SM::H_BYTES / 16; i += MASK_THREADS) reinterpret_cast<uint4*>(sm.img_pm)[i] = make_uint4(0, 0, 0, 0);
 
   // gates of the chunk: rows past the document end count as g = 0, k2 = q2 = beta = 0.  All loads are requested first, from
   // clamped (always valid) addresses, and masked when stored: the block pays one memory round trip, not one per iteration.
@@ -207,9 +208,9 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       if (idx < 64 * E) {
         const int o = idx / E * ES + idx % E;
         const bool ok = idx / E < rows;
-        sm.gc2[o] = ok ? g_in[it] : 0.f;
-        sm.k2[o] = ok ? k2_in[it] : 0.f;
-        sm.q2[o] = ok ? q2_in[it] : 0.f;
+        sm.v.t.gc2[o] = ok ? g_in[it] : 0.f;
+        sm.v.t.k2[o] = ok ? k2_in[it] : 0.f;
+        sm.v.t.q2[o] = ok ? q2_in[it] : 0.f;
       }
     }
     if (tid < 64) sm.beta[tid] = (tid < rows) ? beta_in : 0.f;
@@ -217,10 +218,27 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();                                          // gate values, barriers and the tensor-memory address are visible
   tc_fence_after();
+  // Gram product [K;Q] K^T, under the scan and the first images
+  const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
+  if (warp_u == MASK_THREADS / 32 - 1) {                    // (the last warp: up to seven slices it has no column to scan)
+    mbar_wait(&sm.bar_load, 0, ctl, DEV_TIMEOUT_LOAD);
+    if (elect_one()) {
+      tc_fence_after();
+      const uint64_t desc = make_desc(smem_u32(sm.u.kq), 16, 1024, LAYOUT_SW128);
+      constexpr uint32_t idesc = make_idesc(128, 64, 0, 0);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
+        umma_bf16(tmem, desc_advance(desc, off), desc_advance(desc, off), idesc, kk > 0);
+      }
+      umma_commit(&sm.bar_mma);
+    }
+    __syncwarp();
+  }
   // inclusive scan over the 64 rows, one warp per gate column
   float* gc_out = p.gc + ((static_cast<int64_t>(b) * p.NC + n) * p.H + h) * gate_item_floats(E);
   for (int e = warp; e < E; e += MASK_THREADS / 32) {
-    float v0 = sm.gc2[lane * ES + e], v1 = sm.gc2[(lane + 32) * ES + e];
+    float v0 = sm.v.t.gc2[lane * ES + e], v1 = sm.v.t.gc2[(lane + 32) * ES + e];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const float a0 = __shfl_up_sync(0xffffffffu, v0, o), a1 = __shfl_up_sync(0xffffffffu, v1, o);
@@ -229,8 +247,8 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     v1 += __shfl_sync(0xffffffffu, v0, 31);
     gc_out[lane * E + e] = v0;
     gc_out[(lane + 32) * E + e] = v1;
-    sm.gc2[lane * ES + e] = v0 * LOG2E;
-    sm.gc2[(lane + 32) * ES + e] = v1 * LOG2E;
+    sm.v.t.gc2[lane * ES + e] = v0 * LOG2E;
+    sm.v.t.gc2[(lane + 32) * ES + e] = v1 * LOG2E;
   }
   __syncthreads();
   // Mask sums on the tensor core.  With r0(s) the first row of s's 16-row block,
@@ -244,22 +262,22 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   // flush of the first factor could then hide a product of order one) the CTA takes one exponential per (t, s, e) instead.
   constexpr int KP = SM::KP;
   {
-    const uint32_t hb = smem_u32(sm.img_h());
+    const uint32_t hb = smem_u32(sm.img_pm);
     for (int idx = tid; idx < 64 * E; idx += MASK_THREADS) {
       const int rr = idx / E, e = idx % E, o = rr * ES + e;
-      const float up = sm.gc2[(rr & ~15) * ES + e] - sm.gc2[o];   // >= 0 when gc does not increase
+      const float up = sm.v.t.gc2[(rr & ~15) * ES + e] - sm.v.t.gc2[o];   // >= 0 when gc does not increase
       // too steep, NaN, or not monotone: a log gate above zero anywhere in the chunk makes gc rise from one row to the
       // next, and the factorised form (which clamps its first factor at one) would then be wrong for rows of later blocks
-      if (!(up <= 100.f) || up < 0.f || (rr > 0 && sm.gc2[o] > sm.gc2[o - ES])) sm.steep = 1;
+      if (!(up <= 100.f) || up < 0.f || (rr > 0 && sm.v.t.gc2[o] > sm.v.t.gc2[o - ES])) sm.steep = 1;
       // the gate factors of the recurrences, formed here once instead of by every value block of every recurrence
       {
-        const float eg = fast_exp2(sm.gc2[o]), k2v = sm.k2[o];
+        const float eg = fast_exp2(sm.v.t.gc2[o]), k2v = sm.v.t.k2[o];
         gc_out[64 * E + idx] = k2v * eg;
-        gc_out[128 * E + idx] = k2v * fast_exp2(sm.gc2[63 * ES + e] - sm.gc2[o]);
-        gc_out[192 * E + idx] = p.scale * sm.q2[o] * eg;
-        if (idx < 16) gc_out[256 * E + idx] = idx < E ? fast_exp2(sm.gc2[63 * ES + idx]) : 0.f;
+        gc_out[128 * E + idx] = k2v * fast_exp2(sm.v.t.gc2[63 * ES + e] - sm.v.t.gc2[o]);
+        gc_out[192 * E + idx] = p.scale * sm.v.t.q2[o] * eg;
+        if (idx < 16) gc_out[256 * E + idx] = idx < E ? fast_exp2(sm.v.t.gc2[63 * ES + idx]) : 0.f;
       }
-      const float hv = fast_exp2(up) * sm.k2[o];
+      const float hv = fast_exp2(up) * sm.v.t.k2[o];
       const float hi = round_bf16(hv), lo = hv - hi;
       const uint32_t row = hb + (rr >> 3) * 128 + (rr & 7) * 16;
       st_shared_b16(row + (e >> 3) * 1024 + (e & 7) * 2, hi);                                    // first image:  [hi | hi]
@@ -269,12 +287,14 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   }
   const int t = r & 63;
   const bool isq = r >= 64;
+  mbar_wait_spin(&sm.bar_mma, 0, ctl, DEV_TIMEOUT_MMA);      // the G images take the tile's place
+  tc_fence_after();
   {
     float my2[E], mygc[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      my2[e] = isq ? sm.q2[t * ES + e] : sm.k2[t * ES + e];
-      mygc[e] = sm.gc2[t * ES + e];
+      my2[e] = isq ? sm.v.t.q2[t * ES + e] : sm.v.t.k2[t * ES + e];
+      mygc[e] = sm.v.t.gc2[t * ES + e];
     }
 #pragma unroll
     for (int ii = 0; ii < 2; ++ii) {
@@ -284,11 +304,11 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       for (int k = 0; k < KP; ++k) vals[k] = 0.f;
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        const float g = my2[e] * fast_exp2(fminf(mygc[e] - sm.gc2[(16 * i) * ES + e], 0.f));   // rows above the block are masked later
+        const float g = my2[e] * fast_exp2(fminf(mygc[e] - sm.v.t.gc2[(16 * i) * ES + e], 0.f));   // rows above the block are masked later
         vals[e] = round_bf16(g);
         vals[E + e] = g - vals[e];
       }
-      const uint32_t row = smem_u32(sm.img_g()) + i * SM::G_BYTES + (r >> 3) * 128 + (r & 7) * 16;
+      const uint32_t row = smem_u32(sm.u.g) + i * SM::G_BYTES + (r >> 3) * 128 + (r & 7) * 16;
 #pragma unroll
       for (int kb = 0; kb < KP / 8; ++kb)
         st_shared_v4(row + kb * 2048, pack_bf16(vals[8 * kb], vals[8 * kb + 1]), pack_bf16(vals[8 * kb + 2], vals[8 * kb + 3]),
@@ -300,24 +320,15 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
 
-  // Gram product [K;Q] K^T, then the four mask-sum products
-  mbar_wait(&sm.bar_load, 0, ctl, DEV_TIMEOUT_LOAD);
-  const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
+  // the four mask-sum products
   const uint32_t tmem_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   if (warp_u == 0 && elect_one()) {
     tc_fence_after();
-    const uint64_t desc = make_desc(smem_u32(sm.u.kq), 16, 1024, LAYOUT_SW128);
-    constexpr uint32_t idesc = make_idesc(128, 64, 0, 0);
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-      umma_bf16(tmem, desc_advance(desc, off), desc_advance(desc, off), idesc, kk > 0);
-    }
     constexpr uint32_t idm = make_idesc(128, 16, 0, 0);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint64_t da = make_desc(smem_u32(sm.img_g()) + i * SM::G_BYTES, 2048, 128, LAYOUT_PLAIN);
-      const uint64_t db = make_desc(smem_u32(sm.img_h()) + i * 256, 1024, 128, LAYOUT_PLAIN);
+      const uint64_t da = make_desc(smem_u32(sm.u.g) + i * SM::G_BYTES, 2048, 128, LAYOUT_PLAIN);
+      const uint64_t db = make_desc(smem_u32(sm.img_pm) + i * 256, 1024, 128, LAYOUT_PLAIN);
 #pragma unroll
       for (int kk = 0; kk < KP / 16; ++kk)
         umma_bf16(tmem + 64 + 16 * i, desc_advance(da, kk * 4096), desc_advance(db, kk * 2048), idm, kk > 0);
@@ -328,9 +339,9 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     umma_commit(&sm.bar_mma);
   }
   __syncwarp();                                           // the other lanes must not run ahead into a spin wait
-  mbar_wait_spin(&sm.bar_mma, 0, ctl, DEV_TIMEOUT_MMA);
+  mbar_wait_spin(&sm.bar_mma, 1, ctl, DEV_TIMEOUT_MMA);
   tc_fence_after();
-  // The KQ tile and the operand images are dead from here (every thread has seen the products complete): L, X, the Pm image take
+  // The operand images are dead from here (every thread has seen the products complete): L, X, the Pm image take
   // their places.  Rows 0..63 -> M (strictly lower) -> L, rows 64..127 -> Mp (lower) -> Pm.
   {
     const float rowscale = isq ? p.scale : sm.beta[t];
@@ -371,8 +382,8 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       float my2[E], mygc[E];
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        my2[e] = isq ? sm.q2[t * ES + e] : sm.k2[t * ES + e];
-        mygc[e] = sm.gc2[t * ES + e];
+        my2[e] = isq ? sm.v.t.q2[t * ES + e] : sm.v.t.k2[t * ES + e];
+        mygc[e] = sm.v.t.gc2[t * ES + e];
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -388,7 +399,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
             float acc = 0.f;
 #pragma unroll
             for (int e = 0; e < E; ++e)
-              acc = fmaf(my2[e] * sm.k2[s * ES + e], fast_exp2(mygc[e] - sm.gc2[s * ES + e]), acc);
+              acc = fmaf(my2[e] * sm.v.t.k2[s * ES + e], fast_exp2(mygc[e] - sm.v.t.gc2[s * ES + e]), acc);
             val = rowscale * pr8[c] * acc;
           }
           pr8[c] = val;
@@ -424,23 +435,23 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     float acc = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc = fmaf(L[mat_idx(r0 + 8 + i, r0 + k)], X[mat_idx(r0 + k, r0 + j)], acc);
-    sm.T[tid] = acc;
+    sm.v.T[tid] = acc;
     __syncthreads();
     float acc2 = 0.f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc2 = fmaf(X[mat_idx(r0 + 8 + i, r0 + 8 + k)], sm.T[(tid & ~63) + k * 8 + j], acc2);
+    for (int k = 0; k < 8; ++k) acc2 = fmaf(X[mat_idx(r0 + 8 + i, r0 + 8 + k)], sm.v.T[(tid & ~63) + k * 8 + j], acc2);
     X[mat_idx(r0 + 8 + i, r0 + j)] = -acc2;
   }
   __syncthreads();
-  tri_merge_mma<16>(L, X, sm.T, warp, lane);
-  tri_merge_mma<32>(L, X, sm.T, warp, lane);
+  tri_merge_mma<16>(L, X, sm.v.T, warp, lane);
+  tri_merge_mma<32>(L, X, sm.v.T, warp, lane);
 
   // bf16 image of A (rows 0..63 of the [A;PA] image): one 16-byte piece per thread and step
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int piece = it * MASK_THREADS + tid, i = piece & 63, jb = piece >> 6;
     const float4 a0 = *reinterpret_cast<const float4*>(X + mat_idx(i, jb * 8)), a1 = *reinterpret_cast<const float4*>(X + mat_idx(i, jb * 8 + 4));
-    st_shared_v4(smem_u32(sm.img_ap) + (i >> 3) * 128 + (i & 7) * 16 + jb * 2048, pack_bf16(a0.x, a0.y), pack_bf16(a0.z, a0.w),
+    st_shared_v4(smem_u32(sm.u.img_ap) + (i >> 3) * 128 + (i & 7) * 16 + jb * 2048, pack_bf16(a0.x, a0.y), pack_bf16(a0.z, a0.w),
                  pack_bf16(a1.x, a1.y), pack_bf16(a1.z, a1.w));
   }
   fence_async_smem();
@@ -451,20 +462,20 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   if (warp_u == 0 && elect_one()) {
     tc_fence_after();
     const uint64_t da = make_desc(smem_u32(sm.img_pm), 1024, 128, LAYOUT_PLAIN);   // Pm, K-major (rows past 63: don't care)
-    const uint64_t db = make_desc(smem_u32(sm.img_ap), 128, 2048, LAYOUT_PLAIN);   // A as (K = s, N = j), MN-major
+    const uint64_t db = make_desc(smem_u32(sm.u.img_ap), 128, 2048, LAYOUT_PLAIN);   // A as (K = s, N = j), MN-major
     constexpr uint32_t idesc = make_idesc(128, 64, 0, 1);
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) umma_bf16(tmem + 64, desc_advance(da, kk * 2048), desc_advance(db, kk * 256), idesc, kk > 0);
     umma_commit(&sm.bar_mma);
   }
   __syncwarp();                                           // the other lanes must not run ahead into a spin wait
-  mbar_wait_spin(&sm.bar_mma, 1, ctl, DEV_TIMEOUT_MMA);
+  mbar_wait_spin(&sm.bar_mma, 0, ctl, DEV_TIMEOUT_MMA);
   tc_fence_after();
   if (r < 64) {                                             // PA row r, columns 32*ch .. +32 -> rows 64.. of the image
     float pa[32];
     tmem_ld<32>(tmem_row + 64 + 32 * ch, pa);
     tmem_wait_ld();
-    const uint32_t base = smem_u32(sm.img_ap) + ((64 + r) >> 3) * 128 + (r & 7) * 16;
+    const uint32_t base = smem_u32(sm.u.img_ap) + ((64 + r) >> 3) * 128 + (r & 7) * 16;
 #pragma unroll
     for (int jb = 0; jb < 4; ++jb)
       st_shared_v4(base + (4 * ch + jb) * 2048, pack_bf16(pa[jb * 8], pa[jb * 8 + 1]), pack_bf16(pa[jb * 8 + 2], pa[jb * 8 + 3]),
@@ -477,7 +488,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   const int64_t item = (static_cast<int64_t>(b) * p.NC + n) * p.H + h;
   uint4* ap_out = reinterpret_cast<uint4*>(p.AP + item * (128 * 64));
   uint4* pm_out = reinterpret_cast<uint4*>(p.Pm + item * (64 * 64));
-  const uint4* ap_src = reinterpret_cast<const uint4*>(sm.img_ap);
+  const uint4* ap_src = reinterpret_cast<const uint4*>(sm.u.img_ap);
   const uint4* pm_src = reinterpret_cast<const uint4*>(sm.img_pm);
 #pragma unroll
   for (int it = 0; it < 4; ++it) ap_out[it * MASK_THREADS + tid] = ap_src[it * MASK_THREADS + tid];
