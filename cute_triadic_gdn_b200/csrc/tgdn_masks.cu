@@ -468,6 +468,11 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     for (int kk = 0; kk < 4; ++kk) umma_bf16(tmem + 64, desc_advance(da, kk * 2048), desc_advance(db, kk * 256), idesc, kk > 0);
     umma_commit(&sm.bar_mma);
   }
+  const int64_t item = (static_cast<int64_t>(b) * p.NC + n) * p.H + h;
+  if (warp_u == 2 && elect_one()) {                         // (a warp without PA rows)
+    bulk_store(p.Pm + item * (64 * 64), sm.img_pm, 8192);
+    bulk_commit_group();
+  }
   __syncwarp();                                           // the other lanes must not run ahead into a spin wait
   mbar_wait_spin(&sm.bar_mma, 0, ctl, DEV_TIMEOUT_MMA);
   tc_fence_after();
@@ -481,19 +486,15 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       st_shared_v4(base + (4 * ch + jb) * 2048, pack_bf16(pa[jb * 8], pa[jb * 8 + 1]), pack_bf16(pa[jb * 8 + 2], pa[jb * 8 + 3]),
                    pack_bf16(pa[jb * 8 + 4], pa[jb * 8 + 5]), pack_bf16(pa[jb * 8 + 6], pa[jb * 8 + 7]));
   }
+  fence_async_smem();
   tc_fence_before();
   __syncthreads();
-
-  // images -> global, linear 16-byte copies
-  const int64_t item = (static_cast<int64_t>(b) * p.NC + n) * p.H + h;
-  uint4* ap_out = reinterpret_cast<uint4*>(p.AP + item * (128 * 64));
-  uint4* pm_out = reinterpret_cast<uint4*>(p.Pm + item * (64 * 64));
-  const uint4* ap_src = reinterpret_cast<const uint4*>(sm.u.img_ap);
-  const uint4* pm_src = reinterpret_cast<const uint4*>(sm.img_pm);
-#pragma unroll
-  for (int it = 0; it < 4; ++it) ap_out[it * MASK_THREADS + tid] = ap_src[it * MASK_THREADS + tid];
-#pragma unroll
-  for (int it = 0; it < 2; ++it) pm_out[it * MASK_THREADS + tid] = pm_src[it * MASK_THREADS + tid];
+  if (warp_u == 2 && elect_one()) {                         // the images leave as they are
+    bulk_store(p.AP + item * (128 * 64), sm.u.img_ap, 16384);
+    bulk_commit_group();
+    bulk_wait_group_read();                                 // before the block's shared memory goes to the next one
+  }
+  __syncwarp();
   if (warp == 0) tmem_dealloc(tmem, 128);
 }
 
