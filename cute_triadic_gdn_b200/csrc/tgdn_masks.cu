@@ -76,6 +76,9 @@ __device__ __forceinline__ void mma_step_3x(float* c, FA a_at, FB b_at, int lane
 template <int E>
 struct MaskSmem {
   static constexpr int ES = E == 8 || E == 16 ? E + 4 : E;   // rows of 48 and 80 bytes: 32 lanes read a row each without bank conflicts
+  // Above eight slices gc is stored by rows with the gate factors (a column at a time writes four bytes of every sector: packed E16
+  // 315 -> 302 us; up to eight the scan stores its columns, the detour costs what it gives).
+  static constexpr bool ROWS = E > 8;
   // Operands of the mask-sum products (see the kernel):
   //   G images: four blocks of (128 rows x KP) bf16, image (i = row, j = k), SI = 128, SJ = 2048
   //   H images: two of (64 rows x KP) bf16, image (i = s, j = k), SI = 128, SJ = 1024
@@ -92,6 +95,7 @@ struct MaskSmem {
   union {
     struct {
       float gc2[64 * ES];  // log2-domain cumulative gate
+      float gc[ROWS ? 64 * ES : 1];   // the same as it is stored
       float k2[64 * ES];
       float q2[64 * ES];
     } t;
@@ -245,8 +249,13 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       if (lane >= o) { v0 += a0; v1 += a1; }
     }
     v1 += __shfl_sync(0xffffffffu, v0, 31);
-    gc_out[lane * E + e] = v0;
-    gc_out[(lane + 32) * E + e] = v1;
+    if constexpr (SM::ROWS) {
+      sm.v.t.gc[lane * ES + e] = v0;
+      sm.v.t.gc[(lane + 32) * ES + e] = v1;
+    } else {
+      gc_out[lane * E + e] = v0;
+      gc_out[(lane + 32) * E + e] = v1;
+    }
     sm.v.t.gc2[lane * ES + e] = v0 * LOG2E;
     sm.v.t.gc2[(lane + 32) * ES + e] = v1 * LOG2E;
   }
@@ -272,6 +281,7 @@ masks_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       // the gate factors of the recurrences, formed here once instead of by every value block of every recurrence
       {
         const float eg = fast_exp2(sm.v.t.gc2[o]), k2v = sm.v.t.k2[o];
+        if constexpr (SM::ROWS) gc_out[idx] = sm.v.t.gc[o];
         gc_out[64 * E + idx] = k2v * eg;
         gc_out[128 * E + idx] = k2v * fast_exp2(sm.v.t.gc2[63 * ES + e] - sm.v.t.gc2[o]);
         gc_out[192 * E + idx] = p.scale * sm.v.t.q2[o] * eg;
