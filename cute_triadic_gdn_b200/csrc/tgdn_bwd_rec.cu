@@ -97,7 +97,7 @@ struct RecCfg {
     const int xu = XU_BYTES < 8192 ? 8192 : XU_BYTES;
     const int upto_dt = STAGES * KQ_BYTES + GX_BYTES + nb * (PM_BYTES + A_BYTES) + xu + 2 * STAGES * DOB + DRP_FLOATS * 4;
     const int off_gt = (upto_dt + NCH * 128 + 127) & ~127;
-    return off_gt + STAGES * GT_STRIDE + 256 + 1024;
+    return off_gt + STAGES * (GT_STRIDE + (nb == 1 ? 1024 : 0)) + 256 + 1024;
   }
   // Pm and A get a second copy too where that fits.  Where it does not (eight and sixteen slices) they are single and requested
   // LATE, each on a barrier of its own, when both chains are done with it: Pm after the first products of the chunk, A after (c).
@@ -119,7 +119,13 @@ struct RecCfg {
   static constexpr int OFF_DRP = OFF_DU + STAGES * DOB;
   static constexpr int OFF_DT = OFF_DRP + DRP_FLOATS * 4;     // per chain: exp(gL) of this chunk and the store flags of the next, 2 x 16 words
   static constexpr int OFF_GT = (OFF_DT + NCH * 128 + 127) & ~127;
-  static constexpr int OFF_CTRL = OFF_GT + STAGES * GT_STRIDE;
+  // per stage: the beta rows of the chunk for the four heads h & ~3 .. (TMA when H is a multiple of 4).  At eight and sixteen slices,
+  // whose chunks are bound by the L1 data path: a load per thread of a row of its own costs 32 wavefronts a warp (us, loads -> tile:
+  // 8192 items E8 1055 -> 1031, packed E16 2297 -> 2278); elsewhere one more copy a chunk costs what that gives or a little more
+  // (E12 1004 -> 1019, E2 205 -> 210).
+  static constexpr int BT_BYTES = LATE ? 1024 : 0;
+  static constexpr int OFF_BT = OFF_GT + STAGES * GT_STRIDE;
+  static constexpr int OFF_CTRL = OFF_BT + STAGES * BT_BYTES;
   static constexpr int SMEM_BYTES = OFF_CTRL + 256 + 1024;
 };
 
@@ -141,11 +147,12 @@ template <int E, int VC, int NCH, int NSG, bool PACKED>
 __global__ void __launch_bounds__(512, 1)
 rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
            const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_u,
-           const __grid_constant__ CUtensorMap map_du, const __grid_constant__ CUtensorMap map_a, RecParams p) {
+           const __grid_constant__ CUtensorMap map_du, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_beta, RecParams p) {
   using C = RecCfg<E, VC, NCH, NSG>;
   constexpr int REC_THREADS = C::THREADS, NWG = C::NWG, CT = C::CHAIN_THREADS, CC = C::CC, CV = C::CV, YW = C::YW;
   constexpr int NCOLS = C::NCOLS, CW = C::CW, TPC = C::TPC, ES = C::ES, NCG = C::NCG, EL = C::EL;
   constexpr int NV = HEAD / VC;
+  const bool beta_tma = C::LATE && p.beta_tma;
   constexpr bool TWO_WIDE = TPC * CW < 1024;        // the two-wide multiply-adds of (a) need register pairs: sixteen columns of four slices spill
   constexpr float LOG2E = 1.4426950408889634f;   // the decay threshold below is in the log2 domain
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -258,7 +265,8 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     chunk_info(i, t0, rows);
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
-    mbar_expect_tx(&ctrl.bar_load[st], C::KQ_BYTES + 2 * C::DO_BYTES + C::GT_BYTES + (C::LATE ? 0u : C::A_BYTES + C::PM_BYTES));
+    mbar_expect_tx(&ctrl.bar_load[st], C::KQ_BYTES + 2 * C::DO_BYTES + C::GT_BYTES + (beta_tma ? C::BT_BYTES : 0) + (C::LATE ? 0u : C::A_BYTES + C::PM_BYTES));
+    if (beta_tma) tma_load_4d(smem + C::OFF_BT + st * C::BT_BYTES, &map_beta, &ctrl.bar_load[st], 0, h >> 2, t0, b);
     // (eight value columns x 64 rows = one 1 KB column block of the images)
     tma_load_5d(smem + C::OFF_DO + st * C::DOB, &map_do, &ctrl.bar_load[st], 0, t0, vb * (VC / 8), h, b);
     tma_load_5d(smem + C::OFF_DU + st * C::DOB, &map_u, &ctrl.bar_load[st], 0, static_cast<int>(item * 64), vb * (VC / 8), 0, 0);
@@ -273,7 +281,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     }
   };
   auto prefetch_rows = [&](int i) {                          // the first warpgroup: what threads load themselves, for a later chunk -> L2
-    if (wg != 0) return;
+    if (wg != 0 || beta_tma) return;
     int t0, rows;
     chunk_info(i, t0, rows);
     const int last = max(rows, 1) - 1;
@@ -433,7 +441,8 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       lds_row<E, EL>(gf + (krow ? 0 : C::GF_C), t, e0, ga);
       if (krow) {
         lds_row<E, EL>(gf + C::GF_R, t, e0, gr);
-        bt = __ldg(p.beta + (tok + min(t, max(rows, 1) - 1)) * p.H + h);   // masked where it is used, after (c): nothing here waits for it
+        if (beta_tma) bt = reinterpret_cast<const float*>(smem + C::OFF_BT + st * C::BT_BYTES)[t * 4 + (h & 3)];
+        else bt = __ldg(p.beta + (tok + min(t, max(rows, 1) - 1)) * p.H + h);   // masked where it is used, after (c): nothing here waits for it
         const Piece up = image_piece(duimg);
         // Xu_e = r_e * U -> operand image (i = t, j = n') of (p)
         const uint32_t base = smem_u32(smem + C::OFF_XU) + (t >> 3) * 128 + (t & 7) * 16;
@@ -724,19 +733,19 @@ using namespace tgdn;
 
 template <int E, int VC, int NCH, int NSG, bool PACKED>
 static int launch_rec_rows(const CUtensorMap& mk, const CUtensorMap& mq,
-                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const RecParams& p, cudaStream_t s) {
+                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const CUtensorMap& mb, const RecParams& p, cudaStream_t s) {
   using C = RecCfg<E, VC, NCH, NSG>;
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static bool configured[64] = {};
   if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(rec_kernel<E, VC, NCH, NSG, PACKED>), C::SMEM_BYTES, configured)) return rc;
-  rec_kernel<E, VC, NCH, NSG, PACKED><<<p.n_seq * p.H * (HEAD / VC), C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, ma, p);
+  rec_kernel<E, VC, NCH, NSG, PACKED><<<p.n_seq * p.H * (HEAD / VC), C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, ma, mb, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 template <int E, int VC, int NCH, int NSG = 1>
 static int launch_rec(const CUtensorMap& mk, const CUtensorMap& mq,
-                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const RecParams& p, cudaStream_t s) {
-  return p.cmap != nullptr ? launch_rec_rows<E, VC, NCH, NSG, true>(mk, mq, mdo, mu, mdu, ma, p, s)
-                           : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, ma, p, s);
+                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const CUtensorMap& mb, const RecParams& p, cudaStream_t s) {
+  return p.cmap != nullptr ? launch_rec_rows<E, VC, NCH, NSG, true>(mk, mq, mdo, mu, mdu, ma, mb, p, s)
+                           : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
 }
 
 int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
@@ -762,7 +771,9 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   // dO (token layout) and U, dU (chunk layout: item * 64 + t rows of 128 columns) as operand images of the value block
   const int64_t crows = static_cast<int64_t>(B) * NC * H * 64;
   if (crows > 0x7fffffffLL) return TGDN_ERR_SHAPE;
-  CUtensorMap mdo, mu, mdu, ma;
+  CUtensorMap mdo, mu, mdu, ma, mb = mk;
+  const int beta_tma = H % 4 == 0 && (reinterpret_cast<uintptr_t>(beta) & 15) == 0 ? 1 : 0;
+  if (beta_tma && (rc = tgdn_make_gate_map(&mb, beta, B, T, H / 4, 4, row_tokens))) return rc;   // (B, T, H) read as (B, T, H/4, 4)
   const int blocks = value_block / 8, share = E <= 2 && value_block == 32 ? blocks : blocks / 2;   // dU leaves by chain
   if ((rc = tgdn_make_image_map(&mdo, dO, B, T, H, blocks, row_tokens))) return rc;
   if ((rc = tgdn_make_image_map(&mu, U, 1, static_cast<int>(crows), 1, blocks))) return rc;
@@ -772,23 +783,23 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
               static_cast<const __nv_bfloat16*>(Pm), static_cast<const __nv_bfloat16*>(U),
               static_cast<__nv_bfloat16*>(dV), static_cast<__nv_bfloat16*>(dU), static_cast<__nv_bfloat16*>(ds),
               static_cast<__nv_bfloat16*>(dkg), dr, doc_offsets, chunk_map, B, T, H, NC, packed ? n_docs : B, row_tokens, scale,
-              tgdn_status_word(), grad_state_in, grad_state_out};
+              tgdn_status_word(), grad_state_in, grad_state_out, beta_tma};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1:
-      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
-      return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, ma, p, s);
+      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+      return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
     case 2:
-      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
-      return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, ma, p, s);
+      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+      return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
     case 4:
-      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
-      return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+      return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
     // E = 8: 32 value columns per CTA measured 9% faster than two CTAs per SM of 16 columns each (5.26 -> 4.77 ms at B=8, T=8192, H=32,
     // before the chains), and the state-gradient kernel then adds four value-block images per item instead of eight.
-    case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
-    case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
-    case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, p, s);
+    case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+    case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+    case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
     default: return TGDN_ERR_SHAPE;
   }
 }

@@ -88,6 +88,7 @@ struct RecParams {
   int* status;
   const float* g_in;        // f32 [sequence][H][E][128 d][128 v]: dL/dS after the last token (a later segment's hand-off), or nullptr (zero)
   float* g_out;             // same form: dL/dS before the first token, or nullptr
+  int beta_tma;             // beta rows of a chunk arrive by TMA (H a multiple of 4, base 16-byte aligned), else by global loads
 };
 
 struct SgParams {
