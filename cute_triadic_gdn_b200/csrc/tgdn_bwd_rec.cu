@@ -38,6 +38,7 @@
 // the A half and dU move with one operation each, whatever their width (22 -> 9 a chunk at E = 8); with that and the two-wide f32
 // multiply-adds: E8 1095 -> 1075, E16 2418 -> 2395, E4 291 -> 275, E2 229 -> 209, E1 204 -> 178 us.  (Pulling later chunks into L2 by
 // prefetch instructions made it 3 to 8 % slower: the loads are a chunk ahead already.)
+// dV of a whole chunk leaves as a tile up to eight slices: us, 8192 items E8 1031 -> 1023, 4096 items E4 273 -> 265, E2 206 -> 194, E1 177 -> 171.
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
 #include "tgdn_kernels.h"
@@ -147,12 +148,12 @@ template <int E, int VC, int NCH, int NSG, bool PACKED>
 __global__ void __launch_bounds__(512, 1)
 rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_q,
            const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_u,
-           const __grid_constant__ CUtensorMap map_du, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_beta, RecParams p) {
+           const __grid_constant__ CUtensorMap map_du, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_beta, const __grid_constant__ CUtensorMap map_dv, RecParams p) {
   using C = RecCfg<E, VC, NCH, NSG>;
   constexpr int REC_THREADS = C::THREADS, NWG = C::NWG, CT = C::CHAIN_THREADS, CC = C::CC, CV = C::CV, YW = C::YW;
   constexpr int NCOLS = C::NCOLS, CW = C::CW, TPC = C::TPC, ES = C::ES, NCG = C::NCG, EL = C::EL;
   constexpr int NV = HEAD / VC;
-  const bool beta_tma = C::LATE && p.beta_tma;
+  constexpr bool DV_TILE = NSG == 1;                // (at twelve and sixteen slices the tile costs what it saves)
   constexpr bool TWO_WIDE = TPC * CW < 1024;        // the two-wide multiply-adds of (a) need register pairs: sixteen columns of four slices spill
   constexpr float LOG2E = 1.4426950408889634f;   // the decay threshold below is in the log2 domain
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -265,8 +266,8 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     chunk_info(i, t0, rows);
     uint8_t* kq = smem + C::OFF_KQ + st * C::KQ_BYTES;
     const int64_t item = (static_cast<int64_t>(b) * p.NC + first + i) * p.H + h;
-    mbar_expect_tx(&ctrl.bar_load[st], C::KQ_BYTES + 2 * C::DO_BYTES + C::GT_BYTES + (beta_tma ? C::BT_BYTES : 0) + (C::LATE ? 0u : C::A_BYTES + C::PM_BYTES));
-    if (beta_tma) tma_load_4d(smem + C::OFF_BT + st * C::BT_BYTES, &map_beta, &ctrl.bar_load[st], 0, h >> 2, t0, b);
+    mbar_expect_tx(&ctrl.bar_load[st], C::KQ_BYTES + 2 * C::DO_BYTES + C::GT_BYTES + (C::LATE && p.beta_tma ? C::BT_BYTES : 0) + (C::LATE ? 0u : C::A_BYTES + C::PM_BYTES));
+    if (C::LATE && p.beta_tma) tma_load_4d(smem + C::OFF_BT + st * C::BT_BYTES, &map_beta, &ctrl.bar_load[st], 0, h >> 2, t0, b);
     // (eight value columns x 64 rows = one 1 KB column block of the images)
     tma_load_5d(smem + C::OFF_DO + st * C::DOB, &map_do, &ctrl.bar_load[st], 0, t0, vb * (VC / 8), h, b);
     tma_load_5d(smem + C::OFF_DU + st * C::DOB, &map_u, &ctrl.bar_load[st], 0, static_cast<int>(item * 64), vb * (VC / 8), 0, 0);
@@ -281,7 +282,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     }
   };
   auto prefetch_rows = [&](int i) {                          // the first warpgroup: what threads load themselves, for a later chunk -> L2
-    if (wg != 0 || beta_tma) return;
+    if (wg != 0 || (C::LATE && p.beta_tma)) return;
     int t0, rows;
     chunk_info(i, t0, rows);
     const int last = max(rows, 1) - 1;
@@ -427,7 +428,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     // This chain is done with the previous chunk's stage (its last store of dU has left the stage's buffer); the last chain to say
     // so refills it.
     if (kstep > 0 && warp_u == COPY_WARP && elect_one()) {
-      bulk_wait_group_read();
+      if constexpr (!DV_TILE) bulk_wait_group_read();
       if (atomicAdd(&ctrl.released[st ^ 1], 1u) % NCH == NCH - 1 && kstep + 1 < count) issue_loads(i - 1, st ^ 1);
     }
     __syncwarp();
@@ -441,7 +442,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       lds_row<E, EL>(gf + (krow ? 0 : C::GF_C), t, e0, ga);
       if (krow) {
         lds_row<E, EL>(gf + C::GF_R, t, e0, gr);
-        if (beta_tma) bt = reinterpret_cast<const float*>(smem + C::OFF_BT + st * C::BT_BYTES)[t * 4 + (h & 3)];
+        if (C::LATE && p.beta_tma) bt = reinterpret_cast<const float*>(smem + C::OFF_BT + st * C::BT_BYTES)[t * 4 + (h & 3)];
         else bt = __ldg(p.beta + (tok + min(t, max(rows, 1) - 1)) * p.H + h);   // masked where it is used, after (c): nothing here waits for it
         const Piece up = image_piece(duimg);
         // Xu_e = r_e * U -> operand image (i = t, j = n') of (p)
@@ -597,7 +598,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         if (!live) bt = 0.f;
 #pragma unroll
         for (int c = 0; c < CW; c += 2) xw[c >> 1] = pack_bf16(bt * z[c], bt * z[c + 1]);
-        if (live && sgp == 0) {
+        if (live && sgp == 0 && !(DV_TILE && rows == CHUNK)) {
           __nv_bfloat16* dst = p.dV + ((tok + t) * p.H + h) * HEAD + vb * VC + v0;
 #pragma unroll
           for (int c = 0; c < CW / 2; c += 4) *reinterpret_cast<uint4*>(dst + 2 * c) = make_uint4(xw[c], xw[c + 1], xw[c + 2], xw[c + 3]);
@@ -609,6 +610,10 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       }
       // (p) reads the image of G that X is about to replace
       mbar_wait_spin(&ctrl.bar_ex[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
+      // dV of a whole chunk leaves as an image from the place of Xu, which (p) has read (a row of its own per thread would cost 32
+      // wavefronts a store; a chunk cut short by a document end may not leave as a tile)
+      if (DV_TILE && krow && rows == CHUNK)
+        store_packed(smem_u32(smem + C::OFF_XU) + (TM_C / 8 + (v0 - chain * CV) / 8) * 1024 + (t >> 3) * 128 + (t & 7) * 16, 1024, xw);
       // X image (i = row, j = n'): rows 0..63 -a_e*dW, rows 64..127 c_e*dO
       const uint32_t base = smem_u32(smem + C::OFF_GX) + (row >> 3) * 128 + (row & 7) * 16;
 #pragma unroll
@@ -622,6 +627,11 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     tc_fence_before();
     rec_chain_sync<CT>(chain);
 
+    if (DV_TILE && warp_u == COPY_WARP && rows == CHUNK && elect_one()) {
+      tma_store_5d(&map_dv, smem + C::OFF_XU + TM_C / 8 * 1024, 0, t0, (vb * VC + chain * CV) / 8, h, b);
+      bulk_commit_group();
+    }
+    __syncwarp();
     // ---- (d) dG = [K^T | Q^T] X, G <- d G + dG ------------------------------------------------------------------
     if (warp_u == ISSUE_WARP && elect_one()) {
       tc_fence_after();
@@ -708,6 +718,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         }
       }
     }
+    if (DV_TILE && warp_u == COPY_WARP && elect_one()) bulk_wait_group_read();   // dU and dV have left: their places take the next chunk's U and Xu
     fence_async_smem();
     tc_fence_before();
     rec_chain_sync<CT>(chain);
@@ -733,19 +744,19 @@ using namespace tgdn;
 
 template <int E, int VC, int NCH, int NSG, bool PACKED>
 static int launch_rec_rows(const CUtensorMap& mk, const CUtensorMap& mq,
-                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const CUtensorMap& mb, const RecParams& p, cudaStream_t s) {
+                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mdv, const RecParams& p, cudaStream_t s) {
   using C = RecCfg<E, VC, NCH, NSG>;
   static_assert(C::SMEM_BYTES <= 232448, "shared memory budget of one CTA exceeded");
   static bool configured[64] = {};
   if (const int rc = tgdn_dynamic_smem(reinterpret_cast<const void*>(rec_kernel<E, VC, NCH, NSG, PACKED>), C::SMEM_BYTES, configured)) return rc;
-  rec_kernel<E, VC, NCH, NSG, PACKED><<<p.n_seq * p.H * (HEAD / VC), C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, ma, mb, p);
+  rec_kernel<E, VC, NCH, NSG, PACKED><<<p.n_seq * p.H * (HEAD / VC), C::THREADS, C::SMEM_BYTES, s>>>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p);
   return tgdn_cuda_error(cudaGetLastError());
 }
 template <int E, int VC, int NCH, int NSG = 1>
 static int launch_rec(const CUtensorMap& mk, const CUtensorMap& mq,
-                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const CUtensorMap& mb, const RecParams& p, cudaStream_t s) {
-  return p.cmap != nullptr ? launch_rec_rows<E, VC, NCH, NSG, true>(mk, mq, mdo, mu, mdu, ma, mb, p, s)
-                           : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+                      const CUtensorMap& mdo, const CUtensorMap& mu, const CUtensorMap& mdu, const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mdv, const RecParams& p, cudaStream_t s) {
+  return p.cmap != nullptr ? launch_rec_rows<E, VC, NCH, NSG, true>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s)
+                           : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
 }
 
 int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
@@ -771,13 +782,14 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   // dO (token layout) and U, dU (chunk layout: item * 64 + t rows of 128 columns) as operand images of the value block
   const int64_t crows = static_cast<int64_t>(B) * NC * H * 64;
   if (crows > 0x7fffffffLL) return TGDN_ERR_SHAPE;
-  CUtensorMap mdo, mu, mdu, ma, mb = mk;
+  CUtensorMap mdo, mu, mdu, mdv, ma, mb = mk;
   const int beta_tma = H % 4 == 0 && (reinterpret_cast<uintptr_t>(beta) & 15) == 0 ? 1 : 0;
   if (beta_tma && (rc = tgdn_make_gate_map(&mb, beta, B, T, H / 4, 4, row_tokens))) return rc;   // (B, T, H) read as (B, T, H/4, 4)
   const int blocks = value_block / 8, share = E <= 2 && value_block == 32 ? blocks : blocks / 2;   // dU leaves by chain
   if ((rc = tgdn_make_image_map(&mdo, dO, B, T, H, blocks, row_tokens))) return rc;
   if ((rc = tgdn_make_image_map(&mu, U, 1, static_cast<int>(crows), 1, blocks))) return rc;
   if ((rc = tgdn_make_image_map(&mdu, dU, 1, static_cast<int>(crows), 1, share))) return rc;
+  if ((rc = tgdn_make_image_map(&mdv, dV, B, T, H, share, row_tokens))) return rc;
   if ((rc = tgdn_make_a_half_map(&ma, AP, static_cast<long long>(B) * NC * H))) return rc;
   RecParams p{static_cast<const __nv_bfloat16*>(dO), k2, q2, beta, gc, static_cast<const __nv_bfloat16*>(AP),
               static_cast<const __nv_bfloat16*>(Pm), static_cast<const __nv_bfloat16*>(U),
@@ -787,19 +799,19 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1:
-      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
-      return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+      return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     case 2:
-      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
-      return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+      return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     case 4:
-      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
-      return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+      return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     // E = 8: 32 value columns per CTA measured 9% faster than two CTAs per SM of 16 columns each (5.26 -> 4.77 ms at B=8, T=8192, H=32,
     // before the chains), and the state-gradient kernel then adds four value-block images per item instead of eight.
-    case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
-    case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
-    case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, p, s);
+    case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+    case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+    case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     default: return TGDN_ERR_SHAPE;
   }
 }
