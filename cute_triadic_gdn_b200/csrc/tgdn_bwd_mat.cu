@@ -727,8 +727,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     }
     v0 += __shfl_sync(0xffffffffu, v1, 31);
     const int ra = 63 - lane, rb = 31 - lane;
-    if (ra < rows) p.dg[((tok + ra) * p.H + h) * E + e] = v1;
-    if (rb < rows) p.dg[((tok + rb) * p.H + h) * E + e] = v0;
+    sm.dgc[ra * ES + e] = v1;                              // leaves by rows, below: a column would write four bytes of every sector
+    sm.dgc[rb * ES + e] = v0;
   }
 
   // ---- dk, dq: this thread's row, 32 of the 128 columns ------------------------------------------------------------
@@ -761,6 +761,11 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
+#pragma unroll
+  for (int it = 0; it < GATE_ITERS; ++it) {
+    const int idx = tid + it * MAT_THREADS, rr = idx / E, e = idx % E;
+    if (rr < rows) p.dg[((tok + rr) * p.H + h) * E + e] = sm.dgc[rr * ES + e];
+  }
   if (rows == CHUNK) {
     if (warp_u == 1 && elect_one()) {
       tma_store_4d(&map_dk, sm.kq, 0, h, t0, b);
