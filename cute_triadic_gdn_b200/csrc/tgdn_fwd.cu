@@ -69,7 +69,8 @@ struct FwdCfg {
   static constexpr int S_BYTES = TPC * 256;       // per chain: image (i = d, j = n'), SI = 128, SJ = 2048
   static constexpr int VN_BYTES = TPC * 128;      // per chain: image (i = t, j = n'), SI = 128, SJ = 1024
   static constexpr int BWI_BYTES = UW * 128;      // per chain: image (i = s, j = v), SI = 128, SJ = 1024
-  // W on its way out: in the block that a chain of eight columns leaves unused, else behind the operand where that fits
+  // W on its way out: in the block that a chain of eight columns leaves unused, else behind the operand where that fits, else
+  // (W_OWN false) in the place of the value rows, before o
   static constexpr int WST_OFF = CV == 8 ? 1024 : BWI_BYTES;
   static constexpr int bytes_with(int bw) {
     const int gt = (OFF_BW + NCH * bw + 127) & ~127;
@@ -80,8 +81,8 @@ struct FwdCfg {
   static constexpr int OFF_S = OFF_AP + STAGES * AP_BYTES;
   static constexpr int OFF_VN = OFF_S + NCH * S_BYTES;
   static constexpr int OFF_BW = OFF_VN + NCH * VN_BYTES;
-  static constexpr bool W_TMA = CV == 8 || bytes_with(BWI_BYTES + CV * 128) <= 232448;
-  static constexpr int BW_BYTES = CV == 8 || !W_TMA ? BWI_BYTES : BWI_BYTES + CV * 128;
+  static constexpr bool W_OWN = CV == 8 || bytes_with(BWI_BYTES + CV * 128) <= 232448;
+  static constexpr int BW_BYTES = CV == 8 || !W_OWN ? BWI_BYTES : BWI_BYTES + CV * 128;
   // per stage: the gate factors of the chunk as the masks kernel stored them, a, r, c as 64 dense rows of E floats each,
   // then d (one bulk copy)
   static constexpr int GT_BYTES = gate_factor_bytes(E);
@@ -429,13 +430,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       if (SAVE && p.W != nullptr) {
 #pragma unroll
         for (int c = 0; c < CW; c += 2) w[c >> 1] = pack_bf16(acc[c], acc[c + 1]);
-        if constexpr (C::W_TMA) {
-          put_row(bw_img + C::WST_OFF, w);
-        } else {
-          __nv_bfloat16* dst = p.W + (item * 64 + t) * HEAD + v0g;
-#pragma unroll
-          for (int c = 0; c < CW / 2; c += 4) *reinterpret_cast<uint4*>(dst + 2 * c) = make_uint4(w[c], w[c + 1], w[c + 2], w[c + 3]);
-        }
+        put_row(C::W_OWN ? bw_img + C::WST_OFF : vbox, w);   // (the value row has been read by the same thread)
       }
     }
     fence_async_smem();
@@ -454,8 +449,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       umma_commit(&ctrl.bar_mma[chain]);
     }
     __syncwarp();
-    if (SAVE && C::W_TMA && p.W != nullptr && cwarp_u == COPY_WARP && elect_one())
-      tma_store_4d(&map_w, bw_img + C::WST_OFF, v0c, 0, static_cast<int>(item) * 64, 0);
+    if (SAVE && p.W != nullptr && cwarp_u == COPY_WARP && elect_one()) {
+      tma_store_4d(&map_w, C::W_OWN ? bw_img + C::WST_OFF : vbox, v0c, 0, static_cast<int>(item) * 64, 0);
+      if constexpr (!C::W_OWN) {                     // o takes its place after this product
+        bulk_commit_group();
+        bulk_wait_group_read();
+      }
+    }
     __syncwarp();
     if (PACKED && i + 1 < count) chunk_info(i + 1, t0_next, rows_next);
     if constexpr (LATE_R) {                          // r_e only now, from the stage: sixteen registers fewer are live
