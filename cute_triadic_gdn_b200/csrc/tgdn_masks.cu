@@ -20,7 +20,7 @@
 //   * What bounds it: the chain of these steps, with five block barriers, hidden by four CTAs per SM (three at twelve and sixteen slices:
 //     registers), and the shared-memory wavefronts inside them; hence one buffer for tile, operand images, L and X and [A; PA] in turn,
 //     and padded rows in 16-byte pieces everywhere.  us, before (swizzled single floats, two CTAs per SM) and after: 8192 items E8
-//     355 -> 220; 4096 items E4 179 -> 105, E2 179 -> 96, E1 176 -> 91; packed E16 561 -> 316, E12 238 -> 145.
+//     355 -> 211; 4096 items E4 179 -> 97, E2 179 -> 92, E1 176 -> 90; packed E16 561 -> 301, E12 238 -> 143.
 //   * PA = Pm A: a second tcgen05 MMA group on the bf16 images of Pm and A that are about to be stored anyway.
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
