@@ -33,6 +33,27 @@ def test_wide_value_blocks_of_the_forward(E, docs):
         assert torch.equal(torch.cat([o1, o2], 1), o.detach()) and torch.equal(s2, s_all)
 
 
+@pytest.mark.parametrize("E", [1, 2, 4, 8, 12, 16])
+@pytest.mark.parametrize("H", [3, 4])                      # beta rows by loads, and as tiles of four heads
+def test_saved_and_unsaved_forward_and_ragged_chunks(E, H):
+    """The forward with and without saved tensors (other splits of the block up to eight slices) agree bitwise; whole chunks leave the
+    recurrences as tiles, chunks cut short by a document end row by row."""
+    docs = [0, 1, 64, 128, 191, 256]
+    ins = [t.cuda() for t in orc.make_inputs(1, 256, H, E, seed=90 + E, dist="mild")]
+    do = orc.make_grad_output((1, 256, H, 128), 6)
+    cu = torch.tensor(docs, dtype=torch.int32)
+    with torch.no_grad():
+        plain = gdn_joint_call(*ins, cu_seqlens=cu.cuda())
+    leaves = [t.clone().requires_grad_(True) for t in ins]
+    o = gdn_joint_call(*leaves, cu_seqlens=cu.cuda())
+    o.backward(do.cuda())
+    assert _lib.device_status() == 0 and torch.equal(plain, o.detach())
+    o_ref, g_ref = orc.reference_with_grads(orc.chunk_reference, [t.cpu() for t in ins], do, cu_seqlens=cu, dtype=torch.float32)
+    assert orc.rel_l2(o.detach().float().cpu(), o_ref) < 1e-2
+    for name, leaf, ref in zip("q k v k2 q2 g beta".split(), leaves, g_ref):
+        assert orc.rel_l2(leaf.grad.float().cpu(), ref) < 2e-2, name
+
+
 @pytest.mark.parametrize("B,T,C,act,docs", [
     (2, 37, 1930, 1920, None),                         # 4-byte rows
     (1, 150, 77, 40, [0, 1, 3, 64, 65, 150]),          # 2-byte rows, SiLU ends inside a warp's channels
