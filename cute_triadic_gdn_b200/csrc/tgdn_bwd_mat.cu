@@ -19,8 +19,8 @@
 // five product groups with the sums over the slices between them (f32 on the ordinary pipes).  Hence the two independent chains,
 // the two-wide f32 instructions for those sums, L2 prefetch of the next item, and 16-byte pieces wherever a thread owns a row; the
 // column sums of dA'*A are exchanges inside the warps, before G3, instead of a matrix in shared memory that is walked by columns
-// after it.  us, before (first these, then the two-wide sums) and after: 8192 items E8 575 -> 519; 4096 items E8 mild 303 -> 268,
-// E4 248 -> 231, E1 222 -> 211; packed E16 900 -> 875.
+// after it.  us, before (first these, then the two-wide sums) and after: 8192 items E8 575 -> 506; 4096 items E8 mild 303 -> 262,
+// E4 248 -> 229, E2 228 -> 210, E1 222 -> 205; packed E16 900 -> 837, E12 396 -> 374.
 //
 // Replaces cute_triadic_gdn/kernels/sm100_joint_bwd_parallel.py:80-405 (matrix_kernel),
 // cute_triadic_gdn/kernels/sm90_joint_bwd_parallel.py:278-372 (mask_grad_kernel) and the reverse pass of
@@ -162,11 +162,23 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   const uint32_t tmem_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   WaitCtl ctl{&sm.abort, p.status};
 
-  for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
-  // (items fit in 32 bits, the entry point checks that: 64-bit divisions are a few hundred cycles each on this machine)
-  const int item32 = static_cast<int>(item);
-  const int h = item32 % p.H, n = (item32 / p.H) % p.NC;
-  const int b = item32 / (p.H * p.NC);
+  // (batch row, chunk, head) of an item, the next one found by steps: the two divisions (32-bit: items fit, the entry point checks that)
+  // cost every warp several hundred cycles an item.  us: 4096 items E2 222 -> 210, E1 211 -> 206, packed E12 386 -> 374, E16 841 -> 834.
+  // At four slices the steps' registers spill where the divisions' do not (228 -> 234), so that one divides.
+  constexpr bool STEPS = E != 4;
+  const int step = static_cast<int>(gridDim.x), step_h = step % p.H, step_n = step / p.H % p.NC, step_b = step / (p.H * p.NC);
+  int h = blockIdx.x % p.H, n = blockIdx.x / p.H % p.NC, b = blockIdx.x / (p.H * p.NC);
+  auto advance = [&](int64_t next, int& h1, int& n1, int& b1) {
+    if constexpr (STEPS) {
+      h1 += step_h; n1 += step_n; b1 += step_b;
+      if (h1 >= p.H) { h1 -= p.H; ++n1; }
+      if (n1 >= p.NC) { n1 -= p.NC; ++b1; }
+    } else {
+      const int i = static_cast<int>(next);
+      h1 = i % p.H; n1 = i / p.H % p.NC; b1 = i / (p.H * p.NC);
+    }
+  };
+  for (int64_t item = blockIdx.x; item < n_items; item += step, advance(item, h, n, b)) {
   int t0 = n * CHUNK, rows = CHUNK;
   if (p.cmap != nullptr) {
     t0 = p.cmap[n];
@@ -512,11 +524,10 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     // Pull the inputs of this CTA's next item into L2: its prologue, which nothing on this SM overlaps, then waits for L2
     // instead of for HBM.
     if (warp_u == 1) {
-      const int64_t item2 = item + gridDim.x;              // this CTA's next item
+      const int64_t item2 = item + step;                   // this CTA's next item
       if (item2 < n_items) {
-        const int i2 = static_cast<int>(item2);
-        const int h2 = i2 % p.H, n2 = (i2 / p.H) % p.NC;
-        const int b2 = i2 / (p.H * p.NC);
+        int h2 = h, n2 = n, b2 = b;
+        advance(item2, h2, n2, b2);
         int t2 = n2 * CHUNK, rows2 = CHUNK;
         if (p.cmap != nullptr) { t2 = p.cmap[n2]; rows2 = p.cmap[p.NC + n2]; }
         if (rows2 > 0 && rows2 <= CHUNK && t2 >= 0 && t2 + rows2 <= p.T) {
