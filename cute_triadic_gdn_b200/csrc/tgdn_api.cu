@@ -171,17 +171,7 @@ int tgdn_sm_count() {
   return n;
 }
 
-int tgdn_value_block(int E) { return E > 8 ? 16 : 32; }   // must match the dispatch in tgdn_bwd_rec.cu
-
-// Up to four slices a CTA of 64 columns (two chains of 32) takes 1.35 to 1.4 times as long per chunk as one of 32 for twice the columns,
-// and leaves half as many value-block images to the later stages: it wins when it saves waves (one CTA per SM) by more than that.
-// B=4, T=4096, H=16 (two waves or one), reverse recurrence + state gradients: E = 1 452 -> 350 us, E = 2 500 -> 399, E = 4 639 -> 517.
-int tgdn_value_block_for(int E, long long sequences, int H) {
-  if (E > 4) return tgdn_value_block(E);
-  const long long sms = tgdn_sm_count(), seqs = sequences * H;
-  const long long narrow = (seqs * 4 + sms - 1) / sms, wide = (seqs * 2 + sms - 1) / sms;
-  return wide * 7 < narrow * 5 ? 64 : 32;
-}
+int tgdn_value_block(int E) { return E > 8 ? 16 : 32; }
 
 extern "C" const char* tgdn_error_string(int code) {
   static thread_local char buf[160];

@@ -212,7 +212,7 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   // under the streaming load of the other blocks is microseconds.
   const int64_t tok = static_cast<int64_t>(b) * p.TS + t0;
   constexpr int GATE_ITERS = (64 * E + MAT_THREADS - 1) / MAT_THREADS;
-  constexpr int NV_MAX = 8;                                // value blocks of the reverse recurrence (2, 4 or 8)
+  constexpr int NV_MAX = 8;                                // value blocks of the reverse recurrence (4 or 8)
   float da_in[GATE_ITERS], dc_in[GATE_ITERS];              // row-sum gradients of the state-gradient kernel, used at the end
   const float dd_in = __ldg(p.dd + item * E + min(warp, E - 1));   // warp e adds the chunk-end term of gate column e
   const float beta_in = __ldg(p.beta + (tok + min(tid & 63, rows - 1)) * p.H + h);
@@ -230,7 +230,7 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       dc_in[it] = __ldg(p.dc + item * (64 * E) + idx);
       const float* drp = p.dr + (item * p.NV * 64 + rr) * E + e;   // value block v is 64 * E floats further on
 #pragma unroll
-      for (int v = 0; v < 4; ++v) dr_in[it][v] = v < 2 || p.NV > 2 ? __ldg(drp + v * (64 * E)) : 0.f;
+      for (int v = 0; v < 4; ++v) dr_in[it][v] = __ldg(drp + v * (64 * E));
       if (p.NV > 4) {                                      // four or eight value blocks: the same for every thread
 #pragma unroll
         for (int v = 4; v < NV_MAX; ++v) dr_in[it][v] = __ldg(drp + v * (64 * E));
@@ -825,7 +825,7 @@ static int launch_mat(const CUtensorMap* maps, const MatParams& p, cudaStream_t 
 int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const void* dU, const void* W, const void* U, const void* AP,
                          const float* k2, const float* q2, const float* beta, const float* gc, const void* dkq, const float* da,
                          const float* dc, const float* dd, const float* dr, float scale, const int32_t* chunk_map, int B, int T,
-                         int H, int E, int NC, int row_tokens, int value_block, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
+                         int H, int E, int NC, int row_tokens, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
                          void* stream) {
   if (!q || !k || !dO || !dU || !W || !U || !AP || !k2 || !q2 || !beta || !gc || !dkq || !da || !dc || !dd || !dr ||
       !dq || !dk || !dk2 || !dq2 || !dg || !dbeta)
@@ -849,7 +849,7 @@ int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const voi
   if ((rc = tgdn_make_token_map(&maps[7], dq, B, T, H, 64, 64, 1, row_tokens))) return rc;
   MatParams p{k2, q2, beta, gc, static_cast<const __nv_bfloat16*>(AP), static_cast<const __nv_bfloat16*>(dkq), da, dc, dd, dr,
               static_cast<__nv_bfloat16*>(dq), static_cast<__nv_bfloat16*>(dk), dk2, dq2, dg, dbeta, chunk_map,
-              B, T, H, NC, 128 / value_block, row_tokens, scale, tgdn_status_word(), tgdn_sm_count()};
+              B, T, H, NC, 128 / tgdn_value_block(E), row_tokens, scale, tgdn_status_word(), tgdn_sm_count()};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1: return launch_mat<1>(maps, p, s);
@@ -867,6 +867,6 @@ extern "C" int tgdn_bwd_matrix(const void* q, const void* k, const void* dO, con
                                const void* dkq, const float* da, const float* dc, const float* dd, const float* dr,
                                float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC, void* dq,
                                void* dk, float* dk2, float* dq2, float* dg, float* dbeta, void* stream) {
-  return tgdn_bwd_matrix_rows(q, k, dO, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, scale, chunk_map, B, T, H, E, NC, T, tgdn_value_block(E),
+  return tgdn_bwd_matrix_rows(q, k, dO, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, scale, chunk_map, B, T, H, E, NC, T,
                               dq, dk, dk2, dq2, dg, dbeta, stream);
 }

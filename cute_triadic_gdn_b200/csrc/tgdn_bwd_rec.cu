@@ -33,12 +33,15 @@
 // What bounds it: the dependent chain of a chunk (three MMA -> load -> epilogue round trips) over a shared-memory path that the
 // products' operand reads and the operand images fill to two thirds.  Reverse recurrence, us, one lockstep CTA of four warpgroups
 // that looked the chunk up when it began -> this version: B2 T8192 H32 E8 1241 -> 1092; B1 T32768 packed H8 E12 1132 -> 997;
-// H16 E16 2497 -> 2414; B4 T4096 H16 E4 394 -> 285, E2 318 -> 226, E1 299 -> 202 (the last three with 64 value columns per CTA).
+// H16 E16 2497 -> 2414; B4 T4096 H16 E4 394 -> 285, E2 318 -> 226, E1 299 -> 202 (the last three with 64 value columns per CTA, then one block).
 // Every copy operation costs the warp that issues it some sixty cycles and the chain waits for its last warp, so the images of dO and U,
 // the A half and dU move with one operation each, whatever their width (22 -> 9 a chunk at E = 8); with that and the two-wide f32
 // multiply-adds: E8 1095 -> 1075, E16 2418 -> 2395, E4 291 -> 275, E2 229 -> 209, E1 204 -> 178 us.  (Pulling later chunks into L2 by
 // prefetch instructions made it 3 to 8 % slower: the loads are a chunk ahead already.)
-// dV of a whole chunk leaves as a tile up to eight slices: us, 8192 items E8 1031 -> 1023, 4096 items E4 273 -> 265, E2 206 -> 194, E1 177 -> 171.
+// dV of a whole chunk leaves as a tile up to eight slices: us, 8192 items E8 1031 -> 1023, 4096 items E4 270 -> 255, E2 205 -> 194, E1 177 -> 171.
+// One value block per chain in the 64-column CTA, with sums of its own, instead of one block of 64 columns (whose results depended on
+// the width that the call picked): E4 254 -> 256, E2 193 -> 206, E1 172 -> 188, and the state-gradient kernel adds four images again
+// instead of two (217 -> 247, 164 -> 182, 137 -> 154); four slices on narrow blocks (2048 items), the chains' P in turn: 188 -> 193.
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
 #include "tgdn_kernels.h"
@@ -49,9 +52,14 @@ namespace tgdn {
 // own named barrier.  While one chain's threads are in an epilogue the tensor core works for the other one.  (One lockstep CTA of
 // four warpgroups took 9.5 k cycles per chunk at E = 8, of which its products were in flight for 4.6 k and its epilogues ran for
 // the other 4.9 k, neither overlapping the other.)  The chains share the chunk's tiles (two-stage ring; the last chain to hand a
-// stage back refills it) and two sums over all value columns: P and dr, which both chains read out together (below).  One and two
-// slices on narrow blocks are one chain of four warpgroups: their products are so short that two of everything costs more than
-// the overlap gives.
+// stage back refills it) and, at one block per CTA, two sums over all value columns: P and dr, which both chains read out together
+// (below).  One and two slices on narrow blocks are one chain of four warpgroups: their products are so short that two of everything
+// costs more than the overlap gives.
+// P leaves rounded to bf16 per VALUE BLOCK of 32 columns (16 above eight slices) and dr is summed per block, so the block is part of
+// the results, and the CTA's width must not be: the 64-column CTA (VC = 64, up to four slices, chosen by the number of sequences) is
+// two blocks, one per chain, each with its own P and dr, formed from the same products in the same order as in a CTA of one block.
+// What a sequence gets then does not depend on what runs beside it.  (At four slices the narrow CTA's two chains add into one P in
+// turn, chain 0 first, which is the order of the wide CTA's single chain.)
 // NSG = 2 (twelve and sixteen slices) splits the SLICES of a chain's columns over its two warpgroups: a thread then holds eight
 // value columns of half the slices instead of four columns of all of them, which keeps the 16-byte accesses; the sum over all
 // slices (dU) is completed through shared memory.
@@ -72,9 +80,14 @@ struct RecCfg {
   static constexpr int TPC = EL * CW;             // state columns per thread
   static constexpr int CC = NCOLS / NCH;          // state columns per chain
   static constexpr int CV = VC / NCH;             // value columns per chain
+  static constexpr bool OWN = VC == 64;           // every chain is a value block of its own
+  static constexpr int VBW = OWN ? CV : VC;       // width of a value block
+  static constexpr bool IN_TURN = E == 4 && !OWN; // chain 1 adds its share of P to chain 0's
+  static constexpr bool CROSS = NCH > 1 && !OWN;  // the chains share the sums over the block's columns
   static constexpr int YW = CV < 16 ? 16 : CV;    // columns of Y and Z (the smallest N of an M=128 MMA is 16)
   static_assert(CC % 16 == 0 && CC <= 256 && CV % 8 == 0, "columns of a chain's products");
   static_assert((NCH == 1 && NSG == 1) || NCH == 2, "slice groups are the two warpgroups of a chain");
+  static_assert(!OWN || (NCH == 2 && NSG == 1 && CV == 32), "a wide CTA is two blocks of 32 columns");
   static_assert(CW == 8 || CW == 16, "value columns per thread");
   static constexpr int ES = E | 1;
   static_assert(NWG % NSG == 0 && E % NSG == 0 && (NSG == 1 || EL % 2 == 0), "slice groups split the slices evenly");
@@ -102,6 +115,7 @@ struct RecCfg {
   }
   // Pm and A get a second copy too where that fits.  Where it does not (eight and sixteen slices) they are single and requested
   // LATE, each on a barrier of its own, when both chains are done with it: Pm after the first products of the chunk, A after (c).
+  // (So it is at four slices on 64 columns.)
   // Half a chunk lies between that and the next use by the chain that is ahead.
   static constexpr bool LATE = layout_bytes(2) > LIMIT;
   static constexpr int NB = LATE ? 1 : 2;
@@ -120,8 +134,8 @@ struct RecCfg {
   static constexpr int OFF_DRP = OFF_DU + STAGES * DOB;
   static constexpr int OFF_DT = OFF_DRP + DRP_FLOATS * 4;     // per chain: exp(gL) of this chunk and the store flags of the next, 2 x 16 words
   static constexpr int OFF_GT = (OFF_DT + NCH * 128 + 127) & ~127;
-  // per stage: the beta rows of the chunk for the four heads h & ~3 .. (TMA when H is a multiple of 4).  At eight and sixteen slices,
-  // whose chunks are bound by the L1 data path: a load per thread of a row of its own costs 32 wavefronts a warp (us, loads -> tile:
+  // per stage: the beta rows of the chunk for the four heads h & ~3 .. (TMA when H is a multiple of 4).  With LATE: at eight and sixteen
+  // slices, whose chunks are bound by the L1 data path: a load per thread of a row of its own costs 32 wavefronts a warp (us, loads -> tile:
   // 8192 items E8 1055 -> 1031, packed E16 2297 -> 2278); elsewhere one more copy a chunk costs what that gives or a little more
   // (E12 1004 -> 1019, E2 205 -> 210).
   static constexpr int BT_BYTES = LATE ? 1024 : 0;
@@ -137,6 +151,7 @@ struct RecCtrl {
   uint64_t bar_mma[2];       // per chain: (c)
   uint64_t bar_xu[2];        // per chain: its key-row warps have written the operand Xu of (p), one arrival per warp
   uint64_t bar_ex[2];        // per chain: its share of P is complete and its dr partials are written (four key-row warps and a commit)
+  uint64_t bar_turn;         // P of chain 0 is complete: chain 1 may add to it
   uint64_t bar_done;         // every warp has read its part of P and dr: the next chunk's may be written
   uint32_t released[2], released_pm, released_a;   // chains that are done with a stage, Pm, A (count up forever; a multiple of the chains = all)
   uint32_t tmem_base;
@@ -152,7 +167,8 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   using C = RecCfg<E, VC, NCH, NSG>;
   constexpr int REC_THREADS = C::THREADS, NWG = C::NWG, CT = C::CHAIN_THREADS, CC = C::CC, CV = C::CV, YW = C::YW;
   constexpr int NCOLS = C::NCOLS, CW = C::CW, TPC = C::TPC, ES = C::ES, NCG = C::NCG, EL = C::EL;
-  constexpr int NV = HEAD / VC;
+  constexpr int NV = HEAD / VC, NVB = HEAD / C::VBW;   // CTAs per head, value blocks per head
+  constexpr bool CROSS = C::CROSS;
   constexpr bool DV_TILE = NSG == 1;                // (at twelve and sixteen slices the tile costs what it saves)
   constexpr bool TWO_WIDE = TPC * CW < 1024;        // the two-wide multiply-adds of (a) need register pairs: sixteen columns of four slices spill
   constexpr float LOG2E = 1.4426950408889634f;   // the decay threshold below is in the log2 domain
@@ -198,6 +214,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       mbar_init(&ctrl.bar_ex[c], 8 / NCH + 1);
       ctrl.released[c] = 0;
     }
+    mbar_init(&ctrl.bar_turn, 1);
     mbar_init(&ctrl.bar_done, NWG * 4);
     ctrl.released_pm = ctrl.released_a = 0;
     mbar_fence_init();
@@ -238,7 +255,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   const int warp_u = __shfl_sync(0xffffffffu, warp & (CT / 32 - 1), 0);   // warp index inside the chain as a warp-uniform value
   const uint32_t tmem_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
   const uint32_t TM_C = chain * CC, TM_Y = NCOLS + chain * YW, TM_Z = NCOLS + (NCH + chain) * YW;   // this chain's accumulators
-  constexpr uint32_t TM_P = NCOLS + 2 * NCH * YW;   // P of the chains, 64 columns each
+  constexpr uint32_t TM_P = NCOLS + 2 * NCH * YW;   // P of the chains, 64 columns each (IN_TURN: of both, the first 64)
   WaitCtl ctl{&ctrl.abort, p.status};
 
   auto chunk_info = [&](int i, int& t0, int& rows) {
@@ -412,15 +429,24 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       // (p) P = G Xu^T goes out as soon as the key-row warps have built Xu (they do that first thing in this phase): it runs
       // behind (a), under the epilogue of (a), and nobody waits for it later.  (The previous chunk's P must have been read.)
       mbar_wait(&ctrl.bar_xu[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
-      if (NCH > 1 && kstep > 0) mbar_wait(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);
+      if (CROSS && kstep > 0) mbar_wait(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);
+      const bool add = C::IN_TURN && chain == 1;
+      if (add) mbar_wait(&ctrl.bar_turn, kstep & 1, ctl, DEV_TIMEOUT_MMA);
       if (elect_one()) {
         tc_fence_after();
-        const uint64_t da = make_desc(smem_u32(smem + C::OFF_GX) + TM_C / 8 * 2048, 2048, 128, LAYOUT_PLAIN);   // G: K-major over (i = d, j = n')
-        const uint64_t db = make_desc(smem_u32(smem + C::OFF_XU) + TM_C / 8 * 1024, 1024, 128, LAYOUT_PLAIN);   // Xu: K-major over (i = t, j = n')
+        // A step of K = 16 is two column blocks: the same eight value columns of two slices (of one slice: the next eight columns).
+        // With sixteen columns a thread the two lie two blocks apart; first all slices of the first eight columns, then of the others.
+        constexpr int APART = CW == 16 && EL > 1 ? 2 : 1, EH = EL > 1 ? EL / 2 : 1;
+        const uint64_t da = make_desc(smem_u32(smem + C::OFF_GX) + TM_C / 8 * 2048, APART * 2048, 128, LAYOUT_PLAIN);   // G: K-major over (i = d, j = n')
+        const uint64_t db = make_desc(smem_u32(smem + C::OFF_XU) + TM_C / 8 * 1024, APART * 1024, 128, LAYOUT_PLAIN);   // Xu: K-major over (i = t, j = n')
         constexpr uint32_t idesc = make_idesc(128, 64, 0, 0);
+        const uint32_t tm_p = tmem + TM_P + (C::IN_TURN ? 0 : chain * 64);
 #pragma unroll
-        for (int kk = 0; kk < CC / 16; ++kk)
-          umma_bf16(tmem + TM_P + chain * 64, desc_advance(da, kk * 4096), desc_advance(db, kk * 2048), idesc, kk > 0);
+        for (int kk = 0; kk < CC / 16; ++kk) {
+          const int blk = APART == 1 ? 2 * kk : kk / EL * (2 * EL) + kk % EL / EH + kk % EH * 4;
+          umma_bf16(tm_p, desc_advance(da, blk * 2048), desc_advance(db, blk * 1024), idesc, add || kk > 0);
+        }
+        if (C::IN_TURN && chain == 0) umma_commit(&ctrl.bar_turn);
         umma_commit(&ctrl.bar_ex[chain]);
       }
       __syncwarp();
@@ -487,7 +513,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       constexpr int EP = (8 / CW) < 1 ? 1 : (8 / CW) < EL ? (8 / CW) : EL;   // slices per piece of eight columns
       constexpr int NP = EL / EP;
       float kg[2][EP * CW];
-      if (NCH > 1 && kstep > 0) mbar_wait(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);   // the previous chunk's dr partials have been read
+      if (CROSS && kstep > 0) mbar_wait(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);   // the previous chunk's dr partials have been read
       if (sgp == 0) {
         tmem_ld<CW>(tmem_row + TM_Y + (v0 - chain * CV), du);
       } else {
@@ -502,24 +528,28 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         const float* kp = kg[pc & 1];
 #pragma unroll
         for (int ee = 0; ee < EP; ++ee) {
+          // dr partials: the even and the odd columns of every eight apart, whatever the thread's width
           const float re = gr[pc * EP + ee];
-          if constexpr (TWO_WIDE) {
+          float part = 0.f;
+#pragma unroll
+          for (int c8 = 0; c8 < CW; c8 += 8) {
             float2 dot = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int c = 0; c < CW; c += 2) {
-              fma_pair(du[c], du[c + 1], re, kp[ee * CW + c], kp[ee * CW + c + 1]);
-              dot = __ffma2_rn(make_float2(uv[c], uv[c + 1]), make_float2(kp[ee * CW + c], kp[ee * CW + c + 1]), dot);
+            for (int c = c8; c < c8 + 8; c += 2) {
+              const float k0 = kp[ee * CW + c], k1 = kp[ee * CW + c + 1];
+              if constexpr (TWO_WIDE) {
+                fma_pair(du[c], du[c + 1], re, k0, k1);
+                dot = __ffma2_rn(make_float2(uv[c], uv[c + 1]), make_float2(k0, k1), dot);
+              } else {
+                du[c] = fmaf(re, k0, du[c]);
+                du[c + 1] = fmaf(re, k1, du[c + 1]);
+                dot.x = fmaf(uv[c], k0, dot.x);
+                dot.y = fmaf(uv[c + 1], k1, dot.y);
+              }
             }
-            drp[(cgp * 64 + t) * ES + e0 + pc * EP + ee] = dot.x + dot.y;
-          } else {
-            float dot = 0.f;
-#pragma unroll
-            for (int c = 0; c < CW; ++c) {
-              du[c] = fmaf(re, kp[ee * CW + c], du[c]);
-              dot = fmaf(uv[c], kp[ee * CW + c], dot);
-            }
-            drp[(cgp * 64 + t) * ES + e0 + pc * EP + ee] = dot;
+            part = c8 == 0 ? dot.x + dot.y : part + (dot.x + dot.y);
           }
+          drp[(cgp * 64 + t) * ES + e0 + pc * EP + ee] = part;
         }
       }
       if constexpr (NSG > 1) {
@@ -644,35 +674,50 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       umma_commit(&ctrl.bar_ad[chain]);
     }
     __syncwarp();                                    // the other lanes must not run ahead into a spin wait
-    // meanwhile: the two sums over all value columns of the block, of which each chain takes half of the tokens: P (128 key rows x
-    // 64 tokens, f32, the chains' shares added) -> bf16 operand image (i = d, j = t), SI = 128, SJ = 2048, of this value block (a
-    // warp's 16-byte stores cover 512 contiguous bytes), and dr from the partials of the column groups in a fixed order.
-    if (NCH > 1) mbar_wait_spin(&ctrl.bar_ex[chain ^ 1], kstep & 1, ctl, DEV_TIMEOUT_MMA);
+    // meanwhile: the two sums over all value columns of a block, of which each chain that shares one takes half of the tokens: P (128
+    // key rows x 64 tokens, f32, the chains' shares added) -> bf16 operand image (i = d, j = t), SI = 128, SJ = 2048 (a warp's 16-byte
+    // stores cover 512 contiguous bytes), and dr from the partials of the column groups in a fixed order.
+    if (CROSS) mbar_wait_spin(&ctrl.bar_ex[chain ^ 1], kstep & 1, ctl, DEV_TIMEOUT_MMA);
     {
       tc_fence_after();
-      const int c0 = wg * 16;                        // this warpgroup's sixteen tokens
-      uint8_t* dst = reinterpret_cast<uint8_t*>(p.dkg) + (item * NV + vb) * 16384 + row * 16;
-      float pv[16], pw[16];
-      tmem_ld<16>(tmem_row + TM_P + c0, pv);
-      if constexpr (NCH > 1) tmem_ld<16>(tmem_row + TM_P + 64 + c0, pw);
-      for (int idx = tid & (CT - 1); idx < 64 / NCH * E; idx += CT) {
-        const int r = chain * (64 / NCH) + idx / E, e = idx % E;
-        float s4 = 0.f;
+      const int64_t block = item * NVB + (C::OWN ? vb * 2 + chain : vb);
+      uint8_t* dst = reinterpret_cast<uint8_t*>(p.dkg) + block * 16384 + row * 16;
+      float* dr_out = p.dr + block * (64 * E);
+      constexpr int TOKENS = C::OWN ? 32 : 16;       // of this warpgroup
+      const int c0 = (C::OWN ? wg & 1 : wg) * TOKENS;
 #pragma unroll
-        for (int w = 0; w < NCG; ++w) s4 += drp[(w * 64 + r) * ES + e];
-        p.dr[((item * NV + vb) * 64 + r) * E + e] = s4;
+      for (int cc = 0; cc < TOKENS; cc += 16) {
+        float pv[16], pw[16];
+        tmem_ld<16>(tmem_row + TM_P + (C::OWN ? chain * 64 : 0) + c0 + cc, pv);
+        if constexpr (CROSS && !C::IN_TURN) tmem_ld<16>(tmem_row + TM_P + 64 + c0 + cc, pw);
+        if (cc == 0) {
+          constexpr int ROWS = C::OWN ? 64 : 64 / NCH;
+          for (int idx = tid & (CT - 1); idx < ROWS * E; idx += CT) {
+            const int r = (C::OWN ? 0 : chain * ROWS) + idx / E, e = idx % E;
+            const float* part = drp + r * ES + e;    // group w: 64 * ES floats further on
+            float sum;
+            if constexpr (C::OWN) sum = part[2 * chain * (64 * ES)] + part[(2 * chain + 1) * (64 * ES)];
+            else if constexpr (E <= 4) sum = (part[0] + part[64 * ES]) + (part[2 * 64 * ES] + part[3 * 64 * ES]);   // as the wide CTA adds
+            else {
+              sum = part[0];
+#pragma unroll
+              for (int w = 1; w < NCG; ++w) sum += part[w * (64 * ES)];
+            }
+            dr_out[r * E + e] = sum;
+          }
+        }
+        tmem_wait_ld();
+        if constexpr (CROSS && !C::IN_TURN) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pv[j] += pw[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; j += 8)
+          *reinterpret_cast<uint4*>(dst + ((c0 + cc + j) >> 3) * 2048) =
+              make_uint4(pack_bf16(pv[j], pv[j + 1]), pack_bf16(pv[j + 2], pv[j + 3]), pack_bf16(pv[j + 4], pv[j + 5]),
+                         pack_bf16(pv[j + 6], pv[j + 7]));
       }
-      tmem_wait_ld();
-      if constexpr (NCH > 1) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) pv[j] += pw[j];
-      }
-#pragma unroll
-      for (int j = 0; j < 16; j += 8)
-        *reinterpret_cast<uint4*>(dst + ((c0 + j) >> 3) * 2048) =
-            make_uint4(pack_bf16(pv[j], pv[j + 1]), pack_bf16(pv[j + 2], pv[j + 3]), pack_bf16(pv[j + 4], pv[j + 5]),
-                       pack_bf16(pv[j + 6], pv[j + 7]));
-      if constexpr (NCH > 1) {
+      if constexpr (CROSS) {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctrl.bar_done);
@@ -759,16 +804,28 @@ static int launch_rec(const CUtensorMap& mk, const CUtensorMap& mq,
                            : launch_rec_rows<E, VC, NCH, NSG, false>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
 }
 
+// Two value blocks per CTA?  Up to four slices a CTA of 64 columns (two chains of 32) takes 1.3 to 1.35 times as long per chunk as one
+// of 32 for twice the columns: it wins when it saves waves (one CTA per SM) by more than that.  us, narrow -> wide, B=4, T=4096, H=16
+// (two waves or one): E = 1 289 -> 188, E = 2 306 -> 206, E = 4 378 -> 256.  On packed rows the host knows the number of documents but
+// not their lengths, and where one document's chain sets the time the wide CTA's longer chunk loses: forward + backward, E = 1 / 2 / 4,
+// sixteen documents of 1024 tokens, H=8: 505 / 562 / 655 -> 446 / 499 / 605; one of 8192 and eight of 1024: 834 / 920 / 1126 -> 906 /
+// 994 / 1323.
+static bool rec_wide(int E, long long sequences, int H) {
+  if (E > 4) return false;
+  const long long sms = tgdn_sm_count(), seqs = sequences * H;
+  const long long narrow = (seqs * 4 + sms - 1) / sms, wide = (seqs * 2 + sms - 1) / sms;
+  return wide * 7 < narrow * 5;
+}
+
 int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
                             const float* gc, const void* AP, const void* Pm, const void* U, float scale, const int32_t* doc_offsets,
-                            const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, int value_block, void* dV,
+                            const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, void* dV,
                             void* dU, void* ds, void* dkg, float* dr, const float* grad_state_in, float* grad_state_out,
                             void* stream) {
   if ((reinterpret_cast<uintptr_t>(grad_state_in) | reinterpret_cast<uintptr_t>(grad_state_out)) & 15) return TGDN_ERR_ALIGN;
   if (!q || !k || !dO || !k2 || !q2 || !beta || !gc || !AP || !Pm || !U || !dV || !dU || !ds || !dkg || !dr) return TGDN_ERR_NULL;
   const bool packed = chunk_map != nullptr;
   if (packed && (!doc_offsets || n_docs < 1)) return TGDN_ERR_NULL;
-  if (value_block != tgdn_value_block(E) && !(E <= 4 && value_block == 64)) return TGDN_ERR_SHAPE;
   int rc = tgdn_check_core_shape(B, T, H, E, NC, packed, row_tokens);
   if (rc) return rc;
   if ((reinterpret_cast<uintptr_t>(dO) | reinterpret_cast<uintptr_t>(AP) | reinterpret_cast<uintptr_t>(Pm) |
@@ -785,7 +842,8 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   CUtensorMap mdo, mu, mdu, mdv, ma, mb = mk;
   const int beta_tma = H % 4 == 0 && (reinterpret_cast<uintptr_t>(beta) & 15) == 0 ? 1 : 0;
   if (beta_tma && (rc = tgdn_make_gate_map(&mb, beta, B, T, H / 4, 4, row_tokens))) return rc;   // (B, T, H) read as (B, T, H/4, 4)
-  const int blocks = value_block / 8, share = E <= 2 && value_block == 32 ? blocks : blocks / 2;   // dU leaves by chain
+  const bool wide = rec_wide(E, packed ? n_docs : B, H);
+  const int blocks = (wide ? 64 : tgdn_value_block(E)) / 8, share = E <= 2 && !wide ? blocks : blocks / 2;   // dU leaves by chain
   if ((rc = tgdn_make_image_map(&mdo, dO, B, T, H, blocks, row_tokens))) return rc;
   if ((rc = tgdn_make_image_map(&mu, U, 1, static_cast<int>(crows), 1, blocks))) return rc;
   if ((rc = tgdn_make_image_map(&mdu, dU, 1, static_cast<int>(crows), 1, share))) return rc;
@@ -799,13 +857,13 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1:
-      if (value_block == 64) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+      if (wide) return launch_rec<1, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
       return launch_rec<1, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     case 2:
-      if (value_block == 64) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+      if (wide) return launch_rec<2, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
       return launch_rec<2, 32, 1>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     case 4:
-      if (value_block == 64) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
+      if (wide) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
       return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     // E = 8: 32 value columns per CTA measured 9% faster than two CTAs per SM of 16 columns each (5.26 -> 4.77 ms at B=8, T=8192, H=32,
     // before the chains), and the state-gradient kernel then adds four value-block images per item instead of eight.
@@ -821,7 +879,7 @@ extern "C" int tgdn_bwd_recurrent_state(const void* q, const void* k, const void
                                         float scale, const int32_t* doc_offsets, const int32_t* chunk_map, int n_docs, int B,
                                         int T, int H, int E, int NC, void* dV, void* dU, void* ds, void* dkg, float* dr,
                                         const float* grad_state_in, float* grad_state_out, void* stream) {
-  return tgdn_bwd_recurrent_rows(q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, doc_offsets, chunk_map, n_docs, B, T, H, E, NC, T, tgdn_value_block(E),
+  return tgdn_bwd_recurrent_rows(q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, doc_offsets, chunk_map, n_docs, B, T, H, E, NC, T,
                                  dV, dU, ds, dkg, dr, grad_state_in, grad_state_out, stream);
 }
 

@@ -512,7 +512,7 @@ static int launch_sg(const CUtensorMap& mdv, const CUtensorMap& mdo, const SgPar
 
 int tgdn_bwd_state_grads_rows(const void* q, const void* k, const void* dO, const void* dV, const void* h, const void* ds,
                               const void* dkg, const float* k2, const float* q2, const float* gc, float scale,
-                              const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, int value_block, void* dkq, float* da,
+                              const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, void* dkq, float* da,
                               float* dc, float* dd, void* stream) {
   if (!q || !k || !dO || !dV || !h || !ds || !dkg || !k2 || !q2 || !gc || !dkq || !da || !dc || !dd) return TGDN_ERR_NULL;
   int rc = tgdn_check_core_shape(B, T, H, E, NC, chunk_map != nullptr, row_tokens);
@@ -529,7 +529,7 @@ int tgdn_bwd_state_grads_rows(const void* q, const void* k, const void* dO, cons
   SgParams p{static_cast<const __nv_bfloat16*>(k), static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(dO), static_cast<const __nv_bfloat16*>(dV),
              static_cast<const __nv_bfloat16*>(h),
              static_cast<const __nv_bfloat16*>(ds), static_cast<const __nv_bfloat16*>(dkg), k2, q2, gc,
-             static_cast<__nv_bfloat16*>(dkq), da, dc, dd, chunk_map, B, T, H, NC, HEAD / value_block, row_tokens, scale,
+             static_cast<__nv_bfloat16*>(dkq), da, dc, dd, chunk_map, B, T, H, NC, HEAD / tgdn_value_block(E), row_tokens, scale,
              tgdn_status_word(), tgdn_sm_count()};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
@@ -547,6 +547,6 @@ extern "C" int tgdn_bwd_state_grads(const void* q, const void* k, const void* dO
                                     const void* h, const void* ds, const void* dkg, const float* k2, const float* q2,
                                     const float* gc, float scale, const int32_t* chunk_map, int B, int T, int H, int E, int NC, void* dkq,
                                     float* da, float* dc, float* dd, void* stream) {
-  return tgdn_bwd_state_grads_rows(q, k, dO, dV, h, ds, dkg, k2, q2, gc, scale, chunk_map, B, T, H, E, NC, T, tgdn_value_block(E), dkq, da, dc, dd,
+  return tgdn_bwd_state_grads_rows(q, k, dO, dV, h, ds, dkg, k2, q2, gc, scale, chunk_map, B, T, H, E, NC, T, dkq, da, dc, dd,
                                    stream);
 }

@@ -44,8 +44,6 @@ int tgdn_dynamic_smem(const void* kernel, int bytes, bool* configured);
 // The core stages on a token range of longer rows: the arguments of the entry points of the same name (include/tgdn.h) plus
 // row_tokens >= T, the tokens from one batch row to the next in every token-layout tensor (inputs and outputs; the chunk-layout
 // tensors are those of the T tokens alone).  Dense rows; the entry points of the public ABI are these with row_tokens = T.
-// value_block: value columns per CTA of the reverse recurrence, the same for all three backward stages (dkg and dr have 128/value_block
-// blocks): tgdn_value_block(E), or 64 up to four slices; tgdn_value_block_for picks by the number of sequences.
 int tgdn_masks_rows(const void* q, const void* k, const float* k2, const float* q2, const float* g, const float* beta, float scale,
                     const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, float* gc, void* AP, void* Pm,
                     void* stream);
@@ -55,17 +53,17 @@ int tgdn_fwd_rows(const void* q, const void* k, const void* v, const float* k2, 
                   void* stream);
 int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const float* k2, const float* q2, const float* beta,
                             const float* gc, const void* AP, const void* Pm, const void* U, float scale, const int32_t* doc_offsets,
-                            const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, int value_block, void* dV,
+                            const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, void* dV,
                             void* dU, void* ds, void* dkg, float* dr, const float* grad_state_in, float* grad_state_out,
                             void* stream);
 int tgdn_bwd_state_grads_rows(const void* q, const void* k, const void* dO, const void* dV, const void* h, const void* ds,
                               const void* dkg, const float* k2, const float* q2, const float* gc, float scale,
-                              const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, int value_block, void* dkq, float* da,
+                              const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, void* dkq, float* da,
                               float* dc, float* dd, void* stream);
 int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const void* dU, const void* W, const void* U, const void* AP,
                          const float* k2, const float* q2, const float* beta, const float* gc, const void* dkq, const float* da,
                          const float* dc, const float* dd, const float* dr, float scale, const int32_t* chunk_map, int B, int T,
-                         int H, int E, int NC, int row_tokens, int value_block, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
+                         int H, int E, int NC, int row_tokens, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
                          void* stream);
 
 // The convolution for any channel count, strides and 2-byte aligned rows (weight: 8-byte aligned); the entry points of the public ABI
@@ -84,5 +82,5 @@ int tgdn_glue_bwd(const void* x, const void* weight, const int32_t* cu, int n_do
                   int H, int E, float eps, const void* dq, const void* dk, const void* dv, const float* dk2, const float* dq2, void* dx,
                   void* dw, void* dy_gates, void* scratch, int64_t scratch_bytes, void* stream);
 
+// Value columns of a block of the reverse recurrence: dkg (rounded per block) and dr have 128 / tgdn_value_block(E) of them.
 int tgdn_value_block(int E);
-int tgdn_value_block_for(int E, long long sequences, int H);

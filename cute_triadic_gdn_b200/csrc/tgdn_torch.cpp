@@ -117,7 +117,7 @@ void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.devi
 
 struct Dims {
   int B, T, H, E, NC, row_tokens, n_docs;
-  int value_block() const { return tgdn_value_block_for(E, n_docs ? n_docs : B, H); }      // of the reverse recurrence
+  int64_t blocks() const { return 128 / tgdn_value_block(E); }      // value blocks of the reverse recurrence
 };
 
 // `row_tokens`: q may be a token range of longer rows, (B, T, H, 128) with the batch stride of the whole rows.
@@ -180,8 +180,7 @@ Reverse run_reverse(const Tensor& q, const Tensor& k, const Tensor& dO, const Te
                     const OptTensor& token_map, const OptTensor& grad_state_in, const OptTensor& grad_state_out) {
   const c10::cuda::CUDAGuard guard(q.device());
   const Dims d = dims(q, k2, token_map, chunk_starts);
-  const int VB = d.value_block();
-  const int64_t NV = 128 / VB;
+  const int64_t NV = d.blocks();
   Reverse r;
   r.dV = empty(dO.sizes(), dO, at::kBFloat16);
   r.dU = empty({d.B, d.NC, d.H, CHUNK, 128}, q, at::kBFloat16);
@@ -190,7 +189,7 @@ Reverse run_reverse(const Tensor& q, const Tensor& k, const Tensor& dO, const Te
   r.dr = empty({d.B, d.NC, d.H, NV, CHUNK, d.E}, q, at::kFloat);
   check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U),
                                    static_cast<float>(scale), ptr<int32_t>(chunk_starts), ptr<int32_t>(token_map), d.n_docs, d.B, d.T, d.H,
-                                   d.E, d.NC, d.row_tokens, VB, ptr(r.dV), ptr(r.dU), ptr(r.ds), ptr(r.dkg), ptr<float>(r.dr),
+                                   d.E, d.NC, d.row_tokens, ptr(r.dV), ptr(r.dU), ptr(r.ds), ptr(r.dkg), ptr<float>(r.dr),
                                    ptr<float>(grad_state_in), ptr<float>(grad_state_out), stream_of(q)),
            "tgdn_bwd_recurrent");
   return r;
@@ -210,7 +209,7 @@ StateGrads run_state_grads(const Tensor& q, const Tensor& k, const Tensor& dO, c
   s.dd = empty({d.B, d.NC, d.H, d.E}, q, at::kFloat);
   check_rc(tgdn_bwd_state_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(dV), ptr(h), ptr(ds), ptr(dkg), fptr(k2), fptr(q2), fptr(gc),
                                      static_cast<float>(scale), ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC, d.row_tokens,
-                                     static_cast<int>(128 / dkg.size(3)), ptr(s.dkq), ptr<float>(s.da), ptr<float>(s.dc), ptr<float>(s.dd), stream_of(q)),
+                                     ptr(s.dkq), ptr<float>(s.da), ptr<float>(s.dc), ptr<float>(s.dd), stream_of(q)),
            "tgdn_bwd_state_grads");
   return s;
 }
@@ -238,7 +237,7 @@ void run_matrix(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor
   const Dims d = dims(q, k2, token_map);
   check_rc(tgdn_bwd_matrix_rows(ptr(q), ptr(k), ptr(dO), ptr(dU), ptr(W), ptr(U), ptr(AP), fptr(k2), fptr(q2), fptr(beta), fptr(gc),
                                 ptr(s.dkq), fptr(s.da), fptr(s.dc), fptr(s.dd), fptr(dr), static_cast<float>(scale),
-                                ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC, d.row_tokens, static_cast<int>(128 / dr.size(3)),
+                                ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC, d.row_tokens,
                                 ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2), ptr<float>(out.g), ptr<float>(out.beta), stream_of(q)),
            "tgdn_bwd_matrix");
 }
@@ -258,8 +257,7 @@ void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tens
   // kernel's temporaries matter).
   const c10::cuda::CUDAGuard guard(q.device());
   const Dims d = dims(q, k2, token_map, chunk_starts);
-  const int64_t items = static_cast<int64_t>(d.B) * d.NC * d.H, NV = 128 / d.value_block();
-  const int VB = d.value_block();
+  const int64_t items = static_cast<int64_t>(d.B) * d.NC * d.H, NV = d.blocks();
   const float sc = static_cast<float>(scale);
   const int32_t *starts = ptr<int32_t>(chunk_starts), *map = ptr<int32_t>(token_map);
   void* stream = stream_of(q);
@@ -270,15 +268,15 @@ void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tens
   float *dr = reinterpret_cast<float*>(dkq + items * 32768), *da = dr + items * NV * 64 * d.E, *dc = da + items * 64 * d.E,
         *dd = dc + items * 64 * d.E;
   check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U), sc, starts, map,
-                                   d.n_docs, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, VB, ptr(out.v), dU, ds, dkg, dr, ptr<float>(grad_state_in),
+                                   d.n_docs, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, ptr(out.v), dU, ds, dkg, dr, ptr<float>(grad_state_in),
                                    ptr<float>(grad_state_out), stream),
            "tgdn_bwd_recurrent");
   check_rc(tgdn_bwd_state_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(out.v), ptr(h), ds, dkg, fptr(k2), fptr(q2), fptr(gc), sc, map, d.B, d.T, d.H,
-                                     d.E, d.NC, d.row_tokens, VB, dkq, da, dc, dd, stream),
+                                     d.E, d.NC, d.row_tokens, dkq, da, dc, dd, stream),
            "tgdn_bwd_state_grads");
   big.reset();
   check_rc(tgdn_bwd_matrix_rows(ptr(q), ptr(k), ptr(dO), dU, ptr(W), ptr(U), ptr(AP), fptr(k2), fptr(q2), fptr(beta), fptr(gc), dkq, da, dc, dd, dr,
-                                sc, map, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, VB, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2),
+                                sc, map, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2),
                                 ptr<float>(out.g), ptr<float>(out.beta), stream),
            "tgdn_bwd_matrix");
 }
