@@ -610,9 +610,12 @@ struct ConvInput {
 };
 
 bool aligned(const Tensor& t, uintptr_t bytes) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % bytes == 0; }
-bool rows_aligned(const Tensor& t) { return t.stride(2) == 1 && t.stride(1) % 8 == 0 && t.stride(0) % 8 == 0 && aligned(t, 16); }
+// Strides of the token and the batch axis.  An axis of size one may carry any stride, and contiguous() leaves it: it counts as dense.
+int64_t token_stride(const Tensor& t) { return t.size(1) == 1 ? t.size(2) : t.stride(1); }
+int64_t batch_stride(const Tensor& t) { return t.size(0) == 1 ? t.size(1) * token_stride(t) : t.stride(0); }
+bool rows_aligned(const Tensor& t) { return token_stride(t) % 8 == 0 && batch_stride(t) % 8 == 0 && aligned(t, 16); }
 // Rows of consecutive channels that do not overlap: what the kernels read in place.
-bool rows_readable(const Tensor& t) { return t.stride(2) == 1 && t.stride(1) >= t.size(2); }
+bool rows_readable(const Tensor& t) { return (t.size(2) == 1 || t.stride(2) == 1) && token_stride(t) >= t.size(2); }
 
 // `pieces`: the rows must be whole 16-byte pieces (the fused kernels); otherwise any readable row will do.
 ConvInput conv_prep(const Tensor& x, const Tensor& weight, const OptTensor& cu, bool pieces = false) {
@@ -642,7 +645,7 @@ Tensor conv_fwd(const Tensor& x, const Tensor& weight, int64_t act_channels, con
   const int64_t B = c.x.size(0), T = c.x.size(1), C = c.x.size(2);
   Tensor y = empty({B, T, C}, c.x, at::kBFloat16);
   check_rc(tgdn_conv_fwd_any(ptr(c.x), ptr(c.weight), ptr(y), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T),
-                             static_cast<int>(C), c.x.stride(0), c.x.stride(1), static_cast<int>(act_channels), stream_of(c.x)),
+                             static_cast<int>(C), batch_stride(c.x), token_stride(c.x), static_cast<int>(act_channels), stream_of(c.x)),
            "tgdn_conv_fwd");
   return y;
 }
@@ -656,7 +659,7 @@ std::tuple<Tensor, Tensor> conv_bwd(const Tensor& x, const Tensor& dy_in, const 
   const int64_t nbytes = tgdn_conv_bwd_best_scratch(static_cast<int>(B), static_cast<int>(T), static_cast<int>(C));
   Tensor scratch = empty({nbytes / 4}, c.x, at::kFloat);
   check_rc(tgdn_conv_bwd_any(ptr(c.x), ptr(c.weight), ptr(dy), ptr(dx), ptr(dw), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B),
-                             static_cast<int>(T), static_cast<int>(C), c.x.stride(0), c.x.stride(1), dy.stride(0), dy.stride(1),
+                             static_cast<int>(T), static_cast<int>(C), batch_stride(c.x), token_stride(c.x), batch_stride(dy), token_stride(dy),
                              static_cast<int>(act_channels), ptr(scratch), nbytes, stream_of(c.x)),
            "tgdn_conv_bwd");
   return {dx, dw.to(weight.scalar_type())};
@@ -680,7 +683,7 @@ Five norm_fwd(const Tensor& x, const Tensor& weight, int64_t heads, int64_t slic
          v = empty({B, T, heads, 128}, x, at::kBFloat16), k2 = empty({B, T, heads, slices}, x, at::kFloat),
          q2 = empty({B, T, heads, slices}, x, at::kFloat);
   check_rc(tgdn_glue_fwd(ptr(c.x), ptr(c.weight), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T), static_cast<int>(C),
-                         c.x.stride(0), c.x.stride(1), static_cast<int>(heads), static_cast<int>(slices), static_cast<float>(eps), ptr(q),
+                         batch_stride(c.x), token_stride(c.x), static_cast<int>(heads), static_cast<int>(slices), static_cast<float>(eps), ptr(q),
                          ptr(k), ptr(v), ptr<float>(k2), ptr<float>(q2), stream_of(c.x)),
            "tgdn_glue_fwd");
   return {q, k, v, k2, q2};
@@ -700,7 +703,7 @@ std::tuple<Tensor, Tensor> norm_bwd(const Tensor& x, const Tensor& weight, const
   const int64_t nbytes = tgdn_conv_bwd_best_scratch(static_cast<int>(B), static_cast<int>(T), static_cast<int>(C));
   Tensor scratch = empty({nbytes / 4}, c.x, at::kFloat);
   check_rc(tgdn_glue_bwd(ptr(c.x), ptr(c.weight), ptr<int32_t>(c.cu), c.n_docs, static_cast<int>(B), static_cast<int>(T), static_cast<int>(C),
-                         c.x.stride(0), c.x.stride(1), static_cast<int>(heads), static_cast<int>(slices), static_cast<float>(eps), ptr(q),
+                         batch_stride(c.x), token_stride(c.x), static_cast<int>(heads), static_cast<int>(slices), static_cast<float>(eps), ptr(q),
                          ptr(k), ptr(v), fptr(k2), fptr(q2), ptr(dx), ptr(dw), ptr(dy_gates), ptr(scratch), nbytes, stream_of(c.x)),
            "tgdn_glue_bwd");
   return {dx, dw.to(weight.scalar_type())};

@@ -1,0 +1,41 @@
+"""Forms of a call that a program may use: strides, sizes, argument types, threads and modes around it."""
+import pytest
+import torch
+
+from cute_triadic_gdn_b200 import _lib, conv_split_act_call, conv_split_norm_call
+from oracle import triadic_oracle as orc
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+def conv_step(x, w, act, dy):
+    x, w = x.detach().requires_grad_(True), w.detach().requires_grad_(True)
+    y = conv_split_act_call(x, w, act)
+    return (y.detach(), *torch.autograd.grad(y, (x, w), dy))
+
+
+@pytest.mark.parametrize("B,T,C", [(2, 1, 77), (3, 1, 80), (2, 1, 1), (1, 1, 1), (1, 5, 1), (2, 6, 1), (1, 7, 48)])
+def test_convolution_of_axes_of_size_one(B, T, C):
+    """An axis of size one has whatever stride the tensor was made with, in x and in the gradient (an expanded scalar: zeros)."""
+    g = torch.Generator().manual_seed(C)
+    x, w = torch.randn(B, T, C, generator=g).to(BF16).cuda(), torch.randn(C, 4, generator=g).to(BF16).cuda()
+    ref = conv_step(x, w, C // 2, torch.ones_like(x))
+    views = [x.transpose(1, 2).contiguous().transpose(1, 2), x.permute(2, 1, 0).contiguous().permute(2, 1, 0),
+             torch.cat([x, x], -1)[..., :C], torch.cat([x, x], 1)[:, :T],
+             x.contiguous().as_strided((B, T, C), (x.stride(0) if B > 1 else 3, x.stride(1) if T > 1 else 5, 1 if C > 1 else 7))]
+    for v in views:
+        for dy in (torch.ones_like(x), torch.ones((), dtype=BF16, device="cuda").expand(B, T, C)):
+            for a, b in zip(conv_step(v, w, C // 2, dy), ref):
+                assert torch.equal(a, b)
+    assert _lib.device_status() == 0
+
+
+def test_glue_of_one_token_with_any_stride():
+    H, E = 2, 4
+    C = H * (3 * 128 + 2 * E)
+    g = torch.Generator().manual_seed(3)
+    x, w = torch.randn(2, 1, C, generator=g).to(BF16).cuda(), torch.randn(C, 4, generator=g).to(BF16).cuda()
+    view = x.transpose(1, 2).contiguous().transpose(1, 2)
+    for a, b in zip(conv_split_norm_call(view, w, H, E), conv_split_norm_call(x, w, H, E)):
+        assert torch.equal(a, b)
