@@ -1008,12 +1008,14 @@ static int reduce_dw_launch(const float* partial, void* dw, int n_partial, int C
   return tgdn_cuda_error(cudaGetLastError());
 }
 
-// Tokens per CTA of the walkers: sub-runs of at least 16 rows, a few waves of CTAs.
+// Tokens per CTA of the walkers: sub-runs of at least 16 rows, a few waves of CTAs, and of at most 256 rows as long as the grid holds
+// that many CTAs along the token axis (65535).
 static int walk_run(int B, int T, int columns) {
   int64_t groups = static_cast<int64_t>(32) * tgdn_sm_count() / (static_cast<int64_t>(columns) * B);
   if (groups < 1) groups = 1;
   const int64_t run = (T + groups - 1) / groups;
-  return static_cast<int>(std::min<int64_t>(std::max<int64_t>(run, 16 * CONV_WARPS), 256 * CONV_WARPS));
+  const int64_t longest = std::max<int64_t>(256 * CONV_WARPS, (static_cast<int64_t>(T) + 65534) / 65535);
+  return static_cast<int>(std::min<int64_t>(std::max<int64_t>(run, 16 * CONV_WARPS), longest));
 }
 template <int V>
 static dim3 walk_grid(int B, int C, int groups) { return dim3((C + 32 * V - 1) / (32 * V), groups, B); }

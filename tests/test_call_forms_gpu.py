@@ -39,3 +39,18 @@ def test_glue_of_one_token_with_any_stride():
     view = x.transpose(1, 2).contiguous().transpose(1, 2)
     for a, b in zip(conv_split_norm_call(view, w, H, E), conv_split_norm_call(x, w, H, E)):
         assert torch.equal(a, b)
+
+
+def test_convolution_of_more_tokens_than_a_grid_has_rows():
+    """65535 runs of 2048 tokens and five more: two bytes a token."""
+    T = 65535 * 2048 + 5
+    x = torch.ones(1, T, 1, dtype=BF16, device="cuda")
+    x[0, -1] = 3.0
+    w = torch.tensor([[1.0, 2.0, 4.0, 8.0]], dtype=BF16, device="cuda")
+    y = conv_split_act_call(x, w, 0)
+    dx, dw = torch.ops.tgdn_b200.conv_split_act_bwd(x, x, w, 0, None)
+    assert _lib.device_status() == 0
+    assert y[0, :4, 0].tolist() == [8, 12, 14, 15] and y[0, -2:, 0].tolist() == [15, 31] and bool((y[0, 3:-1] == 15).all())
+    assert dx[0, -5:, 0].tolist() == [15, 17, 18, 20, 24] and bool((dx[0, :-4] == 15).all())
+    # dw[j] = sum of x[t] x[t - 3 + j]: T in f32 partials, rounded to bf16 (2^-9) at the end
+    assert torch.allclose(dw.float(), torch.full_like(dw, T).float(), rtol=2 ** -8)
