@@ -42,16 +42,13 @@ int* tgdn_status_word() {
 
 int tgdn_check_device() {
   static signed char cached[64] = {0};         // per device: 1 = compute capability 10.x, -1 = another one
-  static thread_local int bound = -1;          // the device whose context this thread has made current
   int dev = 0, major = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   // Make the device's primary context current on the calling thread.  The tensor-map encoder is a driver call and
   // fails with "invalid context" on a thread that has not touched the runtime yet (an autograd worker whose tensors all
-  // came out of the allocator's cache); setting the current device again is the documented way to bind the context.
-  if (bound != dev) {
-    if (cudaSetDevice(dev) != cudaSuccess) return 0;
-    bound = dev;
-  }
+  // came out of the allocator's cache, or one from which another library has taken the context away); setting the current
+  // device again is the documented way to bind the context.  On every call: nobody tells this library when a context goes.
+  if (cudaSetDevice(dev) != cudaSuccess) return 0;
   if (dev >= 0 && dev < 64 && cached[dev] != 0) return cached[dev] > 0;
   if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return 0;
   if (dev >= 0 && dev < 64) cached[dev] = major == 10 ? 1 : -1;

@@ -1,8 +1,11 @@
 """Forms of a call that a program may use: strides, sizes, argument types, threads and modes around it."""
+import ctypes
+import threading
+
 import pytest
 import torch
 
-from cute_triadic_gdn_b200 import _lib, conv_split_act_call, conv_split_norm_call
+from cute_triadic_gdn_b200 import _lib, conv_split_act_call, conv_split_norm_call, gdn_joint_call
 from oracle import triadic_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +57,23 @@ def test_convolution_of_more_tokens_than_a_grid_has_rows():
     assert dx[0, -5:, 0].tolist() == [15, 17, 18, 20, 24] and bool((dx[0, :-4] == 15).all())
     # dw[j] = sum of x[t] x[t - 3 + j]: T in f32 partials, rounded to bf16 (2^-9) at the end
     assert torch.allclose(dw.float(), torch.full_like(dw, T).float(), rtol=2 ** -8)
+
+
+def test_thread_whose_context_was_taken_away():
+    """Another library in the process may leave a thread without a current context after the thread's first call."""
+    ins = [t.cuda() for t in orc.make_inputs(1, 64, 2, 2, seed=5)]
+    ref, got = gdn_joint_call(*ins), []
+
+    def work():
+        try:
+            got.append(gdn_joint_call(*ins))
+            assert ctypes.CDLL("libcuda.so.1").cuCtxSetCurrent(None) == 0
+            got.append(gdn_joint_call(*ins))
+            torch.cuda.synchronize()
+        except Exception as e:                               # noqa: BLE001 (shown by the comparison below)
+            got.append(e)
+
+    thread = threading.Thread(target=work)
+    thread.start()
+    thread.join()
+    assert len(got) == 2 and all(torch.equal(o, ref) for o in got), got
