@@ -282,22 +282,26 @@ void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tens
 }
 
 // ---- operators of the core --------------------------------------------------------------------------------------------
+// `covered`: the documents of the chunk map hold every token of the row, as those of prepare_documents do.  Otherwise rows of o and of
+// dV that no document holds are zero; with it nothing has to be filled.
 std::vector<Tensor> joint_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2, const Tensor& g,
-                              const Tensor& beta, double scale, const OptTensor& chunk_starts, const OptTensor& token_map) {
+                              const Tensor& beta, double scale, const OptTensor& chunk_starts, const OptTensor& token_map, bool covered) {
   check_inputs(q, k, v, k2, q2, g, beta, has(token_map));
   check_device_and_e(q, k2.size(3));
   Masks m = run_masks(q, k, k2, q2, g, beta, scale, token_map);
-  Forward f = run_forward(q, k, v, k2, q2, beta, m.gc, m.AP, scale, true, chunk_starts, token_map, std::nullopt, std::nullopt);
+  Forward f = run_forward(q, k, v, k2, q2, beta, m.gc, m.AP, scale, true, chunk_starts, token_map, std::nullopt, std::nullopt,
+                          has(token_map) && !covered ? at::zeros(v.sizes(), v.options()) : Tensor());
   return {f.o, m.gc, m.AP, m.Pm, f.h, f.W, f.U};
 }
 
 // saved: q, k, k2, q2, g, beta, gc, [AP, Pm,] h, W, U
 std::vector<Tensor> joint_bwd(std::vector<Tensor> saved, const Tensor& dO, double scale, const OptTensor& chunk_starts,
-                              const OptTensor& token_map) {
+                              const OptTensor& token_map, bool covered) {
   TORCH_CHECK_VALUE(saved.size() == 12 || saved.size() == 10, "joint_bwd: 12 saved tensors, or 10 without the chunk operators");
   const bool with_masks = saved.size() == 12;
   const int64_t o = with_masks ? 2 : 0;
   Grads out = Grads::like(saved[0], saved[2], saved[5]);
+  if (has(token_map) && !covered) out.v.zero_();
   run_backward(saved[0], saved[1], saved[2], saved[3], saved[4], saved[5], saved[6], with_masks ? saved[7] : Tensor(),
                with_masks ? saved[8] : Tensor(), saved[7 + o], saved[8 + o], saved[9 + o], dO.contiguous(), scale, chunk_starts, token_map,
                std::nullopt, std::nullopt, out);
@@ -320,19 +324,20 @@ std::tuple<Tensor, Tensor, Tensor> joint_metadata(const Tensor& cu, int64_t toke
 }
 
 std::vector<Tensor> call_joint_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2, const Tensor& g,
-                                   const Tensor& beta, double scale, const OptTensor& chunk_starts, const OptTensor& token_map) {
+                                   const Tensor& beta, double scale, const OptTensor& chunk_starts, const OptTensor& token_map,
+                                   bool covered) {
   static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("tgdn_b200::joint_fwd", "").typed<decltype(joint_fwd)>();
-  return op.call(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map);
+  return op.call(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map, covered);
 }
 std::vector<Tensor> call_joint_bwd(at::TensorList saved, const Tensor& dO, double scale, const OptTensor& chunk_starts,
-                                   const OptTensor& token_map) {
-  using Sig = std::vector<Tensor>(at::TensorList, const Tensor&, double, const OptTensor&, const OptTensor&);
+                                   const OptTensor& token_map, bool covered) {
+  using Sig = std::vector<Tensor>(at::TensorList, const Tensor&, double, const OptTensor&, const OptTensor&, bool);
   static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("tgdn_b200::joint_bwd", "").typed<Sig>();
-  return op.call(saved, dO, scale, chunk_starts, token_map);
+  return op.call(saved, dO, scale, chunk_starts, token_map, covered);
 }
 std::vector<Tensor> joint_bwd_entry(at::TensorList saved, const Tensor& dO, double scale, const OptTensor& chunk_starts,
-                                    const OptTensor& token_map) {
-  return joint_bwd(saved.vec(), dO, scale, chunk_starts, token_map);
+                                    const OptTensor& token_map, bool covered) {
+  return joint_bwd(saved.vec(), dO, scale, chunk_starts, token_map, covered);
 }
 
 Tensor or_undefined(const OptTensor& t) { return has(t) ? *t : Tensor(); }
@@ -342,9 +347,9 @@ OptTensor or_nullopt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptT
 struct JointFunction : public torch::autograd::Function<JointFunction> {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                                const Tensor& g, const Tensor& beta, double scale, const OptTensor& chunk_starts,
-                               const OptTensor& token_map) {
+                               const OptTensor& token_map, bool covered) {
     at::AutoDispatchBelowADInplaceOrView below;
-    std::vector<Tensor> out = call_joint_fwd(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map);
+    std::vector<Tensor> out = call_joint_fwd(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map, covered);
     variable_list keep{q, k, k2, q2, g, beta, out[1]};
     if (save_masks()) {
       keep.push_back(out[2]);
@@ -355,19 +360,21 @@ struct JointFunction : public torch::autograd::Function<JointFunction> {
     keep.push_back(or_undefined(token_map));
     ctx->save_for_backward(std::move(keep));
     ctx->saved_data["scale"] = scale;
+    ctx->saved_data["covered"] = covered;
     ctx->mark_non_differentiable(variable_list(out.begin() + 1, out.end()));
     ctx->set_materialize_grads(false);
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    variable_list res(10);
+    variable_list res(11);
     if (!grads[0].defined()) return res;                 // the output was not used
     variable_list kept = ctx->get_saved_variables();      // read exactly once: under activation checkpointing every read unpacks
     const OptTensor token_map = or_nullopt(kept.back());
     kept.pop_back();
     const OptTensor chunk_starts = or_nullopt(kept.back());
     kept.pop_back();
-    std::vector<Tensor> seven = call_joint_bwd(kept, grads[0].contiguous(), ctx->saved_data["scale"].toDouble(), chunk_starts, token_map);
+    std::vector<Tensor> seven = call_joint_bwd(kept, grads[0].contiguous(), ctx->saved_data["scale"].toDouble(), chunk_starts, token_map,
+                                               ctx->saved_data["covered"].toBool());
     for (int i = 0; i < 7; ++i) res[i] = std::move(seven[i]);
     return res;
   }
@@ -375,8 +382,8 @@ struct JointFunction : public torch::autograd::Function<JointFunction> {
 
 std::vector<Tensor> joint_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                                        const Tensor& g, const Tensor& beta, double scale, const OptTensor& chunk_starts,
-                                       const OptTensor& token_map) {
-  return JointFunction::apply(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map);
+                                       const OptTensor& token_map, bool covered) {
+  return JointFunction::apply(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map, covered);
 }
 
 bool any_grad(std::initializer_list<const Tensor*> ts) {
@@ -414,7 +421,7 @@ Tensor joint_call(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   OptTensor chunk_starts, token_map;
   if (has(cu)) std::tie(chunk_starts, token_map) = prepare_documents(qc, *cu);
   return call_joint_fwd(qc, k.contiguous(), v.contiguous(), k2.contiguous(), q2.contiguous(), g.contiguous(), beta.contiguous(),
-                        scale_or_default(scale, qc), chunk_starts, token_map)[0];
+                        scale_or_default(scale, qc), chunk_starts, token_map, true)[0];
 }
 
 void check_state(const Tensor& s, at::IntArrayRef shape, const Tensor& q, const char* name) {
@@ -539,7 +546,7 @@ std::tuple<Tensor, OptTensor> chunk_joint(const Tensor& q, const Tensor& k, cons
       if (*checkpoint_tokens < q.size(1))
         return {CheckpointedFunction::apply(q, k, v, k2, q2, g, beta, scale, *checkpoint_tokens), std::nullopt};
     }
-    return {call_joint_fwd(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map)[0], std::nullopt};
+    return {call_joint_fwd(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map, true)[0], std::nullopt};
   }
   const int64_t n_seq = has(cu) ? cu->numel() - 1 : B;
   OptTensor s_in, s_out;
@@ -765,8 +772,9 @@ Five norm_fwd_autograd(const Tensor& x, const Tensor& weight, int64_t heads, int
 
 TORCH_LIBRARY(tgdn_b200, m) {
   m.def("joint_fwd(Tensor q, Tensor k, Tensor v, Tensor k2, Tensor q2, Tensor g, Tensor beta, float scale, Tensor? chunk_starts=None, "
-        "Tensor? token_map=None) -> Tensor[]");
-  m.def("joint_bwd(Tensor[] saved, Tensor do, float scale, Tensor? chunk_starts=None, Tensor? token_map=None) -> Tensor[]");
+        "Tensor? token_map=None, bool covered=False) -> Tensor[]");
+  m.def("joint_bwd(Tensor[] saved, Tensor do, float scale, Tensor? chunk_starts=None, Tensor? token_map=None, bool covered=False) -> "
+        "Tensor[]");
   m.def("joint_metadata(Tensor cu_seqlens, SymInt tokens) -> (Tensor, Tensor, Tensor)");
   m.def("conv_split_act_fwd(Tensor x, Tensor weight, SymInt act_channels, Tensor? cu_seqlens=None) -> Tensor");
   m.def("conv_split_act_bwd(Tensor x, Tensor dy, Tensor weight, SymInt act_channels, Tensor? cu_seqlens=None) -> (Tensor, Tensor)");

@@ -16,7 +16,7 @@ from .joint_packing import prepare_documents
 
 
 @torch.library.register_fake("tgdn_b200::joint_fwd")
-def _joint_fwd_fake(q, k, v, k2, q2, g, beta, scale, chunk_starts=None, token_map=None):
+def _joint_fwd_fake(q, k, v, k2, q2, g, beta, scale, chunk_starts=None, token_map=None, covered=False):
     B, T, H, D = q.shape
     E = k2.shape[-1]
     NC = token_map.shape[1] if token_map is not None else T // CHUNK
@@ -26,7 +26,7 @@ def _joint_fwd_fake(q, k, v, k2, q2, g, beta, scale, chunk_starts=None, token_ma
 
 
 @torch.library.register_fake("tgdn_b200::joint_bwd")
-def _joint_bwd_fake(saved, do, scale, chunk_starts=None, token_map=None):
+def _joint_bwd_fake(saved, do, scale, chunk_starts=None, token_map=None, covered=False):
     q, k, k2, q2, g, beta = saved[:6]
     return [torch.empty_like(q), torch.empty_like(k), torch.empty_like(do), torch.empty_like(k2), torch.empty_like(q2),
             torch.empty_like(g), torch.empty_like(beta)]
@@ -45,4 +45,4 @@ def gdn_joint_call(q, k, v, k2, q2, g, beta, scale=None, cu_seqlens=None):
     chunk_starts = token_map = None
     if cu_seqlens is not None:
         chunk_starts, token_map = prepare_documents(seven, cu_seqlens)
-    return torch.ops.tgdn_b200.joint_fwd(*seven, float(scale), chunk_starts, token_map)[0]
+    return torch.ops.tgdn_b200.joint_fwd(*seven, float(scale), chunk_starts, token_map, True)[0]

@@ -77,3 +77,30 @@ def test_thread_whose_context_was_taken_away():
     thread.start()
     thread.join()
     assert len(got) == 2 and all(torch.equal(o, ref) for o in got), got
+
+
+@pytest.mark.parametrize("E", [2, 8, 16])
+def test_operator_with_a_chunk_map_that_misses_tokens(E):
+    """Rows of o and dV that no document holds are zero, whatever the allocator hands out."""
+    T, H, cu = 256, 2, torch.tensor([0, 60, 130], dtype=torch.int32).cuda()
+    ins = [t.cuda() for t in orc.make_inputs(1, T, H, E, seed=E)]
+    do = orc.make_grad_output((1, T, H, 128), 1).cuda()
+    offsets, chunk_map, valid = torch.ops.tgdn_b200.joint_metadata(cu, T)
+    assert not bool(valid)
+
+    def litter():                                            # freed blocks of every size full of NaN
+        blocks = [torch.full((1 << n,), float("nan"), device="cuda") for n in range(8, 22) for _ in range(4)]
+        del blocks
+
+    litter()
+    leaves = [t.clone().requires_grad_(True) for t in ins]
+    litter()
+    o = torch.ops.tgdn_b200.joint_fwd(*leaves, 0.1, offsets, chunk_map)[0]
+    litter()
+    dv, = torch.autograd.grad(o, leaves[2], do)
+    assert _lib.device_status() == 0
+    part = [t[:, :130].contiguous().requires_grad_(True) for t in ins]
+    o_part = gdn_joint_call(*part, scale=0.1, cu_seqlens=cu)
+    dv_part, = torch.autograd.grad(o_part, part[2], do[:, :130].contiguous())
+    for whole, head in ((o, o_part), (dv, dv_part)):
+        assert torch.equal(whole[:, :130], head) and bool((whole[:, 130:] == 0).all())
