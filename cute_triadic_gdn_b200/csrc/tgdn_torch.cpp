@@ -14,6 +14,7 @@
 //
 // The device work is the C ABI of libtgdn_b200 (include/tgdn.h), with which this file is linked.
 #include <torch/extension.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/library.h>
 
 #include <ATen/cuda/CUDAContext.h>
@@ -45,6 +46,35 @@ constexpr int64_t CHUNK = 64, HEAD_DIM = 128;
 // packed-row and device / E problems, and TgdnError (_lib.py) when the library rejects a call.
 struct AssertFail : std::runtime_error { using std::runtime_error::runtime_error; };
 struct LibraryFail : std::runtime_error { using std::runtime_error::runtime_error; };
+
+py::handle library_error;                                  // TgdnError, set by _lib.py
+void set_python_error(const AssertFail& e) { PyErr_SetString(PyExc_AssertionError, e.what()); }
+void set_python_error(const LibraryFail& e) { PyErr_SetString(library_error ? library_error.ptr() : PyExc_RuntimeError, e.what()); }
+
+// Impl::forward and Impl::backward as an autograd function.  A backward runs under torch's engine, which keeps the class of a Python
+// error only: the two above are turned into one there (elsewhere the module's translator does it).
+template <typename Impl>
+struct Differentiable : public torch::autograd::Function<Differentiable<Impl>> {
+  template <typename... Args>
+  static auto forward(AutogradContext* ctx, Args&&... args) { return Impl::forward(ctx, std::forward<Args>(args)...); }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    try {
+      return Impl::backward(ctx, std::move(grads));
+    } catch (const AssertFail& e) {
+      rethrow(e);
+    } catch (const LibraryFail& e) {
+      rethrow(e);
+    }
+  }
+  template <typename Fail>
+  [[noreturn]] static void rethrow(const Fail& e) {
+    py::gil_scoped_acquire gil;
+    set_python_error(e);
+    python_error error;
+    error.persist();
+    throw error;
+  }
+};
 
 void check_rc(int rc, const char* what) {
   if (rc != 0) throw LibraryFail(std::string(what) + ": " + tgdn_error_string(rc) + " (code " + std::to_string(rc) + ")");
@@ -344,7 +374,7 @@ Tensor or_undefined(const OptTensor& t) { return has(t) ? *t : Tensor(); }
 OptTensor or_nullopt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
 
 // Differentiates joint_fwd (reference: ops/joint_torch_ops.py:50-80, ops/gdn_joint.py:201-232).
-struct JointFunction : public torch::autograd::Function<JointFunction> {
+struct JointSteps {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                                const Tensor& g, const Tensor& beta, double scale, const OptTensor& chunk_starts,
                                const OptTensor& token_map, bool covered) {
@@ -379,6 +409,7 @@ struct JointFunction : public torch::autograd::Function<JointFunction> {
     return res;
   }
 };
+using JointFunction = Differentiable<JointSteps>;
 
 std::vector<Tensor> joint_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                                        const Tensor& g, const Tensor& beta, double scale, const OptTensor& chunk_starts,
@@ -432,7 +463,7 @@ void check_state(const Tensor& s, at::IntArrayRef shape, const Tensor& q, const 
 // ---- segments and recomputation ---------------------------------------------------------------------------------------
 // The pipeline on ONE SEGMENT of longer sequences: the recurrent state comes in and goes out, and so does its gradient in the
 // backward (f32 (B, H, E, 128, 128) each).  Dense rows only.
-struct SegmentFunction : public torch::autograd::Function<SegmentFunction> {
+struct SegmentSteps {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                                const Tensor& g, const Tensor& beta, const OptTensor& state_in, double scale) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -463,6 +494,7 @@ struct SegmentFunction : public torch::autograd::Function<SegmentFunction> {
     return res;
   }
 };
+using SegmentFunction = Differentiable<SegmentSteps>;
 
 // Backward state recomputation: the forward keeps only the inputs and the f32 state at every segment boundary instead of the
 // per-chunk tensors; the backward walks the segments from the last to the first, runs each segment's forward again with
@@ -471,7 +503,7 @@ struct SegmentFunction : public torch::autograd::Function<SegmentFunction> {
 // The kernels read a segment in place (row_tokens: the batch stride of the whole rows) and write its part of o and of the
 // gradients in place; copying the segments out and the results back was a third of the step (1.0 of 3.0 ms at B=4, T=4096,
 // H=16, E=2 in four segments).
-struct CheckpointedFunction : public torch::autograd::Function<CheckpointedFunction> {
+struct CheckpointedSteps {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                         const Tensor& g, const Tensor& beta, double scale, int64_t seg) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -523,6 +555,7 @@ struct CheckpointedFunction : public torch::autograd::Function<CheckpointedFunct
     return res;
   }
 };
+using CheckpointedFunction = Differentiable<CheckpointedSteps>;
 
 // chunk_gdn_joint: training, recomputation, or inference with the state handed in and out.  Returns (o, final state or None).
 std::tuple<Tensor, OptTensor> chunk_joint(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
@@ -725,7 +758,7 @@ Five call_norm_fwd(const Tensor& x, const Tensor& weight, int64_t heads, int64_t
   return op.call(x, weight, heads, slices, eps, cu);
 }
 
-struct ConvFunction : public torch::autograd::Function<ConvFunction> {
+struct ConvSteps {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, int64_t act_channels, const OptTensor& cu) {
     at::AutoDispatchBelowADInplaceOrView below;
     Tensor y = call_conv_fwd(x, weight, act_channels, cu);
@@ -740,11 +773,12 @@ struct ConvFunction : public torch::autograd::Function<ConvFunction> {
     return {dx, dw, Tensor(), Tensor()};
   }
 };
+using ConvFunction = Differentiable<ConvSteps>;
 Tensor conv_fwd_autograd(const Tensor& x, const Tensor& weight, int64_t act_channels, const OptTensor& cu) {
   return ConvFunction::apply(x, weight, act_channels, cu);
 }
 
-struct NormFunction : public torch::autograd::Function<NormFunction> {
+struct NormSteps {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, int64_t heads, int64_t slices, double eps,
                                const OptTensor& cu) {
     at::AutoDispatchBelowADInplaceOrView below;
@@ -763,6 +797,7 @@ struct NormFunction : public torch::autograd::Function<NormFunction> {
     return {dx, dw, Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
+using NormFunction = Differentiable<NormSteps>;
 Five norm_fwd_autograd(const Tensor& x, const Tensor& weight, int64_t heads, int64_t slices, double eps, const OptTensor& cu) {
   variable_list o = NormFunction::apply(x, weight, heads, slices, eps, cu);
   return {o[0], o[1], o[2], o[3], o[4]};
@@ -804,14 +839,13 @@ TORCH_LIBRARY_IMPL(tgdn_b200, Autograd, m) {
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  static py::handle library_error;                        // TgdnError, set by _lib.py
   py::register_exception_translator([](std::exception_ptr p) {
     try {
       if (p) std::rethrow_exception(p);
     } catch (const AssertFail& e) {
-      PyErr_SetString(PyExc_AssertionError, e.what());
+      set_python_error(e);
     } catch (const LibraryFail& e) {
-      PyErr_SetString(library_error ? library_error.ptr() : PyExc_RuntimeError, e.what());
+      set_python_error(e);
     }
   });
   m.def("set_library_error", [](py::object cls) { library_error = cls.release(); });

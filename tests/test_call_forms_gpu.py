@@ -5,7 +5,8 @@ import threading
 import pytest
 import torch
 
-from cute_triadic_gdn_b200 import _lib, conv_split_act_call, conv_split_norm_call, gdn_joint_call
+from cute_triadic_gdn_b200 import (_lib, chunk_gdn_joint, chunk_gdn_joint_segment, conv_split_act_call, conv_split_norm_call,
+                                   gdn_joint_call)
 from oracle import triadic_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -104,3 +105,17 @@ def test_operator_with_a_chunk_map_that_misses_tokens(E):
     dv_part, = torch.autograd.grad(o_part, part[2], do[:, :130].contiguous())
     for whole, head in ((o, o_part), (dv, dv_part)):
         assert torch.equal(whole[:, :130], head) and bool((whole[:, 130:] == 0).all())
+
+
+@pytest.mark.parametrize("call", [gdn_joint_call, chunk_gdn_joint, lambda *a: chunk_gdn_joint(*a, checkpoint_tokens=64),
+                                  lambda *a: chunk_gdn_joint_segment(*a)[0]], ids=["call", "chunk", "checkpointed", "segment"])
+def test_error_of_the_library_in_a_backward(call):
+    """Its class is the same as in a forward: a gradient at an address that is no multiple of 16 bytes is refused."""
+    leaves = [t.cuda().requires_grad_(True) for t in orc.make_inputs(1, 128, 2, 2, seed=5)]
+    do = torch.empty(128 * 2 * 128 + 1, dtype=BF16, device="cuda")[1:].view(1, 128, 2, 128)
+    o = call(*leaves)
+    with pytest.raises(_lib.TgdnError, match="16-byte aligned"):
+        o.backward(do)
+    o = call(*leaves)                                        # and the next one is fine
+    o.backward(torch.ones_like(o))
+    assert _lib.device_status() == 0
