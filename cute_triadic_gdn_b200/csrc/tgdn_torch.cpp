@@ -373,6 +373,13 @@ std::vector<Tensor> joint_bwd_entry(at::TensorList saved, const Tensor& dO, doub
 Tensor or_undefined(const OptTensor& t) { return has(t) ? *t : Tensor(); }
 OptTensor or_nullopt(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
 
+bool any_grad(std::initializer_list<const Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : ts)
+    if (t->requires_grad()) return true;
+  return false;
+}
+
 // Differentiates joint_fwd (reference: ops/joint_torch_ops.py:50-80, ops/gdn_joint.py:201-232).
 struct JointSteps {
   static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
@@ -414,14 +421,13 @@ using JointFunction = Differentiable<JointSteps>;
 std::vector<Tensor> joint_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k2, const Tensor& q2,
                                        const Tensor& g, const Tensor& beta, double scale, const OptTensor& chunk_starts,
                                        const OptTensor& token_map, bool covered) {
+  // Nothing to differentiate: no autograd function, which would refuse inputs that carry a tangent (forward-mode differentiation),
+  // whatever the caller means to do with it.
+  if (!any_grad({&q, &k, &v, &k2, &q2, &g, &beta})) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return call_joint_fwd(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map, covered);
+  }
   return JointFunction::apply(q, k, v, k2, q2, g, beta, scale, chunk_starts, token_map, covered);
-}
-
-bool any_grad(std::initializer_list<const Tensor*> ts) {
-  if (!at::GradMode::is_enabled()) return false;
-  for (const Tensor* t : ts)
-    if (t->requires_grad()) return true;
-  return false;
 }
 
 double scale_or_default(std::optional<double> scale, const Tensor& q) {
@@ -775,6 +781,10 @@ struct ConvSteps {
 };
 using ConvFunction = Differentiable<ConvSteps>;
 Tensor conv_fwd_autograd(const Tensor& x, const Tensor& weight, int64_t act_channels, const OptTensor& cu) {
+  if (!any_grad({&x, &weight})) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return call_conv_fwd(x, weight, act_channels, cu);
+  }
   return ConvFunction::apply(x, weight, act_channels, cu);
 }
 
@@ -799,6 +809,10 @@ struct NormSteps {
 };
 using NormFunction = Differentiable<NormSteps>;
 Five norm_fwd_autograd(const Tensor& x, const Tensor& weight, int64_t heads, int64_t slices, double eps, const OptTensor& cu) {
+  if (!any_grad({&x, &weight})) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    return call_norm_fwd(x, weight, heads, slices, eps, cu);
+  }
   variable_list o = NormFunction::apply(x, weight, heads, slices, eps, cu);
   return {o[0], o[1], o[2], o[3], o[4]};
 }
