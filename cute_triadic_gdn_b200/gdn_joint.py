@@ -73,7 +73,7 @@ def chunk_gdn_joint_segment(q, k, v, k2, q2, g, beta, state_in=None, scale=None)
     and out of `state_out`, so that segments chained by their states (on one GPU or, with the states sent between
     ranks, on several: `context_parallel.py`) give the outputs and gradients of the unsplit sequences.  T must be a
     multiple of 64; dense rows only."""
-    return _lib.host.joint_segment(q, k, v, k2, q2, g, beta, state_in, scale)
+    return _lib.host.joint_segment(q, k, v, k2, q2, g, beta, state_in, None if scale is None else float(scale))
 
 
 def chunk_gdn_joint(q, k, v, k2, q2, g, beta, scale=None, cu_seqlens=None, reference=False, *, initial_state=None,
@@ -96,8 +96,8 @@ def chunk_gdn_joint(q, k, v, k2, q2, g, beta, scale=None, cu_seqlens=None, refer
     if reference:
         raise NotImplementedError("reference=True: this package has no torch fallback; the CPU oracle used by the "
                                   "tests is oracle/triadic_oracle.py")
-    o, final = _lib.host.chunk_joint(q, k, v, k2, q2, g, beta, scale, cu_seqlens, initial_state, bool(output_final_state),
-                                     checkpoint_tokens)
+    o, final = _lib.host.chunk_joint(q, k, v, k2, q2, g, beta, None if scale is None else float(scale), cu_seqlens, initial_state,
+                                     bool(output_final_state), None if checkpoint_tokens is None else int(checkpoint_tokens))
     return (o, final) if output_final_state else o
 
 
@@ -107,4 +107,4 @@ def gdn_joint_decode(q, k, v, k2, q2, g, beta, state, scale=None):
     q, k, v: bf16 (B, 1, H, 128) or (B, H, 128); k2, q2, g: f32 (B, 1, H, E) or (B, H, E); beta: f32 (B, 1, H) or (B, H);
     `state`: contiguous f32 (B, H, E, 128, 128), the form `chunk_gdn_joint(..., output_final_state=True)` returns; it is
     updated IN PLACE.  Returns o in the shape of v.  Forward only."""
-    return _lib.host.decode(q, k, v, k2, q2, g, beta, state, scale)
+    return _lib.host.decode(q, k, v, k2, q2, g, beta, state, None if scale is None else float(scale))

@@ -38,7 +38,7 @@ def gdn_joint_call(q, k, v, k2, q2, g, beta, scale=None, cu_seqlens=None):
     contiguous), like the reference's entry of the same name (ops/joint_torch_ops.py:83-95).  sm_100 only,
     E in {1, 2, 4, 8, 12, 16}, head dimension 128."""
     if not torch.compiler.is_compiling():              # the same steps natively
-        return _lib.host.joint_call(q, k, v, k2, q2, g, beta, scale, cu_seqlens)
+        return _lib.host.joint_call(q, k, v, k2, q2, g, beta, None if scale is None else float(scale), cu_seqlens)
     seven = [t.contiguous() for t in (q, k, v, k2, q2, g, beta)]
     if scale is None:
         scale = seven[0].shape[-1] ** -0.5

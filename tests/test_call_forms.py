@@ -1,9 +1,11 @@
 """Forms of a call that need no GPU: modes around the operators and types of arguments."""
+import numpy as np
 import pytest
 import torch
 import torch.autograd.forward_ad as forward_ad
 
-from cute_triadic_gdn_b200 import conv_split_act_call, conv_split_norm_call, gdn_joint_call
+from cute_triadic_gdn_b200 import (chunk_gdn_joint, chunk_gdn_joint_segment, conv_split_act_call, conv_split_norm_call, gdn_joint_call,
+                                   gdn_joint_decode)
 
 
 @pytest.fixture
@@ -52,3 +54,20 @@ def test_leaves_are_tracked_only_under_grad_mode(cpu_operators, name):
         assert not call(*leaves).requires_grad
     with torch.inference_mode():
         assert not call(*args).requires_grad
+
+
+@pytest.mark.parametrize("scale", [0.5, 1, "0.5", np.float32(0.5), torch.tensor(0.5)])
+@pytest.mark.parametrize("tokens", [64, 64.0, "64", np.int64(64), torch.tensor(64)])
+def test_whatever_converts_to_a_number_is_one(scale, tokens):
+    """Numbers may be of any type that float() and int() take: these calls come as far as the checks of the inputs (which want a GPU)."""
+    q = torch.ones(1, 64, 2, 128, dtype=torch.bfloat16)
+    k2 = torch.ones(1, 64, 2, 4)
+    args = (q, q, q, k2, k2, k2, k2[..., 0].contiguous())
+    with pytest.raises(AssertionError, match="CUDA device"):
+        chunk_gdn_joint(*args, scale=scale, checkpoint_tokens=tokens)
+    with pytest.raises(AssertionError, match="CUDA device"):
+        chunk_gdn_joint_segment(*args, scale=scale)
+    with pytest.raises(ValueError, match="CUDA device"):
+        gdn_joint_decode(*[t[:, :1] for t in args], torch.zeros(1, 2, 4, 128, 128), scale=scale)
+    with pytest.raises(NotImplementedError, match="CPU"):
+        gdn_joint_call(*args, scale=scale)
