@@ -616,6 +616,9 @@ Tensor decode(Tensor q, Tensor k, Tensor v, Tensor k2, Tensor q2, Tensor g, Tens
   const bool squeeze = q.dim() == 4;
   int64_t t = squeeze ? q.size(1) : 1;
   TORCH_CHECK_VALUE(t == 1, "gdn_joint_decode takes one token per sequence: T must be 1");
+  if (squeeze)                                            // the token axis of the others is dropped at its first token, however long it is
+    for (Tensor* x : {&k, &v, &k2, &q2, &g, &beta})
+      if (x->dim() > 1 && x->size(1) > 1) *x = x->narrow(1, 0, 1);
   // (B, 1, H, X) and (B, H, X) hold the same elements in the same order: shapes are compared with the token axis dropped
   auto sizes3 = [&](const Tensor& x, int64_t b, int64_t h, int64_t w) {
     return squeeze ? x.dim() == 4 && x.size(0) == b && x.size(1) == 1 && x.size(2) == h && x.size(3) == w

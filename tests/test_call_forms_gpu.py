@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from cute_triadic_gdn_b200 import (_lib, chunk_gdn_joint, chunk_gdn_joint_segment, conv_split_act_call, conv_split_norm_call,
-                                   gdn_joint_call)
+                                   gdn_joint_call, gdn_joint_decode)
 from oracle import triadic_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -118,4 +118,19 @@ def test_error_of_the_library_in_a_backward(call):
         o.backward(do)
     o = call(*leaves)                                        # and the next one is fine
     o.backward(torch.ones_like(o))
+    assert _lib.device_status() == 0
+
+
+def test_decode_takes_the_first_token_of_longer_operands():
+    ins = [t.cuda() for t in orc.make_inputs(2, 64, 3, 4, seed=8)]
+    first = [t[:, :1].contiguous() for t in ins]
+    state = torch.randn(2, 3, 4, 128, 128, device="cuda")
+    ref_state = state.clone()
+    ref = gdn_joint_decode(*first, ref_state)
+    for longer in range(1, 7):
+        s = state.clone()
+        assert torch.equal(gdn_joint_decode(*[ins[i][:, :5] if i == longer else t for i, t in enumerate(first)], s), ref)
+        assert torch.equal(s, ref_state)
+    with pytest.raises(ValueError, match="T must be 1"):
+        gdn_joint_decode(*[t[:, :2] for t in ins], state)
     assert _lib.device_status() == 0
