@@ -960,6 +960,7 @@ static int64_t partial_bytes(int B, int groups, int C) { return static_cast<int6
 
 // Scratch with which the backward runs best; tgdn_conv_bwd_scratch_bytes is the least.
 int64_t tgdn_conv_bwd_best_scratch(int B, int T, int C) {
+  if (B <= 0 || T <= 0 || C <= 0) return 0;                            // the entry points refuse these sizes
   return partial_bytes(B, std::max(scratch_groups(B, T, C), bwd_runs(B, T, (C + 127) / 128)), C);
 }
 

@@ -156,7 +156,7 @@ Dims dims(const Tensor& q, const Tensor& k2, const OptTensor& token_map, const O
   d.B = static_cast<int>(q.size(0)); d.T = static_cast<int>(q.size(1)); d.H = static_cast<int>(q.size(2));
   d.E = static_cast<int>(k2.size(3));
   d.NC = has(token_map) ? static_cast<int>(token_map->size(1)) : static_cast<int>(q.size(1) / CHUNK);
-  d.row_tokens = d.B > 1 ? static_cast<int>(q.stride(0) / (q.size(2) * HEAD_DIM)) : d.T;
+  d.row_tokens = d.B > 1 && d.H > 0 ? static_cast<int>(q.stride(0) / (q.size(2) * HEAD_DIM)) : d.T;
   d.n_docs = has(chunk_starts) ? static_cast<int>(chunk_starts->numel() - 1) : 0;
   return d;
 }

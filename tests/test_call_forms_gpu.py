@@ -134,3 +134,29 @@ def test_decode_takes_the_first_token_of_longer_operands():
     with pytest.raises(ValueError, match="T must be 1"):
         gdn_joint_decode(*[t[:, :2] for t in ins], state)
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("B,T,H", [(2, 64, 0), (0, 64, 2), (1, 64, 0)])
+def test_core_without_elements_is_refused(B, T, H):
+    """(A division by the number of heads on the host would end the process.)"""
+    q, k2 = torch.empty(B, T, H, 128, dtype=BF16, device="cuda"), torch.empty(B, T, H, 2, device="cuda")
+    ins = [q, q, q, k2, k2, k2, torch.empty(B, T, H, device="cuda")]
+    for call in (gdn_joint_call, chunk_gdn_joint, lambda *a: chunk_gdn_joint_segment(*a),
+                 lambda *a: chunk_gdn_joint(*[t.clone().requires_grad_(True) for t in a], checkpoint_tokens=64)):
+        with pytest.raises(_lib.TgdnError):
+            call(*ins)
+
+
+@pytest.mark.parametrize("B,T,C", [(0, 8, 16), (2, 0, 16), (2, 8, 0), (0, 8, 784), (1, 0, 784)])
+def test_convolution_without_elements_is_refused(B, T, C):
+    x, w = torch.empty(B, T, C, dtype=BF16, device="cuda"), torch.ones(C, 4, dtype=BF16, device="cuda")
+    with pytest.raises(_lib.TgdnError):
+        conv_split_act_call(x, w, 0)
+    with pytest.raises(_lib.TgdnError):
+        torch.ops.tgdn_b200.conv_split_act_bwd(x, x, w, 0, None)
+    if C == 784:
+        qkv, gates = torch.empty(B, T, 2, 128, dtype=BF16, device="cuda"), torch.empty(B, T, 2, 4, device="cuda")
+        with pytest.raises(_lib.TgdnError):
+            conv_split_norm_call(x, w, 2, 4)
+        with pytest.raises(_lib.TgdnError):
+            torch.ops.tgdn_b200.conv_split_norm_bwd(x, w, qkv, qkv, qkv, gates, gates, 2, 4, 1e-6, None)
