@@ -129,8 +129,10 @@ void check_device_and_e(const Tensor& q, int64_t E) {
 
 // GJ_SAVE_MASKS=1 (default) keeps the chunk operators of the forward for the backward; anything else drops them and lets the
 // backward form them again with the same kernel (bitwise identical).  Read at forward time, like the reference
-// (ops/gdn_joint.py:167-173).
+// (ops/gdn_joint.py:167-173), and under the interpreter's lock: os.environ of another thread writes the same table, and getenv is
+// not safe beside that.
 bool save_masks() {
+  py::gil_scoped_acquire gil;
   const char* s = std::getenv("GJ_SAVE_MASKS");
   return s == nullptr || std::strcmp(s, "1") == 0;
 }
