@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from cute_triadic_gdn_b200 import _lib, chunk_gdn_joint, conv_split_act_call, gdn_joint_call
+from cute_triadic_gdn_b200 import _lib, chunk_gdn_joint, chunk_gdn_joint_segment, conv_split_act_call, gdn_joint_call
 from oracle import triadic_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -11,8 +11,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("E", [1, 2, 4])
 @pytest.mark.parametrize("docs", [None, [0, 1, 64, 129, 200, 263, 384]])
 def test_wide_value_blocks_of_the_forward(E, docs):
-    """Enough sequences for more than one wave of narrow value blocks: the 64-column variant runs, dense and with chunks cut
-    short by document ends, with the state handed in and out."""
+    """Enough sequences for more than one wave of narrow value blocks: the 64-column variants run, dense and with chunks cut
+    short by document ends, the forward also with the state handed in and out."""
     B, T, H = (1, 384, 16) if docs else (6, 128, 16)
     ins = [t.cuda() for t in orc.make_inputs(B, T, H, E, seed=70 + E, dist="mild")]
     do = orc.make_grad_output((B, T, H, 128), 5)
@@ -34,7 +34,7 @@ def test_wide_value_blocks_of_the_forward(E, docs):
 
 
 @pytest.mark.parametrize("E", [1, 2, 4, 8, 12, 16])
-@pytest.mark.parametrize("H", [3, 4])                      # beta rows by loads, and as tiles of four heads
+@pytest.mark.parametrize("H", [3, 4, 16])                  # beta rows by loads, as tiles of four heads, wide blocks up to four slices
 def test_saved_and_unsaved_forward_and_ragged_chunks(E, H):
     """The forward with and without saved tensors (other splits of the block up to eight slices) agree bitwise; whole chunks leave the
     recurrences as tiles, chunks cut short by a document end row by row."""
@@ -42,16 +42,44 @@ def test_saved_and_unsaved_forward_and_ragged_chunks(E, H):
     ins = [t.cuda() for t in orc.make_inputs(1, 256, H, E, seed=90 + E, dist="mild")]
     do = orc.make_grad_output((1, 256, H, 128), 6)
     cu = torch.tensor(docs, dtype=torch.int32)
-    with torch.no_grad():
-        plain = gdn_joint_call(*ins, cu_seqlens=cu.cuda())
+    with torch.no_grad():                              # nothing is saved here; gdn_joint_call always saves
+        plain = chunk_gdn_joint(*ins, cu_seqlens=cu.cuda())
+        stated, _ = chunk_gdn_joint(*ins, cu_seqlens=cu.cuda(), output_final_state=True)
     leaves = [t.clone().requires_grad_(True) for t in ins]
     o = gdn_joint_call(*leaves, cu_seqlens=cu.cuda())
     o.backward(do.cuda())
-    assert _lib.device_status() == 0 and torch.equal(plain, o.detach())
+    assert _lib.device_status() == 0 and torch.equal(plain, o.detach()) and torch.equal(stated, plain)
     o_ref, g_ref = orc.reference_with_grads(orc.chunk_reference, [t.cpu() for t in ins], do, cu_seqlens=cu, dtype=torch.float32)
     assert orc.rel_l2(o.detach().float().cpu(), o_ref) < 1e-2
     for name, leaf, ref in zip("q k v k2 q2 g beta".split(), leaves, g_ref):
         assert orc.rel_l2(leaf.grad.float().cpu(), ref) < 2e-2, name
+
+
+@pytest.mark.parametrize("E", [1, 2, 4])
+def test_wide_value_blocks_with_states_handed_over(E):
+    """64 sequences and heads: recomputation in segments (read and written in place, the last one shorter) and segments chained by
+    hand, both with the state and its gradient handed from one to the next, are the plain call."""
+    B, T, H = 4, 320, 16
+    ins = [t.cuda() for t in orc.make_inputs(B, T, H, E, seed=110 + E, dist="mild")]
+    do = orc.make_grad_output((B, T, H, 128), 7).cuda()
+
+    def step(call):
+        leaves = [t.clone().requires_grad_(True) for t in ins]
+        o = call(*leaves)
+        return [o.detach(), *torch.autograd.grad(o, leaves, do)]
+
+    def chained(*leaves):
+        state, outs = None, []
+        for lo, hi in ((0, 64), (64, 256), (256, T)):
+            o, state = chunk_gdn_joint_segment(*[t[:, lo:hi].contiguous() for t in leaves], state_in=state)
+            outs.append(o)
+        return torch.cat(outs, 1)
+
+    ref = step(gdn_joint_call)
+    for call in (lambda *a: chunk_gdn_joint(*a, checkpoint_tokens=64), lambda *a: chunk_gdn_joint(*a, checkpoint_tokens=192), chained):
+        for name, a, b in zip("o q k v k2 q2 g beta".split(), step(call), ref):
+            assert torch.equal(a, b), name
+    assert _lib.device_status() == 0
 
 
 @pytest.mark.parametrize("B,T,C,act,docs", [
