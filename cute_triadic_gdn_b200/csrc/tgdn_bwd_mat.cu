@@ -163,8 +163,9 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   WaitCtl ctl{&sm.abort, p.status};
 
   // (batch row, chunk, head) of an item, the next one found by steps: the two divisions (32-bit: items fit, the entry point checks that)
-  // cost every warp several hundred cycles an item.  us: 4096 items E2 222 -> 210, E1 211 -> 206, packed E12 386 -> 374, E16 841 -> 834.
-  // At four slices the steps' registers spill where the divisions' do not (228 -> 234), so that one divides.
+  // cost every warp several hundred cycles an item.  us: 4096 items E2 222 -> 210, E1 211 -> 205, packed E12 386 -> 374, E16 841 -> 837.
+  // At four slices the steps' registers spill where the divisions' do not (20 bytes; 228 -> 234), so that one divides.  (Eight, twelve
+  // and sixteen slices spill 8, 16 and 164 bytes with steps, 0, 20 and 184 with divisions.)
   constexpr bool STEPS = E != 4;
   const int step = static_cast<int>(gridDim.x), step_h = step % p.H, step_n = step / p.H % p.NC, step_b = step / (p.H * p.NC);
   int h = blockIdx.x % p.H, n = blockIdx.x / p.H % p.NC, b = blockIdx.x / (p.H * p.NC);

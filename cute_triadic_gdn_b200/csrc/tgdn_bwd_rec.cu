@@ -171,6 +171,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   constexpr bool CROSS = C::CROSS;
   constexpr bool DV_TILE = NSG == 1;                // (at twelve and sixteen slices the tile costs what it saves)
   constexpr bool TWO_WIDE = TPC * CW < 1024;        // the two-wide multiply-adds of (a) need register pairs: sixteen columns of four slices spill
+                                                    // (and on packed rows they spill 36 bytes without)
   constexpr float LOG2E = 1.4426950408889634f;   // the decay threshold below is in the log2 domain
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

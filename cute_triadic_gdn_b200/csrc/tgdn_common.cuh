@@ -43,17 +43,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.b32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 
 // Non-blocking probe: unlike try_wait it never parks the warp, so a spinning waiter sees the flip within a few cycles.
 __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
@@ -130,16 +119,11 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, u
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_group_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-template <int N>       // all but the last N committed groups of this thread
-__device__ __forceinline__ void bulk_wait_group_read_but() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 // 1-D bulk copy shared -> global, in the thread's current bulk group; both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void bulk_wait_group() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
 // 1-D bulk copy global -> shared; both addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -273,14 +257,6 @@ __host__ __device__ constexpr uint32_t make_idesc(int M, int N, int a_major, int
          (static_cast<uint32_t>(M >> 4) << 24);
 }
 
-// Issue `ksteps` MMAs of K=16 each; operand descriptors advance by a_step / b_step bytes per step.
-__device__ __forceinline__ void umma_ksteps(uint32_t d_tmem, uint64_t adesc, uint32_t a_step, uint64_t bdesc,
-                                            uint32_t b_step, uint32_t idesc, int ksteps, bool accumulate) {
-  for (int k = 0; k < ksteps; ++k)
-    umma_bf16(d_tmem, desc_advance(adesc, k * a_step), desc_advance(bdesc, k * b_step), idesc,
-              (accumulate || k > 0) ? 1u : 0u);
-}
-
 // N floats from shared memory; 16-byte loads where N and the address allow, else 8-byte loads (N even) or one float
 template <int N>
 __device__ __forceinline__ void lds_part(const float* p, float* out) {
@@ -346,28 +322,6 @@ __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w 
 __device__ __forceinline__ float round_bf16(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void st_shared_v2(uint32_t saddr, uint32_t a, uint32_t b) {
-  asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(saddr), "r"(a), "r"(b) : "memory");
-}
-
-// Global loads that stay where they are written.  A plain read-only load may be sunk by the compiler to its first use,
-// which turns a prefetch issued one loop iteration ahead back into an exposed memory round trip; volatile asm keeps its
-// program order relative to the barrier and tensor-core instructions around it.
-__device__ __forceinline__ float ldg_pinned_f32(const float* p) {
-  float v;
-  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint2 ldg_pinned_v2(const void* p) {
-  uint2 v;
-  asm volatile("ld.global.nc.v2.b32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint4 ldg_pinned_v4(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
 }
 
 }  // namespace tgdn

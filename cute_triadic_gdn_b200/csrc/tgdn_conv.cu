@@ -860,6 +860,7 @@ __device__ __forceinline__ void reduce_dw(const float2 (&dw)[(V + 1) / 2][CONV_W
 }
 
 template <int V>
+// (Three CTAs per SM leave the walk of single channels 80 registers: it spills 412 bytes.)
 __global__ void __launch_bounds__(CONV_THREADS, V == 4 ? 2 : 3)
 conv_bwd_kernel(ConvArgs a) {
   __shared__ __align__(16) float red[CONV_WARPS * 32 * V * CONV_W];

@@ -196,7 +196,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
 #pragma unroll
     for (int j = 0; j < TPT; ++j) S[j] = 0.f;
   }
-  // a chain of eight columns never writes the second block of the (2) operand: keep it zero (its products land in unused columns)
+  // A chain of eight columns uses the first block of the (2) operand only.  The second starts as zeros and holds W on its way out; its
+  // products land in columns that nobody reads.
   for (int i = (tid & (CT - 1)); i < C::BW_BYTES / 16; i += CT) reinterpret_cast<uint4*>(bw_img)[i] = make_uint4(0, 0, 0, 0);
 
   // Sixteen of this thread's state columns -> h of a chunk, slice e as [v / 8][d][v % 8].  A warp's 16-byte stores cover 512

@@ -12,7 +12,8 @@
 //   * Python functions: what chunk_gdn_joint, gdn_joint_call, gdn_joint_decode and the convolution calls run when they are
 //     not being traced, and the single stages (run_masks, ...) that the tests and the benchmark time one by one.
 //
-// The device work is the C ABI of libtgdn_b200 (include/tgdn.h), with which this file is linked.
+// The device work is libtgdn_b200, with which this file is linked: the entry points of include/tgdn.h in the forms of tgdn_host.h (token
+// ranges of longer rows, rows of any alignment, the glue's backward in one pass).
 #include <torch/extension.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/library.h>
@@ -203,49 +204,6 @@ Forward run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Ten
   return f;
 }
 
-struct Reverse { Tensor dV, dU, ds, dkg, dr; };
-
-// Reverse recurrence.  ds is written only for slices whose chunk decay matters to dg.  Entries of a packed row's chunk map that
-// no document uses are neither written here nor read by the later stages.
-Reverse run_reverse(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& k2, const Tensor& q2, const Tensor& beta,
-                    const Tensor& gc, const Tensor& AP, const Tensor& Pm, const Tensor& U, double scale, const OptTensor& chunk_starts,
-                    const OptTensor& token_map, const OptTensor& grad_state_in, const OptTensor& grad_state_out) {
-  const c10::cuda::CUDAGuard guard(q.device());
-  const Dims d = dims(q, k2, token_map, chunk_starts);
-  const int64_t NV = d.blocks();
-  Reverse r;
-  r.dV = empty(dO.sizes(), dO, at::kBFloat16);
-  r.dU = empty({d.B, d.NC, d.H, CHUNK, 128}, q, at::kBFloat16);
-  r.ds = empty({d.B, d.NC, d.H, d.E, 16, 128, 8}, q, at::kBFloat16);
-  r.dkg = empty({d.B, d.NC, d.H, NV, 8, 128, 8}, q, at::kBFloat16);    // image [token / 8][key row][token % 8] per value block
-  r.dr = empty({d.B, d.NC, d.H, NV, CHUNK, d.E}, q, at::kFloat);
-  check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U),
-                                   static_cast<float>(scale), ptr<int32_t>(chunk_starts), ptr<int32_t>(token_map), d.n_docs, d.B, d.T, d.H,
-                                   d.E, d.NC, d.row_tokens, ptr(r.dV), ptr(r.dU), ptr(r.ds), ptr(r.dkg), ptr<float>(r.dr),
-                                   ptr<float>(grad_state_in), ptr<float>(grad_state_out), stream_of(q)),
-           "tgdn_bwd_recurrent");
-  return r;
-}
-
-struct StateGrads { Tensor dkq, da, dc, dd; };
-
-StateGrads run_state_grads(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dV, const Tensor& h, const Tensor& ds,
-                           const Tensor& dkg, const Tensor& k2, const Tensor& q2, const Tensor& gc, double scale,
-                           const OptTensor& token_map) {
-  const c10::cuda::CUDAGuard guard(q.device());
-  const Dims d = dims(q, k2, token_map);
-  StateGrads s;
-  s.dkq = empty({d.B, d.NC, d.H, 16, 128, 8}, q, at::kBFloat16);       // image [column / 8][row][column % 8]
-  s.da = empty({d.B, d.NC, d.H, CHUNK, d.E}, q, at::kFloat);
-  s.dc = empty({d.B, d.NC, d.H, CHUNK, d.E}, q, at::kFloat);
-  s.dd = empty({d.B, d.NC, d.H, d.E}, q, at::kFloat);
-  check_rc(tgdn_bwd_state_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(dV), ptr(h), ptr(ds), ptr(dkg), fptr(k2), fptr(q2), fptr(gc),
-                                     static_cast<float>(scale), ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC, d.row_tokens,
-                                     ptr(s.dkq), ptr<float>(s.da), ptr<float>(s.dc), ptr<float>(s.dd), stream_of(q)),
-           "tgdn_bwd_state_grads");
-  return s;
-}
-
 // Gradients of the seven inputs, in their order.
 struct Grads {
   Tensor q, k, v, k2, q2, g, beta;
@@ -261,17 +219,88 @@ struct Grads {
   }
 };
 
+// What travels between the three kernels of the backward.
+struct Between {
+  void *dU, *ds, *dkg, *dkq;
+  float *dr, *da, *dc, *dd;
+};
+
+// Reverse recurrence: dV, and dU, ds, dkg, dr of `x`.  ds is written only for slices whose chunk decay matters to dg.  Entries of a
+// packed row's chunk map that no document uses are neither written here nor read by the later stages.
+void launch_reverse(const Dims& d, const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& k2, const Tensor& q2,
+                    const Tensor& beta, const Tensor& gc, const Tensor& AP, const Tensor& Pm, const Tensor& U, double scale,
+                    const OptTensor& chunk_starts, const OptTensor& token_map, const OptTensor& grad_state_in,
+                    const OptTensor& grad_state_out, const Tensor& dV, const Between& x) {
+  check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U),
+                                   static_cast<float>(scale), ptr<int32_t>(chunk_starts), ptr<int32_t>(token_map), d.n_docs, d.B, d.T, d.H,
+                                   d.E, d.NC, d.row_tokens, ptr(dV), x.dU, x.ds, x.dkg, x.dr, ptr<float>(grad_state_in),
+                                   ptr<float>(grad_state_out), stream_of(q)),
+           "tgdn_bwd_recurrent");
+}
+
+// State gradients: dkq, da, dc, dd of `x`.
+void launch_state_grads(const Dims& d, const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dV, const Tensor& h,
+                        const Tensor& k2, const Tensor& q2, const Tensor& gc, double scale, const OptTensor& token_map, const Between& x) {
+  check_rc(tgdn_bwd_state_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(dV), ptr(h), x.ds, x.dkg, fptr(k2), fptr(q2), fptr(gc),
+                                     static_cast<float>(scale), ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC, d.row_tokens, x.dkq,
+                                     x.da, x.dc, x.dd, stream_of(q)),
+           "tgdn_bwd_state_grads");
+}
+
 // Matrix gradients, mask gradients and final assembly, into out's dq, dk, dk2, dq2, dg, dbeta.
+void launch_matrix(const Dims& d, const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& W, const Tensor& U, const Tensor& AP,
+                   const Tensor& k2, const Tensor& q2, const Tensor& beta, const Tensor& gc, double scale, const OptTensor& token_map,
+                   const Between& x, const Grads& out) {
+  check_rc(tgdn_bwd_matrix_rows(ptr(q), ptr(k), ptr(dO), x.dU, ptr(W), ptr(U), ptr(AP), fptr(k2), fptr(q2), fptr(beta), fptr(gc), x.dkq,
+                                x.da, x.dc, x.dd, x.dr, static_cast<float>(scale), ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC,
+                                d.row_tokens, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2), ptr<float>(out.g),
+                                ptr<float>(out.beta), stream_of(q)),
+           "tgdn_bwd_matrix");
+}
+
+// The stages one by one on tensors of their own, for the tests and the benchmark.
+struct Reverse { Tensor dV, dU, ds, dkg, dr; };
+
+Reverse run_reverse(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& k2, const Tensor& q2, const Tensor& beta,
+                    const Tensor& gc, const Tensor& AP, const Tensor& Pm, const Tensor& U, double scale, const OptTensor& chunk_starts,
+                    const OptTensor& token_map, const OptTensor& grad_state_in, const OptTensor& grad_state_out) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const Dims d = dims(q, k2, token_map, chunk_starts);
+  const int64_t NV = d.blocks();
+  Reverse r;
+  r.dV = empty(dO.sizes(), dO, at::kBFloat16);
+  r.dU = empty({d.B, d.NC, d.H, CHUNK, 128}, q, at::kBFloat16);
+  r.ds = empty({d.B, d.NC, d.H, d.E, 16, 128, 8}, q, at::kBFloat16);
+  r.dkg = empty({d.B, d.NC, d.H, NV, 8, 128, 8}, q, at::kBFloat16);    // image [token / 8][key row][token % 8] per value block
+  r.dr = empty({d.B, d.NC, d.H, NV, CHUNK, d.E}, q, at::kFloat);
+  launch_reverse(d, q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, chunk_starts, token_map, grad_state_in, grad_state_out, r.dV,
+                 Between{ptr(r.dU), ptr(r.ds), ptr(r.dkg), nullptr, ptr<float>(r.dr), nullptr, nullptr, nullptr});
+  return r;
+}
+
+struct StateGrads { Tensor dkq, da, dc, dd; };
+
+StateGrads run_state_grads(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dV, const Tensor& h, const Tensor& ds,
+                           const Tensor& dkg, const Tensor& k2, const Tensor& q2, const Tensor& gc, double scale,
+                           const OptTensor& token_map) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const Dims d = dims(q, k2, token_map);
+  StateGrads s;
+  s.dkq = empty({d.B, d.NC, d.H, 16, 128, 8}, q, at::kBFloat16);       // image [column / 8][row][column % 8]
+  s.da = empty({d.B, d.NC, d.H, CHUNK, d.E}, q, at::kFloat);
+  s.dc = empty({d.B, d.NC, d.H, CHUNK, d.E}, q, at::kFloat);
+  s.dd = empty({d.B, d.NC, d.H, d.E}, q, at::kFloat);
+  launch_state_grads(d, q, k, dO, dV, h, k2, q2, gc, scale, token_map,
+                     Between{nullptr, ptr(ds), ptr(dkg), ptr(s.dkq), nullptr, ptr<float>(s.da), ptr<float>(s.dc), ptr<float>(s.dd)});
+  return s;
+}
+
 void run_matrix(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dU, const Tensor& W, const Tensor& U, const Tensor& AP,
                 const Tensor& k2, const Tensor& q2, const Tensor& beta, const Tensor& gc, const StateGrads& s, const Tensor& dr,
                 double scale, const OptTensor& token_map, const Grads& out) {
   const c10::cuda::CUDAGuard guard(q.device());
-  const Dims d = dims(q, k2, token_map);
-  check_rc(tgdn_bwd_matrix_rows(ptr(q), ptr(k), ptr(dO), ptr(dU), ptr(W), ptr(U), ptr(AP), fptr(k2), fptr(q2), fptr(beta), fptr(gc),
-                                ptr(s.dkq), fptr(s.da), fptr(s.dc), fptr(s.dd), fptr(dr), static_cast<float>(scale),
-                                ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC, d.row_tokens,
-                                ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2), ptr<float>(out.g), ptr<float>(out.beta), stream_of(q)),
-           "tgdn_bwd_matrix");
+  launch_matrix(dims(q, k2, token_map), q, k, dO, W, U, AP, k2, q2, beta, gc, scale, token_map,
+                Between{ptr(dU), nullptr, nullptr, ptr(s.dkq), ptr<float>(dr), ptr<float>(s.da), ptr<float>(s.dc), ptr<float>(s.dd)}, out);
 }
 
 // reverse recurrence -> state gradients -> matrix gradients, into `out`.  AP, Pm undefined: GJ_SAVE_MASKS=0, the forward's own
@@ -285,32 +314,19 @@ void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tens
     AP = m.AP;
     Pm = m.Pm;
   }
-  // What travels between the three kernels, in two allocations (the first one, by far the larger, is given back before the last
-  // kernel's temporaries matter).
   const c10::cuda::CUDAGuard guard(q.device());
   const Dims d = dims(q, k2, token_map, chunk_starts);
   const int64_t items = static_cast<int64_t>(d.B) * d.NC * d.H, NV = d.blocks();
-  const float sc = static_cast<float>(scale);
-  const int32_t *starts = ptr<int32_t>(chunk_starts), *map = ptr<int32_t>(token_map);
-  void* stream = stream_of(q);
+  // in two allocations (the first one, by far the larger, is given back before the last kernel's temporaries matter)
   Tensor big = empty({items * (d.E * 32768 + NV * 16384)}, q, at::kByte);              // ds, dkg
   Tensor small = empty({items * (16384 + 32768 + (NV + 2) * 64 * d.E * 4 + d.E * 4)}, q, at::kByte);   // dU, dkq, dr, da, dc, dd
-  uint8_t *ds = ptr<uint8_t>(big), *dkg = ds + items * d.E * 32768;
-  uint8_t *dU = ptr<uint8_t>(small), *dkq = dU + items * 16384;
-  float *dr = reinterpret_cast<float*>(dkq + items * 32768), *da = dr + items * NV * 64 * d.E, *dc = da + items * 64 * d.E,
-        *dd = dc + items * 64 * d.E;
-  check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U), sc, starts, map,
-                                   d.n_docs, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, ptr(out.v), dU, ds, dkg, dr, ptr<float>(grad_state_in),
-                                   ptr<float>(grad_state_out), stream),
-           "tgdn_bwd_recurrent");
-  check_rc(tgdn_bwd_state_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(out.v), ptr(h), ds, dkg, fptr(k2), fptr(q2), fptr(gc), sc, map, d.B, d.T, d.H,
-                                     d.E, d.NC, d.row_tokens, dkq, da, dc, dd, stream),
-           "tgdn_bwd_state_grads");
+  uint8_t *ds = ptr<uint8_t>(big), *dU = ptr<uint8_t>(small), *dkq = dU + items * 16384;
+  float *dr = reinterpret_cast<float*>(dkq + items * 32768), *da = dr + items * NV * 64 * d.E, *dc = da + items * 64 * d.E;
+  const Between x{dU, ds, ds + items * d.E * 32768, dkq, dr, da, dc, dc + items * 64 * d.E};
+  launch_reverse(d, q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, chunk_starts, token_map, grad_state_in, grad_state_out, out.v, x);
+  launch_state_grads(d, q, k, dO, out.v, h, k2, q2, gc, scale, token_map, x);
   big.reset();
-  check_rc(tgdn_bwd_matrix_rows(ptr(q), ptr(k), ptr(dO), dU, ptr(W), ptr(U), ptr(AP), fptr(k2), fptr(q2), fptr(beta), fptr(gc), dkq, da, dc, dd, dr,
-                                sc, map, d.B, d.T, d.H, d.E, d.NC, d.row_tokens, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2),
-                                ptr<float>(out.g), ptr<float>(out.beta), stream),
-           "tgdn_bwd_matrix");
+  launch_matrix(d, q, k, dO, W, U, AP, k2, q2, beta, gc, scale, token_map, x, out);
 }
 
 // ---- operators of the core --------------------------------------------------------------------------------------------
