@@ -61,13 +61,13 @@ KERNEL_U = {
 # shares the eight value blocks of E = 16 where E = 8 has four: its rec and sg figures come out about 64 KB per item low).
 NCU_DRAM_BYTES_PER_ITEM = {
     # kernel: (bytes per item at E = 8, at E = 16); filled from profiles/core_kernels_prof_workload.md
-    "masks": (0.255e9 / 4096, 0.135e9 / 2048), "fwd": (1.518e9 / 4096, 1.282e9 / 2048), "rec": (0.751e9 / 4096, 0.549e9 / 2048),
-    "sg": (1.865e9 / 4096, 1.574e9 / 2048), "mat": (0.824e9 / 4096, 0.495e9 / 2048),
+    "masks": (0.251e9 / 4096, 0.133e9 / 2048), "fwd": (1.516e9 / 4096, 1.284e9 / 2048), "rec": (0.751e9 / 4096, 0.550e9 / 2048),
+    "sg": (1.875e9 / 4096, 1.574e9 / 2048), "mat": (0.827e9 / 4096, 0.495e9 / 2048),
 }
 
 # DRAM bytes (read + write) per element of the conv kernels, from one ncu capture at (1, 8192, 13056)
 # (part of the written lines still sat in L2 when the kernel ended).
-NCU_DRAM_BYTES_PER_ELEMENT_CONV = {"fwd": (215.9 + 162.0) * 1e6 / (8192 * 13056), "bwd": (431.6 + 184.2) * 1e6 / (8192 * 13056)}
+NCU_DRAM_BYTES_PER_ELEMENT_CONV = {"fwd": (214.1 + 167.8) * 1e6 / (8192 * 13056), "bwd": (457.7 + 198.5) * 1e6 / (8192 * 13056)}
 
 
 def ncu_traffic(name, E, items):
@@ -700,7 +700,7 @@ def run_glue_decode(args):
         gf, gb, fms, bms, _ = glue_rates(dev, T=T, reps=args.steps, unfused_too=False)
         line = {"metric": "conv_split_norm GB/s", "value": gf, "unit": "GB/s", "ms_per_step": fms,
                 "config": {"workload": f"conv_split_norm (1,{T},13056) H=32 E=12, {T // 4096} documents"},
-                "roofline": {"bound": "hbm", "kernel": "glue_main + glue_gate (forward)", "achieved": gf, "peak": pk["gbs"],
+                "roofline": {"bound": "hbm", "kernel": "ring_fwd + glue_gate (forward)", "achieved": gf, "peak": pk["gbs"],
                              "unit": "GB/s", "frac": gf / pk["gbs"], "traffic": None, "peak_kind": pk["kind"]},
                 "backward": {"ms": bms, "achieved": gb, "frac": gb / pk["gbs"]}}
     else:
