@@ -10,7 +10,7 @@
 // warp: eleven rows computed for eight in the backward, a CTA barrier per tile, and padded copies of every tensor where the
 // channel count was not a multiple of eight.  Measured at (1, 32768, 13056), of the HBM copy rate: backward 558 -> 424 us (70 ->
 // 92%), forward 302 -> 300 us (87%; two transcendental operations per element are the co-limit); at (3, 1000, 1930), padded
-// copies included, forward and backward 130 -> 32 us.
+// copies included, forward and backward 130 -> 27 us.
 // The weight gradient is accumulated in f32 per run and the runs' partials are summed in a fixed order by a second small kernel.
 #include <algorithm>
 #include <mutex>
