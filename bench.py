@@ -52,17 +52,17 @@ PACKED = {"c3": ("lognormal", 31), "c4": ("uniform", 4096)}   # workload -> how 
 
 # per-kernel algorithmic work, in u per (chunk, head)
 KERNEL_U = {
-    "masks": lambda E: 2, "fwd": lambda E: 2 + 6 * E, "rec": lambda E: 3 + 6 * E, "sg": lambda E: 6 * E, "mat": lambda E: 8,
+    "masks": lambda E: 2, "fwd": lambda E: 2 + 6 * E, "rec": lambda E: 3 + 6 * E, "grads": lambda E: 8 + 6 * E,
 }
 
 # DRAM bytes (read + write) per (chunk, head) item and launch, from ncu captures of each kernel at E = 8 (the `prof`
 # workload, 4096 items) and at E = 16 (B=2, T=4096, H=16: 2048 items).  Traffic grows in proportion to the item count and,
 # between the two captures, linearly in E (the saved states are E * 32 KB per item), so other E are interpolated (E = 12
-# shares the eight value blocks of E = 16 where E = 8 has four: its rec and sg figures come out about 64 KB per item low).
+# shares the eight value blocks of E = 16 where E = 8 has four: its rec and grads figures come out about 64 KB per item low).
 NCU_DRAM_BYTES_PER_ITEM = {
     # kernel: (bytes per item at E = 8, at E = 16); filled from profiles/core_kernels_prof_workload.md
     "masks": (0.251e9 / 4096, 0.133e9 / 2048), "fwd": (1.516e9 / 4096, 1.284e9 / 2048), "rec": (0.751e9 / 4096, 0.550e9 / 2048),
-    "sg": (1.875e9 / 4096, 1.574e9 / 2048), "mat": (0.827e9 / 4096, 0.495e9 / 2048),
+    "grads": (2.103e9 / 4096, 1.574e9 / 2048 + 100e3),
 }
 
 # DRAM bytes (read + write) per element of the conv kernels, from one ncu capture at (1, 8192, 13056)
@@ -77,7 +77,7 @@ def ncu_traffic(name, E, items):
 
 # HBM bytes per (chunk, head) item that each kernel of THIS decomposition must read or write once (bf16 tiles of 64x128
 # are 16 KB; a state slice is 32 KB; NV = value blocks of the reverse recurrence).  The saved forward states h (E * 32 KB
-# written by fwd, read by sg) and the value-block images of the reverse recurrence are consequences of the decomposition,
+# written by fwd, read by grads) and the value-block images of the reverse recurrence are consequences of the decomposition,
 # not of the algorithm: `io_bytes` below counts only what the algorithm itself must move.
 def kernel_bytes(name, E):
     K, NV, gates = 1024, (8 if E > 8 else 4), 3 * 64 * E * 4
@@ -87,8 +87,7 @@ def kernel_bytes(name, E):
         "masks": 32 * K + gates + 256 + packed + 24 * K,
         "fwd": 48 * K + 16 * K + factors + 256 + 48 * K + 32 * K * E,
         "rec": 64 * K + 16 * K + factors + 256 + 32 * K + NV * 16 * K + NV * 64 * E * 4,
-        "sg": 64 * K + 32 * K * E + NV * 16 * K + 2 * 64 * E * 4 + 4 * E + 32 * K + 2 * 64 * E * 4 + 4 * E,
-        "mat": 96 * K + 16 * K + 32 * K + gates + 256 + 2 * 64 * E * 4 + 4 * E + NV * 64 * E * 4 + 32 * K + gates + 256,
+        "grads": 64 * K + 48 * K + 8 * K + 32 * K * E + NV * 16 * K + NV * 64 * E * 4 + 2 * 64 * E * 4 + gates + 256 + 32 * K + gates + 256,
     }[name]
 
 
@@ -248,10 +247,10 @@ def stage_times(leaves, do, E, cu_dev=None, reps=3):
     if cu_dev is not None:
         from cute_triadic_gdn_b200.joint_packing import prepare_documents
         cs, tm = prepare_documents((q, k, v, k2, q2, g, beta), cu_dev)
-    names = ["masks", "fwd", "rec", "sg", "mat"]
+    names = ["masks", "fwd", "rec", "grads"]
     acc = {n: [] for n in names}
     for rep in range(reps + 1):                        # the first repetition warms the allocator and is dropped
-        ev = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
+        ev = [torch.cuda.Event(enable_timing=True) for _ in range(5)]
         ev[0].record()
         gc, AP, Pm = gj._run_masks(q, k, k2, q2, g, beta, scale, tm)
         ev[1].record()
@@ -259,15 +258,13 @@ def stage_times(leaves, do, E, cu_dev=None, reps=3):
         ev[2].record()
         dV, dU, ds, dkg, dr = gj._run_reverse(q, k, do, k2, q2, beta, gc, AP, Pm, U, scale, cs, tm)
         ev[3].record()
-        dkq, da, dc, dd = gj._run_state_grads(q, k, do, dV, h, ds, dkg, k2, q2, gc, scale, tm)
+        gj._run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, tm)
         ev[4].record()
-        gj._run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, scale, tm)
-        ev[5].record()
         torch.cuda.synchronize()
         if rep > 0:
             for i, n in enumerate(names):
                 acc[n].append(ev[i].elapsed_time(ev[i + 1]))
-        del h, ds, dkg, dkq, W, U, dU, o
+        del h, ds, dkg, W, U, dU, o
     return {n: sorted(acc[n])[len(acc[n]) // 2] for n in names}
 
 
@@ -635,7 +632,7 @@ def run_ours(args, rank, world, local_rank):
                     "ms_per_step": ms_e2e / args.steps,
                     "h2d_gbs": h2d / (ms_e2e / args.steps * 1e-3) / 1e9, "d2h_gbs": d2h / (ms_e2e / args.steps * 1e-3) / 1e9,
                     "host_numa": numa},
-            "gpu_launches": args.steps * (5 if backward else 2),
+            "gpu_launches": args.steps * (4 if backward else 2),
             "clocks": clocks, "roofline": roof, "parity": parity, "aux": aux, "device_status": status,
             "reference_kernels": refk,
             "cpu_baseline": {"value": cpu_rate, "unit": "tokens/s", "cores": threads, "kind": "port",

@@ -28,72 +28,16 @@
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
 #include "tgdn_kernels.h"
+#include "tgdn_mat.cuh"
 
 namespace tgdn {
 
 constexpr int MAT_THREADS = 512;
 
-__device__ __forceinline__ float mexp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // 64x64 f32 matrices with rows 68 floats apart: a lane per row writes 16-byte pieces, a lane per column reads floats, both without
 // bank conflicts.
 constexpr int MAT_LD = 68;
 __device__ __forceinline__ int midx(int i, int j) { return i * MAT_LD + j; }
-// Sums of sixteen values over the lanes of a warp by halving exchanges: lanes 2i and 2i + 1 end with the sum of value
-// (bit 4, 3, 2, 1 of the lane).
-__device__ __forceinline__ float warp_sums16(float (&v)[16], int lane) {
-#pragma unroll
-  for (int n = 8, keep = 16; n >= 1; n >>= 1, keep >>= 1) {
-    const bool up = (lane & keep) != 0;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const float send = up ? v[i] : v[i + n], mine = up ? v[i + n] : v[i];
-      v[i] = mine + __shfl_xor_sync(0xffffffffu, send, keep);
-    }
-  }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
-// A row of E gate values as pairs: sums over the slices run on the two-wide f32 instructions, half as many instructions for the
-// same products (each lane an ordinary f32 fma).
-template <int E> struct GateVec {
-  static constexpr int N = (E + 1) / 2;
-  float2 p[N];
-  __device__ __forceinline__ void set(int e, float v) { if (e & 1) p[e / 2].y = v; else p[e / 2].x = v; }
-  __device__ __forceinline__ float get(int e) const { return (e & 1) ? p[e / 2].y : p[e / 2].x; }
-  __device__ __forceinline__ void clear() {
-#pragma unroll
-    for (int i = 0; i < N; ++i) p[i] = make_float2(0.f, 0.f);
-  }
-  __device__ __forceinline__ float dot(const GateVec& o) const {
-    float2 a = __fmul2_rn(p[0], o.p[0]);
-#pragma unroll
-    for (int i = 1; i < N; ++i) a = __ffma2_rn(p[i], o.p[i], a);
-    return E == 1 ? a.x : a.x + a.y;
-  }
-  __device__ __forceinline__ void add_scaled(float f, const GateVec& o) {
-    const float2 ff = make_float2(f, f);
-#pragma unroll
-    for (int i = 0; i < N; ++i) p[i] = __ffma2_rn(ff, o.p[i], p[i]);
-  }
-  __device__ __forceinline__ void load(const float* row) {       // a dense table row (the same row for the whole warp)
-    if constexpr (E % 4 == 0) {
-#pragma unroll
-      for (int i = 0; i < N; i += 2) {
-        const float4 x = *reinterpret_cast<const float4*>(row + 2 * i);
-        p[i] = make_float2(x.x, x.y);
-        p[i + 1] = make_float2(x.z, x.w);
-      }
-    } else if constexpr (E == 2) {
-      p[0] = *reinterpret_cast<const float2*>(row);
-    } else {
-      p[0] = make_float2(row[0], 0.f);
-    }
-  }
-};
 
 template <int E>
 struct MatSmem {
@@ -707,18 +651,15 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       const int rr = idx / E, e = idx % E, o = rr * ES + e;
       const float c2e = ((sm.part[0][0][o] + sm.part[1][0][o]) + (sm.part[0][1][o] + sm.part[1][1][o])) +
                         ((sm.part[0][2][o] + sm.part[1][2][o]) + (sm.part[0][3][o] + sm.part[1][3][o]));
-      const float gcv = sm.gc2[o], gl = sm.gc2[63 * ES + e];
-      const float eg = mexp2(gcv), egr = mexp2(gl - gcv);
-      const float k2v = sm.k2[o], q2v = sm.q2[o];
-      const float dav = da_in[it], dcv = dc_in[it];
-      const float drv = sm.drr[o], r1e = sm.r1[o], c1e = sm.c1[o], r2e = sm.r2[o];
+      const GateGrads gg = gate_gradients(sm.gc2[o], sm.gc2[63 * ES + e], sm.k2[o], sm.q2[o], p.scale, da_in[it], dc_in[it], sm.drr[o], sm.r1[o],
+                                          sm.c1[o], sm.r2[o], c2e);
       if (rr < rows) {
         const int64_t off = ((tok + rr) * p.H + h) * E + e;
-        p.dk2[off] = dav * eg + drv * egr + c1e + r2e + c2e;
-        p.dq2[off] = dcv * p.scale * eg + r1e;
+        p.dk2[off] = gg.dk2;
+        p.dq2[off] = gg.dq2;
       }
-      sm.dgc[o] = dav * (k2v * eg) + dcv * (p.scale * q2v * eg) - drv * (k2v * egr) + q2v * r1e + k2v * (r2e - c1e - c2e);
-      sm.drr[o] = drv * (k2v * egr);                        // dr*r, summed over the rows below
+      sm.dgc[o] = gg.dgc;
+      sm.drr[o] = gg.drr;                                   // dr*r, summed over the rows below
     }
   }
   if (tid < 64 && tid < rows) p.dbeta[(tok + tid) * p.H + h] = (sm.bcolp[0][tid] + sm.bcolp[1][tid]) + sm.brow[tid];
@@ -727,17 +668,8 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   // chunk-end terms sum_t dr*r + dd*exp(gL)
   static_assert(E <= MAT_THREADS / 32, "one warp per gate column");
   for (int e = warp; e < E; e += MAT_THREADS / 32) {
-    float tot = sm.drr[lane * ES + e] + sm.drr[(lane + 32) * ES + e];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     float v1 = sm.dgc[(63 - lane) * ES + e], v0 = sm.dgc[(31 - lane) * ES + e];      // lane l: rows 63-l and 31-l
-    if (lane == 0) v1 += tot + dd_in * mexp2(sm.gc2[63 * ES + e]);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float a1 = __shfl_up_sync(0xffffffffu, v1, o), a0 = __shfl_up_sync(0xffffffffu, v0, o);
-      if (lane >= o) { v1 += a1; v0 += a0; }
-    }
-    v0 += __shfl_sync(0xffffffffu, v1, 31);
+    reverse_scan(v1, v0, sm.drr[lane * ES + e] + sm.drr[(lane + 32) * ES + e], dd_in, mexp2(sm.gc2[63 * ES + e]), lane);
     const int ra = 63 - lane, rb = 31 - lane;
     sm.dgc[ra * ES + e] = v1;                              // leaves by rows, below: a column would write four bytes of every sector
     sm.dgc[rb * ES + e] = v0;

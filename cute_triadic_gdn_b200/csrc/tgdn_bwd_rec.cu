@@ -192,6 +192,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   const int t = row & 63;
 
   const int vb = blockIdx.x % NV, h = (blockIdx.x / NV) % p.H, seq_rank = blockIdx.x / (NV * p.H);
+  if (blockIdx.x == 0 && tid == 0 && p.zeroed != nullptr) *p.zeroed = 0;   // (before any early return)
   int b = seq_rank, first = 0, count = p.NC, seq = seq_rank;
   if constexpr (PACKED) {
     const int doc = p.cmap[2 * p.NC + seq_rank];
@@ -822,7 +823,7 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
                             const float* gc, const void* AP, const void* Pm, const void* U, float scale, const int32_t* doc_offsets,
                             const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, void* dV,
                             void* dU, void* ds, void* dkg, float* dr, const float* grad_state_in, float* grad_state_out,
-                            void* stream) {
+                            void* stream, int* zeroed) {
   if ((reinterpret_cast<uintptr_t>(grad_state_in) | reinterpret_cast<uintptr_t>(grad_state_out)) & 15) return TGDN_ERR_ALIGN;
   if (!q || !k || !dO || !k2 || !q2 || !beta || !gc || !AP || !Pm || !U || !dV || !dU || !ds || !dkg || !dr) return TGDN_ERR_NULL;
   const bool packed = chunk_map != nullptr;
@@ -854,7 +855,7 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
               static_cast<const __nv_bfloat16*>(Pm), static_cast<const __nv_bfloat16*>(U),
               static_cast<__nv_bfloat16*>(dV), static_cast<__nv_bfloat16*>(dU), static_cast<__nv_bfloat16*>(ds),
               static_cast<__nv_bfloat16*>(dkg), dr, doc_offsets, chunk_map, B, T, H, NC, packed ? n_docs : B, row_tokens, scale,
-              tgdn_status_word(), grad_state_in, grad_state_out, beta_tma};
+              tgdn_status_word(), grad_state_in, grad_state_out, beta_tma, zeroed};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (E) {
     case 1:

@@ -86,6 +86,35 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     }
   }
 }
+// The same wait for a warp that has long to wait beside others that work: the probe parks the warp for at most PARK_NS.  A poll is an
+// access to shared memory, and where that path is the bottleneck a dozen polling warps take a third of it.
+constexpr uint32_t PARK_NS = 200;
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      "selp.b32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(PARK_NS)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long start = clock64();
+  for (uint32_t it = 1;; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((it & 63u) == 0u) {
+      if (*ctl.abort) return false;
+      if (clock64() - start > WAIT_LIMIT_CYCLES) {
+        *ctl.abort = 1;
+        atomicCAS(ctl.status, DEV_OK, code);
+        return false;
+      }
+    }
+  }
+}
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
   return mbar_wait(bar, parity, ctl, code);
 }

@@ -55,7 +55,7 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
                             const float* gc, const void* AP, const void* Pm, const void* U, float scale, const int32_t* doc_offsets,
                             const int32_t* chunk_map, int n_docs, int B, int T, int H, int E, int NC, int row_tokens, void* dV,
                             void* dU, void* ds, void* dkg, float* dr, const float* grad_state_in, float* grad_state_out,
-                            void* stream);
+                            void* stream, int* zeroed = nullptr);   // zeroed: a word that the kernel sets to zero, or nullptr
 int tgdn_bwd_state_grads_rows(const void* q, const void* k, const void* dO, const void* dV, const void* h, const void* ds,
                               const void* dkg, const float* k2, const float* q2, const float* gc, float scale,
                               const int32_t* chunk_map, int B, int T, int H, int E, int NC, int row_tokens, void* dkq, float* da,
@@ -65,6 +65,12 @@ int tgdn_bwd_matrix_rows(const void* q, const void* k, const void* dO, const voi
                          const float* dc, const float* dd, const float* dr, float scale, const int32_t* chunk_map, int B, int T,
                          int H, int E, int NC, int row_tokens, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta,
                          void* stream);
+// The state gradients and the matrix gradients in one kernel, bitwise the two above one after the other.  next_item: a word of the call's own
+// that is zero when the kernel starts (tgdn_bwd_recurrent_rows can zero it).
+int tgdn_bwd_grads_rows(const void* q, const void* k, const void* dO, const void* dV, const void* dU, const void* W, const void* U,
+                        const void* AP, const void* h, const void* ds, const void* dkg, const float* k2, const float* q2,
+                        const float* beta, const float* gc, const float* dr, float scale, const int32_t* chunk_map, int B, int T, int H,
+                        int E, int NC, int row_tokens, int* next_item, void* dq, void* dk, float* dk2, float* dq2, float* dg, float* dbeta, void* stream);
 
 // The convolution for any channel count, strides and 2-byte aligned rows (weight: 8-byte aligned); the entry points of the public ABI
 // are these for whole 16-byte pieces.  The backward uses as many weight-gradient partials as the scratch holds, up to

@@ -89,6 +89,7 @@ struct RecParams {
   const float* g_in;        // f32 [sequence][H][E][128 d][128 v]: dL/dS after the last token (a later segment's hand-off), or nullptr (zero)
   float* g_out;             // same form: dL/dS before the first token, or nullptr
   int beta_tma;             // beta rows of a chunk arrive by TMA (H a multiple of 4, base 16-byte aligned), else by global loads
+  int* zeroed;              // set to zero for the kernel that follows, or nullptr
 };
 
 struct SgParams {
@@ -135,6 +136,29 @@ struct MatParams {
   float scale;
   int* status;
   int ahead;                // CTAs to launch (the SM count): the kernel is persistent, CTA c takes items c, c + ahead, ...
+};
+
+struct GradsParams {
+  const __nv_bfloat16* AP;
+  const __nv_bfloat16* h;
+  const __nv_bfloat16* ds;  // read only for slices above DD_MIN_LOG2_DECAY
+  const __nv_bfloat16* dkg; // [item][NV][16 KB image] from the reverse recurrence
+  const float* k2;
+  const float* q2;
+  const float* beta;
+  const float* gc;
+  const float* dr;          // [item][NV][64][E]
+  int* next_item;           // items drawn so far beyond the first of every CTA
+  __nv_bfloat16* dq;        // token layout (out)
+  __nv_bfloat16* dk;
+  float* dk2;               // token layout (out)
+  float* dq2;
+  float* dg;
+  float* dbeta;
+  const int32_t* cmap;
+  int B, T, H, NC, NV, TS;
+  float scale;
+  int* status;
 };
 
 }  // namespace tgdn

@@ -223,6 +223,7 @@ struct Grads {
 struct Between {
   void *dU, *ds, *dkg, *dkq;
   float *dr, *da, *dc, *dd;
+  int* next_item = nullptr;
 };
 
 // Reverse recurrence: dV, and dU, ds, dkg, dr of `x`.  ds is written only for slices whose chunk decay matters to dg.  Entries of a
@@ -234,7 +235,7 @@ void launch_reverse(const Dims& d, const Tensor& q, const Tensor& k, const Tenso
   check_rc(tgdn_bwd_recurrent_rows(ptr(q), ptr(k), ptr(dO), fptr(k2), fptr(q2), fptr(beta), fptr(gc), ptr(AP), ptr(Pm), ptr(U),
                                    static_cast<float>(scale), ptr<int32_t>(chunk_starts), ptr<int32_t>(token_map), d.n_docs, d.B, d.T, d.H,
                                    d.E, d.NC, d.row_tokens, ptr(dV), x.dU, x.ds, x.dkg, x.dr, ptr<float>(grad_state_in),
-                                   ptr<float>(grad_state_out), stream_of(q)),
+                                   ptr<float>(grad_state_out), stream_of(q), x.next_item),
            "tgdn_bwd_recurrent");
 }
 
@@ -256,6 +257,17 @@ void launch_matrix(const Dims& d, const Tensor& q, const Tensor& k, const Tensor
                                 d.row_tokens, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2), ptr<float>(out.g),
                                 ptr<float>(out.beta), stream_of(q)),
            "tgdn_bwd_matrix");
+}
+
+// State gradients and matrix gradients in one kernel: all gradients but dV, into `out` (out.v: the dV of the reverse recurrence).
+void launch_grads(const Dims& d, const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& h, const Tensor& W, const Tensor& U,
+                  const Tensor& AP, const Tensor& k2, const Tensor& q2, const Tensor& beta, const Tensor& gc, double scale,
+                  const OptTensor& token_map, const Between& x, const Grads& out) {
+  check_rc(tgdn_bwd_grads_rows(ptr(q), ptr(k), ptr(dO), ptr(out.v), x.dU, ptr(W), ptr(U), ptr(AP), ptr(h), x.ds, x.dkg, fptr(k2), fptr(q2),
+                               fptr(beta), fptr(gc), x.dr, static_cast<float>(scale), ptr<int32_t>(token_map), d.B, d.T, d.H, d.E, d.NC,
+                               d.row_tokens, x.next_item, ptr(out.q), ptr(out.k), ptr<float>(out.k2), ptr<float>(out.q2),
+                               ptr<float>(out.g), ptr<float>(out.beta), stream_of(q)),
+           "tgdn_bwd_grads");
 }
 
 // The stages one by one on tensors of their own, for the tests and the benchmark.
@@ -303,7 +315,16 @@ void run_matrix(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor
                 Between{ptr(dU), nullptr, nullptr, ptr(s.dkq), ptr<float>(dr), ptr<float>(s.da), ptr<float>(s.dc), ptr<float>(s.dd)}, out);
 }
 
-// reverse recurrence -> state gradients -> matrix gradients, into `out`.  AP, Pm undefined: GJ_SAVE_MASKS=0, the forward's own
+void run_grads(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dU, const Tensor& ds, const Tensor& dkg, const Tensor& dr,
+               const Tensor& h, const Tensor& W, const Tensor& U, const Tensor& AP, const Tensor& k2, const Tensor& q2, const Tensor& beta,
+               const Tensor& gc, double scale, const OptTensor& token_map, const Grads& out) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  Tensor next_item = at::zeros({1}, q.options().dtype(at::kInt));
+  launch_grads(dims(q, k2, token_map), q, k, dO, h, W, U, AP, k2, q2, beta, gc, scale, token_map,
+               Between{ptr(dU), ptr(ds), ptr(dkg), nullptr, ptr<float>(dr), nullptr, nullptr, nullptr, ptr<int>(next_item)}, out);
+}
+
+// reverse recurrence -> state and matrix gradients, into `out`.  AP, Pm undefined: GJ_SAVE_MASKS=0, the forward's own
 // kernel forms them again.
 void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tensor& q2, const Tensor& g, const Tensor& beta,
                   const Tensor& gc, Tensor AP, Tensor Pm, const Tensor& h, const Tensor& W, const Tensor& U, const Tensor& dO, double scale,
@@ -317,16 +338,12 @@ void run_backward(const Tensor& q, const Tensor& k, const Tensor& k2, const Tens
   const c10::cuda::CUDAGuard guard(q.device());
   const Dims d = dims(q, k2, token_map, chunk_starts);
   const int64_t items = static_cast<int64_t>(d.B) * d.NC * d.H, NV = d.blocks();
-  // in two allocations (the first one, by far the larger, is given back before the last kernel's temporaries matter)
-  Tensor big = empty({items * (d.E * 32768 + NV * 16384)}, q, at::kByte);              // ds, dkg
-  Tensor small = empty({items * (16384 + 32768 + (NV + 2) * 64 * d.E * 4 + d.E * 4)}, q, at::kByte);   // dU, dkq, dr, da, dc, dd
-  uint8_t *ds = ptr<uint8_t>(big), *dU = ptr<uint8_t>(small), *dkq = dU + items * 16384;
-  float *dr = reinterpret_cast<float*>(dkq + items * 32768), *da = dr + items * NV * 64 * d.E, *dc = da + items * 64 * d.E;
-  const Between x{dU, ds, ds + items * d.E * 32768, dkq, dr, da, dc, dc + items * 64 * d.E};
+  Tensor between = empty({items * (d.E * 32768 + NV * 16384 + 16384 + NV * 64 * d.E * 4) + 16}, q, at::kByte);   // ds, dkg, dU, dr, the item counter
+  uint8_t *ds = ptr<uint8_t>(between), *dkg = ds + items * d.E * 32768, *dU = dkg + items * NV * 16384;
+  uint8_t *dr = dU + items * 16384, *counter = dr + items * NV * 64 * d.E * 4;
+  const Between x{dU, ds, dkg, nullptr, reinterpret_cast<float*>(dr), nullptr, nullptr, nullptr, reinterpret_cast<int*>(counter)};
   launch_reverse(d, q, k, dO, k2, q2, beta, gc, AP, Pm, U, scale, chunk_starts, token_map, grad_state_in, grad_state_out, out.v, x);
-  launch_state_grads(d, q, k, dO, out.v, h, k2, q2, gc, scale, token_map, x);
-  big.reset();
-  launch_matrix(d, q, k, dO, W, U, AP, k2, q2, beta, gc, scale, token_map, x, out);
+  launch_grads(d, q, k, dO, h, W, U, AP, k2, q2, beta, gc, scale, token_map, x, out);
 }
 
 // ---- operators of the core --------------------------------------------------------------------------------------------
@@ -921,6 +938,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                          const Tensor& da, const Tensor& dc, const Tensor& dd, const Tensor& dr, double scale, const OptTensor& token_map) {
     Grads out = Grads::like(q, k2, beta);
     run_matrix(q, k, dO, dU, W, U, AP, k2, q2, beta, gc, StateGrads{dkq, da, dc, dd}, dr, scale, token_map, out);
+    return std::make_tuple(out.q, out.k, out.k2, out.q2, out.g, out.beta);
+  }, nogil);
+  m.def("run_grads", [](const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dV, const Tensor& dU, const Tensor& ds,
+                        const Tensor& dkg, const Tensor& dr, const Tensor& h, const Tensor& W, const Tensor& U, const Tensor& AP,
+                        const Tensor& k2, const Tensor& q2, const Tensor& beta, const Tensor& gc, double scale, const OptTensor& token_map) {
+    Grads out = Grads::like(q, k2, beta);
+    out.v = dV;
+    run_grads(q, k, dO, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, token_map, out);
     return std::make_tuple(out.q, out.k, out.k2, out.q2, out.g, out.beta);
   }, nogil);
 }

@@ -67,6 +67,12 @@ def _run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, s
     return _lib.host.run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, float(scale), token_map)
 
 
+def _run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, token_map=None):
+    """State and matrix gradients in one kernel, as the backward runs them: (dq, dk, dk2, dq2, dg, dbeta), bitwise those of the two
+    stages above."""
+    return _lib.host.run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, float(scale), token_map)
+
+
 def chunk_gdn_joint_segment(q, k, v, k2, q2, g, beta, state_in=None, scale=None):
     """One segment of longer sequences, differentiable through the state: returns (o, state_out).  `state_in` (None:
     zero) and `state_out` are f32 (B, H, E, 128, 128), S_e as [key row][value column]; gradients flow into `state_in`

@@ -1,0 +1,55 @@
+"""The fused gradient kernel against the two stages it joins (state gradients, then matrix gradients), bit by bit, where its roles have to
+agree on the course of an item: which slices take a trace (none, all, the first, the last, every other), chunks cut short by a document
+end, unused entries of the chunk map, fewer and more items than SMs, and the direct decay path (steep gates, gates above zero)."""
+import pytest
+import torch
+
+from cute_triadic_gdn_b200 import _lib
+from cute_triadic_gdn_b200 import gdn_joint as gj
+from cute_triadic_gdn_b200.joint_packing import prepare_documents
+from oracle import triadic_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+TRACES = {"none": lambda e, E: False, "all": lambda e, E: True, "first": lambda e, E: e == 0, "last": lambda e, E: e == E - 1,
+          "other": lambda e, E: e % 2 == 1}
+
+
+def both(ins, do, docs=None):
+    q, k, v, k2, q2, g, beta = [t.cuda() for t in ins]
+    do, E, scale = do.cuda(), k2.shape[-1], 128 ** -0.5
+    cs = tm = None
+    if docs is not None:
+        cs, tm = prepare_documents((q, k, v, k2, q2, g, beta), torch.tensor(docs, dtype=torch.int32).cuda())
+    gc, AP, Pm = gj._run_masks(q, k, k2, q2, g, beta, scale, tm)
+    _, h, W, U = gj._run_forward(q, k, v, k2, q2, beta, gc, AP, scale, True, cs, tm)
+    dV, dU, ds, dkg, dr = gj._run_reverse(q, k, do, k2, q2, beta, gc, AP, Pm, U, scale, cs, tm)
+    one = gj._run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, tm)
+    dkq, da, dc, dd = gj._run_state_grads(q, k, do, dV, h, ds, dkg, k2, q2, gc, scale, tm)
+    two = gj._run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, scale, tm)
+    assert _lib.device_status() == 0
+    for name, a, b in zip("dq dk dk2 dq2 dg dbeta".split(), one, two):
+        assert torch.isfinite(a.float()).all() and torch.equal(a, b), name
+
+
+@pytest.mark.parametrize("E", [1, 2, 4, 8, 12, 16])
+@pytest.mark.parametrize("traces", list(TRACES))
+@pytest.mark.parametrize("B,T,H,docs", [(2, 64, 1, None), (2, 640, 16, None), (1, 777, 5, [0, 1, 64, 129, 200, 777])])
+def test_one_kernel_is_the_two_stages(E, traces, B, T, H, docs):
+    ins = list(orc.make_inputs(B, T, H, E, seed=40 + E, dist="mild"))
+    taken = torch.tensor([TRACES[traces](e, E) for e in range(E)])
+    ins[5] = torch.where(taken, 0.02, 1.0) * ins[5].abs().neg().clamp(-1.0, -0.4)       # chunk decays above / below 2^-24, none steep
+    both(ins, orc.make_grad_output((B, T, H, 128), 9), docs)
+
+
+@pytest.mark.parametrize("E", [1, 2, 4, 8, 12, 16])
+@pytest.mark.parametrize("kind", ["steep", "rising"])
+def test_direct_decay_path(E, kind):
+    B, T, H = 1, 192, 3
+    ins = list(orc.make_inputs(B, T, H, E, seed=50 + E, dist="mild"))
+    gen = torch.Generator().manual_seed(E)
+    if kind == "steep":
+        ins[5] = torch.where(torch.rand(B, T, H, E, generator=gen) < 0.1, torch.full_like(ins[5], -90.0), ins[5])
+    else:
+        ins[5] = 0.02 * torch.randn(B, T, H, E, generator=gen)
+    both(ins, orc.make_grad_output((B, T, H, 128), 10), None)
