@@ -42,6 +42,9 @@
 // One value block per chain in the 64-column CTA, with sums of its own, instead of one block of 64 columns (whose results depended on
 // the width that the call picked): E4 254 -> 256, E2 193 -> 206, E1 172 -> 188, and the state-gradient kernel adds four images again
 // instead of two (217 -> 247, 164 -> 182, 137 -> 154); four slices on narrow blocks (2048 items), the chains' P in turn: 188 -> 193.
+// Who waits for a product parks (the other chain's epilogue wants the shared-memory path that polls would take); the loads of a chunk are
+// polled, being there already as a rule: us, all waits polled -> E8 1014 -> 987, E12 968 -> 929, E16 1208 -> 1176 (4096 items each),
+// E4 256 -> 247; with the loads parked too E12 977.  (One polling warp and a named barrier for the rest: E8 1133.)
 #include "tgdn_common.cuh"
 #include "tgdn_host.h"
 #include "tgdn_kernels.h"
@@ -430,8 +433,8 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     if (warp_u == ISSUE_WARP) {
       // (p) P = G Xu^T goes out as soon as the key-row warps have built Xu (they do that first thing in this phase): it runs
       // behind (a), under the epilogue of (a), and nobody waits for it later.  (The previous chunk's P must have been read.)
-      mbar_wait(&ctrl.bar_xu[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
-      if (CROSS && kstep > 0) mbar_wait(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);
+      mbar_wait_parked(&ctrl.bar_xu[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
+      if (CROSS && kstep > 0) mbar_wait_parked(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);
       const bool add = C::IN_TURN && chain == 1;
       if (add) mbar_wait(&ctrl.bar_turn, kstep & 1, ctl, DEV_TIMEOUT_MMA);
       if (elect_one()) {
@@ -495,7 +498,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       }
       if (kstep + 2 < count) prefetch_rows(i - 2);
     }
-    mbar_wait_spin(&ctrl.bar_ad[chain], 0, ctl, DEV_TIMEOUT_MMA);      // (a) and (d) of every chunk: even and odd completions
+    mbar_wait_parked(&ctrl.bar_ad[chain], 0, ctl, DEV_TIMEOUT_MMA);      // (a) and (d) of every chunk: even and odd completions
     tc_fence_after();
     if constexpr (C::LATE) {                         // the chain's (a) has read Pm: when both have, the next chunk's copy is asked for
       if (warp_u == COPY_WARP && elect_one()) {
@@ -515,7 +518,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       constexpr int EP = (8 / CW) < 1 ? 1 : (8 / CW) < EL ? (8 / CW) : EL;   // slices per piece of eight columns
       constexpr int NP = EL / EP;
       float kg[2][EP * CW];
-      if (CROSS && kstep > 0) mbar_wait(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);   // the previous chunk's dr partials have been read
+      if (CROSS && kstep > 0) mbar_wait_parked(&ctrl.bar_done, (kstep - 1) & 1, ctl, DEV_TIMEOUT_MMA);   // the previous chunk's dr partials have been read
       if (sgp == 0) {
         tmem_ld<CW>(tmem_row + TM_Y + (v0 - chain * CV), du);
       } else {
@@ -607,7 +610,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
       bulk_commit_group();
     }
     __syncwarp();
-    mbar_wait_spin(&ctrl.bar_mma[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
+    mbar_wait_parked(&ctrl.bar_mma[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
     tc_fence_after();
     if constexpr (C::LATE) {                         // the chain's (c) has read A
       if (warp_u == COPY_WARP && elect_one()) {
@@ -641,7 +644,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         for (int c = 0; c < CW / 2; ++c) xw[c] = w.w[c];
       }
       // (p) reads the image of G that X is about to replace
-      mbar_wait_spin(&ctrl.bar_ex[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
+      mbar_wait_parked(&ctrl.bar_ex[chain], kstep & 1, ctl, DEV_TIMEOUT_MMA);
       // dV of a whole chunk leaves as an image from the place of Xu, which (p) has read (a row of its own per thread would cost 32
       // wavefronts a store; a chunk cut short by a document end may not leave as a tile)
       if (DV_TILE && krow && rows == CHUNK)
@@ -679,7 +682,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     // meanwhile: the two sums over all value columns of a block, of which each chain that shares one takes half of the tokens: P (128
     // key rows x 64 tokens, f32, the chains' shares added) -> bf16 operand image (i = d, j = t), SI = 128, SJ = 2048 (a warp's 16-byte
     // stores cover 512 contiguous bytes), and dr from the partials of the column groups in a fixed order.
-    if (CROSS) mbar_wait_spin(&ctrl.bar_ex[chain ^ 1], kstep & 1, ctl, DEV_TIMEOUT_MMA);
+    if (CROSS) mbar_wait_parked(&ctrl.bar_ex[chain ^ 1], kstep & 1, ctl, DEV_TIMEOUT_MMA);
     {
       tc_fence_after();
       const int64_t block = item * NVB + (C::OWN ? vb * 2 + chain : vb);
@@ -725,7 +728,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
         if (lane == 0) mbar_arrive(&ctrl.bar_done);
       }
     }
-    mbar_wait_spin(&ctrl.bar_ad[chain], 1, ctl, DEV_TIMEOUT_MMA);
+    mbar_wait_parked(&ctrl.bar_ad[chain], 1, ctl, DEV_TIMEOUT_MMA);
     tc_fence_after();
     {
       constexpr int PIECE = TPC < 16 ? TPC : 16;

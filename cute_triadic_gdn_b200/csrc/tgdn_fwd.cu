@@ -308,8 +308,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
 
     // ---- (1) R = [K;Q] S --------------------------------------------------------------------------------------
     // Every thread reads rows of the stage (gates, value row, beta) under the MMA, so every warp waits for the loads itself.
-    // (The MMA completions below are polled by the chain's first warp only: the other three sleep in the chain's hardware
-    // barrier, where they take no issue slots from the chains that are in an epilogue at that moment.)
+    // (The MMA completions below are waited for by the chain's issuing warp only: the others sleep in the chain's hardware
+    // barrier, where they take no issue slots from the chains that are in an epilogue at that moment.  That warp parks: us, polled ->
+    // parked, 4096 items E12 651 -> 636, E16 818 -> 813, 8192 items E8 745 -> 741.  The loads, which are there as a rule, are polled:
+    // parked E16 852.)
     mbar_wait(&ctrl.bar_load[st], (i / STAGES) & 1, ctl, DEV_TIMEOUT_LOAD);
     if (cwarp_u == ISSUE_WARP && elect_one()) {
       tc_fence_after();
@@ -378,7 +380,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       }
       if (i + 2 < count) prefetch_chunk(i + 2);
     }
-    if (cwarp_u == ISSUE_WARP) mbar_wait(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
+    if (cwarp_u == ISSUE_WARP) mbar_wait_parked(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     chain_sync<CT>(chain);
     ++mma_phase;
     tc_fence_after();
@@ -462,7 +464,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
     if constexpr (LATE_R) {                          // r_e only now, from the stage: sixteen registers fewer are live
       if (krow) lds_row<E, ET, E == 16>(gf + C::GF_R, t, e0, gr);   // through the epilogue of (1)
     }
-    if (cwarp_u == ISSUE_WARP) mbar_wait(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
+    if (cwarp_u == ISSUE_WARP) mbar_wait_parked(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     chain_sync<CT>(chain);
     ++mma_phase;
     tc_fence_after();
@@ -523,7 +525,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
       bulk_commit_group();
     }
     __syncwarp();
-    if (cwarp_u == ISSUE_WARP) mbar_wait(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
+    if (cwarp_u == ISSUE_WARP) mbar_wait_parked(&ctrl.bar_mma[chain], mma_phase & 1, ctl, DEV_TIMEOUT_MMA);
     chain_sync<CT>(chain);
     ++mma_phase;
     tc_fence_after();
