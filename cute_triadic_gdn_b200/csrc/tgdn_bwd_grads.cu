@@ -149,6 +149,11 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   SM& sm = *reinterpret_cast<SM*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int ES = SM::ES, NS = SM::NS;
   constexpr float LOG2E = 1.4426950408889634f;
+  // The trace of an item's first slice: up to two slices it is a tile of the double buffer (T0_TILE) and need not wait until dPm' has left the
+  // tensor memory that the other traces use; above, where the chain is what an item waits for, dU, W, U pass before that slice
+  // (TILES_EARLY) so that the chain starts sooner, and its trace waits.  us, slow decays, the second way -> the first: 4096 items E1
+  // 257 -> 235, E2 326 -> 296, E4 461 -> 463; 8192 items E8 1234 -> 1314.
+  constexpr bool T0_TILE = E <= 2, TILES_EARLY = !T0_TILE;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // warp index as a warp-uniform value
   const int NVB = p.NV;
@@ -201,13 +206,13 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   // Barriers, with one completion per item unless noted (so that the parity to wait for is the item's count; a wait for "free" before
   // the first use passes at once):
   //   full / empty[stage]  TMA -> issuer, tensor core -> loads; one per ring entry.  Entries of an item: per slice h, (G), h, (G); dU, W, U
-  //                        behind the first slice, or before it when it has a trace; at the end the value-block images.  (dU, W, U have
+  //                        behind (or before) the first slice; at the end the value-block images.  (dU, W, U have
   //                        another reader than the rest and complete tiles_full instead of full: a waiter that is early by a whole
   //                        round of the ring could not tell the phases of a stage apart.)
   //   kq_full, kq_free     [K;Q] and A; free: eight stream warps (last row sum taken) and G5 complete
   //   xt_full, xt_free     [dW;dO]; free: the item's last P_e complete, and G2
-  //   p_full / p_free[b]   tiles P_e and the value-block sum (E + 1 per item) through the double buffer; free: eight stream warps
-  //   t_full, t_free       trace tile (one per slice with a trace); free: the four stream warps that read it
+  //   p_full / p_free[b]   tiles P_e, the first slice's trace (T0_TILE) and the value-block sum through the double buffer; free: eight stream warps
+  //   t_full, t_free       other traces; free: the four stream warps that read it
   //   g12                  G1, G2 complete;   g2read: the four query-row warps hold dPm': traces may take its place
   //   g34                  G3, then G4 (two per item);   p_ready: the operand of G5 is written;   g5_full: G5
   //   epi_free             the stream warps have read all tiles of the item: the next G1, G2 may be issued
@@ -273,21 +278,31 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
           if (e == 0) mbar_wait_parked(&sm.sums_free, (it & 1) ^ 1, ctl, DEV_TIMEOUT_MMA);
           if (live) atomicAdd(&sm.sums[row * ES + e], krow ? -rowsum : rowsum);
         }
-        if (trace && wg == 0) {                            // <h_e, G_e> = trace(h_e G_e^T): this warp's 32 diagonal elements
-          mbar_wait_parked(&sm.t_full, traces & 1, ctl, DEV_TIMEOUT_MMA);
+        const bool in_tiles = T0_TILE && e == 0;
+        if (trace && (wg == 0 || in_tiles)) {                // <h_e, G_e> = trace(h_e G_e^T): this warp's 32 diagonal elements
+          mbar_wait_parked(in_tiles ? &sm.p_full[tq & 1] : &sm.t_full, (in_tiles ? tq >> 1 : traces) & 1, ctl, DEV_TIMEOUT_MMA);
           tc_fence_after();
-          ++traces;
           float dv[32];
-          tmem_ld<32>(tmem_row + TM_T + (warp & 3) * 32, dv);
-          tmem_wait_ld();
+          if (wg == 0) {
+            tmem_ld<32>(tmem_row + (in_tiles ? (tq & 1) * 128 : TM_T) + (warp & 3) * 32, dv);
+            tmem_wait_ld();
+          }
+          auto take_diagonal = [&]() {
+            if (wg != 0) return;
+            float d = 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) d = (lane == j) ? dv[j] : d;
+            for (int o2 = 16; o2 > 0; o2 >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o2);
+            if (lane == 0) sm.red[e * 4 + (warp & 3)] = d;
+          };
+          // (up to two slices the tile is handed back behind the sum: us, before it -> behind, E1 244 -> 235, E2 331 -> 296; above, before:
+          // E8 1226 against 1249)
+          if constexpr (T0_TILE) take_diagonal();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.t_free);
-          float d = 0.f;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) d = (lane == j) ? dv[j] : d;
-          for (int o2 = 16; o2 > 0; o2 >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o2);
-          if (lane == 0) sm.red[e * 4 + (warp & 3)] = d;
+          if (lane == 0) mbar_arrive(in_tiles ? &sm.p_free[tq & 1] : &sm.t_free);
+          if constexpr (!T0_TILE) take_diagonal();
+          if (in_tiles) ++tq; else ++traces;
         }
       }
       __syncwarp();
@@ -834,8 +849,8 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       sph ^= 1u << st;
       tc_fence_after();
     };
-    // the slice before which dU, W, U pass: the second one, or the first when it has a trace (whose tile must find dPm' read)
-    auto place_of_tiles = [&](uint32_t fmask) { return static_cast<int>(fmask & 1u) ^ 1; };
+    // the slice before which dU, W, U pass: the second one, or (TILES_EARLY) the first when it has a trace
+    auto place_of_tiles = [&](uint32_t fmask) { return TILES_EARLY && (fmask & 1u) ? 0 : 1; };
     constexpr uint32_t id_128 = make_idesc(128, 128, 0, 0), id_64 = make_idesc(128, 64, 0, 0);
     const uint32_t ring = smem_u32(sm.ring[0]);
     const uint64_t dxt = make_desc(smem_u32(sm.xt), 16, 1024, LAYOUT_SW128);
@@ -855,6 +870,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         for (int e = 0; e < E; ++e) {
           const bool trace = (fmask >> e) & 1u;
           if (e == tiles_at) skip_stages(3);
+          const bool in_tiles = T0_TILE && e == 0;
           free_tile();
 #pragma unroll
           for (int vh = 0; vh < 2; ++vh) {
@@ -871,7 +887,12 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
             __syncwarp();
             next_stage();
             if (trace) {                                   // h_e G_e^T over the same value columns
-              if (vh == 0) {
+              const uint32_t tile = in_tiles ? ((tq + 1) & 1) * 128 : TM_T;
+              if (vh == 0 && in_tiles) {
+                ++tq;
+                free_tile();
+                --tq;
+              } else if (vh == 0) {
                 if (first_trace) mbar_wait_parked(&sm.g2read, it & 1, ctl, DEV_TIMEOUT_MMA);
                 first_trace = false;
                 mbar_wait_parked(&sm.t_free, (traces & 1) ^ 1, ctl, DEV_TIMEOUT_MMA);
@@ -881,17 +902,17 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
               if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk)
-                  umma_bf16(tmem + TM_T, desc_advance(dh, kk * 4096), desc_advance(dg, kk * 4096), id_128, (vh > 0 || kk > 0) ? 1u : 0u);
+                  umma_bf16(tmem + tile, desc_advance(dh, kk * 4096), desc_advance(dg, kk * 4096), id_128, (vh > 0 || kk > 0) ? 1u : 0u);
                 umma_commit(&sm.empty[sh]);
                 umma_commit(&sm.empty[st]);
-                if (vh == 1) umma_commit(&sm.t_full);
+                if (vh == 1) umma_commit(in_tiles ? &sm.p_full[(tq + 1) & 1] : &sm.t_full);
               }
               __syncwarp();
               next_stage();
             }
           }
-          ++tq;
-          traces += trace ? 1u : 0u;
+          tq += trace && in_tiles ? 2 : 1;
+          traces += trace && !in_tiles ? 1u : 0u;
         }
         if (elect_one()) umma_commit(&sm.xt_free);
         __syncwarp();
@@ -923,7 +944,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         const typename SM::Place& pl = sm.place[it & 3];
         if (pl.item < 0) break;
         const uint32_t fmask = __shfl_sync(0xffffffffu, pl.traces, 0);
-        const int before = 2 * place_of_tiles(fmask), entries = 2 * E + 2 * __popc(fmask) + 3 + NVB;
+        const int before = place_of_tiles(fmask) * (2 + 2 * (fmask & 1u)), entries = 2 * E + 2 * __popc(fmask) + 3 + NVB;
         mbar_wait_parked(&sm.kq_free, (it & 1) ^ 1, ctl, DEV_TIMEOUT_LOAD);
         if (elect_one()) {
           mbar_expect_tx(&sm.kq_full, 32768 + 8192);
