@@ -61,8 +61,8 @@ KERNEL_U = {
 # shares the eight value blocks of E = 16 where E = 8 has four: its rec and grads figures come out about 64 KB per item low).
 NCU_DRAM_BYTES_PER_ITEM = {
     # kernel: (bytes per item at E = 8, at E = 16); filled from profiles/core_kernels_prof_workload.md
-    "masks": (0.251e9 / 4096, 0.133e9 / 2048), "fwd": (1.516e9 / 4096, 1.284e9 / 2048), "rec": (0.751e9 / 4096, 0.550e9 / 2048),
-    "grads": (2.103e9 / 4096, 1.574e9 / 2048 + 100e3),
+    "masks": (0.251e9 / 4096, 0.133e9 / 2048), "fwd": (1.516e9 / 4096, 1.284e9 / 2048), "rec": (0.750e9 / 4096, 0.550e9 / 2048),
+    "grads": (2.122e9 / 4096, 1.953e9 / 2048),
 }
 
 # DRAM bytes (read + write) per element of the conv kernels, from one ncu capture at (1, 8192, 13056)

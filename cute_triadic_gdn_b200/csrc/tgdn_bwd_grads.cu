@@ -13,15 +13,15 @@
 //   warp 18       loads [K;Q] and A, issues the chain's first products (G1, G2) and its last (G5)
 // The formulas are those of the two kernels, value by value in the same order: the results are bitwise those of running them one after
 // the other (dkq rounded to bf16 included), which tests/test_abi_gpu.py checks.  What need not travel any more: dkq (32 KB an item there and
-// back), da, dc, dd, and the second load of K, Q and dO: 480 KB an item at eight slices instead of 660.
+// back), da, dc, dd, and the second load of K, Q and dO: 520 KB of DRAM traffic an item at eight slices instead of 660.
 //
 // Tensor memory: the tiles P_e and, as the last one, the value-block sum in a double buffer (columns 0..255), G5 (256..383, before that G1
 // in its first 64 columns and dA', Y, dp in turn in its last 64), traces h_e G_e^T (384..511, before that dPm' in the first 64 columns).
 //
-// What bounds it: the memory (480 KB an item at eight slices; 4.8 TB/s) and, close behind, the shared-memory path, which the chain's table
+// What bounds it: the memory (470 KB an item at eight slices; 4.8 TB/s) and, close behind, the shared-memory path, which the chain's table
 // rows, the stream's tensor-memory and K reads, the products' operands and the arriving tiles share; waiting warps park instead of
 // polling for that reason (939 -> 839 us below).  us, state gradients + matrix gradients as two kernels -> this one: 8192 items E8
-// 690 + 505 -> 805, with slow decays 845 + 501 -> 1236; 4096 items E1 148 + 200 -> 236.  Pulling tiles into L2 ahead of the ring, which
+// 690 + 505 -> 805, with slow decays 845 + 501 -> 1226; 4096 items E1 148 + 200 -> 230, E4 238 + 225 -> 293.  Pulling tiles into L2 ahead of the ring, which
 // helped the kernel of the states alone, costs 10 to 20 % here.
 //
 // Replaces cute_triadic_gdn/kernels/sm100_joint_state_grads.py:53-449, sm100_joint_bwd_parallel.py:80-405,

@@ -1,5 +1,6 @@
 // Per-chunk matrix gradients of the Triadic GDN backward, the mask gradients and the final assembly of dq, dk, dk2,
-// dq2, dg, dbeta.
+// dq2, dg, dbeta.  A stage of its own behind the C ABI; the package's backward runs it and the state gradients as one kernel
+// (tgdn_bwd_grads.cu).
 //
 // One CTA of 512 threads per (batch, chunk, head).  Thread (r, cq): r = tensor-memory lane = matrix row (r < 64: key row
 // t = r, r >= 64: query row t = r - 64), cq = which 16 of the 64 columns s it works on.

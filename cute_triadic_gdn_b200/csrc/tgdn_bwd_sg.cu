@@ -1,4 +1,5 @@
 // State gradients of the Triadic GDN backward: everything that contracts over the value axis with the saved forward states.
+// A stage of its own behind the C ABI; the package's backward runs it and the matrix gradients as one kernel (tgdn_bwd_grads.cu).
 //
 // Persistent CTAs (one per SM), each walking (batch, chunk, head) items: 256 worker threads, one warp that only issues the MMAs and one
 // that only issues the bulk loads, so that instruction issue to the tensor core never sits on the workers' path, and the loads of the
