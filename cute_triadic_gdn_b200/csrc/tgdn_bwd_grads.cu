@@ -181,7 +181,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   if (tid == 0) {
     for (int i = 0; i < NS; ++i) { mbar_init(&sm.full[i], 1); mbar_init(&sm.empty[i], 1); }
     mbar_init(&sm.tiles_full, 3); mbar_init(&sm.kq_full, 1); mbar_init(&sm.kq_free, 9);
-    mbar_init(&sm.xt_full, 1); mbar_init(&sm.xt_free, 2);
+    mbar_init(&sm.xt_full, 1); mbar_init(&sm.xt_free, 18);
     for (int i = 0; i < 2; ++i) { mbar_init(&sm.p_full[i], 1); mbar_init(&sm.p_free[i], 8); }
     mbar_init(&sm.t_full, 1); mbar_init(&sm.t_free, 4);
     mbar_init(&sm.g12, 1); mbar_init(&sm.g2read, 4); mbar_init(&sm.g34, 1); mbar_init(&sm.p_ready, 8); mbar_init(&sm.g5_full, 1);
@@ -210,7 +210,8 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   //                        another reader than the rest and complete tiles_full instead of full: a waiter that is early by a whole
   //                        round of the ring could not tell the phases of a stage apart.)
   //   kq_full, kq_free     [K;Q] and A; free: eight stream warps (last row sum taken) and G5 complete
-  //   xt_full, xt_free     [dW;dO]; free: the item's last P_e complete, and G2
+  //   xt_full, xt_free     [dW;dO] and the item's place; free: the item's last P_e complete, G2, and all sixteen stream and chain warps have seen
+  //                        xt_full (with one or two slices nothing else would keep the next item's from completing before they look)
   //   p_full / p_free[b]   tiles P_e, the first slice's trace (T0_TILE) and the value-block sum through the double buffer; free: eight stream warps
   //   t_full, t_free       other traces; free: the four stream warps that read it
   //   g12                  G1, G2 complete;   g2read: the four query-row warps hold dPm': traces may take its place
@@ -231,6 +232,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       mbar_wait_parked(&sm.xt_full, it & 1, ctl, DEV_TIMEOUT_LOAD);
       const typename SM::Place& pl = sm.place[it & 3];
       if (pl.item < 0) break;
+      if (lane == 0) mbar_arrive(&sm.xt_free);
       // this row's gate factors a = k2 exp(gc) (c = scale q2 exp(gc)) as the masks kernel stored them, zero behind a document's end; each
       // asked for a slice ahead
       const float* gates = p.gc + static_cast<int64_t>(pl.item) * gate_item_floats(E) + (krow ? 64 : 192) * E + t * E;
@@ -405,6 +407,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       }
     };
     mbar_wait_parked(&sm.xt_full, 0, ctl, DEV_TIMEOUT_LOAD);
+    if (lane == 0) mbar_arrive(&sm.xt_free);
     if (sm.place[0].item >= 0) request_gates(sm.place[0]);
     for (uint32_t it = 0;; ++it) {
       const typename SM::Place& pl = sm.place[it & 3];     // (seen: xt_full of the item was waited for)
@@ -794,6 +797,8 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       if (E > 4) request_dr();
       mbar_wait_parked(&sm.sg_done, it & 1, ctl, DEV_TIMEOUT_MMA);
       mbar_wait_parked(&sm.xt_full, (it & 1) ^ 1, ctl, DEV_TIMEOUT_LOAD);     // the next item is known
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.xt_free);
       if (sm.place[(it + 1) & 3].item >= 0) request_gates(sm.place[(it + 1) & 3]);
       chain_all();
       // ---- gate gradients: one thread per (row, gate column) ----
@@ -918,6 +923,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         __syncwarp();
         if (tiles_at == E) skip_stages(3);
         // ---- value-block images of the G part of dK, added up, transposed: += [I;0] P_u^T ----
+        if (first_trace) mbar_wait_parked(&sm.g2read, it & 1, ctl, DEV_TIMEOUT_MMA);   // (not behind them: a waiter may not miss a phase)
         free_tile();
         const uint64_t did = make_desc(smem_u32(sm.ident), 1792, 128, LAYOUT_PLAIN);          // K = k
 #pragma unroll 1
@@ -935,7 +941,6 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
           next_stage();
         }
         ++tq;
-        if (first_trace) mbar_wait_parked(&sm.g2read, it & 1, ctl, DEV_TIMEOUT_MMA);   // (a waiter may not miss a phase; long complete)
       }
     } else if (warp_u == 18) {
       // ============================================ products of the chain ============================================
