@@ -238,8 +238,10 @@ mat_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     const int rr = idx / E, e = idx % E, o = rr * ES + e;
     const float up = sm.gc2[(rr & ~15) * ES + e] - sm.gc2[o];    // >= 0 when gc does not increase
     // too steep, NaN, or not monotone (a log gate above zero makes gc rise from one row to the next: the factorised form,
-    // which clamps its first factor at one, would then be wrong for rows of later blocks)
-    if (!(up <= 100.f) || up < 0.f || (rr > 0 && sm.gc2[o] > sm.gc2[o - ES])) sm.steep = 1;
+    // which clamps its first factor at one, would then be wrong for rows of later blocks).  Rows behind a document's end do not
+    // count: their gate factors are zero, and gc, a scan in tree order, rises there by roundings (seven columns of ten at 21 rows),
+    // which sent most short chunks down the direct path for nothing.
+    if (rr < rows && (!(up <= 100.f) || up < 0.f || (rr > 0 && sm.gc2[o] > sm.gc2[o - ES]))) sm.steep = 1;
     sm.hkv[idx] = mexp2(up) * sm.k2[o];
     sm.qxv[idx] = sm.q2[o] * mexp2(-up);
   }

@@ -55,6 +55,31 @@ def test_direct_decay_path(E, kind):
     both(ins, orc.make_grad_output((B, T, H, 128), 10), None)
 
 
+@pytest.mark.parametrize("E", [2, 4, 8, 12, 16])
+@pytest.mark.parametrize("rows", [3, 21, 47, 62])
+def test_roundings_behind_a_documents_end_change_nothing(E, rows):
+    """The cumulative gate of the rows behind a document's end may rise by a rounding.  That is no reason for the direct decay path, whose
+    sums differ in their last bits: a rise there, in a slice without weight, leaves every bit of the gradients as it is."""
+    n, H, scale = 9, 16, 128 ** -0.5
+    q, k, v, k2, q2, g, beta = [t.cuda() for t in orc.make_inputs(1, n * rows, H, E, seed=60 + E, dist="mild")]
+    k2[..., 0] = q2[..., 0] = 0.0
+    g = (g * 256).round().clamp(max=-1) / 256                # sums without roundings: gc does not rise by itself
+    do = orc.make_grad_output((1, n * rows, H, 128), 11).cuda()
+    cs, tm = prepare_documents((q, k, v, k2, q2, g, beta), torch.arange(0, n * rows + 1, rows, dtype=torch.int32, device="cuda"))
+    gc, AP, Pm = gj._run_masks(q, k, k2, q2, g, beta, scale, tm)
+    _, h, W, U = gj._run_forward(q, k, v, k2, q2, beta, gc, AP, scale, True, cs, tm)
+    dV, dU, ds, dkg, dr = gj._run_reverse(q, k, do, k2, q2, beta, gc, AP, Pm, U, scale, cs, tm)
+    risen = gc.clone()
+    gj.chunk_gates(risen, E)[..., rows, 0] *= 1 - 2.0 ** -20
+    assert (gj.chunk_gates(risen, E)[0, :n, :, rows, 0] > gj.chunk_gates(gc, E)[0, :n, :, rows - 1, 0]).all()
+    one, other = (gj._run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, c, scale, tm) for c in (gc, risen))
+    dkq, da, dc, dd = gj._run_state_grads(q, k, do, dV, h, ds, dkg, k2, q2, risen, scale, tm)
+    two = gj._run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, risen, dkq, da, dc, dd, dr, scale, tm)
+    for name, a, b, c in zip("dq dk dk2 dq2 dg dbeta".split(), one, other, two):
+        assert torch.isfinite(a.float()).all() and torch.equal(a, b) and torch.equal(a, c), name
+    assert _lib.device_status() == 0
+
+
 @pytest.mark.parametrize("E", [1, 2, 4])
 @pytest.mark.parametrize("T,docs", [(511, [0, 1, 64, 129, 200, 263, 384, 448, 511]), (64, [0, 1, 64]), (512, None)])
 def test_short_items_again_and_again(E, T, docs):
