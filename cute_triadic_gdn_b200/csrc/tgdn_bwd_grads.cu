@@ -232,6 +232,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       mbar_wait_parked(&sm.xt_full, it & 1, ctl, DEV_TIMEOUT_LOAD);
       const typename SM::Place& pl = sm.place[it & 3];
       if (pl.item < 0) break;
+      __syncwarp();                                        // xt_free: every lane has seen xt_full
       if (lane == 0) mbar_arrive(&sm.xt_free);
       // this row's gate factors a = k2 exp(gc) (c = scale q2 exp(gc)) as the masks kernel stored them, zero behind a document's end; each
       // asked for a slice ahead
@@ -407,6 +408,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       }
     };
     mbar_wait_parked(&sm.xt_full, 0, ctl, DEV_TIMEOUT_LOAD);
+    __syncwarp();
     if (lane == 0) mbar_arrive(&sm.xt_free);
     if (sm.place[0].item >= 0) request_gates(sm.place[0]);
     for (uint32_t it = 0;; ++it) {

@@ -15,6 +15,11 @@ TRACES = {"none": lambda e, E: False, "all": lambda e, E: True, "first": lambda 
           "other": lambda e, E: e % 2 == 1}
 
 
+def repeated(tensors, heads):
+    """The same heads again and again, as many as asked for."""
+    return [t.cuda().repeat([1, 1, heads // t.shape[2]] + [1] * (t.dim() - 3)) for t in tensors]
+
+
 def both(ins, do, docs=None):
     q, k, v, k2, q2, g, beta = [t.cuda() for t in ins]
     do, E, scale = do.cuda(), k2.shape[-1], 128 ** -0.5
@@ -81,11 +86,15 @@ def test_roundings_behind_a_documents_end_change_nothing(E, rows):
 
 
 @pytest.mark.parametrize("E", [1, 2, 4])
+@pytest.mark.parametrize("H,more", [(16, 1), (16, 10)])
 @pytest.mark.parametrize("T,docs", [(511, [0, 1, 64, 129, 200, 263, 384, 448, 511]), (64, [0, 1, 64]), (512, None)])
-def test_short_items_again_and_again(E, T, docs):
-    """With few slices an item is over before a slow warp has looked at its barriers: the same call must give the same bits each time."""
-    ins = [t.cuda() for t in orc.make_inputs(1, T, 16, E, seed=20 + E, dist="mild")]
-    do = orc.make_grad_output((1, T, 16, 128), 4).cuda()
+def test_short_items_again_and_again(E, T, docs, H, more):
+    """With few slices an item is over before a slow warp has looked at its barriers: the same call must give the same bits each time, and
+    the same for the same head.  `more`: at least as many items for each of a B200's 148 persistent blocks."""
+    ins, do = orc.make_inputs(1, T, H, E, seed=20 + E, dist="mild"), orc.make_grad_output((1, T, H, 128), 4)
+    chunks = -(-T // 64) if docs is None else sum(-(-(b - a) // 64) for a, b in zip(docs, docs[1:]))
+    heads = H if more == 1 else H * -(-148 * more // (H * chunks))
+    *ins, do = repeated([*ins, do], heads)
     cu = None if docs is None else torch.tensor(docs, dtype=torch.int32).cuda()
     first = None
     for _ in range(40):
@@ -93,4 +102,5 @@ def test_short_items_again_and_again(E, T, docs):
         grads = torch.autograd.grad(gdn_joint_call(*leaves, cu_seqlens=cu), leaves, do)
         first = first or grads
         assert all(torch.equal(a, b) for a, b in zip(first, grads))
+    assert all(torch.equal(a, b) for a, b in zip(first, repeated([t[:, :, :H] for t in first], heads)))
     assert _lib.device_status() == 0
