@@ -48,6 +48,14 @@ def test_one_kernel_is_the_two_stages(E, traces, B, T, H, docs):
 
 
 @pytest.mark.parametrize("E", [1, 2, 4, 8, 12, 16])
+def test_fourteen_items_a_block(E):
+    """Items enough for every slot of the blocks' item records to be used several times, every other slice with a trace."""
+    ins = list(orc.make_inputs(2, 1024, 8, E, seed=40 + E, dist="mild"))
+    ins[5] = torch.where(torch.arange(E) % 2 == 1, 0.02, 1.0) * ins[5].abs().neg().clamp(-1.0, -0.4)
+    both(repeated(ins, 64), repeated([orc.make_grad_output((2, 1024, 8, 128), 9)], 64)[0])
+
+
+@pytest.mark.parametrize("E", [1, 2, 4, 8, 12, 16])
 @pytest.mark.parametrize("kind", ["steep", "rising"])
 def test_direct_decay_path(E, kind):
     B, T, H = 1, 192, 3
@@ -103,4 +111,35 @@ def test_short_items_again_and_again(E, T, docs, H, more):
         first = first or grads
         assert all(torch.equal(a, b) for a, b in zip(first, grads))
     assert all(torch.equal(a, b) for a, b in zip(first, repeated([t[:, :, :H] for t in first], heads)))
+    assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("E", [1, 8])
+def test_two_streams_and_a_replayed_graph(E):
+    """The counter that items are drawn from belongs to the call: two backwards at a time, and a captured one replayed, give the bits of one."""
+    def step(leaves, do):
+        return torch.autograd.grad(gdn_joint_call(*leaves), leaves, do)
+
+    calls = []
+    for seed in (1, 2):
+        ins = repeated(orc.make_inputs(1, 256, 16, E, seed=seed, dist="mild"), 96)
+        calls.append(([t.requires_grad_(True) for t in ins], repeated([orc.make_grad_output((1, 256, 16, 128), seed)], 96)[0]))
+    alone = [step(*c) for c in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in calls]
+    for _ in range(10):
+        got = []
+        for s, c in zip(streams, calls):
+            with torch.cuda.stream(s):
+                got.append(step(*c))
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for x, y in zip(alone, got) for a, b in zip(x, y))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = step(*calls[0])
+    for _ in range(3):
+        for t in out:
+            t.zero_()
+        graph.replay()
+        assert all(torch.equal(a, b) for a, b in zip(alone[0], out))
     assert _lib.device_status() == 0
