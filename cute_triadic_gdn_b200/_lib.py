@@ -42,6 +42,7 @@ SIGNATURES = {
     "tgdn_selftest_mma": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P]),
     "tgdn_selftest_tma": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _P, _I, _P, _P]),
     "tgdn_selftest_wait": (_I, [_c.c_longlong, _P, _P]),
+    "tgdn_selftest_role": (_I, [_c.c_longlong, _P, _P]),
 }
 
 

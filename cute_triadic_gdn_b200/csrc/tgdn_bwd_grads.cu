@@ -35,8 +35,8 @@ namespace tgdn {
 
 constexpr int GR_THREADS = 20 * 32;   // (warp 19 only completes its warpgroup)
 // Registers a thread: 96 at launch (five warps on each quarter of an SM), then the two warpgroups of a role take what the last one gives
-// back: 2 * 112 + 2 * 104 + 40 = 472 of 480.
-constexpr int GR_STREAM_REGS = 112, GR_CHAIN_REGS = 104, GR_SERVICE_REGS = 40;
+// back: 2 * 112 + 2 * 104 + 48 = 480 of 480 (with 40 for the service warps the loading warp spills).
+constexpr int GR_STREAM_REGS = 112, GR_CHAIN_REGS = 104, GR_SERVICE_REGS = 48;
 static_assert(2 * GR_STREAM_REGS + 2 * GR_CHAIN_REGS + GR_SERVICE_REGS <= 5 * 96, "registers of the block");
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -132,8 +132,10 @@ struct GradsSmem {
   uint64_t full[NS], empty[NS], tiles_full, kq_full, kq_free, xt_full, xt_free, p_full[2], p_free[2], t_full, t_free, g12, g2read, g34, p_ready, g5_full,
       epi_free, stage_free, sums_free, sg_done;
   struct Place { int item, h, b, t0, rows; uint32_t traces; } place[4];   // of the CTA's item `it` in slot it % 4; item -1: the end
+  uint64_t drained;             // all products issued are complete
   uint32_t tmem_base;
-  int abort;
+  int abort, drain_abort;
+  int stream_go, chain_go;      // verdicts of the two roles: on to the item
   int steep;
 };
 
@@ -186,8 +188,10 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     mbar_init(&sm.t_full, 1); mbar_init(&sm.t_free, 4);
     mbar_init(&sm.g12, 1); mbar_init(&sm.g2read, 4); mbar_init(&sm.g34, 1); mbar_init(&sm.p_ready, 8); mbar_init(&sm.g5_full, 1);
     mbar_init(&sm.epi_free, 8); mbar_init(&sm.stage_free, 1); mbar_init(&sm.sums_free, 8); mbar_init(&sm.sg_done, 8);
+    mbar_init(&sm.drained, 3);
     mbar_fence_init();
-    sm.abort = 0;
+    sm.abort = sm.drain_abort = 0;
+    for (int i = 0; i < 4; ++i) sm.place[i].item = -1;
   }
   if (warp_u == 16) { tmem_alloc(&sm.tmem_base, 512); tmem_relinquish(); }
   for (int i = tid; i < (2048 + 3584) / 16; i += GR_THREADS) reinterpret_cast<uint4*>(sm.zero)[i] = make_uint4(0, 0, 0, 0);   // and ident
@@ -201,7 +205,12 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, sm.tmem_base, 0);
   const uint32_t tmem_row = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-  WaitCtl ctl{&sm.abort, p.status};
+  WaitCtl ctl{&sm.abort, p.status}, drain{&sm.drain_abort, p.status};
+  auto seen = [&](uint64_t* bar, uint32_t parity, int code) { return mbar_wait_parked_warp(bar, parity, ctl, code); };
+  // Where a wait gives up, every wait of the CTA that is not met returns at once, and each role ends: the loading warp asks for nothing more
+  // and writes no further item record; a role goes on to an item only when its wait for the record was met (the stream and the
+  // chain by one verdict for all their warps), so that no address comes from a record that was not written; an item that was begun is
+  // gone through to its end.  Loads, stores and products in flight are waited for at the end of the warps that issued them.
 
   // Barriers, with one completion per item unless noted (so that the parity to wait for is the item's count; a wait for "free" before
   // the first use passes at once):
@@ -229,10 +238,17 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
     const uint32_t krow_smem = smem_u32(sm.kq) + wg * 16384 + row * 128;   // this thread's K (Q) row, its 64 columns
     uint32_t tq = 0, traces = 0;                           // tiles, traces read so far
     for (uint32_t it = 0;; ++it) {
-      mbar_wait_parked(&sm.xt_full, it & 1, ctl, DEV_TIMEOUT_LOAD);
       const typename SM::Place& pl = sm.place[it & 3];
-      if (pl.item < 0) break;
-      __syncwarp();                                        // xt_free: every lane has seen xt_full
+      const bool known = seen(&sm.xt_full, it & 1, DEV_TIMEOUT_LOAD);   // (by all lanes, which xt_free says)
+      const bool go = one_verdict<4, 256>(known && pl.item >= 0, tid == 0, &sm.stream_go);
+      // the previous item's dk, dq have left shared memory (waited for behind the verdict: before it, everybody would wait for them;
+      // us, a backward of 4096 items, E2 with slow decays: 703 -> 689)
+      if (it > 0 && warp_u == 3 && elect_one()) {
+        bulk_wait_group_read();
+        mbar_arrive(&sm.stage_free);
+      }
+      __syncwarp();
+      if (!go) break;
       if (lane == 0) mbar_arrive(&sm.xt_free);
       // this row's gate factors a = k2 exp(gc) (c = scale q2 exp(gc)) as the masks kernel stored them, zero behind a document's end; each
       // asked for a slice ahead
@@ -359,16 +375,12 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.epi_free);
       asm volatile("bar.sync 4, 256;" ::: "memory");
-      if (warp_u == 3 && elect_one()) {
-        if (whole) {
-          tma_store_4d(&map_dk, sm.p5, 0, pl.h, pl.t0, pl.b);
-          tma_store_4d(&map_dk, sm.p5 + 8192, 64, pl.h, pl.t0, pl.b);
-          tma_store_4d(&map_dq, sm.dmp, 0, pl.h, pl.t0, pl.b);
-          tma_store_4d(&map_dq, sm.dmp + 8192, 64, pl.h, pl.t0, pl.b);
-          bulk_commit_group();
-          bulk_wait_group_read();
-        }
-        mbar_arrive(&sm.stage_free);
+      if (whole && warp_u == 3 && elect_one()) {
+        tma_store_4d(&map_dk, sm.p5, 0, pl.h, pl.t0, pl.b);
+        tma_store_4d(&map_dk, sm.p5 + 8192, 64, pl.h, pl.t0, pl.b);
+        tma_store_4d(&map_dq, sm.dmp, 0, pl.h, pl.t0, pl.b);
+        tma_store_4d(&map_dq, sm.dmp + 8192, 64, pl.h, pl.t0, pl.b);
+        bulk_commit_group();
       }
       __syncwarp();
     }
@@ -407,13 +419,17 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         q2_in[i] = __ldg(p.q2 + off);
       }
     };
-    mbar_wait_parked(&sm.xt_full, 0, ctl, DEV_TIMEOUT_LOAD);
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&sm.xt_free);
-    if (sm.place[0].item >= 0) request_gates(sm.place[0]);
-    for (uint32_t it = 0;; ++it) {
-      const typename SM::Place& pl = sm.place[it & 3];     // (seen: xt_full of the item was waited for)
-      if (pl.item < 0) break;
+    // the wait for an item's record, its gates asked for and the verdict on it; at its return sm.chain_go says whether there is such an item
+    auto next_item = [&](uint32_t it) {
+      const typename SM::Place& w = sm.place[it & 3];
+      const bool go = seen(&sm.xt_full, it & 1, DEV_TIMEOUT_LOAD) && w.item >= 0;
+      if (lane == 0) mbar_arrive(&sm.xt_free);
+      if (go) request_gates(w);
+      one_verdict<1, 256>(go, mt == 0, &sm.chain_go);
+    };
+    next_item(0);
+    for (uint32_t it = 0; *static_cast<volatile int*>(&sm.chain_go) != 0; ++it) {
+      const typename SM::Place& pl = sm.place[it & 3];
       const int rows = pl.rows;
       // ---- gate tables ----
 #pragma unroll
@@ -800,11 +816,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       }
       if (E > 4) request_dr();
       mbar_wait_parked(&sm.sg_done, it & 1, ctl, DEV_TIMEOUT_MMA);
-      mbar_wait_parked(&sm.xt_full, (it & 1) ^ 1, ctl, DEV_TIMEOUT_LOAD);     // the next item is known
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.xt_free);
-      if (sm.place[(it + 1) & 3].item >= 0) request_gates(sm.place[(it + 1) & 3]);
-      chain_all();
+      next_item(it + 1);
       // ---- gate gradients: one thread per (row, gate column) ----
       const int64_t tok = static_cast<int64_t>(pl.b) * p.TS + pl.t0;
 #pragma unroll
@@ -847,6 +859,8 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         if (rr < rows) p.dg[((tok + rr) * p.H + pl.h) * E + e] = sm.r1[rr * ES + e];
       }
     }
+    if (mw == 0 && elect_one()) umma_commit(&sm.drained);
+    __syncwarp();
   } else {
     regs_down<GR_SERVICE_REGS>();
     int st = 0;                                            // ring stage
@@ -870,8 +884,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       uint32_t tq = 0, traces = 0;                         // tiles, traces issued so far
       auto free_tile = [&]() { mbar_wait_parked(&sm.p_free[tq & 1], ((tq >> 1) & 1) ^ 1, ctl, DEV_TIMEOUT_MMA); };
       for (uint32_t it = 0;; ++it) {
-        mbar_wait_parked(&sm.xt_full, it & 1, ctl, DEV_TIMEOUT_LOAD);
-        if (sm.place[it & 3].item < 0) break;
+        if (!seen(&sm.xt_full, it & 1, DEV_TIMEOUT_LOAD) || sm.place[it & 3].item < 0) break;
         const uint32_t fmask = __shfl_sync(0xffffffffu, sm.place[it & 3].traces, 0);
         const int tiles_at = place_of_tiles(fmask);
         bool first_trace = true;
@@ -946,15 +959,18 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         }
         ++tq;
       }
+      if (elect_one()) umma_commit(&sm.drained);
+      __syncwarp();
     } else if (warp_u == 18) {
       // ============================================ products of the chain ============================================
+      uint32_t kq_loads = 0;
       for (uint32_t it = 0;; ++it) {
-        mbar_wait_parked(&sm.xt_full, it & 1, ctl, DEV_TIMEOUT_LOAD);
         const typename SM::Place& pl = sm.place[it & 3];
-        if (pl.item < 0) break;
+        if (!seen(&sm.xt_full, it & 1, DEV_TIMEOUT_LOAD) || pl.item < 0) break;
         const uint32_t fmask = __shfl_sync(0xffffffffu, pl.traces, 0);
         const int before = place_of_tiles(fmask) * (2 + 2 * (fmask & 1u)), entries = 2 * E + 2 * __popc(fmask) + 3 + NVB;
-        mbar_wait_parked(&sm.kq_free, (it & 1) ^ 1, ctl, DEV_TIMEOUT_LOAD);
+        if (!seen(&sm.kq_free, (it & 1) ^ 1, DEV_TIMEOUT_LOAD)) break;
+        ++kq_loads;
         if (elect_one()) {
           mbar_expect_tx(&sm.kq_full, 32768 + 8192);
           tma_load_4d(sm.kq, &map_k, &sm.kq_full, 0, pl.h, pl.t0, pl.b);
@@ -966,7 +982,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         __syncwarp();
         // ---- G1 = [K;Q] K^T;  G2: dA' = dU W^T (rows 0..63), dPm' = dO U^T (rows 64..127) ----
         mbar_wait_parked(&sm.epi_free, (it & 1) ^ 1, ctl, DEV_TIMEOUT_MMA);
-        mbar_wait_parked(&sm.kq_full, it & 1, ctl, DEV_TIMEOUT_LOAD);
+        if (!seen(&sm.kq_full, it & 1, DEV_TIMEOUT_LOAD)) break;
         tc_fence_after();
         const uint64_t dkq = make_desc(smem_u32(sm.kq), 16, 1024, LAYOUT_SW128);
         if (elect_one()) {
@@ -1026,12 +1042,18 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         }
         __syncwarp();
       }
+      mbar_wait_parked(&sm.kq_full, (kq_loads & 1) ^ 1, drain, DEV_TIMEOUT_LOAD);
+      if (elect_one()) umma_commit(&sm.drained);
+      __syncwarp();
     } else if (warp_u == 17) {
       // ============================================ loads ============================================
-      auto open_stage = [&]() { mbar_wait_parked(&sm.empty[st], sph ^ 1u, ctl, DEV_TIMEOUT_LOAD); };
+      bool open = true;                                    // false: a wait gave up, nothing more is asked for (an entry could meet the last
+                                                           // one of its stage still on its way)
+      uint32_t tiles = 0, tile_stages = 0;                 // tiles asked for, and their parity per stage
+      auto open_stage = [&]() { return open = open && seen(&sm.empty[st], sph ^ 1u, DEV_TIMEOUT_LOAD); };
       auto filled = [&]() { next_stage(); sph ^= st == 0 ? 1u : 0u; };
       auto entry = [&](const uint8_t* src) {               // 16 KB of global memory -> the next stage
-        open_stage();
+        if (!open_stage()) return;
         if (elect_one()) {
           mbar_expect_tx(&sm.full[st], 16384);
           bulk_load(sm.ring[st], src, 16384, &sm.full[st]);
@@ -1040,7 +1062,9 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         filled();
       };
       auto tile_entry = [&](const CUtensorMap* map, int crow) {   // a 64 x 128 tile of a chunk-layout tensor
-        open_stage();
+        if (!open_stage()) return;
+        ++tiles;
+        tile_stages ^= 1u << st;
         if (elect_one()) {
           mbar_expect_tx(&sm.tiles_full, 16384);
           tma_load_4d(sm.ring[st], map, &sm.tiles_full, 0, 0, crow, 0);
@@ -1065,12 +1089,13 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
       cur.item = blockIdx.x;
       if (!place(cur)) cur = draw();
       float my_gl = load_gl(cur);
-      for (uint32_t it = 0;; ++it) {
+      uint32_t it = 0;                                     // item records written
+      for (;; ++it) {
         Walk nxt = cur;
         if (cur.item < n_items) nxt = draw();
         const float next_gl = load_gl(nxt);                // asked for a whole item ahead
         const uint32_t fmask = __ballot_sync(0xffffffffu, lane < E && my_gl * LOG2E >= DD_MIN_LOG2_DECAY);
-        mbar_wait_parked(&sm.xt_free, (it & 1) ^ 1, ctl, DEV_TIMEOUT_LOAD);
+        if (!open || !seen(&sm.xt_free, (it & 1) ^ 1, DEV_TIMEOUT_LOAD)) break;
         const bool end = cur.item >= n_items;
         if (elect_one()) {
           typename SM::Place& pl = sm.place[it & 3];
@@ -1087,7 +1112,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
           }
         }
         __syncwarp();
-        if (end) break;
+        if (end) { ++it; break; }
         // what threads load themselves -> L2: dr of this item, the gates of the next (the tiles and images come without: pulling those
         // ahead made the kernel 10 to 20 % slower)
         for (int l = lane; l < NVB * 2 * E; l += 32) prefetch_l2(p.dr + static_cast<int64_t>(cur.item) * NVB * (64 * E) + l * 32);
@@ -1129,11 +1154,22 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         cur = nxt;
         my_gl = next_gl;
       }
+      // what was asked for has arrived: the last phase of each barrier
+      for (; tiles % 3 != 0; ++tiles)                      // (a set cut short: the arrivals that are missing)
+        if (elect_one()) mbar_arrive(&sm.tiles_full);
+#pragma unroll 1
+      for (int i = 0; i < NS + 2; ++i) {
+        const uint32_t phases = i < NS ? sph ^ (i < st ? 1u : 0u) ^ (tile_stages >> i) : i == NS ? tiles / 3 : it;
+        mbar_wait_parked(i < NS ? &sm.full[i] : i == NS ? &sm.tiles_full : &sm.xt_full, (phases & 1) ^ 1, drain, DEV_TIMEOUT_LOAD);
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp_u == 16) tmem_dealloc(tmem, 512);
+  if (warp_u == 16) {
+    mbar_wait_parked(&sm.drained, 0, drain, DEV_TIMEOUT_MMA);
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 }  // namespace tgdn

@@ -66,8 +66,7 @@ struct WaitCtl {
 constexpr long long WAIT_LIMIT_CYCLES = 1ll << 31;   // about a second of SM clocks
 
 // Wait for `parity` of `bar`; gives up after WAIT_LIMIT_CYCLES, records `code` and raises the CTA's abort flag.
-// Spins on the non-parking probe: the parking form (try_wait) was measured to wake a waiter up to a microsecond after
-// the barrier flipped, which is as long as a whole pipeline phase here.
+// Spins on the non-parking probe, which sees the flip within a few cycles: for waits that are over as a rule when they begin.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code,
                                           long long limit_cycles = WAIT_LIMIT_CYCLES) {
 #pragma unroll 1
@@ -87,7 +86,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 // The same wait for a warp that has long to wait beside others that work: the probe parks the warp for at most PARK_NS.  A poll is an
-// access to shared memory, and where that path is the bottleneck a dozen polling warps take a third of it.
+// access to shared memory, and where that path is the bottleneck a dozen polling warps take a third of it (what each kernel gained, and
+// lost where such a wait took the place of one that is over as a rule, stands in its file).
 constexpr uint32_t PARK_NS = 200;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -100,20 +100,48 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
+__device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code,
+                                                 long long limit_cycles = WAIT_LIMIT_CYCLES) {
   if (mbar_try_wait(bar, parity)) return true;
   const long long start = clock64();
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 0u) {
       if (*ctl.abort) return false;
-      if (clock64() - start > WAIT_LIMIT_CYCLES) {
+      if (clock64() - start > limit_cycles) {
         *ctl.abort = 1;
         atomicCAS(ctl.status, DEV_OK, code);
         return false;
       }
     }
   }
+}
+// The parked wait of a whole warp: its lanes look together and have one outcome.  (A vote on what each lane's own wait returned would come on
+// top of their loops: with the loads of the fused gradient kernel waiting that way, its backward took 0.5 % longer.)
+__device__ __forceinline__ bool mbar_wait_parked_warp(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code,
+                                                      long long limit_cycles = WAIT_LIMIT_CYCLES) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const long long start = clock64();
+  for (uint32_t it = 1;; ++it) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((it & 63u) == 0u) {
+      if (__any_sync(0xffffffffu, *ctl.abort)) return false;
+      if (__any_sync(0xffffffffu, clock64() - start > limit_cycles)) {
+        *ctl.abort = 1;
+        atomicCAS(ctl.status, DEV_OK, code);
+        return false;
+      }
+    }
+  }
+}
+// One verdict for warps that go through named barriers together: that of the thread which leads them.  A wait may be met for one warp and given
+// up by another; whoever acts on its own outcome leaves the others at the next barrier for good.  `word` (shared) is free for the next
+// verdict behind another barrier of the same warps.
+template <int BARRIER, int THREADS>
+__device__ __forceinline__ bool one_verdict(bool mine, bool leads, volatile int* word) {
+  if (leads) *word = mine ? 1 : 0;
+  asm volatile("bar.sync %0, %1;" ::"n"(BARRIER), "n"(THREADS) : "memory");
+  return *word != 0;
 }
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, const WaitCtl& ctl, int code) {
   return mbar_wait(bar, parity, ctl, code);

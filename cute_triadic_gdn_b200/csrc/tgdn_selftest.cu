@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(128) selftest_tma_kernel(const __grid_constant
 
 // A CTA of two warps waits, with a short limit, for a barrier that nothing will ever arrive at: both warps must give up,
 // the status word must read DEV_TIMEOUT_LOAD, the second warp (which starts waiting later) must see the abort flag of
-// the first, and the kernel must end normally.  This is the path every production kernel takes when a pipeline stalls.
+// the first, and the kernel must end normally.  This is the path every production kernel takes when a wait that polls gives up.
 __global__ void __launch_bounds__(64) selftest_wait_kernel(long long limit_cycles, int* status, int* out) {
   __shared__ uint64_t bar;
   __shared__ int abort_s;
@@ -134,9 +134,50 @@ __global__ void __launch_bounds__(64) selftest_wait_kernel(long long limit_cycle
   }
 }
 
+// The parked waits (a lane's in the even warps, a warp's in the odd ones) and the verdict of a role, as the fused gradient kernel uses them.  A role of four warps goes through items; the second
+// warp pair's barrier for the first item, and everybody's for the second, is one that nothing arrives at.  All four warps must go
+// through the first item (the leader's wait is met, that of the second pair gives up), leave before the second, and the kernel must
+// end normally.
+__global__ void __launch_bounds__(128) selftest_role_kernel(long long limit_cycles, int* status, int* out) {
+  __shared__ uint64_t met, never;
+  __shared__ int abort_s, go;
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    mbar_init(&met, 1); mbar_init(&never, 1); mbar_fence_init();
+    abort_s = 0;
+    mbar_arrive(&met);
+  }
+  __syncthreads();
+  WaitCtl ctl{&abort_s, status};
+  const long long t0 = clock64();
+  int items = 0;
+  for (; items < 2; ++items) {
+    uint64_t* bar = items == 0 && warp < 2 ? &met : &never;
+    const bool ok = (warp & 1) ? mbar_wait_parked_warp(bar, 0, ctl, DEV_TIMEOUT_LOAD, limit_cycles)
+                               : __all_sync(0xffffffffu, mbar_wait_parked(bar, 0, ctl, DEV_TIMEOUT_LOAD, limit_cycles));
+    if (!one_verdict<1, 128>(ok, threadIdx.x == 0, &go)) break;
+    asm volatile("bar.sync 1, 128;" ::: "memory");         // the item
+  }
+  const long long waited = clock64() - t0;
+  if ((threadIdx.x & 31) == 0) out[2 + warp] = items;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    out[0] = abort_s;
+    out[1] = waited > 0x7fffffffLL ? 0x7fffffff : static_cast<int>(waited);
+  }
+}
+
 }  // namespace tgdn
 
 using namespace tgdn;
+
+extern "C" int tgdn_selftest_role(long long limit_cycles, int* out6, void* stream) {
+  if (!out6) return TGDN_ERR_NULL;
+  if (limit_cycles < 1 || limit_cycles > (1ll << 28)) return TGDN_ERR_SHAPE;
+  if (!tgdn_check_device()) return TGDN_ERR_DEVICE;
+  selftest_role_kernel<<<1, 128, 0, static_cast<cudaStream_t>(stream)>>>(limit_cycles, tgdn_status_word(), out6);
+  return tgdn_cuda_error(cudaGetLastError());
+}
 
 extern "C" int tgdn_selftest_wait(long long limit_cycles, int* out3, void* stream) {
   if (!out3) return TGDN_ERR_NULL;

@@ -25,6 +25,10 @@ int tgdn_selftest_tma(const void* x, int B, int T, int H, int col0, int head, in
  * [2] the clocks the wait took.  The device status word then reads 1 (a load barrier timed out) until it is read.
  * No counterpart in the reference (its waits are unbounded: cute_triadic_gdn/kernels/sm100_tc.py:116-119). */
 int tgdn_selftest_wait(long long limit_cycles, int* out3, void* stream);
+/* The same for waits that park and for warps that share named barriers: one CTA of four warps goes through two items; two of the warps have
+ * the first item's barrier met, all other waits are for a barrier nothing arrives at.  out6 (device, 6 ints): [0] the abort flag; [1] the
+ * clocks until the end; [2..5] the items each warp went through (1 for all, the leading warp's verdict).  No counterpart in the reference. */
+int tgdn_selftest_role(long long limit_cycles, int* out6, void* stream);
 
 #ifdef __cplusplus
 }

@@ -1,9 +1,10 @@
 """The give-up path of the kernels' bounded waits, exercised without provoking any fault.
 
-Every wait of every kernel here polls an mbarrier with a limit; a wait that runs out raises the CTA's abort flag, records a
-code in the device status word and lets the kernel run to its normal end.  The self-test kernel waits, with a SHORT limit,
-for a barrier nothing arrives at: it must end by itself, report that the wait gave up, leave status 1 (a load barrier
-timed out), and the context must stay usable (the reference's waits are unbounded: kernels/sm100_tc.py:116-119)."""
+Every wait for an mbarrier has a limit, whether it polls or parks; a wait that runs out raises the CTA's abort flag, records a code
+in the device status word and lets the kernel end by itself: kernels whose items come from their block index run to their normal
+end, the fused gradient kernel, whose items are handed out as it runs, finishes the item it is at.  The self-test kernels wait, with a
+SHORT limit, for a barrier nothing arrives at: they must end by themselves, report that the wait gave up, leave status 1 (a load
+barrier timed out), and the context must stay usable (the reference's waits are unbounded: kernels/sm100_tc.py:116-119)."""
 import ctypes
 
 import pytest
@@ -35,9 +36,27 @@ def test_a_wait_that_runs_out_returns_and_reports():
     assert torch.isfinite(o.float()).all() and _lib.device_status() == 0
 
 
+def test_parked_waits_that_run_out_end_a_role_as_one():
+    """Warps that share named barriers go on, and leave, together, although the wait of some was met and that of others gave up."""
+    assert _lib.device_status() == 0
+    out = torch.full((6,), -1, dtype=torch.int32, device="cuda")
+    limit = 1 << 20
+    rc = _lib.lib.tgdn_selftest_role(limit, ctypes.c_void_p(out.data_ptr()),
+                                     ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    abort, waited, *items = out.tolist()
+    assert abort == 1 and items == [1, 1, 1, 1]
+    assert limit < waited < 64 * limit                         # the limit once: the waits behind it return at once
+    assert _lib.device_status() == 1
+    assert _lib.device_status() == 0
+
+
 def test_limits_outside_the_allowed_range_are_rejected():
     out = torch.zeros(3, dtype=torch.int32, device="cuda")
     s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
     assert _lib.lib.tgdn_selftest_wait(0, ctypes.c_void_p(out.data_ptr()), s) == -1
     assert _lib.lib.tgdn_selftest_wait(1 << 40, ctypes.c_void_p(out.data_ptr()), s) == -1
     assert _lib.lib.tgdn_selftest_wait(1 << 10, None, s) == -2
+    assert _lib.lib.tgdn_selftest_role(0, ctypes.c_void_p(out.data_ptr()), s) == -1
+    assert _lib.lib.tgdn_selftest_role(1 << 10, None, s) == -2
