@@ -317,9 +317,8 @@ void run_matrix(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor
 
 void run_grads(const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dU, const Tensor& ds, const Tensor& dkg, const Tensor& dr,
                const Tensor& h, const Tensor& W, const Tensor& U, const Tensor& AP, const Tensor& k2, const Tensor& q2, const Tensor& beta,
-               const Tensor& gc, double scale, const OptTensor& token_map, const Grads& out) {
+               const Tensor& gc, double scale, const OptTensor& token_map, Tensor next_item, const Grads& out) {
   const c10::cuda::CUDAGuard guard(q.device());
-  Tensor next_item = at::zeros({1}, q.options().dtype(at::kInt));
   launch_grads(dims(q, k2, token_map), q, k, dO, h, W, U, AP, k2, q2, beta, gc, scale, token_map,
                Between{ptr(dU), ptr(ds), ptr(dkg), nullptr, ptr<float>(dr), nullptr, nullptr, nullptr, ptr<int>(next_item)}, out);
 }
@@ -942,10 +941,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, nogil);
   m.def("run_grads", [](const Tensor& q, const Tensor& k, const Tensor& dO, const Tensor& dV, const Tensor& dU, const Tensor& ds,
                         const Tensor& dkg, const Tensor& dr, const Tensor& h, const Tensor& W, const Tensor& U, const Tensor& AP,
-                        const Tensor& k2, const Tensor& q2, const Tensor& beta, const Tensor& gc, double scale, const OptTensor& token_map) {
+                        const Tensor& k2, const Tensor& q2, const Tensor& beta, const Tensor& gc, double scale, const OptTensor& token_map,
+                        const OptTensor& next_item) {
     Grads out = Grads::like(q, k2, beta);
     out.v = dV;
-    run_grads(q, k, dO, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, token_map, out);
+    run_grads(q, k, dO, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, token_map,
+              next_item.has_value() ? *next_item : at::zeros({1}, q.options().dtype(at::kInt)), out);
     return std::make_tuple(out.q, out.k, out.k2, out.q2, out.g, out.beta);
   }, nogil);
 }

@@ -67,10 +67,10 @@ def _run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, s
     return _lib.host.run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, float(scale), token_map)
 
 
-def _run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, token_map=None):
+def _run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, token_map=None, next_item=None):
     """State and matrix gradients in one kernel, as the backward runs them: (dq, dk, dk2, dq2, dg, dbeta), bitwise those of the two
-    stages above."""
-    return _lib.host.run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, float(scale), token_map)
+    stages above.  next_item: optional int32 zero that the kernel counts the items drawn in."""
+    return _lib.host.run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, float(scale), token_map, next_item)
 
 
 def chunk_gdn_joint_segment(q, k, v, k2, q2, g, beta, state_in=None, scale=None):

@@ -6,7 +6,7 @@ import torch
 
 from cute_triadic_gdn_b200 import _lib, gdn_joint_call
 from cute_triadic_gdn_b200 import gdn_joint as gj
-from cute_triadic_gdn_b200.joint_packing import prepare_documents
+from cute_triadic_gdn_b200.joint_packing import chunk_capacity, prepare_documents
 from oracle import triadic_oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -20,7 +20,7 @@ def repeated(tensors, heads):
     return [t.cuda().repeat([1, 1, heads // t.shape[2]] + [1] * (t.dim() - 3)) for t in tensors]
 
 
-def both(ins, do, docs=None):
+def both(ins, do, docs=None, drawn=None):
     q, k, v, k2, q2, g, beta = [t.cuda() for t in ins]
     do, E, scale = do.cuda(), k2.shape[-1], 128 ** -0.5
     cs = tm = None
@@ -29,7 +29,7 @@ def both(ins, do, docs=None):
     gc, AP, Pm = gj._run_masks(q, k, k2, q2, g, beta, scale, tm)
     _, h, W, U = gj._run_forward(q, k, v, k2, q2, beta, gc, AP, scale, True, cs, tm)
     dV, dU, ds, dkg, dr = gj._run_reverse(q, k, do, k2, q2, beta, gc, AP, Pm, U, scale, cs, tm)
-    one = gj._run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, tm)
+    one = gj._run_grads(q, k, do, dV, dU, ds, dkg, dr, h, W, U, AP, k2, q2, beta, gc, scale, tm, drawn)
     dkq, da, dc, dd = gj._run_state_grads(q, k, do, dV, h, ds, dkg, k2, q2, gc, scale, tm)
     two = gj._run_matrix(q, k, do, dU, W, U, AP, k2, q2, beta, gc, dkq, da, dc, dd, dr, scale, tm)
     assert _lib.device_status() == 0
@@ -91,6 +91,18 @@ def test_roundings_behind_a_documents_end_change_nothing(E, rows):
     for name, a, b, c in zip("dq dk dk2 dq2 dg dbeta".split(), one, other, two):
         assert torch.isfinite(a.float()).all() and torch.equal(a, b) and torch.equal(a, c), name
     assert _lib.device_status() == 0
+
+
+@pytest.mark.parametrize("E", [1, 8])
+@pytest.mark.parametrize("n,H", [(40, 3), (128, 16)])
+def test_unused_tail_of_the_chunk_map_is_not_drawn(E, n, H):
+    """Half of the map is unused with documents of one chunk each: the blocks draw the items of the other half, and stop."""
+    ins, do = orc.make_inputs(1, 64 * n, H, E, seed=70 + E, dist="mild"), orc.make_grad_output((1, 64 * n, H, 128), 12)
+    drawn = torch.zeros(1, dtype=torch.int32, device="cuda")
+    both(ins, do, list(range(0, 64 * n + 1, 64)), drawn)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    blocks = min(sms, chunk_capacity(64 * n, n) * H)
+    assert drawn.item() == n * H - min(n * H, blocks) + blocks   # (a block's first item is not drawn; each finds the end once)
 
 
 @pytest.mark.parametrize("E", [1, 2, 4])
