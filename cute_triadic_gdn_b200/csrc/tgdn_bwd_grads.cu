@@ -1139,23 +1139,21 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
         const uint8_t* h_item = reinterpret_cast<const uint8_t*>(p.h) + item * (static_cast<int64_t>(E) * 32768);
         const uint8_t* g_item = reinterpret_cast<const uint8_t*>(p.ds) + item * (static_cast<int64_t>(E) * 32768);
         const uint8_t* blocks = reinterpret_cast<const uint8_t*>(p.dkg) + item * (static_cast<int64_t>(NVB) * 16384);
+        // One place in the code asks for entries and one for tiles: five roles' loops share an SM's instruction caches, and what this warp
+        // executes between a free stage and the load into it is waited for.  us, a call in each place -> one: 4096 items E4 303 -> 294, with
+        // slow decays 471 -> 440; 8192 items E8 827 -> 811, 1298 -> 1205; 2048 items E12 342 -> 352, 526 -> 485, E16 416 -> 402, 621 -> 577.
 #pragma unroll 1
-        for (int e = 0; e <= E; ++e) {
+        for (int e = 0; e <= E; ++e) {                     // slices; at E the value-block images
           if (e == tiles_at) {
-            tile_entry(&map_du, crow);
-            tile_entry(&map_w, crow);
-            tile_entry(&map_u, crow);
-          }
-          if (e == E) break;
-          const bool trace = (fmask >> e) & 1u;
 #pragma unroll 1
-          for (int vh = 0; vh < 2; ++vh) {
-            entry(h_item + (2 * e + vh) * 16384);
-            if (trace) entry(g_item + (2 * e + vh) * 16384);
+            for (int i = 0; i < 3; ++i) tile_entry(i == 0 ? &map_du : i == 1 ? &map_w : &map_u, crow);
           }
+          const bool trace = e < E && ((fmask >> e) & 1u);
+          const uint8_t* src = e < E ? h_item + e * 32768 : blocks;
+          const int pieces = e == E ? NVB : trace ? 4 : 2;
+#pragma unroll 1
+          for (int i = 0; i < pieces; ++i) entry(!trace ? src + i * 16384 : (i & 1 ? g_item + e * 32768 : src) + (i >> 1) * 16384);
         }
-#pragma unroll 1
-        for (int u = 0; u < NVB; ++u) entry(blocks + u * 16384);
         cur = nxt;
         my_gl = next_gl;
       }
