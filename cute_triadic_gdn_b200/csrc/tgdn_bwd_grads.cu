@@ -12,17 +12,19 @@
 //                 and the [dW;dO] tile
 //   warp 18       loads [K;Q] and A, issues the chain's first products (G1, G2) and its last (G5)
 // The formulas are those of the two kernels, value by value in the same order: the results are bitwise those of running them one after
-// the other (dkq rounded to bf16 included), which tests/test_abi_gpu.py checks.  What need not travel any more: dkq (32 KB an item there and
-// back), da, dc, dd, and the second load of K, Q and dO: 520 KB of DRAM traffic an item at eight slices instead of 660.
+// the other (dkq rounded to bf16 included), which tests/test_abi_gpu.py and tests/test_grads_gpu.py check.  What need not travel any more: dkq (32 KB an item there and
+// back), da, dc, dd, and the second load of K, Q and dO: 518 KB of DRAM traffic an item at eight slices instead of 660.
 //
 // Tensor memory: the tiles P_e and, as the last one, the value-block sum in a double buffer (columns 0..255), G5 (256..383, before that G1
 // in its first 64 columns and dA', Y, dp in turn in its last 64), traces h_e G_e^T (384..511, before that dPm' in the first 64 columns).
 //
-// What bounds it: the memory (470 KB an item at eight slices; 4.8 TB/s) and, close behind, the shared-memory path, which the chain's table
+// What bounds it: the memory (518 KB an item at eight slices; 5.2 TB/s) and, close behind, the shared-memory path, which the chain's table
 // rows, the stream's tensor-memory and K reads, the products' operands and the arriving tiles share; waiting warps park instead of
-// polling for that reason (939 -> 839 us below).  us, state gradients + matrix gradients as two kernels -> this one: 8192 items E8
-// 690 + 505 -> 805, with slow decays 845 + 501 -> 1226; 4096 items E1 148 + 200 -> 230, E4 238 + 225 -> 293.  Pulling tiles into L2 ahead of the ring, which
-// helped the kernel of the states alone, costs 10 to 20 % here.
+// polling for that reason (8192 items E8 939 -> 839 us when that was done).  us, state gradients + matrix gradients as two kernels -> this
+// one: 8192 items E8 690 + 505 -> 811, with slow decays 845 + 501 -> 1205; 4096 items E1 148 + 200 -> 226, E4 238 + 225 -> 294.  Pulling tiles
+// into L2 ahead of the ring, which helped the kernel of the states alone, costs 10 to 20 % here.  At eight, twelve and sixteen slices the
+// chain does not fit its registers (-Xptxas -v: 48, 132 and 460 bytes of spill stores; 4 to 8 below): with this much
+// shared memory in use a spilled value is a round trip to L2.
 //
 // Replaces cute_triadic_gdn/kernels/sm100_joint_state_grads.py:53-449, sm100_joint_bwd_parallel.py:80-405,
 // sm90_joint_bwd_parallel.py:278-372 (mask_grad_kernel) and the reverse pass of sm90_joint_scan.py:21-80.
@@ -35,7 +37,7 @@ namespace tgdn {
 
 constexpr int GR_THREADS = 20 * 32;   // (warp 19 only completes its warpgroup)
 // Registers a thread: 96 at launch (five warps on each quarter of an SM), then the two warpgroups of a role take what the last one gives
-// back: 2 * 112 + 2 * 104 + 48 = 480 of 480 (with 40 for the service warps the loading warp spills).
+// back: 2 * 112 + 2 * 104 + 48 = 480 of 480 (40 for the service warps spilled 8 bytes more at one slice).
 constexpr int GR_STREAM_REGS = 112, GR_CHAIN_REGS = 104, GR_SERVICE_REGS = 48;
 static_assert(2 * GR_STREAM_REGS + 2 * GR_CHAIN_REGS + GR_SERVICE_REGS <= 5 * 96, "registers of the block");
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -153,8 +155,8 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
   constexpr float LOG2E = 1.4426950408889634f;
   // The trace of an item's first slice: up to two slices it is a tile of the double buffer (T0_TILE) and need not wait until dPm' has left the
   // tensor memory that the other traces use; above, where the chain is what an item waits for, dU, W, U pass before that slice
-  // (TILES_EARLY) so that the chain starts sooner, and its trace waits.  us, slow decays, the second way -> the first: 4096 items E1
-  // 257 -> 235, E2 326 -> 296, E4 461 -> 463; 8192 items E8 1234 -> 1314.
+  // (TILES_EARLY) so that the chain starts sooner, and its trace waits.  Time of the first way against the second, slow decays:
+  // 4096 items E1 -9 %, E2 -9 %, E4 0; 8192 items E8 +6 %.
   constexpr bool T0_TILE = E <= 2, TILES_EARLY = !T0_TILE;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int warp_u = __shfl_sync(0xffffffffu, warp, 0);   // warp index as a warp-uniform value
@@ -314,8 +316,7 @@ grads_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ 
             for (int o2 = 16; o2 > 0; o2 >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o2);
             if (lane == 0) sm.red[e * 4 + (warp & 3)] = d;
           };
-          // (up to two slices the tile is handed back behind the sum: us, before it -> behind, E1 244 -> 235, E2 331 -> 296; above, before:
-          // E8 1226 against 1249)
+          // (up to two slices the tile is handed back behind the sum: E1 -4 %, E2 -11 % against before it; above, before it: behind, E8 +2 %)
           if constexpr (T0_TILE) take_diagonal();
           tc_fence_before();
           __syncwarp();

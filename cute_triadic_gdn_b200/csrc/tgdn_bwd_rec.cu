@@ -9,7 +9,7 @@
 //       dW = beta*Z = dV ;  X = [-a_e*dW ; c_e*dO]
 //   (p) P  = G Xu^T                 tcgen05 M=128 (key rows d), N=64 (tokens), K=E*VC     Xu_e = r_e*U
 //       the value block's share of  sum_e (r_e*U) G_e^T, the part of dK that contracts the gradient state over the
-//       value axis; it leaves as a bf16 operand image (16 KB) and the state-gradient kernel adds the blocks up
+//       value axis; it leaves as a bf16 operand image (16 KB) and the gradient kernel adds the blocks up
 //   (d) dG = [K^T | Q^T] X          tcgen05 M=128, N=E*VC, K=128
 //       G_e <- d_e G_e + dG_e ; bf16 copy -> operand of the next (a)
 //
@@ -40,8 +40,8 @@
 // prefetch instructions made it 3 to 8 % slower: the loads are a chunk ahead already.)
 // dV of a whole chunk leaves as a tile up to eight slices: us, 8192 items E8 1031 -> 1023, 4096 items E4 270 -> 255, E2 205 -> 194, E1 177 -> 171.
 // One value block per chain in the 64-column CTA, with sums of its own, instead of one block of 64 columns (whose results depended on
-// the width that the call picked): E4 254 -> 256, E2 193 -> 206, E1 172 -> 188, and the state-gradient kernel adds four images again
-// instead of two (217 -> 247, 164 -> 182, 137 -> 154); four slices on narrow blocks (2048 items), the chains' P in turn: 188 -> 193.
+// the width that the call picked): E4 254 -> 256, E2 193 -> 206, E1 172 -> 188, and four images are added up behind it again instead
+// of two (in the state-gradient kernel of that time 217 -> 247, 164 -> 182, 137 -> 154); four slices on narrow blocks (2048 items), the chains' P in turn: 188 -> 193.
 // Who waits for a product parks (the other chain's epilogue wants the shared-memory path that polls would take); the loads of a chunk are
 // polled, being there already as a rule: us, all waits polled -> E8 1014 -> 987, E12 968 -> 929, E16 1208 -> 1176 (4096 items each),
 // E4 256 -> 247; with the loads parked too E12 977.  (One polling warp and a named barrier for the rest: E8 1133.)
@@ -335,7 +335,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
     for (int c = 0; c < CW / 2; c += 4)
       st_shared_v4(dst + (c >> 2) * stride, mul_bf16x2(w[c], ff), mul_bf16x2(w[c + 1], ff), mul_bf16x2(w[c + 2], ff), mul_bf16x2(w[c + 3], ff));
   };
-  // G_e of one chunk boundary, for the slices the state-gradient kernel will ask for: slice e as [v/8][d][v%8]
+  // G_e of one chunk boundary, for the slices the gradient kernel will ask for: slice e as [v/8][d][v%8]
   auto store_state = [&](int64_t item, const uint32_t* packed) {
     uint8_t* base = reinterpret_cast<uint8_t*>(p.ds) + item * (static_cast<int64_t>(E) * 32768);
 #pragma unroll
@@ -348,7 +348,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
                                                                       packed[e * (CW / 2) + c + 2], packed[e * (CW / 2) + c + 3]);
     }
   };
-  auto decay_flag = [&](int64_t item, int e) {      // does d_e*dd_e of this chunk matter?  (same expression in the state-gradient kernel)
+  auto decay_flag = [&](int64_t item, int e) {      // does d_e*dd_e of this chunk matter?  (same expression in the gradient kernel)
     return __ldg(p.gc + item * gate_item_floats(E) + 63 * E + e) * LOG2E >= DD_MIN_LOG2_DECAY ? 1 : 0;
   };
 
@@ -754,7 +754,7 @@ rec_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
           const int n0 = wg * TPC + j0 + j;
           st_shared_v4(base + (n0 >> 3) * 2048, packed[j / 2], packed[j / 2 + 1], packed[j / 2 + 2], packed[j / 2 + 3]);
         }
-        // G_e at the end of the previous chunk, for the slices the state-gradient kernel will ask for: [v/8][d][v%8]
+        // G_e at the end of the previous chunk, for the slices the gradient kernel will ask for: [v/8][d][v%8]
         if (sbase != nullptr) {
 #pragma unroll
           for (int j = 0; j < PIECE; j += CW) {
@@ -871,7 +871,7 @@ int tgdn_bwd_recurrent_rows(const void* q, const void* k, const void* dO, const 
       if (wide) return launch_rec<4, 64, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
       return launch_rec<4, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     // E = 8: 32 value columns per CTA measured 9% faster than two CTAs per SM of 16 columns each (5.26 -> 4.77 ms at B=8, T=8192, H=32,
-    // before the chains), and the state-gradient kernel then adds four value-block images per item instead of eight.
+    // before the chains), and the gradient kernel then adds four value-block images per item instead of eight.
     case 8: return launch_rec<8, 32, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     case 12: return launch_rec<12, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);
     case 16: return launch_rec<16, 16, 2, 2>(mk, mq, mdo, mu, mdu, ma, mb, mdv, p, s);

@@ -29,7 +29,7 @@
 // stage with one bulk copy; every thread reads those of its own row (K rows: a, r, beta; Q rows: c) right after its
 // chain's MMA (1) went out.  Nothing couples the chains but the tile ring.  The key-row warps have the longer phases (two
 // gate factors per slice, the operand images of beta*W and r_e*U), so the chain's extra roles sit on its query-row
-// warps: one issues the MMAs and polls their barrier, one hands stages back and issues the loads.
+// warps: one issues the MMAs and waits for them, one hands stages back and issues the loads.
 //
 // Replaces cute_triadic_gdn/kernels/sm100_joint_fwd.py:66-527 (fwd_kernel); math as cute_triadic_gdn/ops/gdn_joint.py:63-90.
 // Column order inside a chain: n' = (w*E + e)*CW + c  <->  (slice e, value column w*CW + c of the chain).
@@ -133,7 +133,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CU
   using C = FwdCfg<E, CW, NCH, WS, WV, STAGES>;
   constexpr int WPC = C::WPC, CV = C::CV, TPC = C::TPC, VC = C::VC, ET = C::ET, TPT = C::TPT, CT = C::CHAIN_THREADS;
   // Roles inside a chain: its key-row warps (0, 1) have the longer epilogues (gate factors r_e, the operand images of W
-  // and of r_e U), so the query-row warps take the extra work: warp 2 issues the MMAs and polls their barrier, warp 3
+  // and of r_e U), so the query-row warps take the extra work: warp 2 issues the MMAs and waits for them, warp 3
   // hands stages back and issues the loads and stores.  (Every copy operation costs its warp some sixty cycles, whatever its size,
   // and the chain waits for its last warp: few and large ones.  Not on the warp that issues the MMAs: 15 % slower.)
   constexpr int ISSUE_WARP = 2, COPY_WARP = 3;

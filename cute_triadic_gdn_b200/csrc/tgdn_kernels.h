@@ -21,7 +21,7 @@ namespace tgdn {
 
 // dd_e = <h_e, G_e>, the gradient of the chunk decay d_e = exp(gL_e), enters the result only as d_e * dd_e.  Where
 // log2(d_e) is below this bound the product is under 2^-24 of <h_e, G_e> and is taken as zero: the reverse recurrence
-// then does not store G_e of that chunk and the state-gradient kernel does not read it.  Both kernels evaluate
+// then does not store G_e of that chunk and the gradient kernel does not read it.  All of them evaluate
 // gc[63][e] * log2(e) >= DD_MIN_LOG2_DECAY on the same f32 value.
 constexpr float DD_MIN_LOG2_DECAY = -24.f;
 

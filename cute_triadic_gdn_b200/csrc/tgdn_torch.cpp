@@ -219,7 +219,8 @@ struct Grads {
   }
 };
 
-// What travels between the three kernels of the backward.
+// What travels between the kernels of the backward: from the reverse recurrence to the gradients; dkq, da, dc, dd between the two stages that
+// the gradients also exist as.
 struct Between {
   void *dU, *ds, *dkg, *dkq;
   float *dr, *da, *dc, *dd;
